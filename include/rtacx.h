@@ -85,8 +85,12 @@ typedef int rtacx_status;
  * Without the flags the 1D pulse is the exact linear interpolation of the
  * table, zero outside it (the evident intent). */
 #define RTACX_FLAG_TEXTURE_CLAMP 4u
+/* A 2D sensor whose pulse taps lie one output range apart and whose windows
+ * hold the pulse takes the range-cell form (one beam lookup per sample and
+ * bearing, the pulse as a filter over the cells; float arithmetic), whatever
+ * the next flag says. */
 /* rtacx_sensor_2d.flags: gather with the FP32 CUDA-core kernel instead of the
- * tensor-core one. By default a 2D ping's gather (output tiles of 64 ranges x
+ * tensor-core one. Otherwise a 2D ping's gather (output tiles of 64 ranges x
  * 128 bearings) forms its sample-by-PSF outer products on the tcgen05 tensor
  * cores from TF32 operands split in hi + lo parts (three products, FP32
  * accumulation: the same accuracy as the FP32 path, the float additions in

@@ -114,6 +114,7 @@ rtacx_status make_pulse_texture_1d(Context& c, const rtacx_sensor_1d* s, float s
 void free_config(Context& c)
 {
     free_precision(c);
+    free_cells(c);
     if(c.psf_tex) cudaDestroyTextureObject(c.psf_tex);
     c.psf_tex = 0;
     if(c.psf_array) cudaFreeArray(c.psf_array);
@@ -404,7 +405,7 @@ rtacx_status rtacx_configure_2d(rtacx_ctx* ctx, const rtacx_sensor_2d* s)
         return RTACX_ERR_OUT_OF_MEMORY;
     c.d_bb_tiles = (c.bearing_tile == 64) ? c.d_bb_tiles64 : c.d_bb_tiles128;
     if(texture_psf && make_psf_texture(c, s) != RTACX_OK) return RTACX_ERR_CUDA;
-    {
+    if(texture_psf || !configure_cells(c, sb)) {
         const uint64_t tiles = (uint64_t)((c.nB + c.bearing_tile - 1) / c.bearing_tile) * ((c.nR + c.range_tile - 1) / c.range_tile);
         if(!upload<uint32_t>(c, c.d_tile_parts, nullptr, tiles) || !upload<uint32_t>(c, c.d_tile_first, nullptr, tiles + 1) ||
            !upload<uint4>(c, c.d_items, nullptr, tiles * 256) || !upload<uint32_t>(c, c.d_item_counter, nullptr, 1))
@@ -465,9 +466,10 @@ rtacx_status rtacx_reduce(rtacx_ctx* ctx, const void* samples, uint64_t n, float
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     for(bool& t : c.traced) t = false;
     st = run_binning(c, samples, n, s);
+    if(st == RTACX_OK && !c.cells_on) st = run_windows(c, s);
     if(st != RTACX_OK) return st;
     c.mark(5, false, s);
-    st = run_reduce(c, out, s);
+    st = c.cells_on ? run_cells(c, n, reinterpret_cast<float2*>(out), s) : run_reduce(c, out, s);
     c.mark(5, true, s);
     return st;
 }

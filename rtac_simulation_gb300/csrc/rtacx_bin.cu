@@ -546,6 +546,13 @@ rtacx_status run_binning(Context& ctx, const void* samples, uint64_t n, cudaStre
         RTACX_CUDA(cudaGetLastError());
         ctx.mark(3, true, stream);
     }
+    return RTACX_OK;
+}
+
+// Effective windows of every output row (the per-row gathers' input).
+rtacx_status run_windows(Context& ctx, cudaStream_t stream)
+{
+    const BinParams& p = ctx.bin;
     ctx.mark(4, false, stream);
     k_windows<<<(ctx.nR + 255) / 256, 256, 0, stream>>>(ctx.d_offsets, p.nBB, ctx.nR, ctx.overlap,
                                                          ctx.d_support, ctx.d_win);

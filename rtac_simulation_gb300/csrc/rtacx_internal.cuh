@@ -287,6 +287,38 @@ struct ReduceParams {
     AxisLerp beam_axis;
 };
 
+// Range cells of a sensor whose pulse taps lie one output range apart
+// (rtacx_cells.cuh).
+struct CellParams {
+    float k_hi, k_lo;                // cells per metre (two floats)
+    float b_frac, b_row;             // cell coordinate of travel 0, plus one: fraction and whole part
+    float knot;                      // fraction of a cell next to a knot that is reduced row by row
+    int cells;                       // storage rows: cells -1 .. nR + taps - 2
+    int taps;                        // pulse taps H
+};
+
+// A ping's arguments of the cell kernels (rtacx_cells.cuh). Positions are
+// the bearings in the order in which the lanes hold them, in segments of
+// 32 BPL positions (pos_bearing -1: padding).
+struct CellPing {
+    CellParams cp;
+    const float4* sorted;
+    float4* cells;                   // [cp.cells][pitch] {T, M}
+    float2* out;
+    const float2* pulse;             // padded pulse table
+    const float* beam;               // padded beam table
+    const float* ranges;
+    const float* row_dev;            // [nR] e_r
+    const float4* taps;              // [cell_tap_entries(H)] {P[i], D[i]}, i = -1 first, zero-padded
+    const float2* seg_reach;         // [segs] bearings that reach a segment's beams
+    const float* pos_theta;          // [pitch]
+    const int* pos_bearing;          // [pitch]
+    AxisLerp range_axis, beam_axis;
+    float theta_lo, theta_hi;        // sample bearings are clamped to these (no beam reaches them)
+    uint32_t nR, nB, pitch;
+    int segs;
+};
+
 // Everything one ping of a batch needs on the device (rtacx_batch_*).
 struct PingDev {
     const float* samples;
@@ -386,6 +418,17 @@ struct Context {
     size_t hist_cols = 0;               // allocated words of d_hist (the write cursors)
     uint32_t* d_hist = nullptr;         // the scatter's per-bin write cursors (cursor_word), nBins x kCursorStride words
 
+    // Cell form of a 2D ping (rtacx_cells.cu).
+    bool cells_on = false;
+    int cell_bpl = 2;                   // bearings per lane
+    CellPing cell{};                    // sorted and out are set per call
+    float4* d_cells = nullptr;
+    float4* d_cell_taps = nullptr;
+    float* d_row_dev = nullptr;
+    float2* d_seg_reach = nullptr;
+    float* d_pos_theta = nullptr;
+    int* d_pos_bearing = nullptr;
+
     // Split persistent gather of 2D pings (see rtacx_reduce.cu).
     uint32_t* d_tile_parts = nullptr;   // [tiles] sample-stream length of each output tile
     uint32_t* d_tile_first = nullptr;   // [tiles + 1] first item of each tile; [tiles] = item count
@@ -468,7 +511,13 @@ rtacx_status run_bin_outputs(Context& ctx, const void* samples, uint64_t n,
 bool ensure_capacity(Context& ctx, uint64_t n);
 
 // Sparse PSF reduction (rtacx_reduce.cu).
+rtacx_status run_windows(Context& ctx, cudaStream_t stream);
 rtacx_status run_reduce(Context& ctx, float* out, cudaStream_t stream);
+
+// Cell form of the plain reduction (rtacx_cells.cu).
+bool configure_cells(Context& ctx, double beam_support);
+void free_cells(Context& ctx);
+rtacx_status run_cells(Context& ctx, uint64_t n, float2* out, cudaStream_t stream);
 
 // Batched plain form. Maps are (ping, index) pairs: count / scatter chunks,
 // column-scan bin blocks of 256, window row blocks of 256; gather items are

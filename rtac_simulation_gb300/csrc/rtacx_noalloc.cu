@@ -272,6 +272,7 @@ extern "C" rtacx_status rtacx_reduce_noalloc(int sample_kind, const void* sensor
     if(e != cudaSuccess) { cudaGetLastError(); return RTACX_ERR_CUDA; }
 
     status = run_binning(ctx, samples, n, st);
+    if(status == RTACX_OK) status = run_windows(ctx, st);
     if(status != RTACX_OK) return status;
     return run_reduce(ctx, out, st);
 }

@@ -1,0 +1,90 @@
+"""Plain 2D form over range cells (pulse taps one output range apart) at the
+edges of its tiles: bearing counts around the 64- and 128-bearing segments,
+range counts around the filter's 8 and 32 rows, the shortest pulses, even and
+odd tables, pings of one unit of samples or a few, samples next to and beyond
+the range window. Each ping against the FP64 oracle at the plain form's
+tolerance, 1e-5 relative L2."""
+import numpy as np
+import pytest
+
+from rtac_simulation_gb300 import workloads as wl
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("needs a GPU", allow_module_level=True)
+
+from helpers_gpu import gpu_reduce, make_context, rel_l2  # noqa: E402
+
+TOL = 1e-5
+
+
+def ping(n, nR, nB, taps, wide, beam_taps=0, seed=3, rmin=0.4, rmax=30.0):
+    res = float(wl.linspace_resolution(rmin, rmax, nR))
+    bearings = wl.arcsin_bearings(nB, 130.0) if nB > 1 else np.zeros(1, np.float32)
+    spacing = 130.0 * wl.DEG / max(nB - 1, 1)
+    if wide:
+        span = 262.0 * wl.DEG
+        beam = wl.beam_sinc2(beam_taps or 701, span, 2.0 * wl.DEG, floor=0.01)
+    else:
+        span = 9 * spacing
+        beam = wl.beam_sinc2(beam_taps or 73, span, 2.0 * spacing)
+    pulse = wl.pulse_at_bin_spacing(taps, res, 1.2e6, 1500.0)
+    rng = np.random.default_rng(seed)
+    t = rng.uniform(rmin - 2 * taps * res, rmax + 2 * taps * res, n)
+    if n > 64:
+        R = wl.linspace(rmin, rmax, nR)
+        t[:64] = R[rng.integers(0, nR, 64)]              # exactly on output ranges
+        t[64 - min(8, n // 8):64] = rmin
+    th = rng.uniform(-70.0 * wl.DEG, 70.0 * wl.DEG, n)
+    re, im = rng.normal(size=(2, n))
+    s = wl.sensor_2d(rmin, rmax, nR, 1500.0, pulse, taps * res, beam, span, bearings)
+    return wl.Workload("cells", 2, s, wl._pack(re, im, t, th))
+
+
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("n,nR,nB,taps,beam_taps", [
+    (2, 2, 1, 2, 0), (31, 7, 3, 1, 0), (128, 8, 31, 2, 0), (129, 9, 33, 3, 72), (1000, 31, 63, 4, 0),
+    (1024, 33, 64, 5, 700), (1025, 64, 65, 8, 0), (3000, 65, 127, 9, 0), (5000, 100, 128, 16, 71),
+    (20000, 257, 129, 33, 0), (40000, 300, 200, 64, 0), (200003, 130, 257, 33, 0),
+])
+def test_cells_match_fp64_oracle(oracle, n, nR, nB, taps, beam_taps, wide):
+    wk = ping(n, nR, nB, taps, wide, beam_taps)
+    got = gpu_reduce(make_context(wk), wk.samples, wk.out_shape)
+    want = oracle.reduce(wk.samples, wk.sensor)
+    assert np.isfinite(got).all()
+    assert rel_l2(got, want) <= TOL, rel_l2(got, want)
+
+
+@pytest.mark.parametrize("change", ["half_margin", "half_tap", "long_pulse"])
+def test_sensors_off_the_cell_rule_match_fp64_oracle(oracle, change):
+    """A margin that cuts the pulse's window, taps that are not one range
+    apart: the per-row gathers, as before."""
+    wk = ping(4000, 100, 65, 17, False)
+    s = wk.sensor
+    if change == "half_margin":
+        s["margin"] = 0.25 * s["margin"]
+    elif change == "half_tap":
+        s["pulse_duration"] = 0.5 * s["pulse_duration"]
+    else:
+        s["pulse_duration"] = 1.01 * s["pulse_duration"]
+    got = gpu_reduce(make_context(wk), wk.samples, wk.out_shape)
+    want = oracle.reduce(wk.samples, wk.sensor)
+    assert rel_l2(got, want) <= TOL
+
+
+def test_cells_drop_samples_without_a_bearing_or_travel():
+    """NaN and far-away bearings and NaN travels carry no weight."""
+    wk = ping(3000, 100, 65, 9, False)
+    bad = wk.samples.copy()
+    bad[::50, 3] = np.nan
+    bad[1::50, 3] = 1e30
+    bad[2::50, 3] = -np.inf
+    clean = bad.copy()
+    clean[~np.isfinite(bad[:, 3]) | (np.abs(bad[:, 3]) > 1e3), :2] = 0.0
+    ctx = make_context(wk)
+    a = gpu_reduce(ctx, bad, wk.out_shape)
+    b = gpu_reduce(ctx, clean, wk.out_shape)
+    assert np.isfinite(a).all()
+    assert rel_l2(a, b) <= 1e-6
