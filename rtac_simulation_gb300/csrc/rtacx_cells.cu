@@ -6,8 +6,8 @@
 //                   reference window zeroed.
 // Measured against the tensor-core gather on the same pings (whole
 // rtacx_reduce, us): 2^20 samples, 512 x 1024, 33 taps, narrow beams: 1384 ->
-// 170; 2^22 samples, 512 x 4096, wide beams: 14433 -> 1278; 150003 samples,
-// 387 x 777, 24 taps: 246 -> 90. k_cells is bound by the beam lookups' shared
+// 152; 2^22 samples, 512 x 4096, wide beams: 14433 -> 1339; 150003 samples,
+// 387 x 777, 24 taps: 246 -> 82. k_cells is bound by the beam lookups' shared
 // memory and issue slots, at one lookup per (sample, bearing).
 #include "rtacx_bin_device.cuh"
 #include "rtacx_cells.cuh"
@@ -21,18 +21,13 @@ namespace rtacx {
 namespace {
 
 constexpr int kCellThreads = 256, kCellWarps = kCellThreads / 32;
-constexpr int kFilterWarps = 4;
 constexpr size_t kMaxCellBytes = (size_t)1 << 30;      // cell rows of one context
 constexpr double kMaxKnot = 0.01;
 
 size_t cells_smem(int W) { return kCellWarps * sizeof(CellWarpSmem) + (size_t)(W + 2) * sizeof(float2); }
 
-// Entries of the tap table: H + 1 taps, kFilterRows - 1 steps of the sliding
-// window beyond them, rounded up to whole blocks of kFilterRows.
-__host__ __device__ __forceinline__ int cell_tap_entries(int H) { return (H + kFilterRows + kFilterRows - 1) / kFilterRows * kFilterRows; }
-
 template <int BPL>
-__global__ void __launch_bounds__(kCellThreads, 2)
+__global__ void __launch_bounds__(kCellThreads, BPL == 2 ? 3 : 2)
 k_cells(const CellPing P, const uint32_t* __restrict__ total)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
@@ -47,24 +42,17 @@ k_cells(const CellPing P, const uint32_t* __restrict__ total)
         accumulate_unit<BPL>(P, u * kUnit, min((uint32_t)kUnit, m - u * kUnit), blockIdx.y, gridDim.y, S, tab, beam);
 }
 
-// One CTA: 32 positions x kFilterWarps * kFilterRows rows, the warps below
-// each other so that they share the cell rows through L1.
 __global__ void __launch_bounds__(32 * kFilterWarps)
 k_cells_filter(const CellPing P, const uint32_t* __restrict__ off, uint32_t nBB, int ov)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    float4* s_taps = reinterpret_cast<float4*>(s_raw);
-    __shared__ int s_on[kFilterWarps * kFilterRows];
-    const int rows0 = blockIdx.y * (kFilterWarps * kFilterRows), warp = threadIdx.x >> 5;
-    for(int i = threadIdx.x; i < cell_tap_entries(P.cp.taps); i += 32 * kFilterWarps) s_taps[i] = P.taps[i];
-    if(threadIdx.x < kFilterWarps * kFilterRows) {
-        const int r = rows0 + threadIdx.x;
+    __shared__ int s_on[kFilterTile];
+    if(threadIdx.x < kFilterTile) {
+        const int r = blockIdx.y * kFilterTile + threadIdx.x;
         int f, l;
         s_on[threadIdx.x] = r < (int)P.nR && ref_window(off, nBB, P.nR, ov, r, f, l) ? 1 : 0;
     }
-    __syncthreads();
-    const int r0 = rows0 + warp * kFilterRows;
-    if(r0 < (int)P.nR) filter_rows(P, blockIdx.x * 32 + (threadIdx.x & 31), r0, s_taps, s_on + warp * kFilterRows);
+    filter_tile(P, blockIdx.x, blockIdx.y, reinterpret_cast<float4*>(s_raw), s_on);   // synchronises before it reads s_on
 }
 
 template <typename T>
@@ -89,8 +77,8 @@ bool put(T*& dst, const std::vector<T>& src)
 
 void free_cells(Context& c)
 {
-    drop(c.d_cells); drop(c.d_cell_taps); drop(c.d_row_dev); drop(c.d_seg_reach);
-    drop(c.d_pos_theta); drop(c.d_pos_bearing);
+    drop(c.d_cells); drop(c.d_cell_taps); drop(c.d_row_dev); drop(c.d_win_reach);
+    drop(c.d_pos_theta); drop(c.d_pos_col); drop(c.d_col_bearing);
     c.cells_on = false;
 }
 
@@ -159,44 +147,81 @@ bool configure_cells(Context& c, double beam_support)
     c.cell.theta_lo = (float)(*mm.first - 2.0 * span);
     c.cell.theta_hi = (float)(*mm.second + 2.0 * span);
 
-    // Bearings per lane: four where a sample reaches most of the fan (fewer
-    // list reads per pair), two where beams are narrow (shorter segments).
-    const bool wide = 4.0 * beam_support >= fan;
-    c.cell_bpl = wide && nB > 64 ? 4 : 2;
-    const int seg_len = 32 * c.cell_bpl, segs = (nB + seg_len - 1) / seg_len;
-    c.cell.segs = segs;
-    c.cell.pitch = (uint32_t)(segs * seg_len);
-    const size_t cell_bytes = (size_t)cp.cells * c.cell.pitch * sizeof(float4);
-    if(cell_bytes > kMaxCellBytes || cells_smem(W) > 200 * 1024) return false;
-
-    // Order of the bearings. For one sample the table entries of two bearings
-    // differ by their distance in taps, whatever the sample; lanes whose
-    // distances differ modulo the 16 eight-byte banks of shared memory never
-    // conflict. Bearings sorted by that remainder and dealt to the groups of
-    // 16 lanes in turn are about one bank apart. Dealt over the whole fan for
-    // wide beams, inside each segment for narrow ones.
+    // Windows. Narrow beams: consecutive bearings, each sample in exactly one
+    // window (the bearings that a window's samples reach are all in it), the
+    // shortest windows that still take half a beam's width of bearings on
+    // average (shorter ones would be flushed after too few samples). Wide
+    // beams: the bearings are shared out among windows that all take every
+    // sample.
+    std::vector<int> sorted_b(nB);
+    std::iota(sorted_b.begin(), sorted_b.end(), 0);
+    std::stable_sort(sorted_b.begin(), sorted_b.end(), [&](int x, int y) { return c.bearings[x] < c.bearings[y]; });
+    std::vector<float2> reach;
+    std::vector<std::vector<int>> members;
+    const float all_lo = (float)(*mm.first - beam_support), all_hi = (float)(*mm.second + beam_support);
+    int bpl = 0;
+    for(int cand = 2; cand <= 4 && !bpl; cand += 2) {
+        const int len = 32 * cand;
+        reach.clear();
+        members.clear();
+        float cur = all_lo;
+        bool ok = true;
+        while(ok && cur < all_hi) {
+            int f = 0;
+            while(f < nB && (double)c.bearings[sorted_b[f]] + beam_support < (double)cur) f++;
+            const int end = std::min(nB, f + len);
+            const float y = end < nB ? (float)((double)c.bearings[sorted_b[end]] - beam_support) : all_hi;
+            ok = y > cur && f < end && reach.size() < 4096;
+            reach.push_back(make_float2(cur, end < nB ? y : std::nextafter(all_hi, INFINITY)));
+            members.emplace_back(sorted_b.begin() + f, sorted_b.begin() + end);
+            cur = y;
+        }
+        if(ok && ((double)all_hi - all_lo) / reach.size() >= 0.5 * beam_support) bpl = cand;
+    }
+    const bool shared_out = bpl == 0;
+    if(shared_out) bpl = nB > 64 ? 4 : 2;
+    const int len = 32 * bpl;
+    // Order of the bearings in a window. For one sample the table entries of
+    // two bearings differ by their distance in taps, whatever the sample;
+    // lanes whose distances differ modulo the 16 eight-byte banks of shared
+    // memory never conflict. Bearings sorted by that remainder and dealt to
+    // the groups of 16 lanes in turn are about one bank apart: 3.1 to 3.5
+    // wavefronts per lookup instead of 3.8 to 4.8 in the bearings' own order
+    // (counted for the tables of the imaging sensors).
     const double kb = (double)c.red.beam_axis.k_hi;
-    std::vector<int> pos(c.cell.pitch, -1);
-    const int scope = wide ? (int)c.cell.pitch : seg_len;
-    for(int s0 = 0; s0 < (int)c.cell.pitch; s0 += scope) {
-        std::vector<int> order;
-        for(int i = s0; i < std::min(nB, s0 + scope); i++) order.push_back(i);
+    auto deal = [&](std::vector<int> order, std::vector<int>& pos, size_t at) {
         auto bank = [&](int i) { const double x = (double)c.bearings[i] * kb; return x - 16.0 * std::floor(x / 16.0); };
         std::stable_sort(order.begin(), order.end(), [&](int a, int d) { return bank(a) < bank(d); });
-        // Deal the bearings to as many whole groups as they fill.
-        const int groups = std::max(1, ((int)order.size() + 15) / 16);
-        for(size_t q = 0; q < order.size(); q++) pos[s0 + (int)(q % groups) * 16 + (int)(q / groups)] = order[q];
+        const size_t groups = std::max<size_t>(1, (order.size() + 15) / 16);
+        for(size_t q = 0; q < order.size(); q++) pos[at + (q % groups) * 16 + q / groups] = order[q];
+    };
+    std::vector<int> pos;
+    if(shared_out) {
+        const int wins = (nB + len - 1) / len;
+        pos.assign((size_t)wins * len, -1);
+        deal(sorted_b, pos, 0);
+        reach.assign(wins, make_float2(all_lo, std::nextafter(all_hi, INFINITY)));
     }
-    std::vector<float> theta(c.cell.pitch, c.bearings[nB - 1]);
-    std::vector<float2> reach(segs, make_float2(INFINITY, -INFINITY));
-    for(int p = 0; p < (int)c.cell.pitch; p++) {
+    else {
+        pos.assign(reach.size() * len, -1);
+        for(size_t w = 0; w < reach.size(); w++) deal(members[w], pos, w * len);
+    }
+    c.cell_bpl = bpl;
+    c.cell.windows = (int)reach.size();
+    // Columns: the lanes' order for shared-out windows (whole rows of 512
+    // bytes per reduction), the bearings' own order for overlapping ones.
+    const uint32_t pitch = shared_out ? (uint32_t)pos.size() : (uint32_t)((nB + 31) / 32 * 32);
+    c.cell.pitch = pitch;
+    std::vector<int> col(pos.size()), col_bearing(pitch, -1);
+    std::vector<float> theta(pos.size(), c.bearings[sorted_b[nB - 1]]);
+    for(size_t p = 0; p < pos.size(); p++) {
+        col[p] = pos[p] < 0 ? -1 : shared_out ? (int)p : pos[p];
         if(pos[p] < 0) continue;
-        const float t = c.bearings[pos[p]];
-        theta[p] = t;
-        float2& s = reach[p / seg_len];
-        s.x = std::min(s.x, (float)(t - beam_support));
-        s.y = std::max(s.y, (float)(t + beam_support));
+        theta[p] = c.bearings[pos[p]];
+        col_bearing[col[p]] = pos[p];
     }
+    const size_t cell_bytes = (size_t)cp.cells * pitch * sizeof(float4);
+    if(cell_bytes > kMaxCellBytes || cells_smem(W) > 200 * 1024 || filter_smem(H) > 200 * 1024) return false;
     std::vector<float4> taps((size_t)cell_tap_entries(H), make_float4(0.f, 0.f, 0.f, 0.f));
     for(int i = -1; i < H; i++) {
         double p[2], d[2];
@@ -207,18 +232,18 @@ bool configure_cells(Context& c, double beam_support)
         }
         taps[i + 1] = make_float4((float)p[0], (float)p[1], (float)d[0], (float)d[1]);
     }
-    bool ok = put(c.d_cell_taps, taps) && put(c.d_row_dev, dev) && put(c.d_seg_reach, reach) &&
-              put(c.d_pos_theta, theta) && put(c.d_pos_bearing, pos);
+    bool ok = put(c.d_cell_taps, taps) && put(c.d_row_dev, dev) && put(c.d_win_reach, reach) &&
+              put(c.d_pos_theta, theta) && put(c.d_pos_col, col) && put(c.d_col_bearing, col_bearing);
     if(ok && cudaMalloc(&c.d_cells, cell_bytes) != cudaSuccess) { cudaGetLastError(); ok = false; }
     const void* fn = c.cell_bpl == 4 ? (const void*)k_cells<4> : (const void*)k_cells<2>;
     if(ok) ok = raise_smem_limit(fn, cells_smem(W)) == cudaSuccess &&
-                raise_smem_limit((const void*)k_cells_filter, cell_tap_entries(H) * sizeof(float4)) == cudaSuccess;
+                raise_smem_limit((const void*)k_cells_filter, filter_smem(H)) == cudaSuccess;
     if(!ok) { free_cells(c); return false; }
     CellPing& P = c.cell;
     P.cells = c.d_cells;
     P.pulse = c.d_pulse; P.beam = c.d_beam; P.ranges = c.d_ranges;
-    P.row_dev = c.d_row_dev; P.taps = c.d_cell_taps; P.seg_reach = c.d_seg_reach;
-    P.pos_theta = c.d_pos_theta; P.pos_bearing = c.d_pos_bearing;
+    P.row_dev = c.d_row_dev; P.taps = c.d_cell_taps; P.win_reach = c.d_win_reach;
+    P.pos_theta = c.d_pos_theta; P.pos_col = c.d_pos_col; P.col_bearing = c.d_col_bearing;
     P.range_axis = c.red.range_axis; P.beam_axis = c.red.beam_axis;
     P.nR = c.nR; P.nB = c.nB;
     c.cells_on = true;
@@ -233,18 +258,18 @@ rtacx_status run_cells(Context& c, uint64_t n, float2* out, cudaStream_t stream)
     cudaError_t e = cudaMemsetAsync(c.d_cells, 0, (size_t)P.cp.cells * P.pitch * sizeof(float4), stream);
     if(e == cudaSuccess) e = cudaMemsetAsync(out, 0, (size_t)c.nR * c.nB * sizeof(float2), stream);
     if(e != cudaSuccess) { c.error = std::string("clearing the cell rows: ") + cudaGetErrorString(e); return RTACX_ERR_CUDA; }
-    // As many units as there are; the segments of a unit are shared out over
+    // As many units as there are; the windows of a unit are shared out over
     // blockIdx.y when there are too few units to fill the SMs.
     const uint64_t ctas = std::max<uint64_t>(1, (n + (uint64_t)kUnit * kCellWarps - 1) / ((uint64_t)kUnit * kCellWarps));
     const uint32_t full = (uint32_t)c.sm_count * 3u;
     const uint32_t gx = (uint32_t)std::min<uint64_t>(ctas, (uint64_t)full * 4u);
-    const uint32_t gy = (uint32_t)std::min<uint64_t>((uint64_t)P.segs, std::max<uint64_t>(1, full / gx));
+    const uint32_t gy = (uint32_t)std::min<uint64_t>((uint64_t)P.windows, std::max<uint64_t>(1, full / gx));
     const dim3 grid(gx, gy);
     const size_t smem = cells_smem(P.beam_axis.n);
     if(c.cell_bpl == 4) k_cells<4><<<grid, kCellThreads, smem, stream>>>(P, c.d_offsets + c.bin.nBins);
     else k_cells<2><<<grid, kCellThreads, smem, stream>>>(P, c.d_offsets + c.bin.nBins);
-    const dim3 fgrid(P.pitch / 32, (c.nR + kFilterWarps * kFilterRows - 1) / (kFilterWarps * kFilterRows));
-    k_cells_filter<<<fgrid, 32 * kFilterWarps, cell_tap_entries(P.cp.taps) * sizeof(float4), stream>>>(
+    const dim3 fgrid(P.pitch / 32, (c.nR + kFilterTile - 1) / kFilterTile);
+    k_cells_filter<<<fgrid, 32 * kFilterWarps, filter_smem(P.cp.taps), stream>>>(
         P, c.d_offsets, c.bin.nBB, c.overlap);
     e = cudaGetLastError();
     if(e != cudaSuccess) { c.error = std::string("cell form: ") + cudaGetErrorString(e); return RTACX_ERR_CUDA; }

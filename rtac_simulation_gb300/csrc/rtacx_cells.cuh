@@ -55,6 +55,13 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
     return r;
 }
 
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 __device__ __forceinline__ void red_add_f4(float4* addr, float x, float y, float z, float w)
 {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
@@ -159,38 +166,30 @@ struct BeamLookup {
 // ---- accumulation of one ping's samples into the cell rows ------------------
 // A warp takes units of kUnit consecutive samples of the sorted order (so of
 // few cells and, with bearing sub-bins, of few bearings) and, one after the
-// other, the segments of 32 BPL bearings that the unit's bearings can reach:
-// lane l holds bearings at positions l, l + 32, ... of the segment and the
-// sums of three consecutive cells for them in registers. Per chunk of 32
-// samples the lanes list the samples of those cells and this segment, in
-// shared memory, each value twice (the packed operands); all lanes then walk
-// the list. A unit's sums go to the cell rows as 16-byte reductions.
+// other, the windows of 32 BPL bearings that hold samples of the unit. Lane l
+// holds the bearings at positions l, l + 32, ... of the window and the sums
+// of three consecutive cells for them in registers. The window's samples are
+// listed by cell in shared memory, each value twice (the packed operands);
+// all lanes then walk the list. The sums go to the cell rows as 16-byte
+// reductions.
 constexpr int kUnit = 128;                 // samples per warp and unit
+constexpr int kUnitLoads = kUnit / 32;
 constexpr int kCellClasses = 3;            // consecutive cells held in registers
 
-struct CellEntry {                          // a listed sample
-    f32x2 theta, w0x, w0y, w1x, w1y, pad;
-};
-
 struct CellWarpSmem {
-    float4 w[kUnit];                        // {w0.x, w0.y, w1.x, w1.y}; row-by-row samples: {v.x, v.y, travel, -}
-    float theta[kUnit];
-    int cell[kUnit];                        // storage row; -1 dropped; -2 - row: reduced row by row
-    CellEntry list[32];
+    ulonglong2 list[kUnit][2];              // {theta, v.x}, {v.y, alpha}, each twice
+    float4 w[kUnit];                        // {v.x, v.y, alpha, -}; row-by-row samples: travel for alpha
 };
 
-// Samples of a unit that fall next to a knot, row by row: the lanes take 32
-// rows at a time, then every row's weight is broadcast and reduced into the
-// (zeroed) ping.
+// One sample next to a knot, row by row: the lanes take 32 rows at a time,
+// then every row's weight is broadcast and reduced into the (zeroed) ping.
 template <int BPL>
-__device__ __forceinline__ void reduce_row_by_row(const CellPing& P, const CellWarpSmem& S, const float2* tab,
+__device__ __forceinline__ void reduce_row_by_row(const CellPing& P, float4 w, float theta, int C, const float2* tab,
                                                   const BeamLookup& beam, const f32x2 (&minus_tb)[BPL / 2],
-                                                  const int* s_b, int s)
+                                                  const int* bearing)
 {
     const int lane = threadIdx.x & 31;
-    const float4 w = S.w[s];
-    const int C = -2 - S.cell[s] - 1;                       // cell index
-    const f32x2 th = pack2(S.theta[s], S.theta[s]);
+    const f32x2 th = pack2(theta, theta);
     float bv[BPL];
 #pragma unroll
     for(int p = 0; p < BPL / 2; p++) {
@@ -212,7 +211,7 @@ __device__ __forceinline__ void reduce_row_by_row(const CellPing& P, const CellW
             if(ux == 0.0f && uy == 0.0f) continue;
 #pragma unroll
             for(int p = 0; p < BPL; p++) {
-                const int b = s_b[p];
+                const int b = bearing[p];
                 if(b >= 0) red_add_f2(P.out + (size_t)(r0 + q) * P.nB + b, ux * bv[p], uy * bv[p]);
             }
         }
@@ -220,154 +219,198 @@ __device__ __forceinline__ void reduce_row_by_row(const CellPing& P, const CellW
 }
 
 // Accumulates samples [first, first + count) (count <= kUnit) of the sorted
-// order into the cell rows, for the segments seg0, seg0 + seg_step, ....
+// order into the cell rows, for the windows win0, win0 + win_step, ....
 template <int BPL>
-__device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t first, uint32_t count, int seg0,
-                                                int seg_step, CellWarpSmem& S, const float2* tab,
+__device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t first, uint32_t count, int win0,
+                                                int win_step, CellWarpSmem& S, const float2* tab,
                                                 const BeamLookup& beam)
 {
     constexpr int NP = BPL / 2;
     const int lane = threadIdx.x & 31;
-    float th_lo = INFINITY, th_hi = -INFINITY;
-    int c_lo = INT_MAX, any_near = 0;
+    const uint32_t below = (1u << lane) - 1u;
+    float th_lo = INFINITY, th_hi = -INFINITY, theta[kUnitLoads];
+    int cell[kUnitLoads];                  // storage row; -1 dropped; -2 - row: reduced row by row
+    bool near_knot = false;
     __syncwarp();
 #pragma unroll
-    for(int q = 0; q < kUnit / 32; q++) {
+    for(int q = 0; q < kUnitLoads; q++) {
         const uint32_t i = (uint32_t)(q * 32 + lane);
-        int cell = -1;
+        cell[q] = -1;
+        theta[q] = 0.0f;
         if(i < count) {
             const float4 rec = __ldcs(P.sorted + first + i);
             float alpha;
-            cell = range_cell(P.cp, rec.z, alpha);
+            const int c = range_cell(P.cp, rec.z, alpha);
             // Bearings far outside (and NaN) move to a bearing that no beam reaches.
             const float th = fminf(fmaxf(rec.w, P.theta_lo), P.theta_hi);
-            S.theta[i] = th;
-            S.w[i] = make_float4(rec.x, rec.y, alpha * rec.x, alpha * rec.y);
-            if(cell >= 0) {
+            const bool near = !(alpha >= P.cp.knot && alpha <= 1.0f - P.cp.knot);
+            theta[q] = th;
+            S.w[i] = make_float4(rec.x, rec.y, near ? rec.z : alpha, 0.0f);
+            if(c >= 0) {
+                cell[q] = near ? -2 - c : c;
+                near_knot |= near;
                 th_lo = fminf(th_lo, th);
                 th_hi = fmaxf(th_hi, th);
-                if(!(alpha >= P.cp.knot && alpha <= 1.0f - P.cp.knot)) {
-                    S.w[i] = make_float4(rec.x, rec.y, rec.z, 0.0f);
-                    cell = -2 - cell;
-                    any_near = 1;
-                }
-                else c_lo = min(c_lo, cell);
             }
         }
-        S.cell[i] = cell;
     }
-    any_near = __any_sync(0xffffffffu, any_near);
+    near_knot = __any_sync(0xffffffffu, near_knot);
     for(int o = 16; o > 0; o >>= 1) {
         th_lo = fminf(th_lo, __shfl_xor_sync(0xffffffffu, th_lo, o));
         th_hi = fmaxf(th_hi, __shfl_xor_sync(0xffffffffu, th_hi, o));
     }
-    c_lo = __reduce_min_sync(0xffffffffu, c_lo);
     __syncwarp();
-    for(int seg = seg0; seg < P.segs; seg += seg_step) {
-        const float2 reach = P.seg_reach[seg];
-        if(!(th_hi >= reach.x && th_lo <= reach.y)) continue;
-        const int pos0 = seg * 32 * BPL + lane;
-        f32x2 minus_tb[NP];
+    for(int g0 = win0; g0 < P.windows; g0 += 32 * win_step) {
+        // Windows g0, g0 + win_step, ... (one per lane) that the unit's bearings touch.
+        const int mine = g0 + lane * win_step;
+        const float2 my_reach = mine < P.windows ? P.win_reach[mine] : make_float2(INFINITY, -INFINITY);
+        uint32_t live = __ballot_sync(0xffffffffu, th_hi >= my_reach.x && th_lo < my_reach.y);
+        for(; live; live &= live - 1u) {
+            const int src = __ffs(live) - 1;
+            const int win = g0 + src * win_step;
+            const float lo = __shfl_sync(0xffffffffu, my_reach.x, src), hi = __shfl_sync(0xffffffffu, my_reach.y, src);
+            uint32_t in_win = 0;                   // bit q: sample q of this lane is in the window
+            int base = INT_MAX;
 #pragma unroll
-        for(int p = 0; p < NP; p++)
-            minus_tb[p] = pack2(-P.pos_theta[pos0 + 64 * p], -P.pos_theta[pos0 + 64 * p + 32]);
-        for(int base = c_lo; base != INT_MAX;) {
-            f32x2 acc[kCellClasses][NP][4];
+            for(int q = 0; q < kUnitLoads; q++) {
+                const bool in = cell[q] != -1 && theta[q] >= lo && theta[q] < hi;
+                in_win |= in ? 1u << q : 0u;
+                if(in && cell[q] >= 0) base = min(base, cell[q]);
+            }
+            if(!__any_sync(0xffffffffu, in_win)) continue;
+            base = __reduce_min_sync(0xffffffffu, base);
+            const int pos0 = win * 32 * BPL + lane;
+            f32x2 minus_tb[NP];
 #pragma unroll
-            for(int k = 0; k < kCellClasses; k++)
+            for(int p = 0; p < NP; p++)
+                minus_tb[p] = pack2(-P.pos_theta[pos0 + 64 * p], -P.pos_theta[pos0 + 64 * p + 32]);
+            while(base != INT_MAX) {
+                // List the samples of cells base .. base + 2, by cell.
+                uint32_t m[kUnitLoads][kCellClasses];
+                int end[kCellClasses] = {0, 0, 0}, next = INT_MAX;
 #pragma unroll
-                for(int p = 0; p < NP; p++)
+                for(int q = 0; q < kUnitLoads; q++) {
+                    const int off = (in_win >> q & 1u) && cell[q] >= base ? cell[q] - base : -1;
+                    if(off >= kCellClasses) next = min(next, cell[q]);
 #pragma unroll
-                    for(int e = 0; e < 4; e++) acc[k][p][e] = 0ull;
-            int next = INT_MAX;
-            uint32_t held = 0;
-#pragma unroll 1
-            for(uint32_t q = 0; q < count; q += 32) {
-                const int i = (int)q + lane;
-                const int cell = S.cell[i];
-                const float th = cell >= 0 ? S.theta[i] : 0.0f;
-                const bool rel = cell >= base && th >= reach.x && th <= reach.y;
-                const int off = cell - base;
-                if(rel && off >= kCellClasses) next = min(next, cell);
-                const uint32_t m0 = __ballot_sync(0xffffffffu, rel && off == 0);
-                const uint32_t m1 = __ballot_sync(0xffffffffu, rel && off == 1);
-                const uint32_t m2 = __ballot_sync(0xffffffffu, rel && off == 2);
-                const int n0 = __popc(m0), n1 = __popc(m1), n2 = __popc(m2);
-                if(n0 + n1 + n2 == 0) continue;
-                if(rel && off < kCellClasses) {
-                    const uint32_t below = (1u << lane) - 1u;
-                    const int at = off == 0 ? __popc(m0 & below)
-                                 : off == 1 ? n0 + __popc(m1 & below) : n0 + n1 + __popc(m2 & below);
-                    const float4 w = S.w[i];
-                    CellEntry* e = S.list + at;
-                    e->theta = pack2(th, th);
-                    e->w0x = pack2(w.x, w.x);
-                    e->w0y = pack2(w.y, w.y);
-                    e->w1x = pack2(w.z, w.z);
-                    e->w1y = pack2(w.w, w.w);
+                    for(int k = 0; k < kCellClasses; k++) {
+                        m[q][k] = __ballot_sync(0xffffffffu, off == k);
+                        end[k] += __popc(m[q][k]);
+                    }
                 }
-                held |= (n0 ? 1u : 0u) | (n1 ? 2u : 0u) | (n2 ? 4u : 0u);
+                int fill[kCellClasses] = {0, end[0], end[0] + end[1]};
+                end[1] += end[0];
+                end[2] += end[1];
+#pragma unroll
+                for(int q = 0; q < kUnitLoads; q++) {
+                    int at = -1;
+#pragma unroll
+                    for(int k = 0; k < kCellClasses; k++) {
+                        if(m[q][k] >> lane & 1u) at = fill[k] + __popc(m[q][k] & below);
+                        fill[k] += __popc(m[q][k]);
+                    }
+                    if(at >= 0) {
+                        const float4 w = S.w[q * 32 + lane];
+                        S.list[at][0] = make_ulonglong2(pack2(theta[q], theta[q]), pack2(w.x, w.x));
+                        S.list[at][1] = make_ulonglong2(pack2(w.y, w.y), pack2(w.z, w.z));
+                    }
+                }
                 __syncwarp();
                 int s = 0;
 #pragma unroll
                 for(int k = 0; k < kCellClasses; k++) {
-                    const int end = k == 0 ? n0 : k == 1 ? n0 + n1 : n0 + n1 + n2;
+                    if(s == end[k]) continue;
+                    f32x2 acc[NP][4];
+#pragma unroll
+                    for(int p = 0; p < NP; p++)
+#pragma unroll
+                        for(int e = 0; e < 4; e++) acc[p][e] = 0ull;
 #pragma unroll 2
-                    for(; s < end; s++) {
-                        const CellEntry& e = S.list[s];
-                        const f32x2 th2 = e.theta, w0x = e.w0x, w0y = e.w0y, w1x = e.w1x, w1y = e.w1y;
+                    for(; s < end[k]; s++) {
+                        const ulonglong2 e0 = S.list[s][0], e1 = S.list[s][1];
 #pragma unroll
                         for(int p = 0; p < NP; p++) {
-                            const f32x2 B = beam(tab, th2, minus_tb[p]);
-                            acc[k][p][0] = fma2(w0x, B, acc[k][p][0]);
-                            acc[k][p][1] = fma2(w0y, B, acc[k][p][1]);
-                            acc[k][p][2] = fma2(w1x, B, acc[k][p][2]);
-                            acc[k][p][3] = fma2(w1y, B, acc[k][p][3]);
+                            const f32x2 B = beam(tab, e0.x, minus_tb[p]), aB = mul2(e1.y, B);
+                            acc[p][0] = fma2(e0.y, B, acc[p][0]);
+                            acc[p][1] = fma2(e1.x, B, acc[p][1]);
+                            acc[p][2] = fma2(e0.y, aB, acc[p][2]);
+                            acc[p][3] = fma2(e1.x, aB, acc[p][3]);
                         }
+                    }
+                    float4* row = P.cells + (size_t)(base + k) * P.pitch;
+#pragma unroll
+                    for(int p = 0; p < NP; p++) {
+                        const float2 a = unpack2(acc[p][0]), b = unpack2(acc[p][1]);
+                        const float2 c = unpack2(acc[p][2]), d = unpack2(acc[p][3]);
+                        const int x = P.pos_col[pos0 + 64 * p], y = P.pos_col[pos0 + 64 * p + 32];
+                        if(x >= 0) red_add_f4(row + x, a.x, b.x, c.x, d.x);
+                        if(y >= 0) red_add_f4(row + y, a.y, b.y, c.y, d.y);
                     }
                 }
                 __syncwarp();
+                base = __reduce_min_sync(0xffffffffu, next);
             }
+            if(near_knot) {
+                int bearing[BPL];
 #pragma unroll
-            for(int k = 0; k < kCellClasses; k++) {
-                if(!(held & (1u << k))) continue;
-                float4* row = P.cells + (size_t)(base + k) * P.pitch + pos0;
-#pragma unroll
-                for(int p = 0; p < NP; p++) {
-                    const float2 a = unpack2(acc[k][p][0]), b = unpack2(acc[k][p][1]);
-                    const float2 c = unpack2(acc[k][p][2]), d = unpack2(acc[k][p][3]);
-                    red_add_f4(row + 64 * p, a.x, b.x, c.x, d.x);
-                    red_add_f4(row + 64 * p + 32, a.y, b.y, c.y, d.y);
+                for(int p = 0; p < BPL; p++) {
+                    const int col = P.pos_col[pos0 + 32 * p];
+                    bearing[p] = col < 0 ? -1 : P.col_bearing[col];
                 }
-            }
-            base = __reduce_min_sync(0xffffffffu, next);
-        }
-        if(any_near) {
-            int s_b[BPL];
+#pragma unroll 1
+                for(int q = 0; q < kUnitLoads; q++) {
+                    // (no register array indexing: the values go through selects)
+                    int c = cell[0];
+                    float th = theta[0];
 #pragma unroll
-            for(int p = 0; p < BPL; p++) s_b[p] = P.pos_bearing[pos0 + 32 * p];
-            for(uint32_t q = 0; q < count; q += 32) {
-                const int i = (int)q + lane;
-                uint32_t m = __ballot_sync(0xffffffffu, S.cell[i] <= -2 && S.theta[i] >= reach.x && S.theta[i] <= reach.y);
-                for(; m; m &= m - 1u)
-                    reduce_row_by_row<BPL>(P, S, tab, beam, minus_tb, s_b, (int)q + __ffs(m) - 1);
+                    for(int z = 1; z < kUnitLoads; z++) {
+                        c = q == z ? cell[z] : c;
+                        th = q == z ? theta[z] : th;
+                    }
+                    uint32_t near = __ballot_sync(0xffffffffu, c <= -2 && (in_win >> q & 1u));
+                    for(; near; near &= near - 1u) {
+                        const int l = __ffs(near) - 1;
+                        reduce_row_by_row<BPL>(P, S.w[q * 32 + l], __shfl_sync(0xffffffffu, th, l),
+                                               -3 - __shfl_sync(0xffffffffu, c, l), tab, beam, minus_tb, bearing);
+                    }
+                }
             }
         }
     }
 }
 
 // ---- range filter over the cell rows ----------------------------------------
-// Thread: one position (bearing) and kFilterRows consecutive output rows. It
-// walks the cells that reach them, one 16-byte load each; the taps of the
-// kFilterRows rows slide through registers (the tap of row q at a cell is the
-// tap of row q + 1 at the next). taps[i] = {P[i], D[i]} for i = -1 ..
-// H - 1, zero beyond on both sides by kFilterRows entries.
-constexpr int kFilterRows = 8;
+// A CTA of kFilterWarps warps filters 32 columns x kFilterWarps * kFilterRows
+// output rows. The cell rows it needs are staged in shared memory by 16-byte
+// asynchronous copies, kFilterChunk rows at a time, all of them in flight
+// together. Each thread holds one column and kFilterRows consecutive output
+// rows and walks the staged cells; the taps of its rows slide through
+// registers (the tap of row q at a cell is the tap of row q + 1 at the next).
+// taps[t] = {P[t - 1], D[t - 1]}, t = 0 .. H, zero beyond.
+constexpr int kFilterWarps = 4, kFilterRows = 8, kFilterTile = kFilterWarps * kFilterRows;
+constexpr int kFilterChunk = 72;           // staged cell rows: a 33-tap pulse's tile in one chunk
 
-__device__ __forceinline__ void filter_rows(const CellPing& P, int pos, int r0, const float4* __restrict__ s_taps,
-                                            const int* __restrict__ s_on)
+// Entries of the tap table: H + 1 taps, the sliding window's steps beyond
+// them, rounded up to whole blocks of kFilterRows.
+__host__ __device__ __forceinline__ int cell_tap_entries(int H) { return (H + 2 * kFilterRows - 1) / kFilterRows * kFilterRows; }
+__host__ __device__ __forceinline__ size_t filter_smem(int H)
 {
-    const int n = P.cp.taps + 1;                              // taps i = -1 .. H - 1
+    return (size_t)cell_tap_entries(H) * sizeof(float4) + (size_t)kFilterChunk * 32 * sizeof(float4);
+}
+
+// Columns [32 tile_c, +32) and rows [kFilterTile tile_r, +kFilterTile) of a
+// ping; on: the rows' flags in shared memory. Called by 32 kFilterWarps threads.
+__device__ __forceinline__ void filter_tile(const CellPing& P, int tile_c, int tile_r, float4* s_raw,
+                                            const int* s_on)
+{
+    constexpr int kThreads = 32 * kFilterWarps;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float4* s_taps = s_raw;
+    float4* s_cells = s_raw + cell_tap_entries(P.cp.taps);
+    const int rows0 = tile_r * kFilterTile, r0 = rows0 + warp * kFilterRows, col = tile_c * 32 + lane;
+    const int span = P.cp.taps + kFilterRows;                  // cells that reach a thread's rows
+    const int total = min(P.cp.taps + kFilterTile, P.cp.cells - rows0);   // cells of the tile
+    for(int i = tid; i < cell_tap_entries(P.cp.taps); i += kThreads) s_taps[i] = P.taps[i];
     float2 acc[kFilterRows];
     float e[kFilterRows];
     float4 c[kFilterRows];
@@ -377,36 +420,46 @@ __device__ __forceinline__ void filter_rows(const CellPing& P, int pos, int r0, 
         e[q] = r0 + q < (int)P.nR ? P.row_dev[r0 + q] : 0.0f;
         c[q] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    // Storage row j of cell C = j - 1; row r takes tap index i + 1 = C - r + 1
-    // = j - r. Cells j = r0 .. r0 + n - 1 + kFilterRows - 1.
-    const float4* col = P.cells + (size_t)r0 * P.pitch + pos;
-    const int last = min(n + kFilterRows - 1, P.cp.cells - r0);
-    for(int j0 = 0; j0 < last; j0 += kFilterRows) {
-        float4 a[kFilterRows];
+    const float4* src = P.cells + (size_t)rows0 * P.pitch + tile_c * 32;
+    for(int k0 = 0; k0 < total; k0 += kFilterChunk) {
+        const int rows = min(kFilterChunk, total - k0);
+        if(k0) __syncthreads();
+        for(int i = warp; i < kFilterChunk; i += kFilterWarps) {
+            float4* dst = s_cells + i * 32 + lane;
+            if(i < rows)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)),
+                             "l"(src + (size_t)(k0 + i) * P.pitch + lane) : "memory");
+            else *dst = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        // The thread's cell j (from its first row) is the tile's cell
+        // j + warp * kFilterRows; output row r0 + q takes tap j - q there.
+        const int j0 = max(0, k0 - warp * kFilterRows), j1 = min(span, k0 + kFilterChunk - warp * kFilterRows);
+        for(int j = j0; j < j1; j += kFilterRows) {
+            const float4* a_row = s_cells + (j + warp * kFilterRows - k0) * 32 + lane;
 #pragma unroll
-        for(int u = 0; u < kFilterRows; u++)
-            a[u] = j0 + u < last ? __ldg(col + (size_t)(j0 + u) * P.pitch) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for(int u = 0; u < kFilterRows; u++) {
+                const float4 a = a_row[u * 32];
+                c[u] = s_taps[j + u];
 #pragma unroll
-        for(int u = 0; u < kFilterRows; u++) {
-            // Row q's tap at cell j0 + u: slot (u - q) mod kFilterRows.
-            c[u] = s_taps[j0 + u];
-#pragma unroll
-            for(int q = 0; q < kFilterRows; q++) {
-                const float4 t = c[(u - q + kFilterRows) % kFilterRows];
-                const float mx = fmaf(e[q], a[u].x, a[u].z), my = fmaf(e[q], a[u].y, a[u].w);
-                acc[q].x = fmaf(t.x, a[u].x, fmaf(-t.y, a[u].y, fmaf(t.z, mx, fmaf(-t.w, my, acc[q].x))));
-                acc[q].y = fmaf(t.x, a[u].y, fmaf(t.y, a[u].x, fmaf(t.z, my, fmaf(t.w, mx, acc[q].y))));
+                for(int q = 0; q < kFilterRows; q++) {
+                    const float4 t = c[(u - q + kFilterRows) % kFilterRows];
+                    const float mx = fmaf(e[q], a.x, a.z), my = fmaf(e[q], a.y, a.w);
+                    acc[q].x = fmaf(t.x, a.x, fmaf(-t.y, a.y, fmaf(t.z, mx, fmaf(-t.w, my, acc[q].x))));
+                    acc[q].y = fmaf(t.x, a.y, fmaf(t.y, a.x, fmaf(t.z, my, fmaf(t.w, mx, acc[q].y))));
+                }
             }
         }
     }
-    const int b = P.pos_bearing[pos];
+    const int b = P.col_bearing[col];
     if(b < 0) return;
 #pragma unroll
     for(int q = 0; q < kFilterRows; q++) {
         if(r0 + q >= (int)P.nR) break;
         float2* o = P.out + (size_t)(r0 + q) * P.nB + b;
         const float2 v = *o;
-        *o = s_on[q] ? make_float2(v.x + acc[q].x, v.y + acc[q].y) : make_float2(0.f, 0.f);
+        *o = s_on[warp * kFilterRows + q] ? make_float2(v.x + acc[q].x, v.y + acc[q].y) : make_float2(0.f, 0.f);
     }
 }
 

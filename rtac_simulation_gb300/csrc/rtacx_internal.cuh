@@ -297,9 +297,10 @@ struct CellParams {
     int taps;                        // pulse taps H
 };
 
-// A ping's arguments of the cell kernels (rtacx_cells.cuh). Positions are
-// the bearings in the order in which the lanes hold them, in segments of
-// 32 BPL positions (pos_bearing -1: padding).
+// A ping's arguments of the cell kernels (rtacx_cells.cuh). A window is a set
+// of 32 BPL bearings, in the order in which a warp's lanes hold them, and the
+// sample bearings that it takes. Columns are the cell rows' order of the
+// bearings.
 struct CellPing {
     CellParams cp;
     const float4* sorted;
@@ -309,14 +310,15 @@ struct CellPing {
     const float* beam;               // padded beam table
     const float* ranges;
     const float* row_dev;            // [nR] e_r
-    const float4* taps;              // [cell_tap_entries(H)] {P[i], D[i]}, i = -1 first, zero-padded
-    const float2* seg_reach;         // [segs] bearings that reach a segment's beams
-    const float* pos_theta;          // [pitch]
-    const int* pos_bearing;          // [pitch]
+    const float4* taps;              // [cell_tap_entries(H)]
+    const float2* win_reach;         // [windows] sample bearings [x, y) that the window takes
+    const float* pos_theta;          // [windows][32 BPL] output bearing at a window's position
+    const int* pos_col;              // ... its column (-1: none)
+    const int* col_bearing;          // [pitch] bearing of a column (-1: padding)
     AxisLerp range_axis, beam_axis;
     float theta_lo, theta_hi;        // sample bearings are clamped to these (no beam reaches them)
     uint32_t nR, nB, pitch;
-    int segs;
+    int windows;
 };
 
 // Everything one ping of a batch needs on the device (rtacx_batch_*).
@@ -425,9 +427,10 @@ struct Context {
     float4* d_cells = nullptr;
     float4* d_cell_taps = nullptr;
     float* d_row_dev = nullptr;
-    float2* d_seg_reach = nullptr;
+    float2* d_win_reach = nullptr;
     float* d_pos_theta = nullptr;
-    int* d_pos_bearing = nullptr;
+    int* d_pos_col = nullptr;
+    int* d_col_bearing = nullptr;
 
     // Split persistent gather of 2D pings (see rtacx_reduce.cu).
     uint32_t* d_tile_parts = nullptr;   // [tiles] sample-stream length of each output tile
