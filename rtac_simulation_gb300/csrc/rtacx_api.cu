@@ -8,7 +8,6 @@
 
 namespace rtacx {
 
-void configure_hist_launch(Context& ctx);
 size_t gather_smem_bytes(uint32_t range_tile, uint32_t bearing_tile, uint32_t H, uint32_t W);
 rtacx_status configure_precision(Context& ctx, const rtacx_precision_desc* d);
 
@@ -30,6 +29,10 @@ void sync_echo(Context& c)
     c.bin.echo_cycles = (c.c > 0.0f) ? 2.0 * c.echo_hz / (double)c.c : 0.0;
     c.bin.echo_k_hi = (float)c.bin.echo_cycles;
     c.bin.echo_k_lo = (float)(c.bin.echo_cycles - (double)c.bin.echo_k_hi);
+    c.cell_bin.echo_flags = c.bin.echo_flags;
+    c.cell_bin.echo_cycles = c.bin.echo_cycles;
+    c.cell_bin.echo_k_hi = c.bin.echo_k_hi;
+    c.cell_bin.echo_k_lo = c.bin.echo_k_lo;
 }
 
 // PSF image of the reference sensor (generate_psf_data,
@@ -199,10 +202,15 @@ bool configure_common(Context& c, const Common& s, float pulse_scale)
 
 bool allocate_bins(Context& c)
 {
-    configure_hist_launch(c);
-    const size_t cols = (size_t)c.bin.nBins * kCursorStride;
-    return upload<uint32_t>(c, c.d_offsets, nullptr, c.bin.nBins + 1) &&
-           upload<uint32_t>(c, c.d_totals, nullptr, c.bin.nBins + c.bin.nBins / 1024 + 1) &&   // + block sums
+    c.sort = sort_shape(c, c.bin.nBins);
+    uint32_t bins = c.bin.nBins;
+    if(c.cells_on) {
+        c.cell_sort = sort_shape(c, c.cell_bin.nBins);
+        bins = std::max(bins, c.cell_bin.nBins);
+    }
+    const size_t cols = (size_t)bins * kCursorStride;
+    return upload<uint32_t>(c, c.d_offsets, nullptr, bins + 1) &&
+           upload<uint32_t>(c, c.d_totals, nullptr, bins + bins / 1024 + 1) &&   // + block sums
            upload<int2>(c, c.d_win, nullptr, c.nR) &&
            upload<uint32_t>(c, c.d_hist, nullptr, cols) &&
            ((c.hist_cols = cols), true);
@@ -396,6 +404,10 @@ rtacx_status rtacx_configure_2d(rtacx_ctx* ctx, const rtacx_sensor_2d* s)
         return bbt;
     };
     const std::vector<int2> bbt64 = tile_ranges(64), bbt128 = tile_ranges(128);
+    if(!texture_psf) {
+        configure_cells(c, sb);
+        sync_echo(c);
+    }
     std::vector<float> bpad(c.W + 2, 0.0f);
     std::memcpy(bpad.data() + 1, s->beam, sizeof(float) * c.W);
     if(!upload(c, c.d_beam, bpad.data(), bpad.size()) ||
@@ -405,7 +417,10 @@ rtacx_status rtacx_configure_2d(rtacx_ctx* ctx, const rtacx_sensor_2d* s)
         return RTACX_ERR_OUT_OF_MEMORY;
     c.d_bb_tiles = (c.bearing_tile == 64) ? c.d_bb_tiles64 : c.d_bb_tiles128;
     if(texture_psf && make_psf_texture(c, s) != RTACX_OK) return RTACX_ERR_CUDA;
-    if(texture_psf || !configure_cells(c, sb)) {
+    if(c.cells_on) {
+        c.cell.pulse = c.d_pulse; c.cell.beam = c.d_beam; c.cell.ranges = c.d_ranges;
+    }
+    else {
         const uint64_t tiles = (uint64_t)((c.nB + c.bearing_tile - 1) / c.bearing_tile) * ((c.nR + c.range_tile - 1) / c.range_tile);
         if(!upload<uint32_t>(c, c.d_tile_parts, nullptr, tiles) || !upload<uint32_t>(c, c.d_tile_first, nullptr, tiles + 1) ||
            !upload<uint4>(c, c.d_items, nullptr, tiles * 256) || !upload<uint32_t>(c, c.d_item_counter, nullptr, 1))
@@ -465,11 +480,12 @@ rtacx_status rtacx_reduce(rtacx_ctx* ctx, const void* samples, uint64_t n, float
     Context& c = ctx->impl;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     for(bool& t : c.traced) t = false;
+    if(c.cells_on) return run_cells(c, samples, n, reinterpret_cast<float2*>(out), s);
     st = run_binning(c, samples, n, s);
-    if(st == RTACX_OK && !c.cells_on) st = run_windows(c, s);
+    if(st == RTACX_OK) st = run_windows(c, s);
     if(st != RTACX_OK) return st;
     c.mark(5, false, s);
-    st = c.cells_on ? run_cells(c, n, reinterpret_cast<float2*>(out), s) : run_reduce(c, out, s);
+    st = run_reduce(c, out, s);
     c.mark(5, true, s);
     return st;
 }
@@ -531,6 +547,8 @@ rtacx_status rtacx_diag_sorted(rtacx_ctx* ctx, float* records, uint64_t max_reco
     if(!ctx || (!records && max_records)) return RTACX_ERR_INVALID_ARGUMENT;
     Context& c = ctx->impl;
     if(set_device(c) != RTACX_OK) return RTACX_ERR_CUDA;
+    const rtacx_status st = restore_sorted(c, static_cast<cudaStream_t>(stream));
+    if(st != RTACX_OK) return st;
     const uint64_t k = std::min(max_records, c.d_sorted ? c.capacity : 0);
     if(k && cudaMemcpyAsync(records, c.d_sorted, k * sizeof(float4), cudaMemcpyDefault,
                             static_cast<cudaStream_t>(stream)) != cudaSuccess) {

@@ -111,7 +111,7 @@ struct Batch {
             d.n = n;
             d.bin = c.bin;
             d.bin.vec4 = (c.dims == 2 && reinterpret_cast<uintptr_t>(pings[i].samples) % 16 == 0) ? 1 : 0;
-            d.chunks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(c.hist_ctas, ceil_div(n, cand.per_cta)));
+            d.chunks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(c.sort.hist_ctas, ceil_div(n, cand.per_cta)));
             d.hist = c.d_hist; d.totals = c.d_totals; d.offsets = c.d_offsets; d.oor = c.d_oor; d.err = c.d_err;
             d.sorted = c.d_sorted;
             d.nR = c.nR; d.overlap = c.overlap; d.support = c.d_support; d.win = c.d_win;
@@ -362,6 +362,7 @@ rtacx_status rtacx_batch_run(rtacx_batch* b, void* stream)
         B.error = "cudaGraphLaunch failed";
         return RTACX_ERR_CUDA;
     }
+    for(const rtacx_ping_desc& p : B.pings) p.ctx->impl.sorted_cells_n = 0;   // the batch sorts in rtacx_bin's order
     return RTACX_OK;
 }
 

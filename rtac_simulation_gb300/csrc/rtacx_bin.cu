@@ -46,11 +46,12 @@ namespace {
 constexpr int kScanThreads = 1024;
 
 __global__ void k_count(const float* __restrict__ samples, uint64_t n, BinParams p,
-                        uint32_t* __restrict__ totals, unsigned long long* __restrict__ oor)
+                        uint32_t* __restrict__ totals, unsigned long long* __restrict__ oor,
+                        uint32_t* __restrict__ nonempty)
 {
     extern __shared__ uint32_t sh[];
     __shared__ unsigned long long s_oor[2];
-    count_chunk(samples, n, p, blockIdx.x, gridDim.x, totals, oor, sh, s_oor);
+    count_chunk(samples, n, p, blockIdx.x, gridDim.x, totals, oor, sh, s_oor, nonempty);
 }
 
 // Exclusive scan of totals[0, nBins) into offsets[0, nBins] by one CTA of
@@ -245,6 +246,13 @@ __global__ void k_oor_out(const unsigned long long* __restrict__ src, uint64_t* 
     if(threadIdx.x < 2) dst[threadIdx.x] = src[threadIdx.x];
 }
 
+// Puts records [*count, n) of the sorted scratch out of every sensor's range.
+__global__ void k_mark_tail(float4* __restrict__ sorted, const uint32_t* __restrict__ count, uint64_t n)
+{
+    for(uint64_t i = *count + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        sorted[i] = make_float4(0.f, 0.f, INFINITY, 0.f);
+}
+
 // ---- batched stages (one launch per stage over every ping of a batch) -----
 
 __global__ void k_count_batch(const PingDev* __restrict__ pings, const uint2* __restrict__ map)
@@ -324,6 +332,7 @@ bool ensure_capacity(Context& ctx, uint64_t n)
     if(ctx.d_sorted) cudaFree(ctx.d_sorted);
     ctx.d_sorted = p;
     ctx.capacity = cap;
+    ctx.sorted_cells_n = 0;
     return true;
 }
 
@@ -503,50 +512,87 @@ constexpr int kNumScatterShapes = sizeof(kScatterShapes) / sizeof(kScatterShapes
 
 } // namespace
 
-void configure_hist_launch(Context& ctx);
-
 rtacx_status run_binning(Context& ctx, const void* samples, uint64_t n, cudaStream_t stream)
 {
     const BinParams& p = ctx.bin;
+    ctx.sorted_cells_n = 0;
     RTACX_CUDA(cudaMemsetAsync(ctx.d_oor, 0, 2 * sizeof(unsigned long long), stream));
     if(n == 0) {
         RTACX_CUDA(cudaMemsetAsync(ctx.d_offsets, 0, (p.nBins + 1) * sizeof(uint32_t), stream));
+        return RTACX_OK;
+    }
+    ctx.mark(1, false, stream);
+    RTACX_CUDA(cudaMemsetAsync(ctx.d_totals, 0, (p.nBins + (p.nBins + kScanBlock - 1) / kScanBlock) * sizeof(uint32_t),
+                               stream));
+    ctx.mark(1, true, stream);
+    return run_sort(ctx, p, ctx.sort, samples, n, nullptr, stream);
+}
+
+rtacx_status run_sort(Context& ctx, const BinParams& p, const SortShape& shape, const void* samples, uint64_t n,
+                      uint32_t* nonempty, cudaStream_t stream)
+{
+    const uint32_t grid = hist_grid(shape.hist_ctas, n);
+    const size_t smem = (size_t)p.nBins * sizeof(uint32_t);
+    const float* s = static_cast<const float*>(samples);
+    const uint32_t scan_blocks = (p.nBins + kScanBlock - 1) / kScanBlock;
+    ctx.mark(0, false, stream);
+    k_count<<<grid, shape.hist_threads, smem + (nonempty ? (p.key.nR + 31) / 32 * sizeof(uint32_t) : 0), stream>>>(
+        s, n, p, ctx.d_totals, ctx.d_oor, nonempty);
+    RTACX_CUDA(cudaGetLastError());
+    ctx.mark(0, true, stream);
+    ctx.mark(2, false, stream);
+    // d_hist holds the per-bin write cursors of the scatter.
+    k_binscan_blocks<<<scan_blocks, kScanBlock, 0, stream>>>(ctx.d_totals, p.nBins, ctx.d_offsets, ctx.d_hist);
+    RTACX_CUDA(cudaGetLastError());
+    ctx.mark(2, true, stream);
+    ctx.mark(3, false, stream);
+    if(shape.scatter_shape) {
+        const ScatterShape& sh = kScatterShapes[shape.scatter_shape - 1];
+        const uint32_t g = hist_grid((uint32_t)ctx.sm_count, n);
+        const bool one_batch = pipe_bins_per_thread(p.nBins, sh.nt) <= (uint32_t)kReserveBatch;
+        const ScatterFn fn = sh.fn[p.echo_flags ? 1 : 0][one_batch ? 1 : 0];
+        fn<<<g, sh.nt, staged_smem_bytes(sh.nt, sh.u, p.nBins), stream>>>(s, n, p, ctx.d_hist, ctx.d_offsets,
+                                                                       ctx.d_sorted, ctx.d_err);
     }
     else {
-        const uint32_t grid = hist_grid(ctx.hist_ctas, n);
-        const size_t smem = (size_t)p.nBins * sizeof(uint32_t);
-        const float* s = static_cast<const float*>(samples);
-        ctx.mark(1, false, stream);
-        const uint32_t scan_blocks = (p.nBins + kScanBlock - 1) / kScanBlock;
-        RTACX_CUDA(cudaMemsetAsync(ctx.d_totals, 0, (p.nBins + scan_blocks) * sizeof(uint32_t), stream));
-        ctx.mark(1, true, stream);
-        ctx.mark(0, false, stream);
-        k_count<<<grid, ctx.hist_threads, smem, stream>>>(s, n, p, ctx.d_totals, ctx.d_oor);
-        RTACX_CUDA(cudaGetLastError());
-        ctx.mark(0, true, stream);
-        ctx.mark(2, false, stream);
-        // d_hist holds the per-bin write cursors of the scatter.
-        k_binscan_blocks<<<scan_blocks, kScanBlock, 0, stream>>>(ctx.d_totals, p.nBins, ctx.d_offsets, ctx.d_hist);
-        RTACX_CUDA(cudaGetLastError());
-        ctx.mark(2, true, stream);
-        ctx.mark(3, false, stream);
-        if(ctx.scatter_shape) {
-            const ScatterShape& sh = kScatterShapes[ctx.scatter_shape - 1];
-            const uint32_t g = hist_grid((uint32_t)ctx.sm_count, n);
-            const bool one_batch = pipe_bins_per_thread(p.nBins, sh.nt) <= (uint32_t)kReserveBatch;
-            const ScatterFn fn = sh.fn[p.echo_flags ? 1 : 0][one_batch ? 1 : 0];
-            fn<<<g, sh.nt, staged_smem_bytes(sh.nt, sh.u, p.nBins), stream>>>(s, n, p, ctx.d_hist, ctx.d_offsets,
-                                                                           ctx.d_sorted, ctx.d_err);
-        }
-        else {
-            k_scatter<<<hist_grid(ctx.scatter_ctas, n), ctx.hist_threads, smem, stream>>>(s, n, p, ctx.d_hist,
-                                                                                           ctx.d_offsets, ctx.d_sorted,
-                                                                                           ctx.d_err);
-        }
-        RTACX_CUDA(cudaGetLastError());
-        ctx.mark(3, true, stream);
+        k_scatter<<<hist_grid(shape.scatter_ctas, n), shape.hist_threads, smem, stream>>>(s, n, p, ctx.d_hist,
+                                                                                          ctx.d_offsets, ctx.d_sorted,
+                                                                                          ctx.d_err);
     }
+    RTACX_CUDA(cudaGetLastError());
+    ctx.mark(3, true, stream);
     return RTACX_OK;
+}
+
+// Brings a sorted scratch that the cell form left in its own order (window x
+// cell block; the same records, each once) into the order that rtacx_bin
+// documents: the records' tail beyond the in-range count is marked out of
+// range, then the reference order's passes run from the scratch itself into
+// a stream-ordered buffer that is copied back.
+rtacx_status restore_sorted(Context& ctx, cudaStream_t stream)
+{
+    const uint64_t n = ctx.sorted_cells_n;
+    if(!n) return RTACX_OK;
+    float4* sorted = ctx.d_sorted;
+    k_mark_tail<<<(uint32_t)std::min<uint64_t>((n + 255) / 256, (uint64_t)ctx.sm_count * 16), 256, 0, stream>>>(
+        sorted, ctx.d_offsets + ctx.cell_bin.nBins, n);
+    RTACX_CUDA(cudaGetLastError());
+    void* tmp = nullptr;
+    RTACX_CUDA(cudaMallocAsync(&tmp, n * sizeof(float4), stream));
+    const BinParams kept = ctx.bin;
+    // The scratch holds 16-byte records with the echo model applied.
+    ctx.bin.stride = 4;
+    ctx.bin.vec4 = 1;
+    ctx.bin.echo_flags = 0;
+    ctx.d_sorted = static_cast<float4*>(tmp);
+    const rtacx_status st = run_binning(ctx, sorted, n, stream);
+    ctx.bin = kept;
+    ctx.d_sorted = sorted;
+    cudaError_t e = cudaSuccess;
+    if(st == RTACX_OK) e = cudaMemcpyAsync(sorted, tmp, n * sizeof(float4), cudaMemcpyDeviceToDevice, stream);
+    cudaFreeAsync(tmp, stream);
+    RTACX_CUDA(e);
+    return st;
 }
 
 // Effective windows of every output row (the per-row gathers' input).
@@ -610,11 +656,12 @@ rtacx_status launch_bin_batch(std::string& error, const PingDev* pings, uint32_t
     return RTACX_OK;
 }
 
-// Launch shape of the count / scatter passes for the configured bin count.
-void configure_hist_launch(Context& ctx)
+// Launch shape of the count / scatter passes for a bin count.
+SortShape sort_shape(const Context& ctx, uint32_t nBins)
 {
-    const size_t smem = (size_t)ctx.bin.nBins * sizeof(uint32_t);
-    raise_smem_limit((const void*)k_count, std::max<size_t>(smem, 1));
+    SortShape shape;
+    const size_t smem = (size_t)nBins * sizeof(uint32_t);
+    raise_smem_limit((const void*)k_count, smem + (size_t)(ctx.nR + 31) / 32 * sizeof(uint32_t) + sizeof(uint32_t));
     raise_smem_limit((const void*)k_scatter, std::max<size_t>(smem, 1));
     // 512-thread CTAs when two histograms fit in one SM's shared memory, one
     // 1024-thread CTA otherwise; each pass gets as many CTAs as are resident
@@ -622,31 +669,31 @@ void configure_hist_launch(Context& ctx)
     // reservation phases of different CTAs overlap and no CTA waits for a
     // second wave.
     const size_t per_sm = 200u * 1024u;
-    ctx.hist_threads = per_sm / (smem + 1024) >= 2 ? 512 : 1024;
+    shape.hist_threads = per_sm / (smem + 1024) >= 2 ? 512 : 1024;
     auto resident = [&](const void* fn) {
         int nb = 0;
-        if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, (int)ctx.hist_threads, std::max<size_t>(smem, 1)) !=
+        if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, (int)shape.hist_threads, std::max<size_t>(smem, 1)) !=
                cudaSuccess || nb < 1)
             nb = 1;
         return (uint32_t)ctx.sm_count * (uint32_t)std::min(nb, 4);
     };
-    ctx.hist_ctas = resident((const void*)k_count);
-    ctx.scatter_ctas = resident((const void*)k_scatter);
+    shape.hist_ctas = resident((const void*)k_count);
+    shape.scatter_ctas = resident((const void*)k_scatter);
     // Staged scatter: the first shape of kScatterShapes whose shared memory
     // fits.
-    ctx.scatter_shape = 0;
     int optin = 0, smem_sm = 0;
     if(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx.device) != cudaSuccess) optin = 0;
     if(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx.device) != cudaSuccess) smem_sm = 0;
-    for(int c = 0; c < kNumScatterShapes && !ctx.scatter_shape; c++) {
+    for(int c = 0; c < kNumScatterShapes && !shape.scatter_shape; c++) {
         const ScatterShape& sh = kScatterShapes[c];
-        const size_t need = staged_smem_bytes(sh.nt, sh.u, ctx.bin.nBins);
+        const size_t need = staged_smem_bytes(sh.nt, sh.u, nBins);
         bool ok = need + 1024 <= (size_t)optin && need + 1024 <= (size_t)smem_sm;
         for(int e = 0; e < 2 && ok; e++)
             for(int b = 0; b < 2 && ok; b++) ok = raise_smem_limit((const void*)sh.fn[e][b], need) == cudaSuccess;
-        if(ok) ctx.scatter_shape = c + 1;
+        if(ok) shape.scatter_shape = c + 1;
     }
     cudaGetLastError();
+    return shape;
 }
 
 } // namespace rtacx

@@ -61,20 +61,31 @@ __device__ __forceinline__ void for_chunk(const float* samples, uint64_t n, cons
 }
 
 // Count pass of chunk c of nc (shared-memory histogram sh of p.nBins
-// words), added into totals[0, nBins) (zeroed by the caller).
+// words), added into totals[0, nBins) (zeroed by the caller). With `nonempty`
+// also the bitmap of the range bins that hold a sample (sh then has
+// (nR + 31) / 32 words more), which the cell order's histogram does not tell.
 __device__ __forceinline__ void count_chunk(const float* __restrict__ samples, uint64_t n, const BinParams& p, uint32_t c,
                             uint32_t nc, uint32_t* __restrict__ totals, unsigned long long* __restrict__ oor,
-                            uint32_t* sh, unsigned long long* s_oor)
+                            uint32_t* sh, unsigned long long* s_oor, uint32_t* __restrict__ nonempty = nullptr)
 {
-    for(uint32_t b = threadIdx.x; b < p.nBins; b += blockDim.x) sh[b] = 0u;
+    const uint32_t words = nonempty ? (p.key.nR + 31) / 32 : 0u;
+    uint32_t* s_bits = sh + p.nBins;
+    for(uint32_t b = threadIdx.x; b < p.nBins + words; b += blockDim.x) sh[b] = 0u;
     if(threadIdx.x < 2) s_oor[threadIdx.x] = 0ull;
     __syncthreads();
 
     uint32_t low = 0, high = 0;
-    for_chunk(samples, n, p, c, nc, [&](const bool* valid, const float4*, const uint32_t* key, const int* side) {
+    for_chunk(samples, n, p, c, nc, [&](const bool* valid, const float4* rec, const uint32_t* key, const int* side) {
 #pragma unroll
         for(int u = 0; u < kTileLoads; u++) {
-            if(valid[u] && key[u] != kOutOfRange) atomicAdd(&sh[key[u]], 1u);
+            if(valid[u] && key[u] != kOutOfRange) {
+                atomicAdd(&sh[key[u]], 1u);
+                if(words) {
+                    int unused;
+                    const uint32_t r = range_key(p.key, rec[u].z, unused), bit = 1u << (r & 31u);
+                    if(!(s_bits[r >> 5] & bit)) atomicOr(&s_bits[r >> 5], bit);
+                }
+            }
             else if(valid[u]) {
                 if(side[u] < 0) low++; else high++;
             }
@@ -95,6 +106,8 @@ __device__ __forceinline__ void count_chunk(const float* __restrict__ samples, u
     }
     for(uint32_t b = threadIdx.x; b < p.nBins; b += blockDim.x)
         if(sh[b]) atomicAdd(&totals[b], sh[b]);
+    for(uint32_t b = threadIdx.x; b < words; b += blockDim.x)
+        if(s_bits[b]) atomicOr(&nonempty[b], s_bits[b]);
     // Per-block sums of kScanBlock bins (totals[nBins + blk]) for the
     // parallel bin scan: one warp per block of bins.
     const uint32_t blocks = (p.nBins + kScanBlock - 1) / kScanBlock;
@@ -180,6 +193,21 @@ __device__ __forceinline__ void scatter_chunk(const float* __restrict__ samples,
 __device__ __forceinline__ uint32_t bin_count(const uint32_t* off, uint32_t nBB, int j)
 {
     return off[(size_t)(j + 1) * nBB] - off[(size_t)j * nBB];
+}
+
+// Does row r's reference window hold at least two non-empty range bins of the
+// bitmap (the view of src/Binner.cu:90-102 is empty otherwise)?
+__device__ __forceinline__ bool row_on(const uint32_t* nonempty, int nR, int ov, int r)
+{
+    const int lo = max(0, r - ov), hi = (int)min((long long)nR - 1, (long long)r + ov);
+    int seen = 0;
+    for(int w = lo >> 5; w <= hi >> 5 && seen < 2; w++) {
+        uint32_t bits = nonempty[w];
+        if(w == lo >> 5) bits &= 0xFFFFFFFFu << (lo & 31);
+        if(w == hi >> 5) bits &= 0xFFFFFFFFu >> (31 - (hi & 31));
+        seen += __popc(bits);
+    }
+    return seen >= 2;
 }
 
 // First / last non-empty range bin of row r's reference window

@@ -23,12 +23,13 @@ namespace {
 constexpr int kCellThreads = 256, kCellWarps = kCellThreads / 32;
 constexpr size_t kMaxCellBytes = (size_t)1 << 30;      // cell rows of one context
 constexpr double kMaxKnot = 0.01;
+constexpr uint32_t kCellBins = 12288;
 
 size_t cells_smem(int W) { return kCellWarps * sizeof(CellWarpSmem) + (size_t)(W + 2) * sizeof(float2); }
 
-template <int BPL>
+template <int BPL, bool SHARED>
 __global__ void __launch_bounds__(kCellThreads, BPL == 2 ? 3 : 2)
-k_cells(const CellPing P, const uint32_t* __restrict__ total)
+k_cells(const CellPing P, const uint32_t* __restrict__ total, uint32_t unit)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     CellWarpSmem& S = reinterpret_cast<CellWarpSmem*>(s_raw)[threadIdx.x >> 5];
@@ -37,20 +38,40 @@ k_cells(const CellPing P, const uint32_t* __restrict__ total)
     __syncthreads();
     BeamLookup beam;
     beam.init(P.beam_axis);
-    const uint32_t m = *total, units = (m + kUnit - 1) / kUnit;
-    for(uint32_t u = blockIdx.x * kCellWarps + (threadIdx.x >> 5); u < units; u += gridDim.x * kCellWarps)
-        accumulate_unit<BPL>(P, u * kUnit, min((uint32_t)kUnit, m - u * kUnit), blockIdx.y, gridDim.y, S, tab, beam);
+    const uint32_t m = *total;
+    for(uint64_t u = (uint64_t)(blockIdx.x * kCellWarps + (threadIdx.x >> 5)) * unit; u < m;
+        u += (uint64_t)gridDim.x * kCellWarps * unit)
+        accumulate_unit<BPL, SHARED>(P, (uint32_t)u, min(unit, m - (uint32_t)u), blockIdx.y, gridDim.y, S, tab, beam);
+}
+
+using CellsFn = void (*)(const CellPing, const uint32_t*, uint32_t);
+CellsFn cells_fn(int bpl, bool shared_out)
+{
+    if(shared_out) return bpl == 4 ? k_cells<4, true> : k_cells<2, true>;
+    return bpl == 4 ? k_cells<4, false> : k_cells<2, false>;
+}
+
+// Zeroes what a ping's passes add into: the bin totals, the range-bin bitmap,
+// the cell rows and the ping (8-byte stores: the ping's alignment).
+__global__ void k_cells_clear(uint32_t* __restrict__ totals, uint32_t n_totals, uint32_t* __restrict__ bits,
+                              uint32_t n_bits, float4* __restrict__ cells, uint64_t n_cells, float2* __restrict__ out,
+                              uint64_t n_out)
+{
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    for(uint64_t i = i0; i < n_totals; i += stride) totals[i] = 0u;
+    for(uint64_t i = i0; i < n_bits; i += stride) bits[i] = 0u;
+    for(uint64_t i = i0; i < n_cells; i += stride) cells[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for(uint64_t i = i0; i < n_out; i += stride) out[i] = make_float2(0.f, 0.f);
 }
 
 __global__ void __launch_bounds__(32 * kFilterWarps)
-k_cells_filter(const CellPing P, const uint32_t* __restrict__ off, uint32_t nBB, int ov)
+k_cells_filter(const CellPing P, const uint32_t* __restrict__ nonempty, int ov)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ int s_on[kFilterTile];
     if(threadIdx.x < kFilterTile) {
         const int r = blockIdx.y * kFilterTile + threadIdx.x;
-        int f, l;
-        s_on[threadIdx.x] = r < (int)P.nR && ref_window(off, nBB, P.nR, ov, r, f, l) ? 1 : 0;
+        s_on[threadIdx.x] = r < (int)P.nR && row_on(nonempty, (int)P.nR, ov, r) ? 1 : 0;
     }
     filter_tile(P, blockIdx.x, blockIdx.y, reinterpret_cast<float4*>(s_raw), s_on);   // synchronises before it reads s_on
 }
@@ -77,9 +98,10 @@ bool put(T*& dst, const std::vector<T>& src)
 
 void free_cells(Context& c)
 {
-    drop(c.d_cells); drop(c.d_cell_taps); drop(c.d_row_dev); drop(c.d_win_reach);
+    drop(c.d_cells); drop(c.d_cell_taps); drop(c.d_row_dev); drop(c.d_nonempty);
     drop(c.d_pos_theta); drop(c.d_pos_col); drop(c.d_col_bearing);
     c.cells_on = false;
+    c.sorted_cells_n = 0;
 }
 
 // Decides whether a configured 2D sensor takes the cell form and builds its
@@ -147,37 +169,34 @@ bool configure_cells(Context& c, double beam_support)
     c.cell.theta_lo = (float)(*mm.first - 2.0 * span);
     c.cell.theta_hi = (float)(*mm.second + 2.0 * span);
 
-    // Windows. Narrow beams: consecutive bearings, each sample in exactly one
-    // window (the bearings that a window's samples reach are all in it), the
-    // shortest windows that still take half a beam's width of bearings on
-    // average (shorter ones would be flushed after too few samples). Wide
-    // beams: the bearings are shared out among windows that all take every
-    // sample.
+    // Windows. Narrow beams: equal intervals of sample bearings, each with the
+    // consecutive output bearings that its samples reach; every sample is in
+    // exactly one. As few as keep the bearings of each within 64 (else 128),
+    // unless a window would be narrower than half a beam's half width (its
+    // sums would be flushed after too few samples). Wide beams: the bearings
+    // are shared out among windows that all take every sample.
     std::vector<int> sorted_b(nB);
     std::iota(sorted_b.begin(), sorted_b.end(), 0);
     std::stable_sort(sorted_b.begin(), sorted_b.end(), [&](int x, int y) { return c.bearings[x] < c.bearings[y]; });
-    std::vector<float2> reach;
-    std::vector<std::vector<int>> members;
-    const float all_lo = (float)(*mm.first - beam_support), all_hi = (float)(*mm.second + beam_support);
+    const double lo = (double)*mm.first - beam_support, hi = (double)*mm.second + beam_support;
+    std::vector<double> theta_sorted(nB);
+    for(int i = 0; i < nB; i++) theta_sorted[i] = c.bearings[sorted_b[i]];
+    const int max_windows = std::max(1, (int)std::min(4096.0, (hi - lo) / (0.5 * beam_support)));
+    std::vector<int2> span_of;              // [first, end) sorted bearings of each window
     int bpl = 0;
-    for(int cand = 2; cand <= 4 && !bpl; cand += 2) {
-        const int len = 32 * cand;
-        reach.clear();
-        members.clear();
-        float cur = all_lo;
-        bool ok = true;
-        while(ok && cur < all_hi) {
-            int f = 0;
-            while(f < nB && (double)c.bearings[sorted_b[f]] + beam_support < (double)cur) f++;
-            const int end = std::min(nB, f + len);
-            const float y = end < nB ? (float)((double)c.bearings[sorted_b[end]] - beam_support) : all_hi;
-            ok = y > cur && f < end && reach.size() < 4096;
-            reach.push_back(make_float2(cur, end < nB ? y : std::nextafter(all_hi, INFINITY)));
-            members.emplace_back(sorted_b.begin() + f, sorted_b.begin() + end);
-            cur = y;
+    for(int cand = 2; cand <= 4 && !bpl; cand += 2)
+        for(int w = std::max(1, nB / (32 * cand)); w <= max_windows && !bpl; w++) {
+            const double step = (hi - lo) / w, slack = 1e-5 * (hi - lo) + beam_support;   // 1e-5: the float window index
+            bool fits = true;
+            span_of.clear();
+            for(int q = 0; q < w && fits; q++) {
+                const auto f = std::lower_bound(theta_sorted.begin(), theta_sorted.end(), lo + q * step - slack);
+                const auto e = std::upper_bound(f, theta_sorted.end(), lo + (q + 1) * step + slack);
+                span_of.push_back(make_int2((int)(f - theta_sorted.begin()), (int)(e - theta_sorted.begin())));
+                fits = e - f <= 32 * cand;
+            }
+            if(fits) bpl = cand;
         }
-        if(ok && ((double)all_hi - all_lo) / reach.size() >= 0.5 * beam_support) bpl = cand;
-    }
     const bool shared_out = bpl == 0;
     if(shared_out) bpl = nB > 64 ? 4 : 2;
     const int len = 32 * bpl;
@@ -200,14 +219,30 @@ bool configure_cells(Context& c, double beam_support)
         const int wins = (nB + len - 1) / len;
         pos.assign((size_t)wins * len, -1);
         deal(sorted_b, pos, 0);
-        reach.assign(wins, make_float2(all_lo, std::nextafter(all_hi, INFINITY)));
     }
     else {
-        pos.assign(reach.size() * len, -1);
-        for(size_t w = 0; w < reach.size(); w++) deal(members[w], pos, w * len);
+        pos.assign(span_of.size() * len, -1);
+        for(size_t w = 0; w < span_of.size(); w++)
+            deal(std::vector<int>(sorted_b.begin() + span_of[w].x, sorted_b.begin() + span_of[w].y), pos, w * len);
     }
     c.cell_bpl = bpl;
-    c.cell.windows = (int)reach.size();
+    c.cell_shared = shared_out;
+    c.cell.windows = (int)(pos.size() / len);
+    // Sort order: window x cell block, with as many bins as the pipelined
+    // scatter takes at one reservation batch per thread.
+    BinParams& bin = c.cell_bin;
+    bin = c.bin;
+    bin.cell = cp;
+    bin.nBB = shared_out ? 1u : (uint32_t)span_of.size();
+    bin.bb_scale = (float)(bin.nBB / (hi - lo));
+    bin.bb_offset = (float)(-lo * (bin.nBB / (hi - lo)));
+    for(bin.cell_shift = 0;; bin.cell_shift++) {
+        bin.cell_blocks = (uint32_t)((cp.cells - 1) >> bin.cell_shift) + 1u;
+        if(bin.nBB * bin.cell_blocks <= kCellBins || bin.cell_blocks == 1u) break;
+    }
+    bin.nBins = bin.nBB * bin.cell_blocks;
+    c.cell.win_scale = bin.bb_scale;
+    c.cell.win_offset = bin.bb_offset;
     // Columns: the lanes' order for shared-out windows (whole rows of 512
     // bytes per reduction), the bearings' own order for overlapping ones.
     const uint32_t pitch = shared_out ? (uint32_t)pos.size() : (uint32_t)((nB + 31) / 32 * 32);
@@ -232,17 +267,15 @@ bool configure_cells(Context& c, double beam_support)
         }
         taps[i + 1] = make_float4((float)p[0], (float)p[1], (float)d[0], (float)d[1]);
     }
-    bool ok = put(c.d_cell_taps, taps) && put(c.d_row_dev, dev) && put(c.d_win_reach, reach) &&
+    bool ok = put(c.d_cell_taps, taps) && put(c.d_row_dev, dev) && put(c.d_nonempty, std::vector<uint32_t>((nR + 31) / 32, 0u)) &&
               put(c.d_pos_theta, theta) && put(c.d_pos_col, col) && put(c.d_col_bearing, col_bearing);
     if(ok && cudaMalloc(&c.d_cells, cell_bytes) != cudaSuccess) { cudaGetLastError(); ok = false; }
-    const void* fn = c.cell_bpl == 4 ? (const void*)k_cells<4> : (const void*)k_cells<2>;
-    if(ok) ok = raise_smem_limit(fn, cells_smem(W)) == cudaSuccess &&
+    if(ok) ok = raise_smem_limit((const void*)cells_fn(bpl, shared_out), cells_smem(W)) == cudaSuccess &&
                 raise_smem_limit((const void*)k_cells_filter, filter_smem(H)) == cudaSuccess;
     if(!ok) { free_cells(c); return false; }
     CellPing& P = c.cell;
     P.cells = c.d_cells;
-    P.pulse = c.d_pulse; P.beam = c.d_beam; P.ranges = c.d_ranges;
-    P.row_dev = c.d_row_dev; P.taps = c.d_cell_taps; P.win_reach = c.d_win_reach;
+    P.row_dev = c.d_row_dev; P.taps = c.d_cell_taps;
     P.pos_theta = c.d_pos_theta; P.pos_col = c.d_pos_col; P.col_bearing = c.d_col_bearing;
     P.range_axis = c.red.range_axis; P.beam_axis = c.red.beam_axis;
     P.nR = c.nR; P.nB = c.nB;
@@ -250,28 +283,42 @@ bool configure_cells(Context& c, double beam_support)
     return true;
 }
 
-rtacx_status run_cells(Context& c, uint64_t n, float2* out, cudaStream_t stream)
+rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out, cudaStream_t stream)
 {
     CellPing P = c.cell;
     P.sorted = c.d_sorted;
     P.out = out;
-    cudaError_t e = cudaMemsetAsync(c.d_cells, 0, (size_t)P.cp.cells * P.pitch * sizeof(float4), stream);
-    if(e == cudaSuccess) e = cudaMemsetAsync(out, 0, (size_t)c.nR * c.nB * sizeof(float2), stream);
-    if(e != cudaSuccess) { c.error = std::string("clearing the cell rows: ") + cudaGetErrorString(e); return RTACX_ERR_CUDA; }
-    // As many units as there are; the windows of a unit are shared out over
-    // blockIdx.y when there are too few units to fill the SMs.
-    const uint64_t ctas = std::max<uint64_t>(1, (n + (uint64_t)kUnit * kCellWarps - 1) / ((uint64_t)kUnit * kCellWarps));
-    const uint32_t full = (uint32_t)c.sm_count * 3u;
-    const uint32_t gx = (uint32_t)std::min<uint64_t>(ctas, (uint64_t)full * 4u);
-    const uint32_t gy = (uint32_t)std::min<uint64_t>((uint64_t)P.windows, std::max<uint64_t>(1, full / gx));
-    const dim3 grid(gx, gy);
-    const size_t smem = cells_smem(P.beam_axis.n);
-    if(c.cell_bpl == 4) k_cells<4><<<grid, kCellThreads, smem, stream>>>(P, c.d_offsets + c.bin.nBins);
-    else k_cells<2><<<grid, kCellThreads, smem, stream>>>(P, c.d_offsets + c.bin.nBins);
-    const dim3 fgrid(P.pitch / 32, (c.nR + kFilterTile - 1) / kFilterTile);
-    k_cells_filter<<<fgrid, 32 * kFilterWarps, filter_smem(P.cp.taps), stream>>>(
-        P, c.d_offsets, c.bin.nBB, c.overlap);
-    e = cudaGetLastError();
+    BinParams bin = c.cell_bin;
+    bin.vec4 = c.bin.vec4;
+    const uint32_t totals = bin.nBins + (bin.nBins + kScanBlock - 1) / kScanBlock;
+    const uint64_t cells = (uint64_t)P.cp.cells * P.pitch, cells_out = (uint64_t)c.nR * c.nB;
+    c.mark(1, false, stream);
+    k_cells_clear<<<(uint32_t)std::min<uint64_t>((cells + 255) / 256, (uint64_t)c.sm_count * 8), 256, 0, stream>>>(
+        c.d_totals, totals, c.d_nonempty, (c.nR + 31) / 32, c.d_cells, cells, out, cells_out);
+    cudaError_t e = cudaGetLastError();
+    c.mark(1, true, stream);
+    c.sorted_cells_n = 0;
+    if(e == cudaSuccess && n) {
+        const rtacx_status st = run_sort(c, bin, c.cell_sort, samples, n, c.d_nonempty, stream);
+        if(st != RTACX_OK) return st;
+        c.sorted_cells_n = n;
+        c.mark(5, false, stream);
+        // Units of fewer samples while that leaves the SMs' warps without one;
+        // wide beams' windows are then also shared out over blockIdx.y.
+        const uint32_t warps = (uint32_t)c.sm_count * 3u * kCellWarps;
+        uint32_t unit = kUnit;
+        while(unit > 32 && n < (uint64_t)warps * unit * 2) unit /= 2;
+        const uint64_t ctas = (n + (uint64_t)unit * kCellWarps - 1) / ((uint64_t)unit * kCellWarps);
+        const uint32_t gx = (uint32_t)std::min<uint64_t>(ctas, (uint64_t)c.sm_count * 12u);
+        const uint32_t gy = c.cell_shared ? (uint32_t)std::min<uint64_t>((uint64_t)P.windows,
+                                                std::max<uint64_t>(1, (uint64_t)c.sm_count * 3u / gx)) : 1u;
+        cells_fn(c.cell_bpl, c.cell_shared)<<<dim3(gx, gy), kCellThreads, cells_smem(P.beam_axis.n), stream>>>(
+            P, c.d_offsets + bin.nBins, unit);
+        const dim3 fgrid(P.pitch / 32, (c.nR + kFilterTile - 1) / kFilterTile);
+        k_cells_filter<<<fgrid, 32 * kFilterWarps, filter_smem(P.cp.taps), stream>>>(P, c.d_nonempty, c.overlap);
+        e = cudaGetLastError();
+        c.mark(5, true, stream);
+    }
     if(e != cudaSuccess) { c.error = std::string("cell form: ") + cudaGetErrorString(e); return RTACX_ERR_CUDA; }
     return RTACX_OK;
 }

@@ -86,24 +86,6 @@ __device__ __forceinline__ float2 pulse_at(const float2* __restrict__ pad, const
     return make_float2(fmaf(alpha, hi.x - lo.x, lo.x), fmaf(alpha, hi.y - lo.y, lo.y));
 }
 
-// Range cell of a travel and its fraction of the cell: floor and fraction of
-// travel * k + b, with the product's exact residual (fmaf) and the low part
-// of k added to the fraction (k * travel reaches the row count, a fraction of
-// which a plain float product would round away). Returns the cell's storage
-// row C + 1 (C = -1: the first cell any row's pulse reaches) or -1 for a
-// travel that reaches no row, NaN and infinities included.
-__device__ __forceinline__ int range_cell(const CellParams& cp, float travel, float& alpha)
-{
-    const float prod = travel * cp.k_hi;
-    const float err = fmaf(travel, cp.k_hi, -prod);
-    const float whole = rintf(prod);
-    const float f = (prod - whole) + (err + fmaf(travel, cp.k_lo, cp.b_frac));
-    const float fl = floorf(f);
-    alpha = f - fl;
-    const float row = whole + fl + cp.b_row;      // whole numbers below 2^22: exact
-    return row >= 0.0f && row < (float)cp.cells ? (int)row : -1;
-}
-
 // ---- the beam table in shared memory ---------------------------------------
 // Entry i of the table is the linear piece left of texel i: {value at its
 // left end, slope}, entry 0 the rise from the zero border to texel 0, entry W
@@ -164,21 +146,22 @@ struct BeamLookup {
 };
 
 // ---- accumulation of one ping's samples into the cell rows ------------------
-// A warp takes units of kUnit consecutive samples of the sorted order (so of
-// few cells and, with bearing sub-bins, of few bearings) and, one after the
-// other, the windows of 32 BPL bearings that hold samples of the unit. Lane l
-// holds the bearings at positions l, l + 32, ... of the window and the sums
-// of three consecutive cells for them in registers. The window's samples are
-// listed by cell in shared memory, each value twice (the packed operands);
-// all lanes then walk the list. The sums go to the cell rows as 16-byte
-// reductions.
-constexpr int kUnit = 128;                 // samples per warp and unit
+// The samples are sorted by (bearing window, block of cells). A warp takes
+// units of up to kUnit consecutive samples, so of one window or two and of
+// few cells. Lane l holds the bearings at positions l, l + 32, ... of a
+// window. The unit's samples are listed by cell in shared memory, each value
+// twice (the packed operands); all lanes then walk a cell's list, summing T
+// and M for their bearings in registers, and add the sums to the cell row in
+// 16-byte reductions. Windows that are shared out (wide beams: every sample
+// reaches every window) walk the same list one after the other.
+constexpr int kUnit = 128;                 // samples per warp and unit, at most
 constexpr int kUnitLoads = kUnit / 32;
-constexpr int kCellClasses = 3;            // consecutive cells held in registers
+constexpr int kListCells = 32;             // cells listed at a time
 
 struct CellWarpSmem {
     ulonglong2 list[kUnit][2];              // {theta, v.x}, {v.y, alpha}, each twice
     float4 w[kUnit];                        // {v.x, v.y, alpha, -}; row-by-row samples: travel for alpha
+    uint32_t count[kListCells], start[kListCells];
 };
 
 // One sample next to a knot, row by row: the lanes take 32 rows at a time,
@@ -219,114 +202,101 @@ __device__ __forceinline__ void reduce_row_by_row(const CellPing& P, float4 w, f
 }
 
 // Accumulates samples [first, first + count) (count <= kUnit) of the sorted
-// order into the cell rows, for the windows win0, win0 + win_step, ....
-template <int BPL>
+// order into the cell rows. SHARED: for the windows win0, win0 + win_step, ...;
+// otherwise for each sample's own window.
+template <int BPL, bool SHARED>
 __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t first, uint32_t count, int win0,
                                                 int win_step, CellWarpSmem& S, const float2* tab,
                                                 const BeamLookup& beam)
 {
     constexpr int NP = BPL / 2;
     const int lane = threadIdx.x & 31;
-    const uint32_t below = (1u << lane) - 1u;
-    float th_lo = INFINITY, th_hi = -INFINITY, theta[kUnitLoads];
+    float theta[kUnitLoads];
     int cell[kUnitLoads];                  // storage row; -1 dropped; -2 - row: reduced row by row
+    int win[kUnitLoads];
+    int cur = INT_MAX;
     bool near_knot = false;
     __syncwarp();
 #pragma unroll
     for(int q = 0; q < kUnitLoads; q++) {
         const uint32_t i = (uint32_t)(q * 32 + lane);
         cell[q] = -1;
+        win[q] = INT_MAX;
         theta[q] = 0.0f;
         if(i < count) {
             const float4 rec = __ldcs(P.sorted + first + i);
             float alpha;
             const int c = range_cell(P.cp, rec.z, alpha);
-            // Bearings far outside (and NaN) move to a bearing that no beam reaches.
-            const float th = fminf(fmaxf(rec.w, P.theta_lo), P.theta_hi);
             const bool near = !(alpha >= P.cp.knot && alpha <= 1.0f - P.cp.knot);
-            theta[q] = th;
+            // Bearings far outside (and NaN) move to a bearing that no beam reaches.
+            theta[q] = fminf(fmaxf(rec.w, P.theta_lo), P.theta_hi);
             S.w[i] = make_float4(rec.x, rec.y, near ? rec.z : alpha, 0.0f);
             if(c >= 0) {
                 cell[q] = near ? -2 - c : c;
                 near_knot |= near;
-                th_lo = fminf(th_lo, th);
-                th_hi = fmaxf(th_hi, th);
+                win[q] = SHARED ? 0 : (int)bearing_bin(P.win_scale, P.win_offset, (uint32_t)P.windows, rec.w);
+                cur = min(cur, win[q]);
             }
         }
     }
     near_knot = __any_sync(0xffffffffu, near_knot);
-    for(int o = 16; o > 0; o >>= 1) {
-        th_lo = fminf(th_lo, __shfl_xor_sync(0xffffffffu, th_lo, o));
-        th_hi = fmaxf(th_hi, __shfl_xor_sync(0xffffffffu, th_hi, o));
-    }
-    __syncwarp();
-    for(int g0 = win0; g0 < P.windows; g0 += 32 * win_step) {
-        // Windows g0, g0 + win_step, ... (one per lane) that the unit's bearings touch.
-        const int mine = g0 + lane * win_step;
-        const float2 my_reach = mine < P.windows ? P.win_reach[mine] : make_float2(INFINITY, -INFINITY);
-        uint32_t live = __ballot_sync(0xffffffffu, th_hi >= my_reach.x && th_lo < my_reach.y);
-        for(; live; live &= live - 1u) {
-            const int src = __ffs(live) - 1;
-            const int win = g0 + src * win_step;
-            const float lo = __shfl_sync(0xffffffffu, my_reach.x, src), hi = __shfl_sync(0xffffffffu, my_reach.y, src);
-            uint32_t in_win = 0;                   // bit q: sample q of this lane is in the window
-            int base = INT_MAX;
+    for(cur = __reduce_min_sync(0xffffffffu, cur); cur != INT_MAX;) {
+        const int w_begin = SHARED ? win0 : cur, w_end = SHARED ? P.windows : cur + 1;
+        int base = INT_MAX, next_win = INT_MAX;
+#pragma unroll
+        for(int q = 0; q < kUnitLoads; q++) {
+            if(win[q] == cur && cell[q] >= 0) base = min(base, cell[q]);
+            if(win[q] > cur) next_win = min(next_win, win[q]);
+        }
+        base = __reduce_min_sync(0xffffffffu, base);
+        while(base != INT_MAX) {
+            // List the window's samples of cells base .. base + kListCells - 1, by cell.
+            uint32_t rank[kUnitLoads];
+            int next = INT_MAX;
+            S.count[lane] = 0u;
+            __syncwarp();
 #pragma unroll
             for(int q = 0; q < kUnitLoads; q++) {
-                const bool in = cell[q] != -1 && theta[q] >= lo && theta[q] < hi;
-                in_win |= in ? 1u << q : 0u;
-                if(in && cell[q] >= 0) base = min(base, cell[q]);
+                const bool in = win[q] == cur && cell[q] >= base;
+                rank[q] = in && cell[q] - base < kListCells ? atomicAdd(&S.count[cell[q] - base], 1u) : 0xFFFFFFFFu;
+                if(in && cell[q] - base >= kListCells) next = min(next, cell[q]);
             }
-            if(!__any_sync(0xffffffffu, in_win)) continue;
-            base = __reduce_min_sync(0xffffffffu, base);
-            const int pos0 = win * 32 * BPL + lane;
-            f32x2 minus_tb[NP];
+            __syncwarp();
+            const uint32_t mine = S.count[lane];
+            uint32_t upto = mine;
+            for(int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, upto, o);
+                if(lane >= o) upto += y;
+            }
+            S.start[lane] = upto - mine;
+            __syncwarp();
 #pragma unroll
-            for(int p = 0; p < NP; p++)
-                minus_tb[p] = pack2(-P.pos_theta[pos0 + 64 * p], -P.pos_theta[pos0 + 64 * p + 32]);
-            while(base != INT_MAX) {
-                // List the samples of cells base .. base + 2, by cell.
-                uint32_t m[kUnitLoads][kCellClasses];
-                int end[kCellClasses] = {0, 0, 0}, next = INT_MAX;
+            for(int q = 0; q < kUnitLoads; q++) {
+                if(rank[q] == 0xFFFFFFFFu) continue;
+                const uint32_t at = S.start[cell[q] - base] + rank[q];
+                const float4 w = S.w[q * 32 + lane];
+                S.list[at][0] = make_ulonglong2(pack2(theta[q], theta[q]), pack2(w.x, w.x));
+                S.list[at][1] = make_ulonglong2(pack2(w.y, w.y), pack2(w.z, w.z));
+            }
+            __syncwarp();
+            const uint32_t filled = __ballot_sync(0xffffffffu, mine != 0u);
+            for(int w = w_begin; w < w_end; w += win_step) {
+                const int pos0 = w * 32 * BPL + lane;
+                f32x2 minus_tb[NP];
 #pragma unroll
-                for(int q = 0; q < kUnitLoads; q++) {
-                    const int off = (in_win >> q & 1u) && cell[q] >= base ? cell[q] - base : -1;
-                    if(off >= kCellClasses) next = min(next, cell[q]);
-#pragma unroll
-                    for(int k = 0; k < kCellClasses; k++) {
-                        m[q][k] = __ballot_sync(0xffffffffu, off == k);
-                        end[k] += __popc(m[q][k]);
-                    }
-                }
-                int fill[kCellClasses] = {0, end[0], end[0] + end[1]};
-                end[1] += end[0];
-                end[2] += end[1];
-#pragma unroll
-                for(int q = 0; q < kUnitLoads; q++) {
-                    int at = -1;
-#pragma unroll
-                    for(int k = 0; k < kCellClasses; k++) {
-                        if(m[q][k] >> lane & 1u) at = fill[k] + __popc(m[q][k] & below);
-                        fill[k] += __popc(m[q][k]);
-                    }
-                    if(at >= 0) {
-                        const float4 w = S.w[q * 32 + lane];
-                        S.list[at][0] = make_ulonglong2(pack2(theta[q], theta[q]), pack2(w.x, w.x));
-                        S.list[at][1] = make_ulonglong2(pack2(w.y, w.y), pack2(w.z, w.z));
-                    }
-                }
-                __syncwarp();
+                for(int p = 0; p < NP; p++)
+                    minus_tb[p] = pack2(-P.pos_theta[pos0 + 64 * p], -P.pos_theta[pos0 + 64 * p + 32]);
                 int s = 0;
-#pragma unroll
-                for(int k = 0; k < kCellClasses; k++) {
-                    if(s == end[k]) continue;
+                for(uint32_t left = filled; left; left &= left - 1u) {
+                    const int k = __ffs(left) - 1;
+                    const int end = (int)__shfl_sync(0xffffffffu, upto, k);
                     f32x2 acc[NP][4];
 #pragma unroll
                     for(int p = 0; p < NP; p++)
 #pragma unroll
                         for(int e = 0; e < 4; e++) acc[p][e] = 0ull;
 #pragma unroll 2
-                    for(; s < end[k]; s++) {
+                    for(; s < end; s++) {
                         const ulonglong2 e0 = S.list[s][0], e1 = S.list[s][1];
 #pragma unroll
                         for(int p = 0; p < NP; p++) {
@@ -347,11 +317,18 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
                         if(y >= 0) red_add_f4(row + y, a.y, b.y, c.y, d.y);
                     }
                 }
-                __syncwarp();
-                base = __reduce_min_sync(0xffffffffu, next);
             }
-            if(near_knot) {
+            base = __reduce_min_sync(0xffffffffu, next);
+            __syncwarp();
+        }
+        if(near_knot) {
+            for(int w = w_begin; w < w_end; w += win_step) {
+                const int pos0 = w * 32 * BPL + lane;
+                f32x2 minus_tb[NP];
                 int bearing[BPL];
+#pragma unroll
+                for(int p = 0; p < NP; p++)
+                    minus_tb[p] = pack2(-P.pos_theta[pos0 + 64 * p], -P.pos_theta[pos0 + 64 * p + 32]);
 #pragma unroll
                 for(int p = 0; p < BPL; p++) {
                     const int col = P.pos_col[pos0 + 32 * p];
@@ -360,14 +337,15 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
 #pragma unroll 1
                 for(int q = 0; q < kUnitLoads; q++) {
                     // (no register array indexing: the values go through selects)
-                    int c = cell[0];
+                    int c = cell[0], v = win[0];
                     float th = theta[0];
 #pragma unroll
                     for(int z = 1; z < kUnitLoads; z++) {
                         c = q == z ? cell[z] : c;
+                        v = q == z ? win[z] : v;
                         th = q == z ? theta[z] : th;
                     }
-                    uint32_t near = __ballot_sync(0xffffffffu, c <= -2 && (in_win >> q & 1u));
+                    uint32_t near = __ballot_sync(0xffffffffu, c <= -2 && v == cur);
                     for(; near; near &= near - 1u) {
                         const int l = __ffs(near) - 1;
                         reduce_row_by_row<BPL>(P, S.w[q * 32 + l], __shfl_sync(0xffffffffu, th, l),
@@ -376,6 +354,7 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
                 }
             }
         }
+        cur = __reduce_min_sync(0xffffffffu, next_win);
     }
 }
 

@@ -90,10 +90,38 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
     return true;
 }
 
+// Range cells of a sensor whose pulse taps lie one output range apart
+// (rtacx_cells.cuh).
+struct CellParams {
+    float k_hi, k_lo;                // cells per metre (two floats)
+    float b_frac, b_row;             // cell coordinate of travel 0, plus one: fraction and whole part
+    float knot;                      // fraction of a cell next to a knot that is reduced row by row
+    int cells;                       // storage rows: cells -1 .. nR + taps - 2
+    int taps;                        // pulse taps H
+};
+
+// Range cell of a travel and its fraction of the cell: floor and fraction of
+// travel * k + b, with the product's exact residual (fmaf) and the low part
+// of k added to the fraction (k * travel reaches the row count, a fraction of
+// which a plain float product would round away). Returns the cell's storage
+// row C + 1 (C = -1: the first cell any row's pulse reaches) or -1 for a
+// travel that reaches no row, NaN and infinities included.
+__device__ __forceinline__ int range_cell(const CellParams& cp, float travel, float& alpha)
+{
+    const float prod = travel * cp.k_hi;
+    const float err = fmaf(travel, cp.k_hi, -prod);
+    const float whole = rintf(prod);
+    const float f = (prod - whole) + (err + fmaf(travel, cp.k_lo, cp.b_frac));
+    const float fl = floorf(f);
+    alpha = f - fl;
+    const float row = whole + fl + cp.b_row;      // whole numbers below 2^22: exact
+    return row >= 0.0f && row < (float)cp.cells ? (int)row : -1;
+}
+
 // Everything the binning kernels need, passed by value.
 struct BinParams {
     KeyParams key;
-    uint32_t nBB;          // bearing sub-bins (1: range key only)
+    uint32_t nBB;          // bearing sub-bins (1: range key only); bearing windows of the cell order
     float bb_scale;        // bearing bin = f(fmaf(bb_scale, bearing, bb_offset))
     float bb_offset;
     uint32_t nBins;        // nR * nBB
@@ -103,6 +131,12 @@ struct BinParams {
     double echo_cycles;    // carrier cycles per metre of travel, 2 f / c
     float echo_k_hi;       // echo_cycles split into two floats (compensated phase)
     float echo_k_lo;
+    // The cell form's order (rtacx_cells.cuh): key = bearing window x cell
+    // block, a block being 2^cell_shift cells. 0 blocks: range bin x bearing
+    // sub-bin, the order of rtacx_bin.
+    uint32_t cell_blocks;
+    int cell_shift;
+    CellParams cell;
 };
 
 // Echo-sample epilogue of the reference's ray generator
@@ -229,11 +263,18 @@ __device__ __forceinline__ uint32_t bearing_bin(float scale, float offset, uint3
     return (uint32_t)__float2int_rz(q);
 }
 
-// Composite (range bin, bearing bin) key; kOutOfRange for out-of-range travel.
+// Composite (range bin, bearing bin) key, or (bearing window, cell block) in
+// the cell order (samples that reach no cell in block 0); kOutOfRange for
+// out-of-range travel either way.
 __device__ __forceinline__ uint32_t sample_key(const BinParams& p, float travel, float bearing, int& side)
 {
     uint32_t rk = range_key(p.key, travel, side);
     if(rk == kOutOfRange) return kOutOfRange;
+    if(p.cell_blocks) {
+        float alpha;
+        const uint32_t block = (uint32_t)max(range_cell(p.cell, travel, alpha), 0) >> p.cell_shift;
+        return (p.nBB > 1u ? bearing_bin(p.bb_scale, p.bb_offset, p.nBB, bearing) * p.cell_blocks : 0u) + block;
+    }
     if(p.nBB == 1u) return rk;
     return rk * p.nBB + bearing_bin(p.bb_scale, p.bb_offset, p.nBB, bearing);
 }
@@ -287,20 +328,9 @@ struct ReduceParams {
     AxisLerp beam_axis;
 };
 
-// Range cells of a sensor whose pulse taps lie one output range apart
-// (rtacx_cells.cuh).
-struct CellParams {
-    float k_hi, k_lo;                // cells per metre (two floats)
-    float b_frac, b_row;             // cell coordinate of travel 0, plus one: fraction and whole part
-    float knot;                      // fraction of a cell next to a knot that is reduced row by row
-    int cells;                       // storage rows: cells -1 .. nR + taps - 2
-    int taps;                        // pulse taps H
-};
-
 // A ping's arguments of the cell kernels (rtacx_cells.cuh). A window is a set
-// of 32 BPL bearings, in the order in which a warp's lanes hold them, and the
-// sample bearings that it takes. Columns are the cell rows' order of the
-// bearings.
+// of 32 BPL bearings, in the order in which a warp's lanes hold them. Columns
+// are the cell rows' order of the bearings.
 struct CellPing {
     CellParams cp;
     const float4* sorted;
@@ -311,14 +341,22 @@ struct CellPing {
     const float* ranges;
     const float* row_dev;            // [nR] e_r
     const float4* taps;              // [cell_tap_entries(H)]
-    const float2* win_reach;         // [windows] sample bearings [x, y) that the window takes
     const float* pos_theta;          // [windows][32 BPL] output bearing at a window's position
     const int* pos_col;              // ... its column (-1: none)
     const int* col_bearing;          // [pitch] bearing of a column (-1: padding)
     AxisLerp range_axis, beam_axis;
     float theta_lo, theta_hi;        // sample bearings are clamped to these (no beam reaches them)
+    float win_scale, win_offset;     // a sample's window: bearing_bin of its bearing
     uint32_t nR, nB, pitch;
     int windows;
+};
+
+// Launch shape of the count / scatter passes for one number of bins.
+struct SortShape {
+    uint32_t hist_ctas = 0;             // CTAs of the count pass (and of the batched passes)
+    uint32_t scatter_ctas = 0;          // CTAs of the per-tile scatter
+    uint32_t hist_threads = 0;
+    int scatter_shape = 0;              // 1 + index of the staged scatter's shape (0: per-tile scatter)
 };
 
 // Everything one ping of a batch needs on the device (rtacx_batch_*).
@@ -411,26 +449,27 @@ struct Context {
     // Sample-sized scratch.
     uint64_t capacity = 0;              // samples the sorted scratch holds
     float4* d_sorted = nullptr;
-    uint32_t hist_ctas = 0;             // CTAs of the count pass (and of the batched passes)
-    uint32_t scatter_ctas = 0;          // CTAs of the scatter pass
-    int scatter_shape = 0;              // 1 + index of the staged scatter's shape (0: per-tile scatter)
+    SortShape sort;
     size_t acc_smem = 0;                // dynamic shared memory of the precision accumulation
     uint32_t acc_blocks_per_sm = 1;
-    uint32_t hist_threads = 0;
     size_t hist_cols = 0;               // allocated words of d_hist (the write cursors)
     uint32_t* d_hist = nullptr;         // the scatter's per-bin write cursors (cursor_word), nBins x kCursorStride words
 
     // Cell form of a 2D ping (rtacx_cells.cu).
     bool cells_on = false;
     int cell_bpl = 2;                   // bearings per lane
+    bool cell_shared = false;           // windows shared out: every sample reaches every window
     CellPing cell{};                    // sorted and out are set per call
     float4* d_cells = nullptr;
     float4* d_cell_taps = nullptr;
     float* d_row_dev = nullptr;
-    float2* d_win_reach = nullptr;
     float* d_pos_theta = nullptr;
     int* d_pos_col = nullptr;
     int* d_col_bearing = nullptr;
+    uint32_t* d_nonempty = nullptr;     // [(nR + 31) / 32] bitmap of non-empty range bins
+    BinParams cell_bin{};               // the cell form's order
+    SortShape cell_sort;
+    uint64_t sorted_cells_n = 0;        // samples of the last ping that left the cell order in d_sorted (0: none)
 
     // Split persistent gather of 2D pings (see rtacx_reduce.cu).
     uint32_t* d_tile_parts = nullptr;   // [tiles] sample-stream length of each output tile
@@ -508,6 +547,12 @@ struct Context {
 
 // Binning pipeline (rtacx_bin.cu): count, scan, scatter, windows.
 rtacx_status run_binning(Context& ctx, const void* samples, uint64_t n, cudaStream_t stream);
+// The passes of one order: count (its totals zeroed by the caller; nonempty:
+// also the bitmap of range bins), scan, scatter.
+rtacx_status run_sort(Context& ctx, const BinParams& p, const SortShape& shape, const void* samples, uint64_t n,
+                      uint32_t* nonempty, cudaStream_t stream);
+SortShape sort_shape(const Context& ctx, uint32_t nBins);
+rtacx_status restore_sorted(Context& ctx, cudaStream_t stream);
 rtacx_status run_bin_outputs(Context& ctx, const void* samples, uint64_t n,
                              uint32_t* keys, uint32_t* segments, uint32_t* windows,
                              uint32_t* counts, uint64_t* oor, cudaStream_t stream);
@@ -520,7 +565,7 @@ rtacx_status run_reduce(Context& ctx, float* out, cudaStream_t stream);
 // Cell form of the plain reduction (rtacx_cells.cu).
 bool configure_cells(Context& ctx, double beam_support);
 void free_cells(Context& ctx);
-rtacx_status run_cells(Context& ctx, uint64_t n, float2* out, cudaStream_t stream);
+rtacx_status run_cells(Context& ctx, const void* samples, uint64_t n, float2* out, cudaStream_t stream);
 
 // Batched plain form. Maps are (ping, index) pairs: count / scatter chunks,
 // column-scan bin blocks of 256, window row blocks of 256; gather items are

@@ -32,7 +32,6 @@
 
 namespace rtacx {
 
-void configure_hist_launch(Context& ctx);
 size_t gather_smem_bytes(uint32_t range_tile, uint32_t bearing_tile, uint32_t H, uint32_t W);
 
 namespace {
@@ -248,8 +247,8 @@ extern "C" rtacx_status rtacx_reduce_noalloc(int sample_kind, const void* sensor
     ctx.d_ranges = reinterpret_cast<float*>(base + kOffRanges);
     ctx.d_support = reinterpret_cast<int2*>(base + kOffSupport);
     ctx.d_bb_tiles = reinterpret_cast<int2*>(base + kOffTiles);
-    configure_hist_launch(ctx);
-    ctx.hist_ctas = std::min(ctx.hist_ctas, kMaxHistCtas);
+    ctx.sort = sort_shape(ctx, ctx.bin.nBins);
+    ctx.sort.hist_ctas = std::min(ctx.sort.hist_ctas, kMaxHistCtas);
     ctx.hist_cols = (size_t)ctx.bin.nBins * kCursorStride;
     if(ctx.hist_cols * sizeof(uint32_t) > kHistBytes) return RTACX_ERR_UNSUPPORTED;
 

@@ -88,3 +88,22 @@ def test_cells_drop_samples_without_a_bearing_or_travel():
     b = gpu_reduce(ctx, clean, wk.out_shape)
     assert np.isfinite(a).all()
     assert rel_l2(a, b) <= 1e-6
+
+
+def test_sorted_scratch_after_a_ping_keeps_its_order(oracle):
+    """rtacx_reduce sorts a cell-form ping in its own order; the diagnostic
+    copy of the sorted scratch still has every in-range sample once, grouped
+    by ascending (range bin, bearing sub-bin), and pings after it are right."""
+    from test_gpu_sorted import KEY_OOR, composite_keys, record_hash
+    wk = ping(20001, 257, 200, 17, False)
+    ctx = make_context(wk)
+    first = gpu_reduce(ctx, wk.samples, wk.out_shape)
+    buf = torch.zeros((wk.n, 4), device="cuda")
+    ctx.diag_sorted(buf, wk.n, stream=torch.cuda.current_stream())
+    recs = buf.cpu().numpy()
+    key = composite_keys(oracle, wk, wk.samples)
+    inside = wk.samples[key != KEY_OOR]
+    got = recs[:len(inside)]
+    assert np.all(np.diff(composite_keys(oracle, wk, got).astype(np.int64)) >= 0)
+    assert np.array_equal(np.sort(record_hash(got)), np.sort(record_hash(inside)))
+    assert rel_l2(gpu_reduce(ctx, wk.samples, wk.out_shape), first) <= 1e-6
