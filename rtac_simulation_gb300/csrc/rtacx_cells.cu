@@ -25,15 +25,18 @@ constexpr size_t kMaxCellBytes = (size_t)1 << 30;      // cell rows of one conte
 constexpr double kMaxKnot = 0.01;
 constexpr uint32_t kCellBins = 12288;
 
-size_t cells_smem(int W) { return kCellWarps * sizeof(CellWarpSmem) + (size_t)(W + 2) * sizeof(float2); }
+size_t cells_smem(int W, bool pairs)
+{
+    return kCellWarps * (pairs ? sizeof(CellWarpSmem<true>) : sizeof(CellWarpSmem<false>)) + (size_t)(W + 2) * sizeof(float2);
+}
 
-template <int BPL, bool SHARED>
+template <int BPL, bool SHARED, bool PAIR>
 __global__ void __launch_bounds__(kCellThreads, BPL == 2 ? 3 : 2)
 k_cells(const CellPing P, const uint32_t* __restrict__ total, uint32_t unit)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    CellWarpSmem& S = reinterpret_cast<CellWarpSmem*>(s_raw)[threadIdx.x >> 5];
-    float2* tab = reinterpret_cast<float2*>(s_raw + kCellWarps * sizeof(CellWarpSmem));
+    CellWarpSmem<PAIR>& S = reinterpret_cast<CellWarpSmem<PAIR>*>(s_raw)[threadIdx.x >> 5];
+    float2* tab = reinterpret_cast<float2*>(s_raw + kCellWarps * sizeof(CellWarpSmem<PAIR>));
     load_beam_table(tab, P.beam, P.beam_axis.n, threadIdx.x, kCellThreads);
     __syncthreads();
     BeamLookup beam;
@@ -41,14 +44,19 @@ k_cells(const CellPing P, const uint32_t* __restrict__ total, uint32_t unit)
     const uint32_t m = *total;
     for(uint64_t u = (uint64_t)(blockIdx.x * kCellWarps + (threadIdx.x >> 5)) * unit; u < m;
         u += (uint64_t)gridDim.x * kCellWarps * unit)
-        accumulate_unit<BPL, SHARED>(P, (uint32_t)u, min(unit, m - (uint32_t)u), blockIdx.y, gridDim.y, S, tab, beam);
+        accumulate_unit<BPL, SHARED, PAIR>(P, (uint32_t)u, min(unit, m - (uint32_t)u), blockIdx.y, gridDim.y, S, tab, beam);
 }
 
 using CellsFn = void (*)(const CellPing, const uint32_t*, uint32_t);
-CellsFn cells_fn(int bpl, bool shared_out)
+template <bool PAIR>
+CellsFn cells_fn_of(int bpl, bool shared_out)
 {
-    if(shared_out) return bpl == 4 ? k_cells<4, true> : k_cells<2, true>;
-    return bpl == 4 ? k_cells<4, false> : k_cells<2, false>;
+    if(shared_out) return bpl == 4 ? k_cells<4, true, PAIR> : k_cells<2, true, PAIR>;
+    return bpl == 4 ? k_cells<4, false, PAIR> : k_cells<2, false, PAIR>;
+}
+CellsFn cells_fn(int bpl, bool shared_out, bool pairs)
+{
+    return pairs ? cells_fn_of<true>(bpl, shared_out) : cells_fn_of<false>(bpl, shared_out);
 }
 
 // Zeroes what a ping's passes add into: the bin totals, the range-bin bitmap,
@@ -74,6 +82,19 @@ k_cells_filter(const CellPing P, const uint32_t* __restrict__ nonempty, int ov)
         s_on[threadIdx.x] = r < (int)P.nR && row_on(nonempty, (int)P.nR, ov, r) ? 1 : 0;
     }
     filter_tile(P, blockIdx.x, blockIdx.y, reinterpret_cast<float4*>(s_raw), s_on);   // synchronises before it reads s_on
+}
+
+// Row pairs into the ping: row r takes T of storage row r + 1 and M of storage
+// row r.
+__global__ void __launch_bounds__(256)
+k_pairs_join(const CellPing P, const uint32_t* __restrict__ nonempty, int ov)
+{
+    const int r = blockIdx.y, col = blockIdx.x * blockDim.x + threadIdx.x;
+    if(col >= (int)P.pitch) return;
+    const int b = P.col_bearing[col];
+    if(b < 0) return;
+    const float4 t = P.cells[(size_t)(r + 1) * P.pitch + col], m = P.cells[(size_t)r * P.pitch + col];
+    P.out[(size_t)r * P.nB + b] = row_on(nonempty, (int)P.nR, ov, r) ? make_float2(t.x + m.z, t.y + m.w) : make_float2(0.f, 0.f);
 }
 
 template <typename T>
@@ -112,6 +133,7 @@ void free_cells(Context& c)
 //     per row and pair, so it is kept under a hundredth of a cell);
 //   * every row's PSF support lies inside its reference window, so the window
 //     only decides whether the row is on;
+//   or (row pairs) no travel reaches more than two rows;
 //   * the cell rows and the beam table fit.
 // Returns whether the form is on; a failed allocation leaves it off.
 bool configure_cells(Context& c, double beam_support)
@@ -139,28 +161,45 @@ bool configure_cells(Context& c, double beam_support)
         dev[r] = (float)e;
         worst = std::max(worst, std::fabs(e));
     }
-    // What moves a row's knots against the grid: its own deviation, the tap
-    // spacing's over half the pulse, and the rounding of travel - range.
-    const double knot = 1.01 * (worst + std::fabs(kappa - 1.0) * (0.5 * H + 1.0)) + 2e-6 + 1.5e-7 * H;
-    if(!(knot <= kMaxKnot)) return false;
-    // Rows' supports inside their windows.
-    for(int r = 0; r < nR; r++) {
-        const double ext = 1.0 / (k / H), half = 0.5 * ext * (1.0 + 1.0 / H) * (1.0 + 1e-4);
-        const double slack = 1e-6 * (std::fabs(R[r]) + half) + 1e-30;
-        const int lo = (int)host_range_key_clamped(c.key, (float)(R[r] - half - slack));
-        const int hi = (int)host_range_key_clamped(c.key, (float)(R[r] + half + slack));
-        if(lo < std::max(0ll, (long long)r - c.overlap) || hi > std::min((long long)nR - 1, (long long)r + c.overlap)) return false;
-    }
-    // Cell coordinate y = travel / spacing + b; storage row = cell + 1.
+    const double ext = (double)H / k;
     CellParams& cp = c.cell.cp;
-    const double kc = 1.0 / spacing, b = center - kc * R0;
+    const double kc = 1.0 / spacing;
     cp.k_hi = (float)kc;
     cp.k_lo = (float)(kc - (double)cp.k_hi);
-    cp.b_row = (float)(std::floor(b) + 1.0);
+    double b;                                // cell coordinate y = travel / spacing + b
+    // Row pairs: no travel within `half` of three rows (a hair of the spacing
+    // covers the float cell index and the rows' deviations). Storage row
+    // floor(y) + 2 = first row reached + 1.
+    const double half = 0.5 * ext * (1.0 + 1.0 / H) + 1e-4 * spacing + worst / k + 1e-6 * std::fabs(R[nR - 1]);
+    c.cell_pairs = half < spacing;
+    if(c.cell_pairs) {
+        b = -(half + R0) / spacing;
+        cp.b_row = (float)(std::floor(b) + 2.0);
+        cp.knot = 0.0f;
+        cp.cells = nR + 1;
+    }
+    else {
+        // What moves a row's knots against the grid: its own deviation, the tap
+        // spacing's over half the pulse, and the rounding of travel - range.
+        const double knot = 1.01 * (worst + std::fabs(kappa - 1.0) * (0.5 * H + 1.0)) + 2e-6 + 1.5e-7 * H;
+        if(!(knot <= kMaxKnot)) return false;
+        // Rows' supports inside their windows.
+        for(int r = 0; r < nR; r++) {
+            const double reach = 0.5 * ext * (1.0 + 1.0 / H) * (1.0 + 1e-4);
+            const double slack = 1e-6 * (std::fabs(R[r]) + reach) + 1e-30;
+            const int lo = (int)host_range_key_clamped(c.key, (float)(R[r] - reach - slack));
+            const int hi = (int)host_range_key_clamped(c.key, (float)(R[r] + reach + slack));
+            if(lo < std::max(0ll, (long long)r - c.overlap) || hi > std::min((long long)nR - 1, (long long)r + c.overlap)) return false;
+        }
+        b = center - kc * R0;                // storage row = cell + 1
+        cp.b_row = (float)(std::floor(b) + 1.0);
+        cp.knot = (float)knot;
+        cp.cells = nR + H;
+    }
     cp.b_frac = (float)(b - std::floor(b));
-    cp.knot = (float)knot;
-    cp.cells = nR + H;
     cp.taps = H;
+    c.cell.key = c.key;
+    c.cell.overlap = c.overlap;
     if(std::fabs(b) + cp.cells > (double)(1 << 21)) return false;
     // Beam coordinates far below the rounding trick's 2^22.
     const auto mm = std::minmax_element(c.bearings.begin(), c.bearings.end());
@@ -256,7 +295,8 @@ bool configure_cells(Context& c, double beam_support)
         col_bearing[col[p]] = pos[p];
     }
     const size_t cell_bytes = (size_t)cp.cells * pitch * sizeof(float4);
-    if(cell_bytes > kMaxCellBytes || cells_smem(W) > 200 * 1024 || filter_smem(H) > 200 * 1024) return false;
+    if(cell_bytes > kMaxCellBytes || cells_smem(W, c.cell_pairs) > 200 * 1024 ||
+       (!c.cell_pairs && filter_smem(H) > 200 * 1024)) return false;
     std::vector<float4> taps((size_t)cell_tap_entries(H), make_float4(0.f, 0.f, 0.f, 0.f));
     for(int i = -1; i < H; i++) {
         double p[2], d[2];
@@ -270,8 +310,9 @@ bool configure_cells(Context& c, double beam_support)
     bool ok = put(c.d_cell_taps, taps) && put(c.d_row_dev, dev) && put(c.d_nonempty, std::vector<uint32_t>((nR + 31) / 32, 0u)) &&
               put(c.d_pos_theta, theta) && put(c.d_pos_col, col) && put(c.d_col_bearing, col_bearing);
     if(ok && cudaMalloc(&c.d_cells, cell_bytes) != cudaSuccess) { cudaGetLastError(); ok = false; }
-    if(ok) ok = raise_smem_limit((const void*)cells_fn(bpl, shared_out), cells_smem(W)) == cudaSuccess &&
-                raise_smem_limit((const void*)k_cells_filter, filter_smem(H)) == cudaSuccess;
+    if(ok) ok = raise_smem_limit((const void*)cells_fn(bpl, shared_out, c.cell_pairs), cells_smem(W, c.cell_pairs)) == cudaSuccess &&
+                (c.cell_pairs ||
+                 raise_smem_limit((const void*)k_cells_filter, filter_smem(H)) == cudaSuccess);
     if(!ok) { free_cells(c); return false; }
     CellPing& P = c.cell;
     P.cells = c.d_cells;
@@ -291,7 +332,7 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
     BinParams bin = c.cell_bin;
     bin.vec4 = c.bin.vec4;
     const uint32_t totals = bin.nBins + (bin.nBins + kScanBlock - 1) / kScanBlock;
-    const uint64_t cells = (uint64_t)P.cp.cells * P.pitch, cells_out = (uint64_t)c.nR * c.nB;
+    const uint64_t cells = (uint64_t)P.cp.cells * P.pitch, cells_out = c.cell_pairs && n ? 0 : (uint64_t)c.nR * c.nB;   // (the pairs' join writes every cell)
     c.mark(1, false, stream);
     k_cells_clear<<<(uint32_t)std::min<uint64_t>((cells + 255) / 256, (uint64_t)c.sm_count * 8), 256, 0, stream>>>(
         c.d_totals, totals, c.d_nonempty, (c.nR + 31) / 32, c.d_cells, cells, out, cells_out);
@@ -312,10 +353,12 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
         const uint32_t gx = (uint32_t)std::min<uint64_t>(ctas, (uint64_t)c.sm_count * 12u);
         const uint32_t gy = c.cell_shared ? (uint32_t)std::min<uint64_t>((uint64_t)P.windows,
                                                 std::max<uint64_t>(1, (uint64_t)c.sm_count * 3u / gx)) : 1u;
-        cells_fn(c.cell_bpl, c.cell_shared)<<<dim3(gx, gy), kCellThreads, cells_smem(P.beam_axis.n), stream>>>(
+        cells_fn(c.cell_bpl, c.cell_shared, c.cell_pairs)<<<dim3(gx, gy), kCellThreads,
+                                                            cells_smem(P.beam_axis.n, c.cell_pairs), stream>>>(
             P, c.d_offsets + bin.nBins, unit);
         const dim3 fgrid(P.pitch / 32, (c.nR + kFilterTile - 1) / kFilterTile);
-        k_cells_filter<<<fgrid, 32 * kFilterWarps, filter_smem(P.cp.taps), stream>>>(P, c.d_nonempty, c.overlap);
+        if(c.cell_pairs) k_pairs_join<<<dim3((P.pitch + 255) / 256, c.nR), 256, 0, stream>>>(P, c.d_nonempty, c.overlap);
+        else k_cells_filter<<<fgrid, 32 * kFilterWarps, filter_smem(P.cp.taps), stream>>>(P, c.d_nonempty, c.overlap);
         e = cudaGetLastError();
         c.mark(5, true, stream);
     }

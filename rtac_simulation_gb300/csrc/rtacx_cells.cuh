@@ -15,6 +15,11 @@
 // whatever the pulse's length, instead of one product per output row.
 // Samples within `knot` of a grid knot, which the rows' e_r put into
 // different pieces for different rows, are reduced row by row.
+//
+// Row pairs: a pulse that reaches at most two output rows (the reference's
+// adaptive duration, one range bin) uses the same accumulation with the
+// cells between rows: T and M then hold the sample's contributions to the
+// cell's two rows, with the rows' own pulse weights, whatever the table.
 #pragma once
 
 #include "rtacx_internal.cuh"
@@ -158,9 +163,14 @@ constexpr int kUnit = 128;                 // samples per warp and unit, at most
 constexpr int kUnitLoads = kUnit / 32;
 constexpr int kListCells = 32;             // cells listed at a time
 
+// A listed sample, each value twice: theta, v.x, v.y, alpha; for row pairs
+// theta and the two rows' weighted values.
+template <bool PAIR> struct CellEntry { ulonglong2 v[PAIR ? 3 : 2]; };
+
+template <bool PAIR>
 struct CellWarpSmem {
-    ulonglong2 list[kUnit][2];              // {theta, v.x}, {v.y, alpha}, each twice
-    float4 w[kUnit];                        // {v.x, v.y, alpha, -}; row-by-row samples: travel for alpha
+    CellEntry<PAIR> list[kUnit];
+    float4 w[kUnit];                        // {v.x, v.y, alpha, -}; row-by-row samples: travel for alpha; pairs: both rows'
     uint32_t count[kListCells], start[kListCells];
 };
 
@@ -204,9 +214,9 @@ __device__ __forceinline__ void reduce_row_by_row(const CellPing& P, float4 w, f
 // Accumulates samples [first, first + count) (count <= kUnit) of the sorted
 // order into the cell rows. SHARED: for the windows win0, win0 + win_step, ...;
 // otherwise for each sample's own window.
-template <int BPL, bool SHARED>
+template <int BPL, bool SHARED, bool PAIR>
 __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t first, uint32_t count, int win0,
-                                                int win_step, CellWarpSmem& S, const float2* tab,
+                                                int win_step, CellWarpSmem<PAIR>& S, const float2* tab,
                                                 const BeamLookup& beam)
 {
     constexpr int NP = BPL / 2;
@@ -227,10 +237,24 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
             const float4 rec = __ldcs(P.sorted + first + i);
             float alpha;
             const int c = range_cell(P.cp, rec.z, alpha);
-            const bool near = !(alpha >= P.cp.knot && alpha <= 1.0f - P.cp.knot);
+            const bool near = !PAIR && !(alpha >= P.cp.knot && alpha <= 1.0f - P.cp.knot);
             // Bearings far outside (and NaN) move to a bearing that no beam reaches.
             theta[q] = fminf(fmaxf(rec.w, P.theta_lo), P.theta_hi);
-            S.w[i] = make_float4(rec.x, rec.y, near ? rec.z : alpha, 0.0f);
+            if(PAIR) {
+                // Storage row c holds the shares of output rows c - 1 and c.
+                float2 f[2];
+                int side;
+                const int key = (int)range_key(P.key, rec.z, side);
+#pragma unroll
+                for(int k = 0; k < 2; k++) {
+                    const int r = c - 1 + k;
+                    const bool on = c >= 0 && r >= 0 && r < (int)P.nR && abs(key - r) <= P.overlap;
+                    f[k] = on ? pulse_at(P.pulse, P.range_axis, rec.z - P.ranges[on ? r : 0]) : make_float2(0.f, 0.f);
+                }
+                S.w[i] = make_float4(rec.x * f[0].x - rec.y * f[0].y, rec.x * f[0].y + rec.y * f[0].x,
+                                     rec.x * f[1].x - rec.y * f[1].y, rec.x * f[1].y + rec.y * f[1].x);
+            }
+            else S.w[i] = make_float4(rec.x, rec.y, near ? rec.z : alpha, 0.0f);
             if(c >= 0) {
                 cell[q] = near ? -2 - c : c;
                 near_knot |= near;
@@ -275,8 +299,9 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
                 if(rank[q] == 0xFFFFFFFFu) continue;
                 const uint32_t at = S.start[cell[q] - base] + rank[q];
                 const float4 w = S.w[q * 32 + lane];
-                S.list[at][0] = make_ulonglong2(pack2(theta[q], theta[q]), pack2(w.x, w.x));
-                S.list[at][1] = make_ulonglong2(pack2(w.y, w.y), pack2(w.z, w.z));
+                S.list[at].v[0] = make_ulonglong2(pack2(theta[q], theta[q]), pack2(w.x, w.x));
+                S.list[at].v[1] = make_ulonglong2(pack2(w.y, w.y), pack2(w.z, w.z));
+                if constexpr(PAIR) S.list[at].v[2].x = pack2(w.w, w.w);
             }
             __syncwarp();
             const uint32_t filled = __ballot_sync(0xffffffffu, mine != 0u);
@@ -295,16 +320,25 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
                     for(int p = 0; p < NP; p++)
 #pragma unroll
                         for(int e = 0; e < 4; e++) acc[p][e] = 0ull;
-#pragma unroll 2
+#pragma unroll BPL
                     for(; s < end; s++) {
-                        const ulonglong2 e0 = S.list[s][0], e1 = S.list[s][1];
+                        const ulonglong2 e0 = S.list[s].v[0], e1 = S.list[s].v[1];
+                        f32x2 e2 = 0ull;
+                        if constexpr(PAIR) e2 = S.list[s].v[2].x;
 #pragma unroll
                         for(int p = 0; p < NP; p++) {
-                            const f32x2 B = beam(tab, e0.x, minus_tb[p]), aB = mul2(e1.y, B);
+                            const f32x2 B = beam(tab, e0.x, minus_tb[p]);
                             acc[p][0] = fma2(e0.y, B, acc[p][0]);
                             acc[p][1] = fma2(e1.x, B, acc[p][1]);
-                            acc[p][2] = fma2(e0.y, aB, acc[p][2]);
-                            acc[p][3] = fma2(e1.x, aB, acc[p][3]);
+                            if constexpr(PAIR) {
+                                acc[p][2] = fma2(e1.y, B, acc[p][2]);
+                                acc[p][3] = fma2(e2, B, acc[p][3]);
+                            }
+                            else {
+                                const f32x2 aB = mul2(e1.y, B);
+                                acc[p][2] = fma2(e0.y, aB, acc[p][2]);
+                                acc[p][3] = fma2(e1.x, aB, acc[p][3]);
+                            }
                         }
                     }
                     float4* row = P.cells + (size_t)(base + k) * P.pitch;
@@ -321,7 +355,7 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
             base = __reduce_min_sync(0xffffffffu, next);
             __syncwarp();
         }
-        if(near_knot) {
+        if(!PAIR && near_knot) {
             for(int w = w_begin; w < w_end; w += win_step) {
                 const int pos0 = w * 32 * BPL + lane;
                 f32x2 minus_tb[NP];

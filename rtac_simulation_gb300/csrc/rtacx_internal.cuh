@@ -347,6 +347,8 @@ struct CellPing {
     AxisLerp range_axis, beam_axis;
     float theta_lo, theta_hi;        // sample bearings are clamped to these (no beam reaches them)
     float win_scale, win_offset;     // a sample's window: bearing_bin of its bearing
+    KeyParams key;                   // row pairs: a row takes the range bins within `overlap` of it
+    int overlap;
     uint32_t nR, nB, pitch;
     int windows;
 };
@@ -459,6 +461,7 @@ struct Context {
     bool cells_on = false;
     int cell_bpl = 2;                   // bearings per lane
     bool cell_shared = false;           // windows shared out: every sample reaches every window
+    bool cell_pairs = false;            // row pairs instead of knot cells
     CellPing cell{};                    // sorted and out are set per call
     float4* d_cells = nullptr;
     float4* d_cell_taps = nullptr;

@@ -107,3 +107,21 @@ def test_sorted_scratch_after_a_ping_keeps_its_order(oracle):
     assert np.all(np.diff(composite_keys(oracle, wk, got).astype(np.int64)) >= 0)
     assert np.array_equal(np.sort(record_hash(got)), np.sort(record_hash(inside)))
     assert rel_l2(gpu_reduce(ctx, wk.samples, wk.out_shape), first) <= 1e-6
+
+
+@pytest.mark.parametrize("margin", [1.0, 0.999, 3.0])
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("n,nR,nB,H", [(1, 2, 1, 3), (33, 5, 33, 2), (1000, 64, 65, 17), (30000, 300, 129, 164)])
+def test_row_pairs_match_fp64_oracle(oracle, n, nR, nB, H, wide, margin):
+    """Pulses one output range long (the adaptive duration): every sample
+    reaches at most two rows; a margin under one bin switches every row off."""
+    wk = ping(n, nR, nB, 5, wide)
+    s = wk.sensor
+    res = float(wl.linspace_resolution(s["range_min"], s["range_max"], nR))
+    s["pulse"] = np.exp(1j * np.linspace(0.0, 40.0, H)).astype(np.complex64)
+    s["pulse_duration"] = float(np.float32(np.float32(res) / np.float32(1500.0)))
+    s["margin"] = margin * float(np.float32(1500.0) * np.float32(s["pulse_duration"]))
+    got = gpu_reduce(make_context(wk), wk.samples, wk.out_shape)
+    want = oracle.reduce(wk.samples, s)
+    assert np.isfinite(got).all()
+    assert rel_l2(got, want) <= TOL, rel_l2(got, want)
