@@ -310,6 +310,7 @@ rtacx_status rtacx_configure_1d(rtacx_ctx* ctx, const rtacx_sensor_1d* s)
     sync_echo(c);
     if(c.nR > kMaxSmemBins) { c.error = "range_count above the shared-memory histogram limit"; return RTACX_ERR_UNSUPPORTED; }
     std::vector<float> one(1, 0.0f);
+    free_cells(c);
     if(!upload(c, c.d_beam, one.data(), 1) || !upload(c, c.d_bearings, one.data(), 1) || !allocate_bins(c))
         return RTACX_ERR_OUT_OF_MEMORY;
     if((s->flags & RTACX_FLAG_TEXTURE_PSF) && make_pulse_texture_1d(c, s, scale) != RTACX_OK) return RTACX_ERR_CUDA;
@@ -319,6 +320,9 @@ rtacx_status rtacx_configure_1d(rtacx_ctx* ctx, const rtacx_sensor_1d* s)
         // bins that hold the pulse's support.
         std::vector<int2> whole(c.nR, make_int2(0, (int)c.nR - 1));
         if(!upload(c, c.d_support, whole.data(), whole.size())) return RTACX_ERR_OUT_OF_MEMORY;
+    }
+    if(!(s->flags & RTACX_FLAG_TEXTURE_PSF) && configure_cells_1d(c)) {
+        c.cell.pulse = c.d_pulse; c.cell.ranges = c.d_ranges;
     }
     c.configured = true;
     return RTACX_OK;
@@ -480,7 +484,7 @@ rtacx_status rtacx_reduce(rtacx_ctx* ctx, const void* samples, uint64_t n, float
     Context& c = ctx->impl;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     for(bool& t : c.traced) t = false;
-    if(c.cells_on) return run_cells(c, samples, n, reinterpret_cast<float2*>(out), s);
+    if(takes_cells(c, n)) return run_cells(c, samples, n, reinterpret_cast<float2*>(out), s);
     st = run_binning(c, samples, n, s);
     if(st == RTACX_OK) st = run_windows(c, s);
     if(st != RTACX_OK) return st;

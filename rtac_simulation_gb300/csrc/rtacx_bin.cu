@@ -565,18 +565,20 @@ rtacx_status run_sort(Context& ctx, const BinParams& p, const SortShape& shape, 
 }
 
 // Brings a sorted scratch that the cell form left in its own order (window x
-// cell block; the same records, each once) into the order that rtacx_bin
-// documents: the records' tail beyond the in-range count is marked out of
-// range, then the reference order's passes run from the scratch itself into
+// cell block of the in-range records, or, 1D, the input order of all) into
+// the order that rtacx_bin documents: the tail beyond the in-range count is
+// marked out of range, then the reference order's passes run from the scratch itself into
 // a stream-ordered buffer that is copied back.
 rtacx_status restore_sorted(Context& ctx, cudaStream_t stream)
 {
     const uint64_t n = ctx.sorted_cells_n;
     if(!n) return RTACX_OK;
     float4* sorted = ctx.d_sorted;
-    k_mark_tail<<<(uint32_t)std::min<uint64_t>((n + 255) / 256, (uint64_t)ctx.sm_count * 16), 256, 0, stream>>>(
-        sorted, ctx.d_offsets + ctx.cell_bin.nBins, n);
-    RTACX_CUDA(cudaGetLastError());
+    if(!ctx.sorted_input_order) {
+        k_mark_tail<<<(uint32_t)std::min<uint64_t>((n + 255) / 256, (uint64_t)ctx.sm_count * 16), 256, 0, stream>>>(
+            sorted, ctx.d_offsets + ctx.cell_bin.nBins, n);
+        RTACX_CUDA(cudaGetLastError());
+    }
     void* tmp = nullptr;
     RTACX_CUDA(cudaMallocAsync(&tmp, n * sizeof(float4), stream));
     const BinParams kept = ctx.bin;

@@ -1,15 +1,18 @@
-// Plain 2D reduction over range cells (see rtacx_cells.cuh): configuration
-// and the single-ping kernels.
+// Plain reduction over range cells (see rtacx_cells.cuh): configuration and
+// the single-ping kernels.
 //
 //   k_cells         the sorted samples of one ping into the cell rows;
 //   k_cells_filter  the pulse's taps over the cell rows, rows without a
-//                   reference window zeroed.
+//                   reference window zeroed (k_pairs_join: row pairs);
+//   k_cells_1d, k_cells_filter_1d, k_rows_off_1d  the same for 1D sensors,
+//                   from the input order.
 // Measured against the tensor-core gather on the same pings (whole
 // rtacx_reduce, us): 2^20 samples, 512 x 1024, 33 taps, narrow beams: 1384 ->
-// 152; 2^22 samples, 512 x 4096, wide beams: 14433 -> 1339; 150003 samples,
-// 387 x 777, 24 taps: 246 -> 82. k_cells is bound by the beam lookups' shared
-// memory and issue slots, at one lookup per (sample, bearing).
-#include "rtacx_bin_device.cuh"
+// 135; 2^22 samples, 512 x 4096, wide beams: 14433 -> 1247; 150003 samples,
+// 387 x 777, 24 taps: 246 -> 62; 20000 samples, 256 x 500, row pairs: 91 -> 38. k_cells is bound by the beam lookups' shared
+// memory and issue slots, at one lookup per (sample, bearing). 1D, us: 20000
+// samples 1049 ranges (row by row) 32.1 -> 13.5; 3e6 samples 4096 ranges, 65
+// taps 380 -> 43.
 #include "rtacx_cells.cuh"
 
 #include <algorithm>
@@ -97,6 +100,39 @@ k_pairs_join(const CellPing P, const uint32_t* __restrict__ nonempty, int ov)
     P.out[(size_t)r * P.nB + b] = row_on(nonempty, (int)P.nR, ov, r) ? make_float2(t.x + m.z, t.y + m.w) : make_float2(0.f, 0.f);
 }
 
+// 1D pings: the samples into the cells (or rows), then the taps.
+constexpr int kThreads1D = 256;
+template <bool ROWS>
+__global__ void __launch_bounds__(kThreads1D)
+k_cells_1d(const CellPing P, const BinParams p, const float* __restrict__ samples, uint64_t n,
+           uint32_t* __restrict__ nonempty, float4* __restrict__ copy)
+{
+    extern __shared__ uint32_t s_bits[];
+    const uint32_t words = (P.nR + 31) / 32;
+    for(uint32_t i = threadIdx.x; i < words; i += kThreads1D) s_bits[i] = 0u;
+    __syncthreads();
+    const uint64_t chunk = (n + gridDim.x - 1) / gridDim.x, begin = blockIdx.x * chunk;
+    accumulate_1d<ROWS>(P, p, samples, begin, min(begin + chunk, n), P.cells + (size_t)(blockIdx.x % P.replicas) * P.cp.cells,
+                        s_bits, copy);
+    __syncthreads();
+    for(uint32_t i = threadIdx.x; i < words; i += kThreads1D)
+        if(s_bits[i]) atomicOr(&nonempty[i], s_bits[i]);
+}
+
+__global__ void __launch_bounds__(4 * kFilterRows1D)
+k_cells_filter_1d(const CellPing P, const uint32_t* __restrict__ nonempty)
+{
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    filter_rows_1d(P, blockIdx.x, reinterpret_cast<float4*>(s_raw), nonempty);
+}
+
+// Rows of a 1D ping without a reference window.
+__global__ void k_rows_off_1d(const CellPing P, const uint32_t* __restrict__ nonempty)
+{
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if(r < (int)P.nR && !row_on(nonempty, (int)P.nR, P.overlap, r)) P.out[r] = make_float2(0.f, 0.f);
+}
+
 template <typename T>
 void drop(T*& p)
 {
@@ -125,82 +161,169 @@ void free_cells(Context& c)
     c.sorted_cells_n = 0;
 }
 
+namespace {
+
+// The best line (least squares) through the rows' float ranges, and how far
+// each row lies from it, in taps.
+struct RowFit {
+    double k = 0.0, spacing = 0.0, R0 = 0.0, worst = 0.0, last = 0.0;   // taps per metre; metres; taps; metres
+    std::vector<double> R;
+    std::vector<float> dev;
+};
+
+bool fit_rows(const Context& c, RowFit& f)
+{
+    const int nR = (int)c.nR;
+    if(nR < 2 || c.H < 1) return false;
+    f.k = (double)c.red.range_axis.k_hi + (double)c.red.range_axis.k_lo;
+    f.R.resize(nR);
+    double sr = 0.0, sx = 0.0;
+    for(int r = 0; r < nR; r++) {
+        f.R[r] = host_linspace_at(c.rmin, c.rmax, c.nR, (uint32_t)r);
+        sr += f.R[r];
+        sx += ((double)r - 0.5 * (nR - 1)) * f.R[r];
+    }
+    f.spacing = sx / ((double)nR * ((double)nR * nR - 1.0) / 12.0);
+    f.R0 = sr / nR - 0.5 * (nR - 1) * f.spacing;
+    if(!(f.spacing > 0.0) || !std::isfinite(f.spacing)) return false;
+    f.dev.resize(nR);
+    for(int r = 0; r < nR; r++) {
+        const double e = f.k * (f.R0 + r * f.spacing - f.R[r]);
+        f.dev[r] = (float)e;
+        f.worst = std::max(f.worst, std::fabs(e));
+        f.last = std::max(f.last, std::fabs(f.R[r]));
+    }
+    return true;
+}
+
+// Cell coordinate y = travel / spacing + b, storage row floor(y) + shift.
+bool set_cell_axis(CellParams& cp, const RowFit& f, double b, int shift, int cells, double knot, int taps)
+{
+    const double kc = 1.0 / f.spacing;
+    cp.k_hi = (float)kc;
+    cp.k_lo = (float)(kc - (double)cp.k_hi);
+    cp.b_row = (float)(std::floor(b) + shift);
+    cp.b_frac = (float)(b - std::floor(b));
+    cp.knot = (float)knot;
+    cp.cells = cells;
+    cp.taps = taps;
+    return std::fabs(b) + cells <= (double)(1 << 21);
+}
+
+// Half of the travels that reach a row, with a hair of the spacing for the
+// float cell index and the rows' deviations.
+double row_reach(const Context& c, const RowFit& f)
+{
+    return 0.5 * ((double)c.H / f.k) * (1.0 + 1.0 / c.H) + 1e-4 * f.spacing + f.worst / f.k + 1e-6 * f.last;
+}
+
+// Knot cells: the pulse's taps one output range apart, up to what the knot
+// band covers (it costs one product per row and pair, so it is kept under a
+// hundredth of a cell), and every row's PSF support inside its reference
+// window, so that the window only decides whether the row is on.
+bool knot_cells(Context& c, const RowFit& f)
+{
+    const int nR = (int)c.nR, H = (int)c.H;
+    // What moves a row's knots against the grid: its own deviation, the tap
+    // spacing's over half the pulse, and the rounding of travel - range.
+    const double knot = 1.01 * (f.worst + std::fabs(f.k * f.spacing - 1.0) * (0.5 * H + 1.0)) + 2e-6 + 1.5e-7 * H;
+    if(!(knot <= kMaxKnot)) return false;
+    for(int r = 0; r < nR; r++) {
+        const double reach = 0.5 * ((double)H / f.k) * (1.0 + 1.0 / H) * (1.0 + 1e-4);
+        const double slack = 1e-6 * (std::fabs(f.R[r]) + reach) + 1e-30;
+        const int lo = (int)host_range_key_clamped(c.key, (float)(f.R[r] - reach - slack));
+        const int hi = (int)host_range_key_clamped(c.key, (float)(f.R[r] + reach + slack));
+        if(lo < std::max(0ll, (long long)r - c.overlap) || hi > std::min((long long)nR - 1, (long long)r + c.overlap)) return false;
+    }
+    return set_cell_axis(c.cell.cp, f, 0.5 * H - 0.5 - f.R0 / f.spacing, 1, nR + H, knot, H);
+}
+
+// Taps of the knot cells' filter.
+std::vector<float4> cell_taps(const Context& c, const RowFit& f)
+{
+    const int H = (int)c.H;
+    const double kappa = f.k * f.spacing;
+    std::vector<float4> taps((size_t)cell_tap_entries(H), make_float4(0.f, 0.f, 0.f, 0.f));
+    for(int i = -1; i < H; i++) {
+        double p[2], d[2];
+        for(int q = 0; q < 2; q++) {
+            const double lo = i >= 0 ? c.pulse[2 * (size_t)i + q] : 0.0, hi = i + 1 < H ? c.pulse[2 * ((size_t)i + 1) + q] : 0.0;
+            p[q] = lo + (hi - lo) * (kappa - 1.0) * ((double)i - (0.5 * H - 0.5));
+            d[q] = (hi - lo) * kappa;
+        }
+        taps[i + 1] = make_float4((float)p[0], (float)p[1], (float)d[0], (float)d[1]);
+    }
+    return taps;
+}
+
+void set_ping_params(Context& c)
+{
+    CellPing& P = c.cell;
+    P.cells = c.d_cells;
+    P.row_dev = c.d_row_dev; P.taps = c.d_cell_taps;
+    P.pos_theta = c.d_pos_theta; P.pos_col = c.d_pos_col; P.col_bearing = c.d_col_bearing;
+    P.range_axis = c.red.range_axis; P.beam_axis = c.red.beam_axis;
+    P.key = c.key; P.overlap = c.overlap;
+    P.nR = c.nR; P.nB = c.nB;
+}
+
+} // namespace
+
+// 1D sensors: knot cells where the pulse's taps allow them, else row by row.
+bool configure_cells_1d(Context& c)
+{
+    free_cells(c);
+    RowFit f;
+    if(c.dims != 1 || !fit_rows(c, f)) return false;
+    const int nR = (int)c.nR;
+    bool ok = filter_smem_1d((int)c.H) <= 200 * 1024 && knot_cells(c, f);
+    c.cell_pairs = false;
+    c.cell_rows = !ok;
+    if(c.cell_rows) {
+        const double reach = row_reach(c, f), rows = std::floor(2.0 * reach / f.spacing) + 1.0;
+        if(!(rows <= 64.0)) return false;
+        c.cell.rows = (int)rows;
+        // First row reached: floor(y) + 1 with y = (travel - reach - R0) / spacing.
+        ok = set_cell_axis(c.cell.cp, f, -(reach + f.R0) / f.spacing, c.cell.rows, nR + c.cell.rows - 1, 0.0, (int)c.H);
+    }
+    ok = ok && put(c.d_row_dev, f.dev) && put(c.d_cell_taps, cell_taps(c, f)) &&
+         put(c.d_nonempty, std::vector<uint32_t>((nR + 31) / 32, 0u)) &&
+         put(c.d_cells, std::vector<float4>(c.cell_rows ? 1 : (size_t)kReplicas1D * c.cell.cp.cells)) &&
+         raise_smem_limit((const void*)k_cells_filter_1d, filter_smem_1d(c.cell_rows ? 1 : (int)c.H)) == cudaSuccess;
+    if(!ok) { free_cells(c); return false; }
+    set_ping_params(c);
+    c.cell.pitch = 1;
+    c.cells_on = true;
+    return true;
+}
+
+// Row by row is bound by the reductions queueing at the output rows, the
+// sorted gather by its launches until the samples outweigh them. Whole pings,
+// us, row by row / sorted: 1049 ranges, 5 rows, 2^15 samples 19 / 33, 2^17 31 /
+// 35, 2^19 134 / 51; 4096 ranges, 32 rows, 2^15 32 / 33, 2^17 82 / 40; 9 rows
+// 2^17 30 / 35. They meet near 512 reductions per row, or a million in all.
+bool takes_cells(const Context& c, uint64_t n)
+{
+    return c.cells_on && (!c.cell_rows || n * (uint64_t)c.cell.rows <= std::min<uint64_t>(512ull * c.nR, 1ull << 20));
+}
+
 // Decides whether a configured 2D sensor takes the cell form and builds its
-// tables. The rule (everything else keeps the per-row gathers):
-//   * the pulse's taps are one output range apart: the best line through the
-//     rows' float ranges has k * spacing = 1 up to what the knot band covers,
-//     and every row lies within the band of it (the band costs one product
-//     per row and pair, so it is kept under a hundredth of a cell);
-//   * every row's PSF support lies inside its reference window, so the window
-//     only decides whether the row is on;
-//   or (row pairs) no travel reaches more than two rows;
-//   * the cell rows and the beam table fit.
-// Returns whether the form is on; a failed allocation leaves it off.
+// tables: row pairs where no travel reaches three rows, else knot cells where
+// the pulse's taps allow them, and the cell rows and the beam table have to
+// fit (everything else keeps the per-row gathers). Returns whether the form
+// is on; a failed allocation leaves it off.
 bool configure_cells(Context& c, double beam_support)
 {
     free_cells(c);
     const int nR = (int)c.nR, nB = (int)c.nB, H = (int)c.H, W = (int)c.W;
-    if(c.dims != 2 || nR < 2 || H < 1) return false;
-    const double k = (double)c.red.range_axis.k_hi + (double)c.red.range_axis.k_lo, center = 0.5 * H - 0.5;
-    // Least-squares line through the rows' float ranges.
-    std::vector<double> R(nR);
-    double sr = 0.0, sx = 0.0;
-    for(int r = 0; r < nR; r++) {
-        R[r] = host_linspace_at(c.rmin, c.rmax, c.nR, (uint32_t)r);
-        sr += R[r];
-        sx += ((double)r - 0.5 * (nR - 1)) * R[r];
-    }
-    const double spacing = sx / ((double)nR * ((double)nR * nR - 1.0) / 12.0);
-    const double R0 = sr / nR - 0.5 * (nR - 1) * spacing;
-    if(!(spacing > 0.0) || !std::isfinite(spacing)) return false;
-    const double kappa = k * spacing;
-    double worst = 0.0;
-    std::vector<float> dev(nR);
-    for(int r = 0; r < nR; r++) {
-        const double e = k * (R0 + r * spacing - R[r]);
-        dev[r] = (float)e;
-        worst = std::max(worst, std::fabs(e));
-    }
-    const double ext = (double)H / k;
+    RowFit f;
+    if(c.dims != 2 || !fit_rows(c, f)) return false;
     CellParams& cp = c.cell.cp;
-    const double kc = 1.0 / spacing;
-    cp.k_hi = (float)kc;
-    cp.k_lo = (float)(kc - (double)cp.k_hi);
-    double b;                                // cell coordinate y = travel / spacing + b
-    // Row pairs: no travel within `half` of three rows (a hair of the spacing
-    // covers the float cell index and the rows' deviations). Storage row
-    // floor(y) + 2 = first row reached + 1.
-    const double half = 0.5 * ext * (1.0 + 1.0 / H) + 1e-4 * spacing + worst / k + 1e-6 * std::fabs(R[nR - 1]);
-    c.cell_pairs = half < spacing;
-    if(c.cell_pairs) {
-        b = -(half + R0) / spacing;
-        cp.b_row = (float)(std::floor(b) + 2.0);
-        cp.knot = 0.0f;
-        cp.cells = nR + 1;
-    }
-    else {
-        // What moves a row's knots against the grid: its own deviation, the tap
-        // spacing's over half the pulse, and the rounding of travel - range.
-        const double knot = 1.01 * (worst + std::fabs(kappa - 1.0) * (0.5 * H + 1.0)) + 2e-6 + 1.5e-7 * H;
-        if(!(knot <= kMaxKnot)) return false;
-        // Rows' supports inside their windows.
-        for(int r = 0; r < nR; r++) {
-            const double reach = 0.5 * ext * (1.0 + 1.0 / H) * (1.0 + 1e-4);
-            const double slack = 1e-6 * (std::fabs(R[r]) + reach) + 1e-30;
-            const int lo = (int)host_range_key_clamped(c.key, (float)(R[r] - reach - slack));
-            const int hi = (int)host_range_key_clamped(c.key, (float)(R[r] + reach + slack));
-            if(lo < std::max(0ll, (long long)r - c.overlap) || hi > std::min((long long)nR - 1, (long long)r + c.overlap)) return false;
-        }
-        b = center - kc * R0;                // storage row = cell + 1
-        cp.b_row = (float)(std::floor(b) + 1.0);
-        cp.knot = (float)knot;
-        cp.cells = nR + H;
-    }
-    cp.b_frac = (float)(b - std::floor(b));
-    cp.taps = H;
-    c.cell.key = c.key;
-    c.cell.overlap = c.overlap;
-    if(std::fabs(b) + cp.cells > (double)(1 << 21)) return false;
+    c.cell_rows = false;
+    const double reach = row_reach(c, f);
+    c.cell_pairs = reach < f.spacing;
+    // Pairs: the first row reached is floor(y) + 1, its storage row one more.
+    if(!(c.cell_pairs ? set_cell_axis(cp, f, -(reach + f.R0) / f.spacing, 2, nR + 1, 0.0, H) : knot_cells(c, f))) return false;
     // Beam coordinates far below the rounding trick's 2^22.
     const auto mm = std::minmax_element(c.bearings.begin(), c.bearings.end());
     const double fan = (double)*mm.second - (double)*mm.first, span = c.span;
@@ -297,35 +420,51 @@ bool configure_cells(Context& c, double beam_support)
     const size_t cell_bytes = (size_t)cp.cells * pitch * sizeof(float4);
     if(cell_bytes > kMaxCellBytes || cells_smem(W, c.cell_pairs) > 200 * 1024 ||
        (!c.cell_pairs && filter_smem(H) > 200 * 1024)) return false;
-    std::vector<float4> taps((size_t)cell_tap_entries(H), make_float4(0.f, 0.f, 0.f, 0.f));
-    for(int i = -1; i < H; i++) {
-        double p[2], d[2];
-        for(int q = 0; q < 2; q++) {
-            const double lo = i >= 0 ? c.pulse[2 * (size_t)i + q] : 0.0, hi = i + 1 < H ? c.pulse[2 * ((size_t)i + 1) + q] : 0.0;
-            p[q] = lo + (hi - lo) * (kappa - 1.0) * ((double)i - center);
-            d[q] = (hi - lo) * kappa;
-        }
-        taps[i + 1] = make_float4((float)p[0], (float)p[1], (float)d[0], (float)d[1]);
-    }
-    bool ok = put(c.d_cell_taps, taps) && put(c.d_row_dev, dev) && put(c.d_nonempty, std::vector<uint32_t>((nR + 31) / 32, 0u)) &&
+    bool ok = put(c.d_cell_taps, cell_taps(c, f)) && put(c.d_row_dev, f.dev) && put(c.d_nonempty, std::vector<uint32_t>((nR + 31) / 32, 0u)) &&
               put(c.d_pos_theta, theta) && put(c.d_pos_col, col) && put(c.d_col_bearing, col_bearing);
     if(ok && cudaMalloc(&c.d_cells, cell_bytes) != cudaSuccess) { cudaGetLastError(); ok = false; }
     if(ok) ok = raise_smem_limit((const void*)cells_fn(bpl, shared_out, c.cell_pairs), cells_smem(W, c.cell_pairs)) == cudaSuccess &&
                 (c.cell_pairs ||
                  raise_smem_limit((const void*)k_cells_filter, filter_smem(H)) == cudaSuccess);
     if(!ok) { free_cells(c); return false; }
-    CellPing& P = c.cell;
-    P.cells = c.d_cells;
-    P.row_dev = c.d_row_dev; P.taps = c.d_cell_taps;
-    P.pos_theta = c.d_pos_theta; P.pos_col = c.d_pos_col; P.col_bearing = c.d_col_bearing;
-    P.range_axis = c.red.range_axis; P.beam_axis = c.red.beam_axis;
-    P.nR = c.nR; P.nB = c.nB;
+    set_ping_params(c);
     c.cells_on = true;
     return true;
 }
 
+static rtacx_status run_cells_1d(Context& c, const void* samples, uint64_t n, float2* out, cudaStream_t stream)
+{
+    CellPing P = c.cell;
+    P.out = out;
+    P.replicas = !c.cell_rows && n >= kReplicateFrom1D ? kReplicas1D : 1;
+    const uint64_t cells = c.cell_rows ? 0 : (uint64_t)P.cp.cells * P.replicas;
+    c.mark(1, false, stream);
+    k_cells_clear<<<(uint32_t)std::min<uint64_t>((cells + c.nR + 255) / 256, (uint64_t)c.sm_count * 8), 256, 0, stream>>>(
+        c.d_totals, 0, c.d_nonempty, (c.nR + 31) / 32, c.d_cells, cells, out, c.nR);
+    cudaError_t e = cudaGetLastError();
+    c.mark(1, true, stream);
+    c.sorted_cells_n = n;
+    c.sorted_input_order = true;
+    if(e == cudaSuccess && n) {
+        c.mark(5, false, stream);
+        // One record per thread while that fills the SMs, more beyond.
+        const uint32_t grid = (uint32_t)std::min<uint64_t>((n + kThreads1D - 1) / kThreads1D, (uint64_t)c.sm_count * 8);
+        const size_t bits = (c.nR + 31) / 32 * sizeof(uint32_t);
+        auto fn = c.cell_rows ? k_cells_1d<true> : k_cells_1d<false>;
+        fn<<<grid, kThreads1D, bits, stream>>>(P, c.bin, static_cast<const float*>(samples), n, c.d_nonempty, c.d_sorted);
+        if(c.cell_rows) k_rows_off_1d<<<(c.nR + 255) / 256, 256, 0, stream>>>(P, c.d_nonempty);
+        else k_cells_filter_1d<<<(c.nR + kFilterRows1D - 1) / kFilterRows1D, 4 * kFilterRows1D, filter_smem_1d(P.cp.taps),
+                                 stream>>>(P, c.d_nonempty);
+        e = cudaGetLastError();
+        c.mark(5, true, stream);
+    }
+    if(e != cudaSuccess) { c.error = std::string("cell form: ") + cudaGetErrorString(e); return RTACX_ERR_CUDA; }
+    return RTACX_OK;
+}
+
 rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out, cudaStream_t stream)
 {
+    if(c.dims == 1) return run_cells_1d(c, samples, n, out, stream);
     CellPing P = c.cell;
     P.sorted = c.d_sorted;
     P.out = out;
@@ -343,6 +482,7 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
         const rtacx_status st = run_sort(c, bin, c.cell_sort, samples, n, c.d_nonempty, stream);
         if(st != RTACX_OK) return st;
         c.sorted_cells_n = n;
+        c.sorted_input_order = false;
         c.mark(5, false, stream);
         // Units of fewer samples while that leaves the SMs' warps without one;
         // wide beams' windows are then also shared out over blockIdx.y.

@@ -22,6 +22,7 @@
 // cell's two rows, with the rows' own pulse weights, whatever the table.
 #pragma once
 
+#include "rtacx_bin_device.cuh"
 #include "rtacx_internal.cuh"
 
 namespace rtacx {
@@ -67,14 +68,16 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
     return r;
 }
 
+// Reductions into buffers that the reducing kernel never reads: no memory
+// clobber, so that loads move across them.
 __device__ __forceinline__ void red_add_f4(float4* addr, float x, float y, float z, float w)
 {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(x), "f"(y), "f"(z), "f"(w));
 }
 
 __device__ __forceinline__ void red_add_f2(float2* addr, float x, float y)
 {
-    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(addr), "f"(x), "f"(y) : "memory");
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(addr), "f"(x), "f"(y));
 }
 
 // Pulse weight at delta = travel - output range: the lerp of the zero-padded
@@ -389,6 +392,123 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
             }
         }
         cur = __reduce_min_sync(0xffffffffu, next_win);
+    }
+}
+
+// ---- 1D sensors --------------------------------------------------------------
+// Without bearings a sample's sums are two complex numbers, so nothing is
+// gained by sorting: each sample is one 16-byte reduction {v, alpha v} into
+// its cell (ROWS: one 8-byte reduction per output row it reaches), straight
+// from the input order. Samples [begin, end) by one CTA, kLoads1D records per
+// thread in flight. cells: the copy of the cell rows that the CTA adds into
+// (see kReplicas1D). s_bits: the CTA's bitmap of range bins. The records (echo
+// model applied) are kept in `copy` for the diagnostic copy of the sorted scratch.
+constexpr int kLoads1D = 4;
+// Copies of the cell rows on large pings: with one, 3e6 samples on 4161 cells
+// queue at the same L2 addresses (whole ping 55.5 us; 41.6 with 8 copies, 41.1
+// with 32, 33 without the reductions); below 2^18 samples the copies' clearing
+// costs more than it saves.
+constexpr int kReplicas1D = 8;
+constexpr uint64_t kReplicateFrom1D = 1ull << 18;
+
+template <bool ROWS>
+__device__ __forceinline__ void accumulate_1d(const CellPing& P, const BinParams& p, const float* __restrict__ samples,
+                                              uint64_t begin, uint64_t end, float4* cells, uint32_t* s_bits,
+                                              float4* copy)
+{
+    const int lane = threadIdx.x & 31;
+    // Whole warps run every iteration (the row-by-row samples are shared out
+    // over the lanes).
+    for(uint64_t i0 = begin + threadIdx.x - lane; i0 < end; i0 += (uint64_t)blockDim.x * kLoads1D) {
+        float4 rec[kLoads1D];
+#pragma unroll
+        for(int u = 0; u < kLoads1D; u++) {
+            const uint64_t i = i0 + (uint64_t)u * blockDim.x + lane;
+            rec[u] = i < end ? load_record(samples, i, p) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for(int u = 0; u < kLoads1D; u++) {
+            const uint64_t i = i0 + (uint64_t)u * blockDim.x + lane;
+            const float t = rec[u].z;
+            int side;
+            const uint32_t key = i < end ? range_key(p.key, t, side) : kOutOfRange;
+            float2 v = make_float2(rec[u].x, rec[u].y);
+            if(p.echo_flags) v = apply_echo(p, v, t);
+            if(i < end) __stcs(copy + i, make_float4(v.x, v.y, t, 0.0f));
+            float alpha = 0.5f;
+            const int row = key != kOutOfRange ? range_cell(P.cp, t, alpha) : -1;
+            if(key != kOutOfRange) {
+                const uint32_t bit = 1u << (key & 31u);
+                if(!(s_bits[key >> 5] & bit)) atomicOr(&s_bits[key >> 5], bit);
+            }
+            if(ROWS) {
+                if(row < 0) continue;
+                const int r0 = row - (P.rows - 1);
+#pragma unroll 4
+                for(int r = max(r0, 0); r < min(r0 + P.rows, (int)P.nR); r++) {
+                    if(abs((int)key - r) > P.overlap) continue;
+                    const float2 f = pulse_at(P.pulse, P.range_axis, t - P.ranges[r]);
+                    if(f.x != 0.0f || f.y != 0.0f) red_add_f2(P.out + r, v.x * f.x - v.y * f.y, v.x * f.y + v.y * f.x);
+                }
+                continue;
+            }
+            const bool near = row >= 0 && !(alpha >= P.cp.knot && alpha <= 1.0f - P.cp.knot);
+            if(row >= 0 && !near) red_add_f4(cells + row, v.x, v.y, alpha * v.x, alpha * v.y);
+            // Next to a knot: row by row (rows whose pulse reaches cells C - 1 .. C + 1).
+            for(uint32_t m = __ballot_sync(0xffffffffu, near); m; m &= m - 1u) {
+                const int l = __ffs(m) - 1;
+                const float vx = __shfl_sync(0xffffffffu, v.x, l), vy = __shfl_sync(0xffffffffu, v.y, l);
+                const float tl = __shfl_sync(0xffffffffu, t, l);
+                const int C = __shfl_sync(0xffffffffu, row, l) - 1;
+                for(int r = max(0, C - P.cp.taps - 1) + lane; r <= min((int)P.nR - 1, C + 2); r += 32) {
+                    const float2 f = pulse_at(P.pulse, P.range_axis, tl - P.ranges[r]);
+                    if(f.x != 0.0f || f.y != 0.0f) red_add_f2(P.out + r, vx * f.x - vy * f.y, vx * f.y + vy * f.x);
+                }
+            }
+        }
+    }
+}
+
+// Range filter of a 1D ping: four threads per output row, every fourth tap
+// each. s: the cells of the CTA's rows and the taps.
+constexpr int kFilterRows1D = 32;          // rows per CTA of 4 * kFilterRows1D threads
+__host__ __device__ __forceinline__ size_t filter_smem_1d(int H)
+{
+    return (size_t)(kFilterRows1D + 2 * (H + 1)) * sizeof(float4);
+}
+
+__device__ __forceinline__ void filter_rows_1d(const CellPing& P, int tile, float4* s, const uint32_t* nonempty)
+{
+    const int n = P.cp.taps + 1, rows0 = tile * kFilterRows1D;
+    float4 *s_cells = s, *s_taps = s + kFilterRows1D + n;
+    for(int i = threadIdx.x; i < kFilterRows1D + n; i += 4 * kFilterRows1D)
+    {
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+        if(rows0 + i < P.cp.cells)
+            for(int k = 0; k < P.replicas; k++) {
+                const float4 x = P.cells[(size_t)k * P.cp.cells + rows0 + i];
+                a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
+            }
+        s_cells[i] = a;
+    }
+    for(int i = threadIdx.x; i < n; i += 4 * kFilterRows1D) s_taps[i] = P.taps[i];
+    __syncthreads();
+    const int q = threadIdx.x >> 2, r = rows0 + q;
+    const float e = r < (int)P.nR ? P.row_dev[r] : 0.0f;
+    float2 acc = make_float2(0.f, 0.f);
+    for(int t = threadIdx.x & 3; t < n; t += 4) {
+        const float4 c = s_taps[t], a = s_cells[q + t];
+        const float mx = fmaf(e, a.x, a.z), my = fmaf(e, a.y, a.w);
+        acc.x = fmaf(c.x, a.x, fmaf(-c.y, a.y, fmaf(c.z, mx, fmaf(-c.w, my, acc.x))));
+        acc.y = fmaf(c.x, a.y, fmaf(c.y, a.x, fmaf(c.z, my, fmaf(c.w, mx, acc.y))));
+    }
+    for(int o = 1; o < 4; o <<= 1) {
+        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+        acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+    }
+    if((threadIdx.x & 3) == 0 && r < (int)P.nR) {
+        const float2 v = P.out[r];
+        P.out[r] = row_on(nonempty, (int)P.nR, P.overlap, r) ? make_float2(v.x + acc.x, v.y + acc.y) : make_float2(0.f, 0.f);
     }
 }
 

@@ -349,6 +349,8 @@ struct CellPing {
     float win_scale, win_offset;     // a sample's window: bearing_bin of its bearing
     KeyParams key;                   // row pairs: a row takes the range bins within `overlap` of it
     int overlap;
+    int rows;                        // 1D, row by row: rows that a travel reaches, at most
+    int replicas;                    // 1D: copies of the cell rows, taken in turn by the CTAs
     uint32_t nR, nB, pitch;
     int windows;
 };
@@ -462,6 +464,7 @@ struct Context {
     int cell_bpl = 2;                   // bearings per lane
     bool cell_shared = false;           // windows shared out: every sample reaches every window
     bool cell_pairs = false;            // row pairs instead of knot cells
+    bool cell_rows = false;             // 1D without knot cells: row by row
     CellPing cell{};                    // sorted and out are set per call
     float4* d_cells = nullptr;
     float4* d_cell_taps = nullptr;
@@ -472,7 +475,8 @@ struct Context {
     uint32_t* d_nonempty = nullptr;     // [(nR + 31) / 32] bitmap of non-empty range bins
     BinParams cell_bin{};               // the cell form's order
     SortShape cell_sort;
-    uint64_t sorted_cells_n = 0;        // samples of the last ping that left the cell order in d_sorted (0: none)
+    uint64_t sorted_cells_n = 0;        // samples of the last ping that left another order in d_sorted (0: none)
+    bool sorted_input_order = false;    // ... all of them in input order (1D) instead of the in-range ones in cell order
 
     // Split persistent gather of 2D pings (see rtacx_reduce.cu).
     uint32_t* d_tile_parts = nullptr;   // [tiles] sample-stream length of each output tile
@@ -567,6 +571,8 @@ rtacx_status run_reduce(Context& ctx, float* out, cudaStream_t stream);
 
 // Cell form of the plain reduction (rtacx_cells.cu).
 bool configure_cells(Context& ctx, double beam_support);
+bool configure_cells_1d(Context& ctx);
+bool takes_cells(const Context& ctx, uint64_t n);
 void free_cells(Context& ctx);
 rtacx_status run_cells(Context& ctx, const void* samples, uint64_t n, float2* out, cudaStream_t stream);
 

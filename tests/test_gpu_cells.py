@@ -125,3 +125,46 @@ def test_row_pairs_match_fp64_oracle(oracle, n, nR, nB, H, wide, margin):
     want = oracle.reduce(wk.samples, s)
     assert np.isfinite(got).all()
     assert rel_l2(got, want) <= TOL, rel_l2(got, want)
+
+
+def ping_1d(n, nR, taps, H=0, ext_bins=0.0, seed=5):
+    rmin, rmax = 0.4, 30.0
+    res = float(wl.linspace_resolution(rmin, rmax, nR))
+    pulse = wl.pulse_at_bin_spacing(H or taps, res, 38e3, 1500.0)
+    rng = np.random.default_rng(seed)
+    t = rng.uniform(rmin - 2 * taps * res, rmax + 2 * taps * res, n)
+    if n > 64:
+        t[:32] = wl.linspace(rmin, rmax, nR)[rng.integers(0, nR, 32)]
+    re, im = rng.normal(size=(2, n))
+    return wl.Workload("cells_1d", 1, wl.sensor_1d(rmin, rmax, nR, 1500.0, pulse, (ext_bins or taps) * res),
+                       wl._pack(re, im, t))
+
+
+@pytest.mark.parametrize("n,nR,taps,H,ext", [
+    (1, 2, 1, 0, 0), (2, 31, 2, 0, 0), (33, 32, 3, 0, 0), (255, 33, 8, 0, 0), (1025, 100, 65, 0, 0),
+    (70001, 1025, 33, 0, 0), (1 << 20, 300, 9, 0, 0),                       # taps one range apart
+    (33, 31, 1, 7, 0.9), (1000, 64, 2, 40, 2.0), (5000, 257, 4, 77, 4.03),   # row by row
+    (200000, 500, 30, 77, 29.7), (2000, 3000, 200, 77, 150.2),               # the sorted gather again
+])
+def test_1d_pings_match_fp64_oracle(oracle, n, nR, taps, H, ext):
+    wk = ping_1d(n, nR, taps, H, ext)
+    for offset in (0, 1):
+        got = gpu_reduce(make_context(wk), wk.samples, wk.out_shape, offset_floats=offset)
+        want = oracle.reduce(wk.samples, wk.sensor)
+        assert np.isfinite(got).all()
+        assert rel_l2(got, want) <= TOL, rel_l2(got, want)
+
+
+def test_1d_sorted_scratch_after_a_ping(oracle):
+    from test_gpu_sorted import KEY_OOR, composite_keys, record_hash
+    wk = ping_1d(5000, 257, 17)
+    ctx = make_context(wk)
+    gpu_reduce(ctx, wk.samples, wk.out_shape)
+    buf = torch.zeros((wk.n, 4), device="cuda")
+    ctx.diag_sorted(buf, wk.n, stream=torch.cuda.current_stream())
+    recs = np.zeros((wk.n, 4), np.float32)
+    recs[:, :3] = wk.samples
+    inside = recs[composite_keys(oracle, wk, recs) != KEY_OOR]
+    got = buf.cpu().numpy()[:len(inside)]
+    assert np.all(np.diff(composite_keys(oracle, wk, got).astype(np.int64)) >= 0)
+    assert np.array_equal(np.sort(record_hash(got)), np.sort(record_hash(inside)))
