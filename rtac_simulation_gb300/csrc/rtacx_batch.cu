@@ -11,7 +11,9 @@
 // kernel: k_batch_fused, a cooperative persistent launch (one or two CTAs per
 // SM, all resident) that runs every phase of every ping, taking work from
 // atomic queues and separating the phases with bounded grid barriers (and a
-// 24-byte memset node that resets the barrier and the queues). With
+// memset node that resets the barrier and the queues). Pings that rtacx_reduce
+// takes through the cell form go through it here too (choose_form): 16 mixed
+// pings of 2^13 to 2^20 samples 10.0 -> 0.63 ms. With
 // RTACX_BATCH_STAGED the graph holds one launch per binning stage and a
 // persistent gather kernel instead. rtacx_batch_run replays the graph with one
 // cudaGraphLaunch. With RTACX_BATCH_AUTOTUNE the plan times every candidate
@@ -50,9 +52,15 @@ struct Batch {
     uint2* d_win_map = nullptr;
     uint2* d_scan_map = nullptr;
     uint4* d_items = nullptr;
+    uint4* d_filters = nullptr;
+    ZeroItem* d_zero16 = nullptr;
+    ZeroItem* d_zero8 = nullptr;
     uint32_t* d_counter = nullptr;
     BatchSync* d_sync = nullptr;
     uint32_t* d_status = nullptr;
+    uint32_t n_chunks_all = 0, n_filters = 0, n_zero16 = 0, n_zero8 = 0;
+    bool cells = false;             // the fused kernel with the cell form
+    bool per_row_2d = false;        // some 2D ping takes the per-row gather
     uint32_t n_chunks = 0, n_col = 0, n_win = 0, n_scan = 0, n_items = 0, max_bins = 0;
     size_t gather_smem = 0;
     uint32_t gather_grid = 0;
@@ -75,6 +83,7 @@ struct Batch {
         if(exec) cudaGraphExecDestroy(exec);
         exec = nullptr;
         drop(d_pings); drop(d_chunk_map); drop(d_col_map); drop(d_win_map); drop(d_scan_map); drop(d_items);
+        drop(d_filters); drop(d_zero16); drop(d_zero8);
         graph_kernels = 0;
     }
 
@@ -92,13 +101,44 @@ struct Batch {
         return true;
     }
 
+    // Samples of a ping's cell form that one work item takes: about 2048
+    // samples of a 64-bearing window's work, in whole rounds of the CTA's warps.
+    static uint32_t cells_per_item(const Context& c)
+    {
+        const uint64_t pairs = c.cell_shared ? c.cell.pitch : 32u * (uint32_t)c.cell_bpl;
+        const uint64_t want = 2048u * 64u / std::max<uint64_t>(pairs, 64u);
+        return want >= 2048 ? 2048u : want >= 1024 ? 1024u : want >= 512 ? 512u : 256u;
+    }
+
+    // Whether the batch runs on the fused kernel with the cell form: when the
+    // per-row gathers' share of the work (samples x bearings) is at most half,
+    // since that kernel keeps fewer of their CTAs resident.
+    void choose_form()
+    {
+        double per_row = 0.0, cell = 0.0;
+        for(const rtacx_ping_desc& p : pings) {
+            const Context& c = p.ctx->impl;
+            (takes_cells(c, p.n) ? cell : per_row) += (double)p.n * c.nB;
+        }
+        cells = !staged && cell > 0.0 && per_row <= cell;
+        per_row_2d = false;
+        for(const rtacx_ping_desc& p : pings)
+            if(p.ctx->impl.dims == 2 && !(cells && takes_cells(p.ctx->impl, p.n))) per_row_2d = true;
+    }
+
     // Descriptors, maps and work items for one candidate; captures the graph.
     rtacx_status build(const Candidate& cand)
     {
         free_plan();
         const int TR = gather_shape_rows(cand.shape), TB = gather_shape_bearings(cand.shape);
         std::vector<PingDev> descs;
-        std::vector<uint2> chunk_map, col_map, win_map, scan_map;
+        std::vector<uint2> chunk_map, chunk_map_1d, col_map, win_map, scan_map;
+        std::vector<uint4> filters;
+        std::vector<ZeroItem> zero16, zero8;
+        auto zero = [](std::vector<ZeroItem>& list, void* p, uint64_t n, size_t elem) {
+            for(uint64_t i = 0; i < n; i += 4096)
+                list.push_back(ZeroItem{static_cast<unsigned char*>(p) + i * elem, std::min<uint64_t>(4096, n - i)});
+        };
         struct Item { uint4 v; double cost; };
         std::vector<Item> items;
         max_bins = 1;
@@ -107,9 +147,12 @@ struct Batch {
             Context& c = pings[i].ctx->impl;
             const uint64_t n = pings[i].n;
             PingDev d{};
+            const bool cell_form = cells && takes_cells(c, n);
+            d.form = !cell_form ? kPerRow
+                   : c.dims == 1 ? (c.cell_rows ? kRows1D : kCells1D) : (c.cell_pairs ? kPairs2D : kCells2D);
             d.samples = static_cast<const float*>(pings[i].samples);
             d.n = n;
-            d.bin = c.bin;
+            d.bin = cell_form && c.dims == 2 ? c.cell_bin : c.bin;
             d.bin.vec4 = (c.dims == 2 && reinterpret_cast<uintptr_t>(pings[i].samples) % 16 == 0) ? 1 : 0;
             d.chunks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(c.sort.hist_ctas, ceil_div(n, cand.per_cta)));
             d.hist = c.d_hist; d.totals = c.d_totals; d.offsets = c.d_offsets; d.oor = c.d_oor; d.err = c.d_err;
@@ -118,13 +161,45 @@ struct Batch {
             d.red = c.red; d.bb_tiles = c.d_bb_tiles; d.ranges = c.d_ranges; d.bearings = c.d_bearings;
             d.pulse = c.d_pulse; d.beam = c.d_beam; d.out = reinterpret_cast<float2*>(pings[i].out);
             if(c.dims == 2) d.bb_tiles = (TB == 64) ? c.d_bb_tiles64 : c.d_bb_tiles128;   // ranges for width TB
-            descs.push_back(d);
+            if(cell_form) {
+                d.cell = c.cell;
+                d.cell.sorted = c.d_sorted;
+                d.cell.out = d.out;
+                d.cell.replicas = c.dims == 1 ? cell_replicas(c, n) : 1;
+                d.nonempty = c.d_nonempty;
+                d.bpl = c.cell_bpl;
+                d.shared = c.cell_shared ? 1 : 0;
+                zero(zero16, c.d_nonempty, (c.nR + 127) / 128, 16);
+                if(d.form != kRows1D) zero(zero16, c.d_cells, (uint64_t)c.cell.cp.cells * c.cell.pitch * d.cell.replicas, 16);
+                if(d.form != kPairs2D) zero(zero8, d.out, (uint64_t)c.nR * c.nB, 8);
+                uint32_t columns;
+                const uint32_t rows = batch_filter_tiles(c, columns);
+                for(uint32_t y = 0; y < rows; y++)
+                    for(uint32_t x = 0; x < columns; x++) filters.push_back(make_uint4(i, x, y, 0));
+                gather_smem = std::max(gather_smem, batch_cells_smem(c));
+            }
+            if(cell_form && c.dims == 1) {
+                d.chunks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sm_count * 8, ceil_div(n, cand.per_cta)));
+                for(uint32_t k = 0; k < d.chunks; k++) chunk_map_1d.push_back(make_uint2(i, k));
+                descs.push_back(d);
+                continue;
+            }
             for(uint32_t k = 0; k < d.chunks; k++) chunk_map.push_back(make_uint2(i, k));
-            for(uint32_t k = 0; k < ceil_div(c.bin.nBins, 256); k++) col_map.push_back(make_uint2(i, k));
-            for(uint32_t k = 0; k < ceil_div(c.nR, 256); k++) win_map.push_back(make_uint2(i, k));
-            for(uint32_t k = 0; k < ceil_div(c.bin.nBins, kScanBlock); k++) scan_map.push_back(make_uint2(i, k));
-            max_bins = std::max(max_bins, c.bin.nBins);
+            for(uint32_t k = 0; k < ceil_div(d.bin.nBins, 256); k++) col_map.push_back(make_uint2(i, k));
+            for(uint32_t k = 0; k < ceil_div(d.bin.nBins, kScanBlock); k++) scan_map.push_back(make_uint2(i, k));
+            max_bins = std::max(max_bins, d.bin.nBins);
             const double density = (double)n / c.nR;     // samples per range bin
+            if(cell_form) {
+                d.per_item = cells_per_item(c);
+                d.unit = std::min(128u, std::max(32u, d.per_item / 8));
+                const double pairs = c.cell_shared ? c.cell.pitch : 32.0 * c.cell_bpl;
+                for(uint64_t k = 0; k < ceil_div(n, d.per_item); k++)
+                    items.push_back({make_uint4(i, (uint32_t)k, 0, 2), (double)std::min<uint64_t>(n, d.per_item) * pairs / 64.0});
+                descs.push_back(d);
+                continue;
+            }
+            descs.push_back(d);
+            for(uint32_t k = 0; k < ceil_div(c.nR, 256); k++) win_map.push_back(make_uint2(i, k));
             if(c.dims == 2) {
                 const uint32_t tb = (c.nB + TB - 1) / TB, tr = (c.nR + TR - 1) / TR;
                 for(uint32_t y = 0; y < tr; y++)
@@ -139,10 +214,15 @@ struct Batch {
         std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.cost > b.cost; });
         std::vector<uint4> iv(items.size());
         for(size_t k = 0; k < items.size(); k++) iv[k] = items[k].v;
-        n_chunks = (uint32_t)chunk_map.size(); n_col = (uint32_t)col_map.size();
+        n_chunks = (uint32_t)chunk_map.size();
+        chunk_map.insert(chunk_map.end(), chunk_map_1d.begin(), chunk_map_1d.end());
+        n_chunks_all = (uint32_t)chunk_map.size();
+        n_filters = (uint32_t)filters.size(); n_zero16 = (uint32_t)zero16.size(); n_zero8 = (uint32_t)zero8.size();
+        n_col = (uint32_t)col_map.size();
         n_win = (uint32_t)win_map.size(); n_scan = (uint32_t)scan_map.size(); n_items = (uint32_t)iv.size();
         if(!put(d_pings, descs) || !put(d_chunk_map, chunk_map) || !put(d_col_map, col_map) ||
-           !put(d_win_map, win_map) || !put(d_scan_map, scan_map) || !put(d_items, iv))
+           !put(d_win_map, win_map) || !put(d_scan_map, scan_map) || !put(d_items, iv) || !put(d_filters, filters) ||
+           !put(d_zero16, zero16) || !put(d_zero8, zero8))
             return RTACX_ERR_OUT_OF_MEMORY;
         if(gather_smem > 227 * 1024) { error = "PSF tables too large for the batched gather"; return RTACX_ERR_UNSUPPORTED; }
         if(staged && (size_t)max_bins * 4 > 227 * 1024) { error = "histograms too large for the batched binning"; return RTACX_ERR_UNSUPPORTED; }
@@ -155,12 +235,15 @@ struct Batch {
     rtacx_status capture_fused(const Candidate& cand)
     {
         fused_smem = gather_smem;
-        rtacx_status prep = prepare_fused_batch(error, cand.shape, fused_smem, sm_count, fused_grid);
+        rtacx_status prep = prepare_fused_batch(error, cand.shape, cells, fused_smem, sm_count, fused_grid);
         if(prep != RTACX_OK) return prep;
         fb = FusedBatch{};
         fb.pings = d_pings;
         fb.col_map = d_col_map; fb.n_col = n_col;
-        fb.chunk_map = d_chunk_map; fb.n_chunks = n_chunks;
+        fb.chunk_map = d_chunk_map; fb.n_chunks = n_chunks; fb.n_chunks_all = n_chunks_all;
+        fb.zero16 = d_zero16; fb.n_zero16 = n_zero16;
+        fb.zero8 = d_zero8; fb.n_zero8 = n_zero8;
+        fb.filters = d_filters; fb.n_filters = n_filters;
         fb.scan_map = d_scan_map; fb.n_scan = n_scan;
         fb.win_map = d_win_map; fb.n_win = n_win;
         fb.items = d_items; fb.n_items = n_items;
@@ -176,7 +259,7 @@ struct Batch {
         }
         rtacx_status st = RTACX_OK;
         if(cudaMemsetAsync(d_sync, 0, sizeof(BatchSync), stream) != cudaSuccess) st = RTACX_ERR_CUDA;
-        if(st == RTACX_OK) st = launch_fused_batch(error, cand.shape, fb, fused_smem, fused_grid, stream);
+        if(st == RTACX_OK) st = launch_fused_batch(error, cand.shape, cells, fb, fused_smem, fused_grid, stream);
         return finish_capture(st, graph);
     }
 
@@ -330,6 +413,7 @@ rtacx_status rtacx_batch_plan(rtacx_batch* b, const rtacx_ping_desc* pings, uint
     }
     B.pings.assign(pings, pings + count);
     B.staged = (flags & RTACX_BATCH_STAGED) != 0;
+    B.choose_form();
     if(!(flags & RTACX_BATCH_AUTOTUNE)) {
         const rtacx_status st = B.build(Candidate{2, 4096});
         B.tuned_ms = 0.0f;
@@ -338,7 +422,7 @@ rtacx_status rtacx_batch_plan(rtacx_batch* b, const rtacx_ping_desc* pings, uint
     // Autotune: every candidate is built, captured and timed on this batch.
     Candidate best{2, 4096};
     float best_ms = 1e30f;
-    for(int shape = 0; shape < 3; shape++)
+    for(int shape = 0; shape < (B.per_row_2d ? 3 : 1); shape++)     // (the tile shape is the per-row 2D gather's)
         for(uint32_t per : {2048u, 4096u, 8192u}) {
             const Candidate cand{shape, per};
             if(B.build(cand) != RTACX_OK) continue;
@@ -362,7 +446,12 @@ rtacx_status rtacx_batch_run(rtacx_batch* b, void* stream)
         B.error = "cudaGraphLaunch failed";
         return RTACX_ERR_CUDA;
     }
-    for(const rtacx_ping_desc& p : B.pings) p.ctx->impl.sorted_cells_n = 0;   // the batch sorts in rtacx_bin's order
+    // The order that the batch leaves in the pings' sorted scratch.
+    for(const rtacx_ping_desc& p : B.pings) {
+        Context& c = p.ctx->impl;
+        c.sorted_cells_n = B.cells && takes_cells(c, p.n) ? p.n : 0;
+        c.sorted_input_order = c.dims == 1;
+    }
     return RTACX_OK;
 }
 

@@ -290,18 +290,27 @@ __device__ __forceinline__ void scan_bin_block(const uint32_t* __restrict__ tota
 
 // Count pass of chunk c of nc straight into totals[0, nBins) with one global
 // atomic per sample (no shared histogram: the fused batched kernel keeps its
-// shared memory for the gather). Out-of-range counts as count_chunk.
+// shared memory for the gather). Out-of-range counts and the bitmap as
+// count_chunk's (a set bit is read before it is written again).
 __device__ __forceinline__ void count_chunk_global(const float* __restrict__ samples, uint64_t n, const BinParams& p,
                                                    uint32_t c, uint32_t nc, uint32_t* __restrict__ totals,
-                                                   unsigned long long* __restrict__ oor, unsigned long long* s_oor)
+                                                   unsigned long long* __restrict__ oor, unsigned long long* s_oor,
+                                                   uint32_t* nonempty = nullptr)
 {
     if(threadIdx.x < 2) s_oor[threadIdx.x] = 0ull;
     __syncthreads();
     uint32_t low = 0, high = 0;
-    for_chunk(samples, n, p, c, nc, [&](const bool* valid, const float4*, const uint32_t* key, const int* side) {
+    for_chunk(samples, n, p, c, nc, [&](const bool* valid, const float4* rec, const uint32_t* key, const int* side) {
 #pragma unroll
         for(int u = 0; u < kTileLoads; u++) {
-            if(valid[u] && key[u] != kOutOfRange) atomicAdd(&totals[key[u]], 1u);
+            if(valid[u] && key[u] != kOutOfRange) {
+                atomicAdd(&totals[key[u]], 1u);
+                if(nonempty) {
+                    int unused;
+                    const uint32_t r = range_key(p.key, rec[u].z, unused), bit = 1u << (r & 31u);
+                    if(!(__ldcg(nonempty + (r >> 5)) & bit)) atomicOr(nonempty + (r >> 5), bit);
+                }
+            }
             else if(valid[u]) {
                 if(side[u] < 0) low++; else high++;
             }

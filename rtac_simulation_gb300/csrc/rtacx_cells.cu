@@ -76,28 +76,17 @@ __global__ void k_cells_clear(uint32_t* __restrict__ totals, uint32_t n_totals, 
 }
 
 __global__ void __launch_bounds__(32 * kFilterWarps)
-k_cells_filter(const CellPing P, const uint32_t* __restrict__ nonempty, int ov)
+k_cells_filter(const CellPing P, const uint32_t* __restrict__ nonempty)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    __shared__ int s_on[kFilterTile];
-    if(threadIdx.x < kFilterTile) {
-        const int r = blockIdx.y * kFilterTile + threadIdx.x;
-        s_on[threadIdx.x] = r < (int)P.nR && row_on(nonempty, (int)P.nR, ov, r) ? 1 : 0;
-    }
-    filter_tile(P, blockIdx.x, blockIdx.y, reinterpret_cast<float4*>(s_raw), s_on);   // synchronises before it reads s_on
+    filter_tile<kFilterWarps>(P, blockIdx.x, blockIdx.y, reinterpret_cast<float4*>(s_raw), nonempty);
 }
 
-// Row pairs into the ping: row r takes T of storage row r + 1 and M of storage
-// row r.
+// One CTA per output row.
 __global__ void __launch_bounds__(256)
-k_pairs_join(const CellPing P, const uint32_t* __restrict__ nonempty, int ov)
+k_pairs_join(const CellPing P, const uint32_t* __restrict__ nonempty)
 {
-    const int r = blockIdx.y, col = blockIdx.x * blockDim.x + threadIdx.x;
-    if(col >= (int)P.pitch) return;
-    const int b = P.col_bearing[col];
-    if(b < 0) return;
-    const float4 t = P.cells[(size_t)(r + 1) * P.pitch + col], m = P.cells[(size_t)r * P.pitch + col];
-    P.out[(size_t)r * P.nB + b] = row_on(nonempty, (int)P.nR, ov, r) ? make_float2(t.x + m.z, t.y + m.w) : make_float2(0.f, 0.f);
+    join_pairs(P, blockIdx.x, nonempty);
 }
 
 // 1D pings: the samples into the cells (or rows), then the taps.
@@ -123,7 +112,7 @@ __global__ void __launch_bounds__(4 * kFilterRows1D)
 k_cells_filter_1d(const CellPing P, const uint32_t* __restrict__ nonempty)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    filter_rows_1d(P, blockIdx.x, reinterpret_cast<float4*>(s_raw), nonempty);
+    filter_rows_1d<kFilterRows1D>(P, blockIdx.x, reinterpret_cast<float4*>(s_raw), nonempty);
 }
 
 // Rows of a 1D ping without a reference window.
@@ -276,7 +265,7 @@ bool configure_cells_1d(Context& c)
     RowFit f;
     if(c.dims != 1 || !fit_rows(c, f)) return false;
     const int nR = (int)c.nR;
-    bool ok = filter_smem_1d((int)c.H) <= 200 * 1024 && knot_cells(c, f);
+    bool ok = filter_smem_1d((int)c.H, kFilterRows1D) <= 200 * 1024 && knot_cells(c, f);
     c.cell_pairs = false;
     c.cell_rows = !ok;
     if(c.cell_rows) {
@@ -287,9 +276,9 @@ bool configure_cells_1d(Context& c)
         ok = set_cell_axis(c.cell.cp, f, -(reach + f.R0) / f.spacing, c.cell.rows, nR + c.cell.rows - 1, 0.0, (int)c.H);
     }
     ok = ok && put(c.d_row_dev, f.dev) && put(c.d_cell_taps, cell_taps(c, f)) &&
-         put(c.d_nonempty, std::vector<uint32_t>((nR + 31) / 32, 0u)) &&
+         put(c.d_nonempty, std::vector<uint32_t>((nR + 127) / 128 * 4, 0u)) &&
          put(c.d_cells, std::vector<float4>(c.cell_rows ? 1 : (size_t)kReplicas1D * c.cell.cp.cells)) &&
-         raise_smem_limit((const void*)k_cells_filter_1d, filter_smem_1d(c.cell_rows ? 1 : (int)c.H)) == cudaSuccess;
+         raise_smem_limit((const void*)k_cells_filter_1d, filter_smem_1d(c.cell_rows ? 1 : (int)c.H, kFilterRows1D)) == cudaSuccess;
     if(!ok) { free_cells(c); return false; }
     set_ping_params(c);
     c.cell.pitch = 1;
@@ -306,6 +295,8 @@ bool takes_cells(const Context& c, uint64_t n)
 {
     return c.cells_on && (!c.cell_rows || n * (uint64_t)c.cell.rows <= std::min<uint64_t>(512ull * c.nR, 1ull << 20));
 }
+
+int cell_replicas(const Context& c, uint64_t n) { return !c.cell_rows && n >= kReplicateFrom1D ? kReplicas1D : 1; }
 
 // Decides whether a configured 2D sensor takes the cell form and builds its
 // tables: row pairs where no travel reaches three rows, else knot cells where
@@ -420,7 +411,7 @@ bool configure_cells(Context& c, double beam_support)
     const size_t cell_bytes = (size_t)cp.cells * pitch * sizeof(float4);
     if(cell_bytes > kMaxCellBytes || cells_smem(W, c.cell_pairs) > 200 * 1024 ||
        (!c.cell_pairs && filter_smem(H) > 200 * 1024)) return false;
-    bool ok = put(c.d_cell_taps, cell_taps(c, f)) && put(c.d_row_dev, f.dev) && put(c.d_nonempty, std::vector<uint32_t>((nR + 31) / 32, 0u)) &&
+    bool ok = put(c.d_cell_taps, cell_taps(c, f)) && put(c.d_row_dev, f.dev) && put(c.d_nonempty, std::vector<uint32_t>((nR + 127) / 128 * 4, 0u)) &&
               put(c.d_pos_theta, theta) && put(c.d_pos_col, col) && put(c.d_col_bearing, col_bearing);
     if(ok && cudaMalloc(&c.d_cells, cell_bytes) != cudaSuccess) { cudaGetLastError(); ok = false; }
     if(ok) ok = raise_smem_limit((const void*)cells_fn(bpl, shared_out, c.cell_pairs), cells_smem(W, c.cell_pairs)) == cudaSuccess &&
@@ -436,7 +427,7 @@ static rtacx_status run_cells_1d(Context& c, const void* samples, uint64_t n, fl
 {
     CellPing P = c.cell;
     P.out = out;
-    P.replicas = !c.cell_rows && n >= kReplicateFrom1D ? kReplicas1D : 1;
+    P.replicas = cell_replicas(c, n);
     const uint64_t cells = c.cell_rows ? 0 : (uint64_t)P.cp.cells * P.replicas;
     c.mark(1, false, stream);
     k_cells_clear<<<(uint32_t)std::min<uint64_t>((cells + c.nR + 255) / 256, (uint64_t)c.sm_count * 8), 256, 0, stream>>>(
@@ -453,7 +444,7 @@ static rtacx_status run_cells_1d(Context& c, const void* samples, uint64_t n, fl
         auto fn = c.cell_rows ? k_cells_1d<true> : k_cells_1d<false>;
         fn<<<grid, kThreads1D, bits, stream>>>(P, c.bin, static_cast<const float*>(samples), n, c.d_nonempty, c.d_sorted);
         if(c.cell_rows) k_rows_off_1d<<<(c.nR + 255) / 256, 256, 0, stream>>>(P, c.d_nonempty);
-        else k_cells_filter_1d<<<(c.nR + kFilterRows1D - 1) / kFilterRows1D, 4 * kFilterRows1D, filter_smem_1d(P.cp.taps),
+        else k_cells_filter_1d<<<(c.nR + kFilterRows1D - 1) / kFilterRows1D, 4 * kFilterRows1D, filter_smem_1d(P.cp.taps, kFilterRows1D),
                                  stream>>>(P, c.d_nonempty);
         e = cudaGetLastError();
         c.mark(5, true, stream);
@@ -496,9 +487,9 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
         cells_fn(c.cell_bpl, c.cell_shared, c.cell_pairs)<<<dim3(gx, gy), kCellThreads,
                                                             cells_smem(P.beam_axis.n, c.cell_pairs), stream>>>(
             P, c.d_offsets + bin.nBins, unit);
-        const dim3 fgrid(P.pitch / 32, (c.nR + kFilterTile - 1) / kFilterTile);
-        if(c.cell_pairs) k_pairs_join<<<dim3((P.pitch + 255) / 256, c.nR), 256, 0, stream>>>(P, c.d_nonempty, c.overlap);
-        else k_cells_filter<<<fgrid, 32 * kFilterWarps, filter_smem(P.cp.taps), stream>>>(P, c.d_nonempty, c.overlap);
+        const dim3 fgrid(P.pitch / 32, (c.nR + kFilterWarps * kFilterRows - 1) / (kFilterWarps * kFilterRows));
+        if(c.cell_pairs) k_pairs_join<<<c.nR, std::min(256u, P.pitch), 0, stream>>>(P, c.d_nonempty);
+        else k_cells_filter<<<fgrid, 32 * kFilterWarps, filter_smem(P.cp.taps), stream>>>(P, c.d_nonempty);
         e = cudaGetLastError();
         c.mark(5, true, stream);
     }

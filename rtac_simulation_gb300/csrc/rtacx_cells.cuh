@@ -471,27 +471,28 @@ __device__ __forceinline__ void accumulate_1d(const CellPing& P, const BinParams
 
 // Range filter of a 1D ping: four threads per output row, every fourth tap
 // each. s: the cells of the CTA's rows and the taps.
-constexpr int kFilterRows1D = 32;          // rows per CTA of 4 * kFilterRows1D threads
-__host__ __device__ __forceinline__ size_t filter_smem_1d(int H)
+constexpr int kFilterRows1D = 32;          // rows per CTA of 4 kFilterRows1D threads
+__host__ __device__ __forceinline__ size_t filter_smem_1d(int H, int rows)
 {
-    return (size_t)(kFilterRows1D + 2 * (H + 1)) * sizeof(float4);
+    return (size_t)(rows + 2 * (H + 1)) * sizeof(float4);
 }
 
+template <int ROWS>
 __device__ __forceinline__ void filter_rows_1d(const CellPing& P, int tile, float4* s, const uint32_t* nonempty)
 {
-    const int n = P.cp.taps + 1, rows0 = tile * kFilterRows1D;
-    float4 *s_cells = s, *s_taps = s + kFilterRows1D + n;
-    for(int i = threadIdx.x; i < kFilterRows1D + n; i += 4 * kFilterRows1D)
+    const int n = P.cp.taps + 1, rows0 = tile * ROWS;
+    float4 *s_cells = s, *s_taps = s + ROWS + n;
+    for(int i = threadIdx.x; i < ROWS + n; i += 4 * ROWS)
     {
         float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
         if(rows0 + i < P.cp.cells)
             for(int k = 0; k < P.replicas; k++) {
-                const float4 x = P.cells[(size_t)k * P.cp.cells + rows0 + i];
+                const float4 x = __ldcg(P.cells + (size_t)k * P.cp.cells + rows0 + i);
                 a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
             }
         s_cells[i] = a;
     }
-    for(int i = threadIdx.x; i < n; i += 4 * kFilterRows1D) s_taps[i] = P.taps[i];
+    for(int i = threadIdx.x; i < n; i += 4 * ROWS) s_taps[i] = P.taps[i];
     __syncthreads();
     const int q = threadIdx.x >> 2, r = rows0 + q;
     const float e = r < (int)P.nR ? P.row_dev[r] : 0.0f;
@@ -507,20 +508,19 @@ __device__ __forceinline__ void filter_rows_1d(const CellPing& P, int tile, floa
         acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
     }
     if((threadIdx.x & 3) == 0 && r < (int)P.nR) {
-        const float2 v = P.out[r];
+        const float2 v = __ldcg(P.out + r);
         P.out[r] = row_on(nonempty, (int)P.nR, P.overlap, r) ? make_float2(v.x + acc.x, v.y + acc.y) : make_float2(0.f, 0.f);
     }
 }
 
 // ---- range filter over the cell rows ----------------------------------------
-// A CTA of kFilterWarps warps filters 32 columns x kFilterWarps * kFilterRows
-// output rows. The cell rows it needs are staged in shared memory by 16-byte
+// A CTA of WARPS warps filters 32 columns x WARPS * kFilterRows output rows. The cell rows it needs are staged in shared memory by 16-byte
 // asynchronous copies, kFilterChunk rows at a time, all of them in flight
 // together. Each thread holds one column and kFilterRows consecutive output
 // rows and walks the staged cells; the taps of its rows slide through
 // registers (the tap of row q at a cell is the tap of row q + 1 at the next).
 // taps[t] = {P[t - 1], D[t - 1]}, t = 0 .. H, zero beyond.
-constexpr int kFilterWarps = 4, kFilterRows = 8, kFilterTile = kFilterWarps * kFilterRows;
+constexpr int kFilterWarps = 4, kFilterRows = 8;
 constexpr int kFilterChunk = 72;           // staged cell rows: a 33-tap pulse's tile in one chunk
 
 // Entries of the tap table: H + 1 taps, the sliding window's steps beyond
@@ -531,18 +531,24 @@ __host__ __device__ __forceinline__ size_t filter_smem(int H)
     return (size_t)cell_tap_entries(H) * sizeof(float4) + (size_t)kFilterChunk * 32 * sizeof(float4);
 }
 
-// Columns [32 tile_c, +32) and rows [kFilterTile tile_r, +kFilterTile) of a
-// ping; on: the rows' flags in shared memory. Called by 32 kFilterWarps threads.
+// Columns [32 tile_c, +32) and rows [8 WARPS tile_r, +8 WARPS) of a ping. Called
+// by 32 WARPS threads; synchronises.
+template <int WARPS>
 __device__ __forceinline__ void filter_tile(const CellPing& P, int tile_c, int tile_r, float4* s_raw,
-                                            const int* s_on)
+                                            const uint32_t* nonempty)
 {
-    constexpr int kThreads = 32 * kFilterWarps;
+    constexpr int kThreads = 32 * WARPS, kFilterTile = WARPS * kFilterRows;
+    __shared__ int s_on[kFilterTile];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float4* s_taps = s_raw;
     float4* s_cells = s_raw + cell_tap_entries(P.cp.taps);
     const int rows0 = tile_r * kFilterTile, r0 = rows0 + warp * kFilterRows, col = tile_c * 32 + lane;
     const int span = P.cp.taps + kFilterRows;                  // cells that reach a thread's rows
     const int total = min(P.cp.taps + kFilterTile, P.cp.cells - rows0);   // cells of the tile
+    if(tid < kFilterTile) {
+        const int r = rows0 + tid;
+        s_on[tid] = r < (int)P.nR && row_on(nonempty, (int)P.nR, P.overlap, r) ? 1 : 0;
+    }
     for(int i = tid; i < cell_tap_entries(P.cp.taps); i += kThreads) s_taps[i] = P.taps[i];
     float2 acc[kFilterRows];
     float e[kFilterRows];
@@ -557,7 +563,7 @@ __device__ __forceinline__ void filter_tile(const CellPing& P, int tile_c, int t
     for(int k0 = 0; k0 < total; k0 += kFilterChunk) {
         const int rows = min(kFilterChunk, total - k0);
         if(k0) __syncthreads();
-        for(int i = warp; i < kFilterChunk; i += kFilterWarps) {
+        for(int i = warp; i < kFilterChunk; i += WARPS) {
             float4* dst = s_cells + i * 32 + lane;
             if(i < rows)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)),
@@ -591,8 +597,21 @@ __device__ __forceinline__ void filter_tile(const CellPing& P, int tile_c, int t
     for(int q = 0; q < kFilterRows; q++) {
         if(r0 + q >= (int)P.nR) break;
         float2* o = P.out + (size_t)(r0 + q) * P.nB + b;
-        const float2 v = *o;
+        const float2 v = __ldcg(o);
         *o = s_on[warp * kFilterRows + q] ? make_float2(v.x + acc[q].x, v.y + acc[q].y) : make_float2(0.f, 0.f);
+    }
+}
+
+// Row pairs of output row r into the ping, by every thread of the CTA: T of
+// storage row r + 1 and M of storage row r.
+__device__ __forceinline__ void join_pairs(const CellPing& P, int r, const uint32_t* nonempty)
+{
+    const bool on = row_on(nonempty, (int)P.nR, P.overlap, r);
+    for(int col = threadIdx.x; col < (int)P.pitch; col += blockDim.x) {
+        const int b = P.col_bearing[col];
+        if(b < 0) continue;
+        const float4 t = __ldcg(P.cells + (size_t)(r + 1) * P.pitch + col), m = __ldcg(P.cells + (size_t)r * P.pitch + col);
+        P.out[(size_t)r * P.nB + b] = on ? make_float2(t.x + m.z, t.y + m.w) : make_float2(0.f, 0.f);
     }
 }
 

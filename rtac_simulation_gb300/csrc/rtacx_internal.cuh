@@ -363,8 +363,17 @@ struct SortShape {
     int scatter_shape = 0;              // 1 + index of the staged scatter's shape (0: per-tile scatter)
 };
 
+// How a ping of a batch is reduced: sorted by range and gathered per row
+// (kPerRow), or in the cell form (rtacx_cells.cuh).
+enum PingForm : int { kPerRow = 0, kCells2D, kPairs2D, kCells1D, kRows1D };
+
 // Everything one ping of a batch needs on the device (rtacx_batch_*).
 struct PingDev {
+    int form;
+    int bpl, shared;                 // cell form, 2D: bearings per lane; shared-out windows
+    uint32_t per_item, unit;         // ... samples per work item and per warp's unit
+    CellPing cell;
+    uint32_t* nonempty;
     const float* samples;
     uint64_t n;
     BinParams bin;
@@ -390,18 +399,30 @@ struct PingDev {
 
 // Grid-barrier and work-queue state of the fused batched kernel (zeroed
 // before every launch): barrier arrivals and generation, then one work
-// counter per dynamically scheduled phase (count, scan, scatter, gather).
+// counter per dynamically scheduled phase (count, scan, scatter, gather,
+// filter).
 struct BatchSync {
     uint32_t arrived;
     uint32_t generation;
-    uint32_t next[4];
+    uint32_t next[5];
+};
+
+// A stretch of memory to zero: n elements of 16 (cell rows, bitmaps) or 8
+// bytes (pings).
+struct ZeroItem {
+    void* p;
+    uint64_t n;
 };
 
 // Parameters of the fused batched kernel. Maps are (ping, index) pairs.
 struct FusedBatch {
     const PingDev* pings;
     const uint2* col_map;   uint32_t n_col;      // 256-bin groups of the totals to zero
-    const uint2* chunk_map; uint32_t n_chunks;   // chunks of the count and scatter passes
+    const uint2* chunk_map; uint32_t n_chunks;   // chunks of the count and scatter passes; from n_chunks to
+    uint32_t n_chunks_all;                       // n_chunks_all the 1D cell-form pings' chunks (scatter phase only)
+    const ZeroItem* zero16; uint32_t n_zero16;   // cell form: zeroed in phase 0
+    const ZeroItem* zero8; uint32_t n_zero8;     // ... its pings, zeroed in phase 1
+    const uint4* filters;   uint32_t n_filters;  // ... {ping, column tile, row tile, -}
     const uint2* scan_map;  uint32_t n_scan;     // kScanBlock-bin blocks of the bin scan
     const uint2* win_map;   uint32_t n_win;      // 256-row groups of the windows
     const uint4* items;     uint32_t n_items;    // gather items (2D tiles, 1D row groups)
@@ -573,6 +594,7 @@ rtacx_status run_reduce(Context& ctx, float* out, cudaStream_t stream);
 bool configure_cells(Context& ctx, double beam_support);
 bool configure_cells_1d(Context& ctx);
 bool takes_cells(const Context& ctx, uint64_t n);
+int cell_replicas(const Context& ctx, uint64_t n);       // 1D: copies of the cell rows that a ping uses
 void free_cells(Context& ctx);
 rtacx_status run_cells(Context& ctx, const void* samples, uint64_t n, float2* out, cudaStream_t stream);
 
@@ -590,9 +612,12 @@ rtacx_status launch_gather_batch(std::string& error, int shape, const PingDev* p
                                  cudaStream_t stream);
 // Fused batched form: the whole batch (zeroing, count, scan, windows,
 // scatter, gather) in one cooperative persistent launch.
-rtacx_status prepare_fused_batch(std::string& error, int shape, size_t smem, int sm_count, uint32_t& grid);
-rtacx_status launch_fused_batch(std::string& error, int shape, const FusedBatch& fb, size_t smem, uint32_t grid,
-                                cudaStream_t stream);
+// cells: the kernel that takes the cell form's pings too.
+rtacx_status prepare_fused_batch(std::string& error, int shape, bool cells, size_t smem, int sm_count, uint32_t& grid);
+rtacx_status launch_fused_batch(std::string& error, int shape, bool cells, const FusedBatch& fb, size_t smem,
+                                uint32_t grid, cudaStream_t stream);
+size_t batch_cells_smem(const Context& c);       // shared memory of a cell-form ping's items
+uint32_t batch_filter_tiles(const Context& c, uint32_t& columns);   // filter items: row tiles, column tiles
 int gather_shape_rows(int shape);
 int gather_shape_bearings(int shape);
 

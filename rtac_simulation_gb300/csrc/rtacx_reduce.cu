@@ -20,6 +20,7 @@
 // acc[r][b] += U[k][r] * B[k][b]. A warp skips a chunk whose range bins lie
 // outside its rows' windows.
 #include "rtacx_bin_device.cuh"
+#include "rtacx_cells.cuh"
 #include "rtacx_internal.cuh"
 #include "rtacx_tcgen05.cuh"
 
@@ -970,24 +971,109 @@ __device__ __forceinline__ uint32_t claim(uint32_t* counter, uint32_t* s_item)
     return *s_item;
 }
 
+// ---- the cell form's items in the fused kernel ------------------------------
+// Noinline: one copy for every tile shape of the per-row gather.
+__device__ __noinline__ void batch_cells_item(const CellPing& P, int form, int bpl, int shared, uint32_t first,
+                                              uint32_t end, uint32_t unit, unsigned char* smem_raw)
+{
+    const int warp = threadIdx.x >> 5;
+    const size_t per_warp = form == kPairs2D ? sizeof(CellWarpSmem<true>) : sizeof(CellWarpSmem<false>);
+    float2* tab = reinterpret_cast<float2*>(smem_raw + kWarps * per_warp);
+    load_beam_table(tab, P.beam, P.beam_axis.n, threadIdx.x, kThreads);
+    __syncthreads();
+    BeamLookup beam;
+    beam.init(P.beam_axis);
+    unsigned char* own = smem_raw + warp * per_warp;
+    auto& S = *reinterpret_cast<CellWarpSmem<false>*>(own);
+    auto& S2 = *reinterpret_cast<CellWarpSmem<true>*>(own);
+    for(uint32_t u = first + warp * unit; u < end; u += kWarps * unit) {
+        const uint32_t count = min(unit, end - u);
+        if(form == kPairs2D) {
+            if(shared) {
+                if(bpl == 4) accumulate_unit<4, true, true>(P, u, count, 0, 1, S2, tab, beam);
+                else accumulate_unit<2, true, true>(P, u, count, 0, 1, S2, tab, beam);
+            }
+            else if(bpl == 4) accumulate_unit<4, false, true>(P, u, count, 0, 1, S2, tab, beam);
+            else accumulate_unit<2, false, true>(P, u, count, 0, 1, S2, tab, beam);
+        }
+        else if(shared) {
+            if(bpl == 4) accumulate_unit<4, true, false>(P, u, count, 0, 1, S, tab, beam);
+            else accumulate_unit<2, true, false>(P, u, count, 0, 1, S, tab, beam);
+        }
+        else if(bpl == 4) accumulate_unit<4, false, false>(P, u, count, 0, 1, S, tab, beam);
+        else accumulate_unit<2, false, false>(P, u, count, 0, 1, S, tab, beam);
+    }
+}
+
+__device__ __noinline__ void batch_chunk_1d(const PingDev& D, const CellPing& P, uint32_t chunk, unsigned char* smem_raw)
+{
+    uint32_t* s_bits = reinterpret_cast<uint32_t*>(smem_raw);
+    const uint32_t words = (P.nR + 31) / 32;
+    for(uint32_t i = threadIdx.x; i < words; i += kThreads) s_bits[i] = 0u;
+    __syncthreads();
+    const uint64_t per = (D.n + D.chunks - 1) / D.chunks, begin = chunk * per, end = min(begin + per, D.n);
+    float4* cells = P.cells + (size_t)(chunk % P.replicas) * P.cp.cells;
+    if(D.form == kRows1D) accumulate_1d<true>(P, D.bin, D.samples, begin, end, cells, s_bits, D.sorted);
+    else accumulate_1d<false>(P, D.bin, D.samples, begin, end, cells, s_bits, D.sorted);
+    __syncthreads();
+    for(uint32_t i = threadIdx.x; i < words; i += kThreads)
+        if(s_bits[i]) atomicOr(&D.nonempty[i], s_bits[i]);
+}
+
+constexpr int kBatchFilterRows = kWarps * kFilterRows;      // output rows of a 2D filter item
+constexpr int kBatchPairRows = 32;                           // ... of a row-pair item
+constexpr int kBatchRows1D = kThreads / 4;                   // ... of a 1D filter item
+
+__device__ __noinline__ void batch_filter_item(const PingDev& D, const CellPing& P, uint4 item, unsigned char* smem_raw)
+{
+    float4* s = reinterpret_cast<float4*>(smem_raw);
+    const int r0 = (int)item.z * (D.form == kPairs2D ? kBatchPairRows : kThreads);
+    switch(D.form) {
+    case kCells2D: filter_tile<kWarps>(P, (int)item.y, (int)item.z, s, D.nonempty); break;
+    case kPairs2D:
+        for(int r = r0; r < min(r0 + kBatchPairRows, (int)P.nR); r++) join_pairs(P, r, D.nonempty);
+        break;
+    case kCells1D: filter_rows_1d<kBatchRows1D>(P, (int)item.z, s, D.nonempty); break;
+    case kRows1D: {
+        const int r = r0 + (int)threadIdx.x;
+        if(r < (int)P.nR && !row_on(D.nonempty, (int)P.nR, P.overlap, r)) P.out[r] = make_float2(0.f, 0.f);
+        break;
+    }
+    default: break;
+    }
+}
+
 // The whole batched plain form in one cooperative persistent launch:
-//   phase 0  zero every ping's bin totals and out-of-range counts
+//   phase 0  zero every ping's bin totals and out-of-range counts (cell
+//            form: its cell rows and bitmaps)
 //   phase 1  count chunks (a global atomic per sample)       dynamic queue
+//            (cell form: zero its pings first)
 //   phase 2  bin-scan blocks of kScanBlock bins              dynamic queue
 //   phase 3  reference windows (static), scatter chunks      dynamic queue
-//            (a global cursor atomic per sample)
-//   phase 4  gather items, heaviest first                    dynamic queue
+//            (a global cursor atomic per sample; 1D cell-form pings: the
+//            samples into their cells or rows)
+//   phase 4  gather items, heaviest first (cell form: units  dynamic queue
+//            of sorted samples into the cell rows)
+//   phase 5  cell form: range filters                        dynamic queue
 // separated by bounded grid barriers. The binning phases use no shared
 // histogram, so the dynamic shared memory is the gather's and as many CTAs
 // per SM stay resident as for a gather alone.
-template <int TR, int TB>
-__global__ void __launch_bounds__(kThreads) k_batch_fused(const FusedBatch fb)
+template <int TR, int TB, bool CELLS>
+__device__ __forceinline__ void batch_fused(const FusedBatch& fb, unsigned char* smem_raw)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned long long s_oor[2];
     __shared__ uint32_t s_warp[32];
     __shared__ uint32_t s_prefix, s_item;
     __shared__ int s_ok;
+    __shared__ CellPing s_cell;
+    // The item's cell parameters in shared memory (they are read in loops).
+    auto cell_of = [&](const PingDev& P) -> const CellPing& {
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(&P.cell);
+        uint32_t* dst = reinterpret_cast<uint32_t*>(&s_cell);
+        for(uint32_t i = threadIdx.x; i < sizeof(CellPing) / 4; i += kThreads) dst[i] = src[i];
+        __syncthreads();
+        return s_cell;
+    };
 
     for(uint32_t k = blockIdx.x; k < fb.n_col; k += gridDim.x) {
         const uint2 m = fb.col_map[k];
@@ -997,14 +1083,25 @@ __global__ void __launch_bounds__(kThreads) k_batch_fused(const FusedBatch fb)
         if(b < (P.bin.nBins + kScanBlock - 1) / kScanBlock) P.totals[P.bin.nBins + b] = 0u;
         if(m.y == 0 && threadIdx.x < 2) P.oor[threadIdx.x] = 0ull;
     }
+    if(CELLS)
+        for(uint32_t k = blockIdx.x; k < fb.n_zero16; k += gridDim.x) {
+            const ZeroItem z = fb.zero16[k];
+            for(uint64_t i = threadIdx.x; i < z.n; i += kThreads) static_cast<float4*>(z.p)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
     if(!grid_barrier(fb, &s_ok)) return;
 
+    if(CELLS)
+        for(uint32_t k = blockIdx.x; k < fb.n_zero8; k += gridDim.x) {
+            const ZeroItem z = fb.zero8[k];
+            for(uint64_t i = threadIdx.x; i < z.n; i += kThreads) static_cast<float2*>(z.p)[i] = make_float2(0.f, 0.f);
+        }
     for(;;) {
         const uint32_t k = claim(&fb.sync->next[0], &s_item);
         if(k >= fb.n_chunks) break;
         const uint2 m = fb.chunk_map[k];
         const PingDev& P = fb.pings[m.x];
-        count_chunk_global(P.samples, P.n, P.bin, m.y, P.chunks, P.totals, P.oor, s_oor);
+        count_chunk_global(P.samples, P.n, P.bin, m.y, P.chunks, P.totals, P.oor, s_oor,
+                           CELLS && P.form != kPerRow ? P.nonempty : nullptr);
     }
     if(!grid_barrier(fb, &s_ok)) return;
 
@@ -1024,10 +1121,11 @@ __global__ void __launch_bounds__(kThreads) k_batch_fused(const FusedBatch fb)
     }
     for(;;) {
         const uint32_t k = claim(&fb.sync->next[2], &s_item);
-        if(k >= fb.n_chunks) break;
+        if(k >= fb.n_chunks_all) break;
         const uint2 m = fb.chunk_map[k];
         const PingDev& P = fb.pings[m.x];
-        scatter_chunk_global(P.samples, P.n, P.bin, m.y, P.chunks, P.hist, P.offsets, P.sorted, P.err);
+        if(CELLS && k >= fb.n_chunks) batch_chunk_1d(P, cell_of(P), m.y, smem_raw);
+        else scatter_chunk_global(P.samples, P.n, P.bin, m.y, P.chunks, P.hist, P.offsets, P.sorted, P.err);
     }
     if(!grid_barrier(fb, &s_ok)) return;
 
@@ -1040,6 +1138,13 @@ __global__ void __launch_bounds__(kThreads) k_batch_fused(const FusedBatch fb)
             gather_tile_2d<TR, TB>(P.sorted, P.offsets, P.win, P.bb_tiles, P.ranges, P.bearings, P.pulse, P.beam,
                                    P.red, P.bin.nBB, P.out, (int)item.y, (int)item.z, smem_raw);
         }
+        else if(CELLS && item.w == 2) {
+            const uint32_t total = P.offsets[P.bin.nBins];
+            const uint64_t first = (uint64_t)item.y * P.per_item;
+            if(first >= total) continue;
+            batch_cells_item(cell_of(P), P.form, P.bpl, P.shared, (uint32_t)first,
+                             (uint32_t)min(first + P.per_item, (uint64_t)total), P.unit, smem_raw);
+        }
         else {
             float2* s_pulse = reinterpret_cast<float2*>(smem_raw);
             for(int i = threadIdx.x; i < P.red.range_axis.n + 2; i += kThreads) s_pulse[i] = P.pulse[i];
@@ -1047,18 +1152,47 @@ __global__ void __launch_bounds__(kThreads) k_batch_fused(const FusedBatch fb)
             gather_rows_1d(P.sorted, P.offsets, P.win, P.ranges, s_pulse, P.red, P.out, (int)item.y * kWarps);
         }
     }
+    if(!CELLS) return;
+    if(!grid_barrier(fb, &s_ok)) return;
+
+    for(;;) {
+        const uint32_t it = claim(&fb.sync->next[4], &s_item);
+        if(it >= fb.n_filters) break;
+        const uint4 item = fb.filters[it];
+        const PingDev& P = fb.pings[item.x];
+        batch_filter_item(P, cell_of(P), item, smem_raw);
+    }
 }
 
 template <int TR, int TB>
+__global__ void __launch_bounds__(kThreads) k_batch_fused(const FusedBatch fb)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    batch_fused<TR, TB, false>(fb, smem_raw);
+}
+
+// With the cell form, two CTAs per SM (its registers); the kernel above keeps
+// the per-row gather's occupancy for batches that are mostly per-row.
+template <int TR, int TB>
+__global__ void __launch_bounds__(kThreads, 2) k_batch_cells(const FusedBatch fb)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    batch_fused<TR, TB, true>(fb, smem_raw);
+}
+
+template <int TR, int TB, bool CELLS>
+constexpr auto batch_kernel() { return CELLS ? k_batch_cells<TR, TB> : k_batch_fused<TR, TB>; }
+
+template <int TR, int TB, bool CELLS>
 rtacx_status prepare_fused_shape(std::string& error, size_t smem, int sm_count, uint32_t& grid)
 {
-    if(raise_smem_limit((const void*)k_batch_fused<TR, TB>, smem) != cudaSuccess) {
+    if(raise_smem_limit((const void*)batch_kernel<TR, TB, CELLS>(), smem) != cudaSuccess) {
         cudaGetLastError();
         error = "shared memory of the fused batched kernel (" + std::to_string(smem) + " B) not available";
         return RTACX_ERR_UNSUPPORTED;
     }
     int per_sm = 0;
-    if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_fused<TR, TB>, kThreads, smem) != cudaSuccess ||
+    if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel<TR, TB, CELLS>(), kThreads, smem) != cudaSuccess ||
        per_sm < 1) {
         cudaGetLastError();
         error = "the fused batched kernel does not fit on an SM";
@@ -1068,7 +1202,7 @@ rtacx_status prepare_fused_shape(std::string& error, size_t smem, int sm_count, 
     return RTACX_OK;
 }
 
-template <int TR, int TB>
+template <int TR, int TB, bool CELLS>
 rtacx_status launch_fused_shape(std::string& error, const FusedBatch& fb, size_t smem, uint32_t grid,
                                 cudaStream_t stream)
 {
@@ -1082,7 +1216,7 @@ rtacx_status launch_fused_shape(std::string& error, const FusedBatch& fb, size_t
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_batch_fused<TR, TB>, fb);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, batch_kernel<TR, TB, CELLS>(), fb);
     if(e != cudaSuccess) {
         cudaGetLastError();
         error = std::string("k_batch_fused: ") + cudaGetErrorString(e);
@@ -1093,19 +1227,37 @@ rtacx_status launch_fused_shape(std::string& error, const FusedBatch& fb, size_t
 
 } // namespace
 
-rtacx_status prepare_fused_batch(std::string& error, int shape, size_t smem, int sm_count, uint32_t& grid)
+rtacx_status prepare_fused_batch(std::string& error, int shape, bool cells, size_t smem, int sm_count, uint32_t& grid)
 {
-    if(shape == 2) return prepare_fused_shape<32, 128>(error, smem, sm_count, grid);
-    if(shape == 1) return prepare_fused_shape<16, 128>(error, smem, sm_count, grid);
-    return prepare_fused_shape<16, 64>(error, smem, sm_count, grid);
+    auto fn = shape == 2 ? (cells ? prepare_fused_shape<32, 128, true> : prepare_fused_shape<32, 128, false>)
+            : shape == 1 ? (cells ? prepare_fused_shape<16, 128, true> : prepare_fused_shape<16, 128, false>)
+                         : (cells ? prepare_fused_shape<16, 64, true> : prepare_fused_shape<16, 64, false>);
+    return fn(error, smem, sm_count, grid);
 }
 
-rtacx_status launch_fused_batch(std::string& error, int shape, const FusedBatch& fb, size_t smem, uint32_t grid,
-                                cudaStream_t stream)
+rtacx_status launch_fused_batch(std::string& error, int shape, bool cells, const FusedBatch& fb, size_t smem,
+                                uint32_t grid, cudaStream_t stream)
 {
-    if(shape == 2) return launch_fused_shape<32, 128>(error, fb, smem, grid, stream);
-    if(shape == 1) return launch_fused_shape<16, 128>(error, fb, smem, grid, stream);
-    return launch_fused_shape<16, 64>(error, fb, smem, grid, stream);
+    auto fn = shape == 2 ? (cells ? launch_fused_shape<32, 128, true> : launch_fused_shape<32, 128, false>)
+            : shape == 1 ? (cells ? launch_fused_shape<16, 128, true> : launch_fused_shape<16, 128, false>)
+                         : (cells ? launch_fused_shape<16, 64, true> : launch_fused_shape<16, 64, false>);
+    return fn(error, fb, smem, grid, stream);
+}
+
+size_t batch_cells_smem(const Context& c)
+{
+    if(c.dims == 1)
+        return std::max(c.cell_rows ? 0 : filter_smem_1d((int)c.H, kBatchRows1D), (size_t)(c.nR + 31) / 32 * sizeof(uint32_t));
+    const size_t units = kWarps * (c.cell_pairs ? sizeof(CellWarpSmem<true>) : sizeof(CellWarpSmem<false>)) +
+                         (size_t)(c.W + 2) * sizeof(float2);
+    return c.cell_pairs ? units : std::max(units, filter_smem((int)c.H));
+}
+
+uint32_t batch_filter_tiles(const Context& c, uint32_t& columns)
+{
+    columns = c.dims == 2 && !c.cell_pairs ? c.cell.pitch / 32 : 1;
+    const uint32_t rows = c.dims == 1 ? (c.cell_rows ? kThreads : kBatchRows1D) : c.cell_pairs ? kBatchPairRows : kBatchFilterRows;
+    return (c.nR + rows - 1) / rows;
 }
 
 // Batched gather tile shapes: 0 = 16 x 64, 1 = 16 x 128, 2 = 32 x 128.

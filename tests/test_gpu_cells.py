@@ -168,3 +168,37 @@ def test_1d_sorted_scratch_after_a_ping(oracle):
     got = buf.cpu().numpy()[:len(inside)]
     assert np.all(np.diff(composite_keys(oracle, wk, got).astype(np.int64)) >= 0)
     assert np.array_equal(np.sort(record_hash(got)), np.sort(record_hash(inside)))
+
+
+@pytest.mark.parametrize("autotune", [False, True])
+def test_batch_of_every_form_matches_fp64_oracle(oracle, autotune):
+    """One batch with a ping of every form (narrow and wide cells, row pairs,
+    a 2D sensor off the rule, 1D cells, row by row and sorted), run twice."""
+    from rtac_simulation_gb300 import _lib
+    pair = ping(3000, 100, 65, 5, True)
+    res = float(wl.linspace_resolution(0.4, 30.0, 100))
+    pair.sensor["pulse"] = np.exp(1j * np.linspace(0.0, 9.0, 20)).astype(np.complex64)
+    pair.sensor["pulse_duration"] = float(np.float32(res) / np.float32(1500.0))
+    off = ping(2000, 64, 40, 9, False)
+    off.sensor["pulse_duration"] *= 0.5
+    pings = [ping(70001, 257, 129, 33, False), ping(9000, 200, 200, 17, True), pair, off,
+             ping_1d(300000, 300, 33), ping_1d(999, 64, 2, 40, 2.0), ping_1d(200000, 500, 30, 77, 29.7),
+             ping(1, 9, 33, 3, False)]
+    ctxs = [make_context(wk) for wk in pings]
+    devs = [torch.from_numpy(wk.samples.reshape(-1)).cuda() for wk in pings]
+    outs = [torch.full(wk.out_shape + (2,), float("nan"), device="cuda") for wk in pings]
+    batch = _lib.Batch(0)
+    batch.plan([(c, d, wk.n, o) for wk, c, d, o in zip(pings, ctxs, devs, outs)], autotune=autotune)
+    assert batch.graph_kernels() == 1
+    for _ in range(2):
+        batch.run(torch.cuda.current_stream())
+        batch.status(torch.cuda.current_stream())
+        for wk, o in zip(pings, outs):
+            got = o.cpu().numpy()
+            got = got[..., 0].astype(np.float64) + 1j * got[..., 1]
+            want = oracle.reduce(wk.samples, wk.sensor)
+            assert rel_l2(got, want) <= TOL, (wk.name, wk.n, rel_l2(got, want))
+    # A single ping on a context that the batch used, and the batch again.
+    one = gpu_reduce(ctxs[0], pings[0].samples, pings[0].out_shape)
+    assert rel_l2(one, oracle.reduce(pings[0].samples, pings[0].sensor)) <= TOL
+    batch.close()
