@@ -51,7 +51,9 @@ __global__ void k_count(const float* __restrict__ samples, uint64_t n, BinParams
 {
     extern __shared__ uint32_t sh[];
     __shared__ unsigned long long s_oor[2];
-    count_chunk(samples, n, p, blockIdx.x, gridDim.x, totals, oor, sh, s_oor, nonempty);
+    chain_next();
+    chain_wait();
+    count_chunk(after_chain(samples), n, p, blockIdx.x, gridDim.x, totals, oor, sh, s_oor, nonempty);
 }
 
 // Exclusive scan of totals[0, nBins) into offsets[0, nBins] by one CTA of
@@ -103,7 +105,9 @@ __global__ void __launch_bounds__(kScanBlock) k_binscan_blocks(const uint32_t* _
 {
     __shared__ uint32_t s_warp[32];
     __shared__ uint32_t s_prefix;
-    scan_bin_block(totals, nBins, blockIdx.x, offsets, cursor, s_warp, &s_prefix);
+    chain_next();
+    chain_wait();
+    scan_bin_block(after_chain(totals), nBins, blockIdx.x, offsets, cursor, s_warp, &s_prefix);
 }
 
 __global__ void k_scatter(const float* __restrict__ samples, uint64_t n, BinParams p,
@@ -111,7 +115,9 @@ __global__ void k_scatter(const float* __restrict__ samples, uint64_t n, BinPara
                           float4* __restrict__ sorted, uint32_t* __restrict__ err)
 {
     extern __shared__ uint32_t sh[];
-    scatter_chunk(samples, n, p, blockIdx.x, gridDim.x, cursor, offsets, sorted, err, sh);
+    chain_next();
+    chain_wait();
+    scatter_chunk(after_chain(samples), n, p, blockIdx.x, gridDim.x, cursor, after_chain(offsets), sorted, err, sh);
 }
 
 // Staged scatter (single ping; one 1024-thread CTA per SM): tiles of
@@ -144,7 +150,10 @@ k_scatter_staged(const float* __restrict__ samples, uint64_t n, BinParams p, uin
     uint32_t* s_delta = s_start + nb;                                     // global base - local start
     const uint32_t tid = threadIdx.x;
     const uint32_t per = (nb + NT - 1) / NT, b0 = min(tid * per, nb), b1 = min(b0 + per, nb);
-    const uint32_t total = offsets[nb];
+    chain_next();
+    chain_wait();
+    samples = after_chain(samples);
+    const uint32_t total = *after_chain(offsets + nb);
     const uint64_t chunk = (n + gridDim.x - 1) / gridDim.x;
     const uint64_t begin = (uint64_t)blockIdx.x * chunk, end = min(begin + chunk, n);
     for(uint32_t b = tid; b < nb; b += NT) s_start[b] = 0u;
@@ -409,10 +418,13 @@ k_scatter_pipe(const float* __restrict__ samples, uint64_t n, BinParams p, uint3
     uint32_t* s_delta = s_start + nb;                                     // global base - local start
     const uint32_t tid = threadIdx.x;
     const uint32_t per = pipe_bins_per_thread(nb, NT), b0 = min(tid * per, nb), b1 = min(b0 + per, nb);
-    const uint32_t total = offsets[nb];
+    for(uint32_t b = b0; b < b1; b++) s_start[b] = 0u;
+    chain_next();
+    chain_wait();
+    samples = after_chain(samples);
+    const uint32_t total = *after_chain(offsets + nb);
     const uint64_t chunk = (n + gridDim.x - 1) / gridDim.x;
     const uint64_t begin = (uint64_t)blockIdx.x * chunk, end = min(begin + chunk, n);
-    for(uint32_t b = b0; b < b1; b++) s_start[b] = 0u;
     uint32_t prev = 0;                       // sorted slots of the previous tile
     for(uint64_t t0 = begin;; t0 += (uint64_t)NT * U) {
         const bool more = t0 < end;
@@ -536,14 +548,14 @@ rtacx_status run_sort(Context& ctx, const BinParams& p, const SortShape& shape, 
     const float* s = static_cast<const float*>(samples);
     const uint32_t scan_blocks = (p.nBins + kScanBlock - 1) / kScanBlock;
     ctx.mark(0, false, stream);
-    k_count<<<grid, shape.hist_threads, smem + (nonempty ? (p.key.nR + 31) / 32 * sizeof(uint32_t) : 0), stream>>>(
-        s, n, p, ctx.d_totals, ctx.d_oor, nonempty);
-    RTACX_CUDA(cudaGetLastError());
+    RTACX_CUDA(launch_chained(k_count, grid, shape.hist_threads,
+                              smem + (nonempty ? (p.key.nR + 31) / 32 * sizeof(uint32_t) : 0), stream, s, n, p,
+                              ctx.d_totals, ctx.d_oor, nonempty));
     ctx.mark(0, true, stream);
     ctx.mark(2, false, stream);
     // d_hist holds the per-bin write cursors of the scatter.
-    k_binscan_blocks<<<scan_blocks, kScanBlock, 0, stream>>>(ctx.d_totals, p.nBins, ctx.d_offsets, ctx.d_hist);
-    RTACX_CUDA(cudaGetLastError());
+    RTACX_CUDA(launch_chained(k_binscan_blocks, scan_blocks, kScanBlock, 0, stream, ctx.d_totals, p.nBins,
+                              ctx.d_offsets, ctx.d_hist));
     ctx.mark(2, true, stream);
     ctx.mark(3, false, stream);
     if(shape.scatter_shape) {
@@ -551,15 +563,13 @@ rtacx_status run_sort(Context& ctx, const BinParams& p, const SortShape& shape, 
         const uint32_t g = hist_grid((uint32_t)ctx.sm_count, n);
         const bool one_batch = pipe_bins_per_thread(p.nBins, sh.nt) <= (uint32_t)kReserveBatch;
         const ScatterFn fn = sh.fn[p.echo_flags ? 1 : 0][one_batch ? 1 : 0];
-        fn<<<g, sh.nt, staged_smem_bytes(sh.nt, sh.u, p.nBins), stream>>>(s, n, p, ctx.d_hist, ctx.d_offsets,
-                                                                       ctx.d_sorted, ctx.d_err);
+        RTACX_CUDA(launch_chained(fn, g, sh.nt, staged_smem_bytes(sh.nt, sh.u, p.nBins), stream, s, n, p, ctx.d_hist,
+                                  ctx.d_offsets, ctx.d_sorted, ctx.d_err));
     }
     else {
-        k_scatter<<<hist_grid(shape.scatter_ctas, n), shape.hist_threads, smem, stream>>>(s, n, p, ctx.d_hist,
-                                                                                          ctx.d_offsets, ctx.d_sorted,
-                                                                                          ctx.d_err);
+        RTACX_CUDA(launch_chained(k_scatter, hist_grid(shape.scatter_ctas, n), shape.hist_threads, smem, stream, s, n,
+                                  p, ctx.d_hist, ctx.d_offsets, ctx.d_sorted, ctx.d_err));
     }
-    RTACX_CUDA(cudaGetLastError());
     ctx.mark(3, true, stream);
     return RTACX_OK;
 }

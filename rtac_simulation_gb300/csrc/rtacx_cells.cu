@@ -35,16 +35,20 @@ size_t cells_smem(int W, bool pairs)
 
 template <int BPL, bool SHARED, bool PAIR>
 __global__ void __launch_bounds__(kCellThreads, BPL == 2 ? 3 : 2)
-k_cells(const CellPing P, const uint32_t* __restrict__ total, uint32_t unit)
+k_cells(const CellPing ping, const uint32_t* __restrict__ total, uint32_t unit)
 {
+    CellPing P = ping;
     extern __shared__ __align__(16) unsigned char s_raw[];
     CellWarpSmem<PAIR>& S = reinterpret_cast<CellWarpSmem<PAIR>*>(s_raw)[threadIdx.x >> 5];
     float2* tab = reinterpret_cast<float2*>(s_raw + kCellWarps * sizeof(CellWarpSmem<PAIR>));
+    chain_next();
     load_beam_table(tab, P.beam, P.beam_axis.n, threadIdx.x, kCellThreads);
     __syncthreads();
+    chain_wait();
+    P.sorted = after_chain(P.sorted);
     BeamLookup beam;
     beam.init(P.beam_axis);
-    const uint32_t m = *total;
+    const uint32_t m = *after_chain(total);
     for(uint64_t u = (uint64_t)(blockIdx.x * kCellWarps + (threadIdx.x >> 5)) * unit; u < m;
         u += (uint64_t)gridDim.x * kCellWarps * unit)
         accumulate_unit<BPL, SHARED, PAIR>(P, (uint32_t)u, min(unit, m - (uint32_t)u), blockIdx.y, gridDim.y, S, tab, beam);
@@ -69,6 +73,8 @@ __global__ void k_cells_clear(uint32_t* __restrict__ totals, uint32_t n_totals, 
                               uint64_t n_out)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    chain_next();
+    chain_wait();
     for(uint64_t i = i0; i < n_totals; i += stride) totals[i] = 0u;
     for(uint64_t i = i0; i < n_bits; i += stride) bits[i] = 0u;
     for(uint64_t i = i0; i < n_cells; i += stride) cells[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -76,17 +82,26 @@ __global__ void k_cells_clear(uint32_t* __restrict__ totals, uint32_t n_totals, 
 }
 
 __global__ void __launch_bounds__(32 * kFilterWarps)
-k_cells_filter(const CellPing P, const uint32_t* __restrict__ nonempty)
+k_cells_filter(const CellPing ping, const uint32_t* nonempty)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    filter_tile<kFilterWarps>(P, blockIdx.x, blockIdx.y, reinterpret_cast<float4*>(s_raw), nonempty);
+    CellPing P = ping;
+    chain_next();
+    chain_wait();
+    P.cells = after_chain(P.cells);
+    P.out = after_chain(P.out);
+    filter_tile<kFilterWarps>(P, blockIdx.x, blockIdx.y, reinterpret_cast<float4*>(s_raw), after_chain(nonempty));
 }
 
 // One CTA per output row.
 __global__ void __launch_bounds__(256)
-k_pairs_join(const CellPing P, const uint32_t* __restrict__ nonempty)
+k_pairs_join(const CellPing ping, const uint32_t* nonempty)
 {
-    join_pairs(P, blockIdx.x, nonempty);
+    CellPing P = ping;
+    chain_next();
+    chain_wait();
+    P.cells = after_chain(P.cells);
+    join_pairs(P, blockIdx.x, after_chain(nonempty));
 }
 
 // 1D pings: the samples into the cells (or rows), then the taps.
@@ -98,10 +113,12 @@ k_cells_1d(const CellPing P, const BinParams p, const float* __restrict__ sample
 {
     extern __shared__ uint32_t s_bits[];
     const uint32_t words = (P.nR + 31) / 32;
+    chain_next();
     for(uint32_t i = threadIdx.x; i < words; i += kThreads1D) s_bits[i] = 0u;
     __syncthreads();
+    chain_wait();
     const uint64_t chunk = (n + gridDim.x - 1) / gridDim.x, begin = blockIdx.x * chunk;
-    accumulate_1d<ROWS>(P, p, samples, begin, min(begin + chunk, n), P.cells + (size_t)(blockIdx.x % P.replicas) * P.cp.cells,
+    accumulate_1d<ROWS>(P, p, after_chain(samples), begin, min(begin + chunk, n), P.cells + (size_t)(blockIdx.x % P.replicas) * P.cp.cells,
                         s_bits, copy);
     __syncthreads();
     for(uint32_t i = threadIdx.x; i < words; i += kThreads1D)
@@ -109,17 +126,24 @@ k_cells_1d(const CellPing P, const BinParams p, const float* __restrict__ sample
 }
 
 __global__ void __launch_bounds__(4 * kFilterRows1D)
-k_cells_filter_1d(const CellPing P, const uint32_t* __restrict__ nonempty)
+k_cells_filter_1d(const CellPing ping, const uint32_t* nonempty)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    filter_rows_1d<kFilterRows1D>(P, blockIdx.x, reinterpret_cast<float4*>(s_raw), nonempty);
+    CellPing P = ping;
+    chain_next();
+    chain_wait();
+    P.cells = after_chain(P.cells);
+    P.out = after_chain(P.out);
+    filter_rows_1d<kFilterRows1D>(P, blockIdx.x, reinterpret_cast<float4*>(s_raw), after_chain(nonempty));
 }
 
 // Rows of a 1D ping without a reference window.
-__global__ void k_rows_off_1d(const CellPing P, const uint32_t* __restrict__ nonempty)
+__global__ void k_rows_off_1d(const CellPing P, const uint32_t* nonempty)
 {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if(r < (int)P.nR && !row_on(nonempty, (int)P.nR, P.overlap, r)) P.out[r] = make_float2(0.f, 0.f);
+    chain_next();
+    chain_wait();
+    if(r < (int)P.nR && !row_on(after_chain(nonempty), (int)P.nR, P.overlap, r)) P.out[r] = make_float2(0.f, 0.f);
 }
 
 template <typename T>
@@ -430,9 +454,9 @@ static rtacx_status run_cells_1d(Context& c, const void* samples, uint64_t n, fl
     P.replicas = cell_replicas(c, n);
     const uint64_t cells = c.cell_rows ? 0 : (uint64_t)P.cp.cells * P.replicas;
     c.mark(1, false, stream);
-    k_cells_clear<<<(uint32_t)std::min<uint64_t>((cells + c.nR + 255) / 256, (uint64_t)c.sm_count * 8), 256, 0, stream>>>(
-        c.d_totals, 0, c.d_nonempty, (c.nR + 31) / 32, c.d_cells, cells, out, c.nR);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_chained(k_cells_clear, (uint32_t)std::min<uint64_t>((cells + c.nR + 255) / 256, (uint64_t)c.sm_count * 8),
+                                   256, 0, stream, c.d_totals, 0u, c.d_nonempty, (c.nR + 31) / 32, c.d_cells, cells, out,
+                                   (uint64_t)c.nR);
     c.mark(1, true, stream);
     c.sorted_cells_n = n;
     c.sorted_input_order = true;
@@ -442,14 +466,15 @@ static rtacx_status run_cells_1d(Context& c, const void* samples, uint64_t n, fl
         const uint32_t grid = (uint32_t)std::min<uint64_t>((n + kThreads1D - 1) / kThreads1D, (uint64_t)c.sm_count * 8);
         const size_t bits = (c.nR + 31) / 32 * sizeof(uint32_t);
         auto fn = c.cell_rows ? k_cells_1d<true> : k_cells_1d<false>;
-        fn<<<grid, kThreads1D, bits, stream>>>(P, c.bin, static_cast<const float*>(samples), n, c.d_nonempty, c.d_sorted);
-        if(c.cell_rows) k_rows_off_1d<<<(c.nR + 255) / 256, 256, 0, stream>>>(P, c.d_nonempty);
-        else k_cells_filter_1d<<<(c.nR + kFilterRows1D - 1) / kFilterRows1D, 4 * kFilterRows1D, filter_smem_1d(P.cp.taps, kFilterRows1D),
-                                 stream>>>(P, c.d_nonempty);
-        e = cudaGetLastError();
+        e = launch_chained(fn, grid, kThreads1D, bits, stream, P, c.bin, static_cast<const float*>(samples), n,
+                           c.d_nonempty, c.d_sorted);
+        if(e == cudaSuccess)
+            e = c.cell_rows ? launch_chained(k_rows_off_1d, (c.nR + 255) / 256, 256, 0, stream, P, c.d_nonempty)
+                            : launch_chained(k_cells_filter_1d, (c.nR + kFilterRows1D - 1) / kFilterRows1D, 4 * kFilterRows1D,
+                                             filter_smem_1d(P.cp.taps, kFilterRows1D), stream, P, c.d_nonempty);
         c.mark(5, true, stream);
     }
-    if(e != cudaSuccess) { c.error = std::string("cell form: ") + cudaGetErrorString(e); return RTACX_ERR_CUDA; }
+    if(e != cudaSuccess) { cudaGetLastError(); c.error = std::string("cell form: ") + cudaGetErrorString(e); return RTACX_ERR_CUDA; }
     return RTACX_OK;
 }
 
@@ -464,9 +489,9 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
     const uint32_t totals = bin.nBins + (bin.nBins + kScanBlock - 1) / kScanBlock;
     const uint64_t cells = (uint64_t)P.cp.cells * P.pitch, cells_out = c.cell_pairs && n ? 0 : (uint64_t)c.nR * c.nB;   // (the pairs' join writes every cell)
     c.mark(1, false, stream);
-    k_cells_clear<<<(uint32_t)std::min<uint64_t>((cells + 255) / 256, (uint64_t)c.sm_count * 8), 256, 0, stream>>>(
-        c.d_totals, totals, c.d_nonempty, (c.nR + 31) / 32, c.d_cells, cells, out, cells_out);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_chained(k_cells_clear, (uint32_t)std::min<uint64_t>((cells + 255) / 256, (uint64_t)c.sm_count * 8),
+                                   256, 0, stream, c.d_totals, totals, c.d_nonempty, (c.nR + 31) / 32, c.d_cells, cells,
+                                   out, cells_out);
     c.mark(1, true, stream);
     c.sorted_cells_n = 0;
     if(e == cudaSuccess && n) {
@@ -484,16 +509,16 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
         const uint32_t gx = (uint32_t)std::min<uint64_t>(ctas, (uint64_t)c.sm_count * 12u);
         const uint32_t gy = c.cell_shared ? (uint32_t)std::min<uint64_t>((uint64_t)P.windows,
                                                 std::max<uint64_t>(1, (uint64_t)c.sm_count * 3u / gx)) : 1u;
-        cells_fn(c.cell_bpl, c.cell_shared, c.cell_pairs)<<<dim3(gx, gy), kCellThreads,
-                                                            cells_smem(P.beam_axis.n, c.cell_pairs), stream>>>(
-            P, c.d_offsets + bin.nBins, unit);
+        e = launch_chained(cells_fn(c.cell_bpl, c.cell_shared, c.cell_pairs), dim3(gx, gy), kCellThreads,
+                           cells_smem(P.beam_axis.n, c.cell_pairs), stream, P, c.d_offsets + bin.nBins, unit);
         const dim3 fgrid(P.pitch / 32, (c.nR + kFilterWarps * kFilterRows - 1) / (kFilterWarps * kFilterRows));
-        if(c.cell_pairs) k_pairs_join<<<c.nR, std::min(256u, P.pitch), 0, stream>>>(P, c.d_nonempty);
-        else k_cells_filter<<<fgrid, 32 * kFilterWarps, filter_smem(P.cp.taps), stream>>>(P, c.d_nonempty);
-        e = cudaGetLastError();
+        if(e == cudaSuccess)
+            e = c.cell_pairs ? launch_chained(k_pairs_join, c.nR, std::min(256u, P.pitch), 0, stream, P, c.d_nonempty)
+                             : launch_chained(k_cells_filter, fgrid, 32 * kFilterWarps, filter_smem(P.cp.taps), stream, P,
+                                              c.d_nonempty);
         c.mark(5, true, stream);
     }
-    if(e != cudaSuccess) { c.error = std::string("cell form: ") + cudaGetErrorString(e); return RTACX_ERR_CUDA; }
+    if(e != cudaSuccess) { cudaGetLastError(); c.error = std::string("cell form: ") + cudaGetErrorString(e); return RTACX_ERR_CUDA; }
     return RTACX_OK;
 }
 

@@ -3,6 +3,7 @@
 
 #include <cstdint>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -48,6 +49,51 @@ inline cudaError_t raise_smem_limit(const void* fn, size_t bytes)
         e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if(e != cudaSuccess) cudaGetLastError();
     return e;
+}
+
+// Chained launches (programmatic dependent launch). A kernel launched with
+// launch_chained may start before the kernel ahead of it in the stream has
+// ended: it sets itself up (shared memory, tables written at configuration)
+// and calls chain_wait before it touches anything that a kernel writes, which
+// returns once everything ahead is complete and visible. Every kernel that is
+// launched so calls chain_next (the next kernel's blocks may be scheduled once
+// all of its own are) and chain_wait, in every thread, so the order of a chain
+// is that of the stream. Saves about 1.5 us of the 2 us between two kernels.
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// A pointer to what kernels ahead in the chain write, for use after
+// chain_wait: read-only loads (__restrict__, __ldg, __ldcg) are invariant to
+// the compiler, which may move them above the wait unless their address comes
+// from behind it.
+template <typename T>
+__device__ __forceinline__ T* after_chain(T* p)
+{
+    asm volatile("" : "+l"(p));
+    return p;
+}
+
+inline cudaLaunchConfig_t chained_config(dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                         cudaLaunchAttribute* attr)
+{
+    attr->id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr->val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args)
+{
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = chained_config(grid, block, smem, stream, &attr);
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
 // mbarrier helpers of the TMA pipelines (tensor-core GEMM, staged

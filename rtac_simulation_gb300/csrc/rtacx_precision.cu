@@ -126,6 +126,10 @@ k_prec_accumulate(const float* __restrict__ samples, uint64_t n, BinParams p, Gr
     extern __shared__ __align__(16) unsigned char s_raw[];
     uint32_t* s_bits = reinterpret_cast<uint32_t*>(s_raw);
     int hot_lo = 0, hot_len = 0;
+    chain_next();
+    chain_wait();
+    samples = after_chain(samples);
+    hot = after_chain(hot);
     if(hot) { const int2 h = *hot; hot_lo = h.x; hot_len = h.y; }
     const uint32_t rsel = (blockIdx.x + (threadIdx.x >> 5)) & (kHotReplicas - 1);   // by CTA and warp
     const uint32_t pitch = g.pitch;
@@ -221,10 +225,14 @@ k_prec_accumulate_staged(const float4* __restrict__ samples, uint64_t n, BinPara
                        "l"(stream_pol)
                      : "memory");
     };
+    chain_next();
     if(threadIdx.x == 0) {
         for(int i = 0; i < kStages; i++) mbar_init(smem_u32(&s_full[i]), 1);
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    chain_wait();
+    if(threadIdx.x == 0) {
         for(int i = 0; i < kStages; i++) {
             const uint64_t c = blockIdx.x + (uint64_t)i * gridDim.x;
             if(c < stages) issue(c, i);
@@ -351,6 +359,8 @@ __global__ void k_prec_clear(float4* __restrict__ G, uint64_t quads, uint32_t* _
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    chain_next();
+    chain_wait();
     for(uint64_t i = i0; i < quads; i += stride) G[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     for(uint64_t i = i0; i < words; i += stride) bits[i] = 0u;
 }
@@ -365,6 +375,9 @@ __global__ void k_hot_count(const float* __restrict__ samples, uint64_t n, BinPa
                             uint32_t* __restrict__ cnt)
 {
     const uint64_t m = (n + step - 1) / step;
+    chain_next();
+    chain_wait();
+    samples = after_chain(samples);
     for(uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s < m; s += (uint64_t)gridDim.x * blockDim.x) {
         const float4 rec = load_record(samples, s * step, p);
         int side;
@@ -409,6 +422,9 @@ __global__ void __launch_bounds__(kHotPickThreads) k_hot_pick(uint32_t* __restri
 {
     extern __shared__ uint32_t s_pre[];           // [nR + 1] inclusive prefix: s_pre[j + 1] = sum cnt[0..j]
     __shared__ unsigned long long s_best;
+    chain_next();
+    chain_wait();
+    cnt = after_chain(cnt);
     const uint32_t per = (nR + blockDim.x - 1) / blockDim.x;
     const uint32_t b0 = min(threadIdx.x * per, nR), b1 = min(b0 + per, nR);
     uint32_t sum = 0;
@@ -440,7 +456,11 @@ __global__ void __launch_bounds__(kHotPickThreads) k_hot_pick(uint32_t* __restri
 __global__ void k_hot_fold(const int2* __restrict__ hot, uint32_t pitch, const float4* __restrict__ rep,
                            float4* __restrict__ G)
 {
-    const int2 h = *hot;
+    chain_next();
+    chain_wait();
+    rep = after_chain(rep);
+    G = after_chain(G);
+    const int2 h = *after_chain(hot);
     const uint64_t total = (uint64_t)h.y * pitch;
     for(uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t row = i / pitch, k = i % pitch;
@@ -458,7 +478,9 @@ __global__ void k_hot_fold(const int2* __restrict__ hot, uint32_t pitch, const f
 // Zeroes the replicas of the hot rows (nothing when the interval is empty).
 __global__ void k_hot_zero(const int2* __restrict__ hot, uint32_t pitch, float4* __restrict__ rep)
 {
-    const uint64_t total = (uint64_t)hot->y * kHotReplicas * pitch;
+    chain_next();
+    chain_wait();
+    const uint64_t total = (uint64_t)after_chain(hot)->y * kHotReplicas * pitch;
     for(uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x)
         rep[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
@@ -532,6 +554,9 @@ __global__ void k_prec_split(const float4* __restrict__ G, uint32_t rows, uint32
 {
     const uint32_t m = blockIdx.y;                   // node rows 2m, 2m + 1
     const uint32_t k2 = blockIdx.x * blockDim.x + threadIdx.x;
+    chain_next();
+    chain_wait();
+    G = after_chain(G);
     if(2 * m >= rows || 2 * k2 >= cells) return;
     float2 a0, a1, b0, b1;                           // rows 2m, 2m + 1 at grid bearings 2 k2, 2 k2 + 1
     pair_values(G, m, 2 * k2, pitch, a0, b0);
@@ -561,6 +586,9 @@ k_prec_split_f16(const float4* __restrict__ G, uint32_t rows, uint32_t cells, ui
 {
     __shared__ float s_max[2][kSplitF16Threads / 32];
     const uint32_t m = blockIdx.x;                   // node rows 2m, 2m + 1
+    chain_next();
+    chain_wait();
+    G = after_chain(G);
     if(2 * m >= rows) return;
     const bool second = 2 * m + 1 < rows;
     float mx0 = 0.0f, mx1 = 0.0f;
@@ -640,6 +668,10 @@ k_prec_filter(const float2* __restrict__ C, uint32_t ldc2, uint32_t c_rows, size
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int par = warp >> 3, wl = warp & 7;                           // parity, warp within it
     const int r0 = blockIdx.y * kFiltRows, k0 = blockIdx.x * kFiltCols;
+    chain_next();
+    chain_wait();
+    C = after_chain(C);
+    nonempty = after_chain(nonempty);
     if(tid < 2 * kFiltRows) {
         const int p = tid / kFiltRows, m = tid % kFiltRows;
         const int r = 2 * (r0 + m) + p;
@@ -1172,8 +1204,7 @@ rtacx_status precision_begin(Context& ctx, cudaStream_t stream)
 {
     const uint64_t quads = grid_quads(ctx.grid_rows, ctx.grid.pitch);
     const uint32_t blocks = (uint32_t)std::min<uint64_t>((quads + 255) / 256, (uint64_t)ctx.sm_count * 32);
-    k_prec_clear<<<blocks, 256, 0, stream>>>(ctx.d_G, quads, ctx.d_flags, (ctx.nR + 31) / 32);
-    RTACX_CUDA(cudaGetLastError());
+    RTACX_CUDA(launch_chained(k_prec_clear, blocks, 256, 0, stream, ctx.d_G, quads, ctx.d_flags, (ctx.nR + 31) / 32));
     return RTACX_OK;
 }
 
@@ -1190,16 +1221,16 @@ rtacx_status precision_accumulate(Context& ctx, const void* samples, uint64_t n,
             const uint32_t blocks = (uint32_t)std::min<uint64_t>(stages, (uint64_t)ctx.sm_count * ctx.acc_staged_blocks[m]);
             void* args[] = {(void*)&samples, (void*)&n, (void*)&ctx.bin, (void*)&ctx.grid, (void*)&ctx.d_G,
                             (void*)&ctx.d_flags, (void*)&ctx.d_err, (void*)&ctx.diag_drop_stage};
-            RTACX_CUDA(cudaLaunchKernel(accumulate_staged_kernel(m), dim3(blocks), dim3(kStagedThreads), args,
-                                        ctx.acc_staged_smem, stream));
+            cudaLaunchAttribute attr;
+            const cudaLaunchConfig_t cfg = chained_config(blocks, kStagedThreads, ctx.acc_staged_smem, stream, &attr);
+            RTACX_CUDA(cudaLaunchKernelExC(&cfg, accumulate_staged_kernel(m), args));
             return RTACX_OK;
         }
     }
     const uint32_t blocks = (uint32_t)std::min<uint64_t>(want, (uint64_t)ctx.sm_count * ctx.acc_blocks_per_sm);
-    k_prec_accumulate<<<blocks, kAccThreads, ctx.acc_smem, stream>>>(static_cast<const float*>(samples), n, ctx.bin,
-                                                                     ctx.grid, ctx.d_G, ctx.d_flags,
-                                                                     ctx.prec_hot ? ctx.d_hot : nullptr, ctx.d_rep);
-    RTACX_CUDA(cudaGetLastError());
+    RTACX_CUDA(launch_chained(k_prec_accumulate, blocks, kAccThreads, ctx.acc_smem, stream,
+                              static_cast<const float*>(samples), n, ctx.bin, ctx.grid, ctx.d_G, ctx.d_flags,
+                              ctx.prec_hot ? ctx.d_hot : nullptr, ctx.d_rep));
     return RTACX_OK;
 }
 
@@ -1212,15 +1243,12 @@ rtacx_status precision_hot_scan(Context& ctx, const void* samples, uint64_t n, c
     const uint64_t m = n ? (n + step - 1) / step : 0;
     if(m) {
         const uint32_t blocks = (uint32_t)std::min<uint64_t>((m + 255) / 256, (uint64_t)ctx.sm_count * 4);
-        k_hot_count<<<blocks, 256, 0, stream>>>(static_cast<const float*>(samples), n, ctx.bin, ctx.grid, step,
-                                                ctx.d_hotcnt);
-        RTACX_CUDA(cudaGetLastError());
+        RTACX_CUDA(launch_chained(k_hot_count, blocks, 256, 0, stream, static_cast<const float*>(samples), n, ctx.bin,
+                                  ctx.grid, step, ctx.d_hotcnt));
     }
-    k_hot_pick<<<1, kHotPickThreads, (ctx.grid_rows + 1) * sizeof(uint32_t), stream>>>(ctx.d_hotcnt, ctx.grid_rows,
-                                                                                        ctx.d_hot);
-    RTACX_CUDA(cudaGetLastError());
-    k_hot_zero<<<ctx.sm_count * 4, 256, 0, stream>>>(ctx.d_hot, ctx.grid.pitch, ctx.d_rep);
-    RTACX_CUDA(cudaGetLastError());
+    RTACX_CUDA(launch_chained(k_hot_pick, 1, kHotPickThreads, (ctx.grid_rows + 1) * sizeof(uint32_t), stream, ctx.d_hotcnt,
+                              ctx.grid_rows, ctx.d_hot));
+    RTACX_CUDA(launch_chained(k_hot_zero, ctx.sm_count * 4, 256, 0, stream, ctx.d_hot, ctx.grid.pitch, ctx.d_rep));
     return RTACX_OK;
 }
 
@@ -1244,19 +1272,18 @@ rtacx_status precision_finish(Context& ctx, float* out, cudaStream_t stream)
 {
     const uint32_t nR = ctx.nR, nB = ctx.nB, cells = ctx.grid.cells;
     if(ctx.prec_hot) {
-        k_hot_fold<<<ctx.sm_count * 4, 256, 0, stream>>>(ctx.d_hot, ctx.grid.pitch, ctx.d_rep, ctx.d_G);
-        RTACX_CUDA(cudaGetLastError());
+        RTACX_CUDA(launch_chained(k_hot_fold, ctx.sm_count * 4, 256, 0, stream, ctx.d_hot, ctx.grid.pitch, ctx.d_rep, ctx.d_G));
     }
     ctx.mark(1, false, stream);
     if(!ctx.prec_f16) {
         const dim3 sgrid((cells / 2 + 255) / 256, (ctx.grid_rows + 1) / 2);
-        k_prec_split<<<sgrid, 256, 0, stream>>>(ctx.d_G, ctx.grid_rows, cells, ctx.grid.pitch, ctx.Kp, ctx.d_A);
+        RTACX_CUDA(launch_chained(k_prec_split, sgrid, 256, 0, stream, ctx.d_G, ctx.grid_rows, cells, ctx.grid.pitch,
+                                  ctx.Kp, ctx.d_A));
     }
     else {
-        k_prec_split_f16<<<(ctx.grid_rows + 1) / 2, kSplitF16Threads, 0, stream>>>(ctx.d_G, ctx.grid_rows, cells, ctx.grid.pitch,
-                                                                         ctx.Kp, ctx.d_A, ctx.d_row_scale);
+        RTACX_CUDA(launch_chained(k_prec_split_f16, (ctx.grid_rows + 1) / 2, kSplitF16Threads, 0, stream, ctx.d_G,
+                                  ctx.grid_rows, cells, ctx.grid.pitch, ctx.Kp, ctx.d_A, ctx.d_row_scale));
     }
-    RTACX_CUDA(cudaGetLastError());
     ctx.mark(1, true, stream);
     ctx.mark(3, false, stream);
     rtacx_status st = gemm_tn(ctx.error, ctx.d_A, ctx.d_B, ctx.d_C, (int)ctx.Mpad, (int)ctx.Npad, (int)ctx.Kp,
@@ -1267,10 +1294,10 @@ rtacx_status precision_finish(Context& ctx, float* out, cudaStream_t stream)
     ctx.mark(2, false, stream);
     const dim3 fgrid((nB + kFiltCols - 1) / kFiltCols, (range_nodes(nR) + kFiltRows - 1) / kFiltRows);
     auto filter = ctx.ksplit == 2 ? k_prec_filter<2> : k_prec_filter<1>;
-    filter<<<fgrid, kFiltThreads, filter_smem_bytes(ctx.taps), stream>>>(
-        reinterpret_cast<const float2*>(ctx.d_C), ctx.Npad / 2, ctx.grid_rows, (size_t)ctx.Mpad * ctx.Npad / 2,
-        ctx.d_flags, ctx.overlap, ctx.d_taps, ctx.taps, nR, nB, reinterpret_cast<float2*>(out));
-    RTACX_CUDA(cudaGetLastError());
+    RTACX_CUDA(launch_chained(filter, fgrid, kFiltThreads, filter_smem_bytes(ctx.taps), stream,
+                              reinterpret_cast<const float2*>(ctx.d_C), ctx.Npad / 2, ctx.grid_rows,
+                              (size_t)ctx.Mpad * ctx.Npad / 2, ctx.d_flags, ctx.overlap, ctx.d_taps, ctx.taps, nR, nB,
+                              reinterpret_cast<float2*>(out)));
     ctx.mark(2, true, stream);
     return RTACX_OK;
 }

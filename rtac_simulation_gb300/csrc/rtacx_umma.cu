@@ -123,10 +123,13 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    chain_next();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    chain_wait();
+    row_scale = after_chain(row_scale);
 
     if(warp == 0 && lane == 0) {
         // TMA producer.
@@ -306,16 +309,11 @@ rtacx_status gemm_tn(std::string& error, const void* A, const void* B, float* C,
         attr_done.fetch_or(1ull << dev);
     }
     dim3 grid(N / bn, M / BM, ksplit);
-    if(wide) {
-        if(f16) k_gemm_tn<true, TileWide><<<grid, kThreads, TileWide::SMEM_BYTES, stream>>>(ma, mb, C, M, N, K, ldc, row_scale, col_scale, err);
-        else k_gemm_tn<false, TileWide><<<grid, kThreads, TileWide::SMEM_BYTES, stream>>>(ma, mb, C, M, N, K, ldc, row_scale, col_scale, err);
-    }
-    else {
-        if(f16) k_gemm_tn<true, TileNarrow><<<grid, kThreads, TileNarrow::SMEM_BYTES, stream>>>(ma, mb, C, M, N, K, ldc, row_scale, col_scale, err);
-        else k_gemm_tn<false, TileNarrow><<<grid, kThreads, TileNarrow::SMEM_BYTES, stream>>>(ma, mb, C, M, N, K, ldc, row_scale, col_scale, err);
-    }
-    const cudaError_t e = cudaGetLastError();
-    if(e != cudaSuccess) { error = std::string("k_gemm_tn: ") + cudaGetErrorString(e); return RTACX_ERR_CUDA; }
+    auto fn = wide ? (f16 ? k_gemm_tn<true, TileWide> : k_gemm_tn<false, TileWide>)
+                   : (f16 ? k_gemm_tn<true, TileNarrow> : k_gemm_tn<false, TileNarrow>);
+    const cudaError_t e = launch_chained(fn, grid, kThreads, wide ? TileWide::SMEM_BYTES : TileNarrow::SMEM_BYTES, stream,
+                                         ma, mb, C, M, N, K, ldc, row_scale, col_scale, err);
+    if(e != cudaSuccess) { cudaGetLastError(); error = std::string("k_gemm_tn: ") + cudaGetErrorString(e); return RTACX_ERR_CUDA; }
     return RTACX_OK;
 }
 

@@ -202,3 +202,37 @@ def test_batch_of_every_form_matches_fp64_oracle(oracle, autotune):
     one = gpu_reduce(ctxs[0], pings[0].samples, pings[0].out_shape)
     assert rel_l2(one, oracle.reduce(pings[0].samples, pings[0].sensor)) <= TOL
     batch.close()
+
+
+@pytest.mark.parametrize("maker", [
+    lambda: ping(20001, 257, 200, 17, False), lambda: ping(5000, 300, 128, 9, True),
+    lambda: ping_1d(5000, 257, 17), lambda: ping_1d(1000, 64, 2, 40, 2.0),
+])
+def test_chained_pings_read_what_the_kernel_ahead_wrote(maker):
+    """Samples written by a kernel right before the ping, two different ones in
+    turn through the same context, sample buffer and ping, without a pause."""
+    wk = maker()
+    ctx = make_context(wk)
+    stream = torch.cuda.current_stream()
+    a = torch.from_numpy(wk.samples).cuda()
+    b = a.flip(0).contiguous()
+    b[:, :2] *= -0.5
+    b[:, 2] = b[:, 2] * 0.75 + 0.5
+    buf = torch.empty_like(a)
+    out = torch.empty(wk.out_shape + (2,), device="cuda")
+    want = []
+    for src in (a, b):
+        torch.mul(src, 1.0, out=buf)
+        torch.cuda.synchronize()
+        ctx.reduce(buf, wk.n, out, stream=stream)
+        torch.cuda.synchronize()
+        want.append(out.clone())
+    got = []
+    for _ in range(40):
+        for src in (a, b):
+            torch.mul(src, 1.0, out=buf)
+            ctx.reduce(buf, wk.n, out, stream=stream)
+            got.append(out.clone())
+    torch.cuda.synchronize()
+    for i, g in enumerate(got):
+        assert float((g - want[i % 2]).norm() / want[i % 2].norm()) <= 2e-6, i
