@@ -174,27 +174,29 @@ k_prec_accumulate(const float* __restrict__ samples, uint64_t n, BinParams p, Gr
 
 // The accumulation for the common case: 16-byte aligned records, no hot
 // range, and the echo model kEcho fixed at compile time. The records reach
-// shared memory by bulk copies (cp.async.bulk, the TMA engine) into a ring of
-// kStages stages of kStageRecs records, so the bytes in flight per SM depend
-// neither on registers nor on how long the threads compute. Each thread
-// computes the key, grid coordinates and weighted values of its records of a
-// stage without branches (invalid and tail records only clear a predicate),
-// then issues the bitmap bits and the reductions; the results are those of
-// k_prec_accumulate. One persistent CTA takes stages c = blockIdx.x,
-// blockIdx.x + gridDim.x, ...; thread 0 issues the copy of the stage kStages
-// ahead as soon as every thread has read the stage it refills. Each wait is
-// bounded (kAccWaitCycles); a timeout sets kErrAccumulateTimeout in the error
-// word, the CTA stops, and thread 0 waits (bounded again) for its copies
-// still in flight before the CTA exits.
-constexpr int kStageRecs = 1024;                 // 16 KB of records per stage
+// shared memory by bulk copies (cp.async.bulk, the TMA engine): every warp has
+// its own ring of kStages stages of kStageRecs records, so that no barrier
+// of the CTA is in the loop and the bytes in flight per SM depend neither on
+// registers nor on how long the threads compute. Each thread computes the
+// key, grid coordinates and weighted values of its records of a stage without
+// branches (invalid and tail records only clear a predicate), then issues the
+// bitmap bits and the reductions; the results are those of k_prec_accumulate.
+// Warp w of the grid takes stages w, w + warps, ...; its lane 0 issues the
+// copy of the stage kStages ahead as soon as every lane has read the stage it
+// refills. Each wait is bounded (kAccWaitCycles); a timeout sets
+// kErrAccumulateTimeout in the error word, the CTA's warps stop at their next
+// stage, and each waits (bounded again) for its copies still in flight.
+constexpr int kStageRecs = 32;                   // 512 B of records per stage: one per lane
 constexpr int kStages = 4;
-constexpr int kStagedThreads = 512;
-constexpr int kStagedPerThread = kStageRecs / kStagedThreads;
+constexpr int kStagedThreads = 512, kStagedWarps = kStagedThreads / 32;
+constexpr int kStagedPerThread = kStageRecs / 32;
+constexpr int kDiagStageRecs = 1024;             // records of a stage of rtacx_diag_drop_accumulation_stage
 constexpr long long kAccWaitCycles = 2000000000ll;   // about one second
+constexpr uint32_t kNoEntry = 0xFFFFFFFFu;
 
 size_t staged_smem_bytes(uint32_t nR)
 {
-    return (size_t)kStages * kStageRecs * sizeof(float4) + (size_t)((nR + 31) / 32) * sizeof(uint32_t);
+    return (size_t)kStagedWarps * kStages * kStageRecs * sizeof(float4) + (size_t)((nR + 31) / 32) * sizeof(uint32_t);
 }
 
 template <uint32_t kEcho>
@@ -204,20 +206,22 @@ k_prec_accumulate_staged(const float4* __restrict__ samples, uint64_t n, BinPara
                          uint32_t drop_stage)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    __shared__ __align__(8) uint64_t s_full[kStages];
+    __shared__ __align__(8) uint64_t s_full[kStagedWarps][kStages];
     __shared__ int s_abort;
-    float4* s_ring = reinterpret_cast<float4*>(s_raw);
-    uint32_t* s_bits = reinterpret_cast<uint32_t*>(s_ring + kStages * kStageRecs);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float4* s_ring = reinterpret_cast<float4*>(s_raw) + warp * (kStages * kStageRecs);
+    uint32_t* s_bits = reinterpret_cast<uint32_t*>(reinterpret_cast<float4*>(s_raw) + kStagedWarps * kStages * kStageRecs);
     const uint32_t words = (p.key.nR + 31) / 32;
     const uint64_t stages = (n + kStageRecs - 1) / kStageRecs;
+    const uint64_t stride = (uint64_t)gridDim.x * kStagedWarps, c0 = (uint64_t)blockIdx.x * kStagedWarps + warp;
     const uint32_t pitch = g.pitch;
-    const uint64_t stream_pol = policy_evict_first(), keep = policy_evict_last();
+    const uint64_t stream_pol = policy_evict_first(), keep_pol = policy_evict_last();
     auto issue = [&](uint64_t c, int slot) {
-        if(c == drop_stage) return;      // failure-path test: this stage's copy never comes
+        if(c / (kDiagStageRecs / kStageRecs) == drop_stage) return;   // failure-path test: this copy never comes
         const uint64_t first = c * kStageRecs;
         const uint64_t left = n - first;
         const uint32_t bytes = (uint32_t)(left < (uint64_t)kStageRecs ? left : (uint64_t)kStageRecs) * (uint32_t)sizeof(float4);
-        const uint32_t bar = smem_u32(&s_full[slot]);
+        const uint32_t bar = smem_u32(&s_full[warp][slot]);
         mbar_expect_tx(bar, bytes);
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
                      " [%0], [%1], %2, [%3], %4;"
@@ -226,97 +230,92 @@ k_prec_accumulate_staged(const float4* __restrict__ samples, uint64_t n, BinPara
                      : "memory");
     };
     chain_next();
-    if(threadIdx.x == 0) {
-        for(int i = 0; i < kStages; i++) mbar_init(smem_u32(&s_full[i]), 1);
-        s_abort = 0;
+    if(lane == 0) {
+        for(int i = 0; i < kStages; i++) mbar_init(smem_u32(&s_full[warp][i]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    chain_wait();
-    if(threadIdx.x == 0) {
-        for(int i = 0; i < kStages; i++) {
-            const uint64_t c = blockIdx.x + (uint64_t)i * gridDim.x;
-            if(c < stages) issue(c, i);
-        }
-    }
+    if(threadIdx.x == 0) s_abort = 0;
     for(uint32_t i = threadIdx.x; i < words; i += blockDim.x) s_bits[i] = 0u;
+    chain_wait();
     __syncthreads();
+    if(lane == 0) {
+        for(int i = 0; i < kStages; i++)
+            if(c0 + (uint64_t)i * stride < stages) issue(c0 + (uint64_t)i * stride, i);
+    }
     int it = 0;
     bool aborted = false;
-    for(uint64_t c = blockIdx.x; c < stages; c += gridDim.x, it++) {
+    for(uint64_t c = c0; c < stages; c += stride, it++) {
         const int slot = it % kStages;
-        const bool ready = mbar_wait_bounded(smem_u32(&s_full[slot]), (uint32_t)(it / kStages) & 1u, &s_abort,
-                                             kAccWaitCycles);
+        aborted = *(volatile int*)&s_abort != 0 ||
+                  !mbar_wait_bounded(smem_u32(&s_full[warp][slot]), (uint32_t)(it / kStages) & 1u, &s_abort, kAccWaitCycles);
+        if(__any_sync(0xffffffffu, aborted)) { aborted = true; break; }
         const uint64_t left = n - c * kStageRecs;
         const uint32_t count = left < (uint64_t)kStageRecs ? (uint32_t)left : (uint32_t)kStageRecs;
         uint32_t key[kStagedPerThread];
-        int row[kStagedPerThread], cell[kStagedPerThread];
+        uint32_t at0[kStagedPerThread], at1[kStagedPerThread];   // grid entries of the sample's two nodes (kNoEntry: none)
         float wgt[kStagedPerThread];
         float4 add[kStagedPerThread];
 #pragma unroll
         for(int u = 0; u < kStagedPerThread; u++) {
-            const uint32_t idx = threadIdx.x + (uint32_t)u * kStagedThreads;
-            const float4 rec = s_ring[slot * kStageRecs + min(idx, (uint32_t)kStageRecs - 1u)];
-            const uint32_t k = range_key_select(p.key, rec.z);
-            const bool live = ready && idx < count && k != kOutOfRange;
+            const uint32_t idx = (uint32_t)lane + (uint32_t)u * 32u;
+            const float4 rec = s_ring[slot * kStageRecs + idx];
+            int side;
+            const uint32_t k = range_key(p.key, rec.z, side);
+            const bool live = idx < count && k != kOutOfRange;
             key[u] = live ? k : kOutOfRange;
             int jg, q;
             float alpha, w;
             const bool ok = grid_coords(g, rec.z, rec.w, jg, alpha, q, w) && live;
             const float2 v = apply_echo(p, make_float2(rec.x, rec.y), rec.z, kEcho);
-            row[u] = ok ? jg : -1;
-            cell[u] = q;
+            const uint32_t e = ((uint32_t)(jg >> 1) * pitch + (uint32_t)q) * 2u;
+            at0[u] = ok ? e + (uint32_t)(jg & 1) : kNoEntry;
+            at1[u] = ok ? e + ((jg & 1) ? 2u * pitch : 1u) : kNoEntry;
             wgt[u] = w;
             const float a0 = 1.0f - alpha;
             add[u] = make_float4(a0 * v.x, a0 * v.y, alpha * v.x, alpha * v.y);
         }
-        // Every thread has read the slot: refill it kStages stages ahead.
-        aborted = __syncthreads_or(!ready) != 0;
-        if(threadIdx.x == 0 && !aborted) {
+        // Every lane has read the slot: refill it kStages stages ahead.
+        __syncwarp();
+        if(lane == 0) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            const uint64_t next = c + (uint64_t)kStages * gridDim.x;
+            const uint64_t next = c + (uint64_t)kStages * stride;
             if(next < stages) issue(next, slot);
         }
         // Lanes 2k and 2k + 1 deposit together: first the even lane's
         // sample (row jg from the even lane, jg + 1 from the odd one), then
         // the odd lane's, so each reduction instruction sends a sample's two
-        // rows of an interval as one sector when jg is even.
-        const bool odd = (threadIdx.x & 1u) != 0u;
+        // rows of an interval as one sector when jg is even. Each lane keeps
+        // one node's share of its own sample and trades the other's.
+        const bool odd = (lane & 1) != 0;
 #pragma unroll
         for(int u = 0; u < kStagedPerThread; u++) {
-            if(key[u] != kOutOfRange) atomicOr(&s_bits[key[u] >> 5], 1u << (key[u] & 31));
-            const int row_p = __shfl_xor_sync(0xffffffffu, row[u], 1);
-            const int cell_p = __shfl_xor_sync(0xffffffffu, cell[u], 1);
-            const float wgt_p = __shfl_xor_sync(0xffffffffu, wgt[u], 1);
-            float4 add_p;
-            add_p.x = __shfl_xor_sync(0xffffffffu, add[u].x, 1);
-            add_p.y = __shfl_xor_sync(0xffffffffu, add[u].y, 1);
-            add_p.z = __shfl_xor_sync(0xffffffffu, add[u].z, 1);
-            add_p.w = __shfl_xor_sync(0xffffffffu, add[u].w, 1);
-#pragma unroll
-            for(int h = 0; h < 2; h++) {
-                // h = 0: the even lane's sample; h = 1: the odd lane's.
-                const bool mine = odd == (h == 1);
-                const int r = mine ? row[u] : row_p;
-                if(r >= 0) {
-                    const float4 a = mine ? add[u] : add_p;
-                    deposit(G + grid_at(r + (odd ? 1 : 0), mine ? cell[u] : cell_p, pitch), mine ? wgt[u] : wgt_p,
-                            odd ? make_float2(a.z, a.w) : make_float2(a.x, a.y), keep);
-                }
-            }
+            // (Set once the first samples are in: a read instead of an atomic.)
+            if(key[u] != kOutOfRange && !(s_bits[key[u] >> 5] >> (key[u] & 31) & 1u))
+                atomicOr(&s_bits[key[u] >> 5], 1u << (key[u] & 31));
+            const uint32_t keep = odd ? at1[u] : at0[u];
+            const float2 keep_v = odd ? make_float2(add[u].z, add[u].w) : make_float2(add[u].x, add[u].y);
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? at0[u] : at1[u], 1);
+            float2 got_v;
+            got_v.x = __shfl_xor_sync(0xffffffffu, odd ? add[u].x : add[u].z, 1);
+            got_v.y = __shfl_xor_sync(0xffffffffu, odd ? add[u].y : add[u].w, 1);
+            const float got_w = __shfl_xor_sync(0xffffffffu, wgt[u], 1);
+            const uint32_t first = odd ? got : keep, second = odd ? keep : got;
+            if(first != kNoEntry) deposit(G + first, odd ? got_w : wgt[u], odd ? got_v : keep_v, keep_pol);
+            if(second != kNoEntry) deposit(G + second, odd ? wgt[u] : got_w, odd ? keep_v : got_v, keep_pol);
         }
-        if(aborted) break;
     }
-    if(aborted && threadIdx.x == 0) {
+    if(aborted && lane == 0) {
         atomicOr(err, kErrAccumulateTimeout);
+        s_abort = 1;
         // Let the copies still in flight land before the CTA's shared memory
         // is released: those of iterations it .. it + kStages - 1 (the refill
         // of the aborted iteration was not issued). Each wait is bounded on
         // its own; a copy that was never issued (or never lands) costs one
         // more timeout.
         for(int i = it; i < it + kStages; i++) {
-            if(blockIdx.x + (uint64_t)i * gridDim.x >= stages) break;
+            if(c0 + (uint64_t)i * stride >= stages) break;
             volatile int keep_waiting = 0;
-            mbar_wait_bounded(smem_u32(&s_full[i % kStages]), (uint32_t)(i / kStages) & 1u, &keep_waiting,
+            mbar_wait_bounded(smem_u32(&s_full[warp][i % kStages]), (uint32_t)(i / kStages) & 1u, &keep_waiting,
                               kAccWaitCycles);
         }
     }
@@ -1218,7 +1217,8 @@ rtacx_status precision_accumulate(Context& ctx, const void* samples, uint64_t n,
         const int m = accumulate_echo_model(ctx.bin.echo_flags);
         if(ctx.acc_staged_blocks[m] > 0) {
             const uint64_t stages = (n + kStageRecs - 1) / kStageRecs;
-            const uint32_t blocks = (uint32_t)std::min<uint64_t>(stages, (uint64_t)ctx.sm_count * ctx.acc_staged_blocks[m]);
+            const uint32_t blocks = (uint32_t)std::min<uint64_t>((stages + kStagedWarps - 1) / kStagedWarps,
+                                                                 (uint64_t)ctx.sm_count * ctx.acc_staged_blocks[m]);
             void* args[] = {(void*)&samples, (void*)&n, (void*)&ctx.bin, (void*)&ctx.grid, (void*)&ctx.d_G,
                             (void*)&ctx.d_flags, (void*)&ctx.d_err, (void*)&ctx.diag_drop_stage};
             cudaLaunchAttribute attr;
