@@ -248,7 +248,7 @@ typedef struct {
 } rtacx_precision_desc;
 /* Contract in FP16 instead of BF16: each row of the filtered grid and each
  * column of the directivity is scaled by a power of two to [2^14, 2^15)
- * before the fp16 [hi | hi | lo] x [hi | lo | hi] split (11-bit halves,
+ * before the fp16 hi + lo split (11-bit halves,
  * products exact in the FP32 accumulator) and the scales are undone exactly
  * in the GEMM epilogue. */
 #define RTACX_PRECISION_FP16_ROWSCALE 1u

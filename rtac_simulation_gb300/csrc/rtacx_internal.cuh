@@ -6,6 +6,7 @@
 #include <utility>
 #include <vector>
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include "../../include/rtacx.h"
@@ -505,6 +506,13 @@ struct FusedBatch {
     unsigned long long wait_ns;                  // bound of one barrier wait
 };
 
+// Plan of the precision form's contraction (plan_gemm_split).
+struct GemmPlan {
+    CUtensorMap ma, mb;
+    int bn = 0, ksplit = 1;             // tile width; K parts (partial products summed by the filter)
+    std::vector<uint16_t> lists;        // [column tiles][1 + blocks of K]: count, then the blocks where B is not zero
+};
+
 // Scratch and configuration owned by one context.
 struct Context {
     int device = 0;
@@ -598,8 +606,9 @@ struct Context {
     // Precision form (rtacx_configure_precision).
     bool prec_configured = false;
     uint32_t taps = 0, tap_center = 0;   // taps per output-row parity, index of node offset 0
-    uint32_t Mpad = 0, Npad = 0, Kp = 0;
-    uint32_t ksplit = 1;                // K parts of the contraction (partial products summed by the filter)
+    uint32_t Mpad = 0, Npad = 0, Kp = 0;    // contraction sizes; Kp: one half (hi or lo) of the operands' rows
+    GemmPlan gemm;
+    uint16_t* d_blocks = nullptr;       // gemm.lists
     GridParams grid{};                  // range nodes (two output bins apart) and uniform bearing grid
     uint32_t grid_rows = 0;             // (nR - 1) / 2 + 1 + taps + 1 node rows of the binned grid
     float4* d_G = nullptr;              // [grid_rows][grid.cells] bearing intervals: {left, right} shares (complex)
@@ -607,9 +616,9 @@ struct Context {
     uint32_t acc_staged_blocks[6] = {}; // resident CTAs per SM of each staged accumulation (0: not used)
     size_t acc_staged_smem = 0;
     uint32_t diag_drop_stage = 0xFFFFFFFFu; // failure-path test: stage whose copy the staged accumulation skips
-    uint16_t* d_A = nullptr;            // [Mpad][Kp] bf16 [hi | hi | lo] split of the binned grid
-    uint16_t* d_B = nullptr;            // [Npad][Kp] bf16 [hi | lo | hi] split of the directivity
-    float* d_C = nullptr;               // [ksplit][Mpad][Npad] GEMM partial outputs: the grid contracted over bearings
+    uint16_t* d_A = nullptr;            // [Mpad][2 Kp] bf16 [hi | lo] split of the binned grid
+    uint16_t* d_B = nullptr;            // [Npad][2 Kp] bf16 [hi | lo] split of the directivity
+    float* d_C = nullptr;               // [gemm.ksplit][Mpad][Npad] GEMM partial outputs: the grid contracted over bearings
     float2* d_taps = nullptr;           // [2][taps] range taps per output-row parity at node offsets t - tap_center
     // FP16 per-row-scaled contraction (RTACX_PRECISION_FP16_ROWSCALE): A and B
     // hold fp16 splits instead of bf16 ones.
@@ -703,13 +712,11 @@ rtacx_status precision_finish(Context& ctx, float* out, cudaStream_t stream);
 void free_streaming(Context& ctx);
 void free_precision(Context& ctx);
 
-// Tensor-core GEMM (rtacx_umma.cu): C = row_scale * col_scale * (A * B^T),
-// K-major operands, both bf16 or both fp16 (f16); scales optional; ksplit
-// partial products at C + z M ldc.
-rtacx_status gemm_tn(std::string& error, const void* A, const void* B, float* C, int M, int N, int K, int ldc,
-                     cudaStream_t stream, uint32_t* err, bool f16, const float* row_scale, const float* col_scale,
-                     int ksplit);
-size_t gemm_smem_bytes();
+// Split contraction of the precision form (rtacx_umma.cu).
+rtacx_status plan_gemm_split(std::string& error, GemmPlan& g, const void* A, const void* B, const uint16_t* b, int M, int N,
+                             int K, bool f16, int sm_count);
+rtacx_status gemm_split(std::string& error, const GemmPlan& g, const uint16_t* d_blocks, float* C, int M, int N, int K,
+                        cudaStream_t stream, uint32_t* err, bool f16, const float* row_scale, const float* col_scale);
 
 } // namespace rtacx
 

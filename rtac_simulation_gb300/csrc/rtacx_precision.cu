@@ -17,7 +17,7 @@
 //                      when its nodes share a pair. No sort.
 //   k_prec_split       grid bearing q of a node = left share of interval q +
 //                      right share of interval q - 1, as the bf16 A operand
-//                      [hi | hi | lo] of the three-term split product
+//                      [hi | lo] of the three-term split product
 //                      (k_prec_split_f16: fp16 with a power-of-two scale per
 //                      row).
 //   gemm_tn            C = A x B^T on tcgen05 (rtacx_umma.cu), B the
@@ -527,12 +527,12 @@ __device__ __forceinline__ void pair_values(const float4* __restrict__ G, uint32
     v1 = make_float2(a1.x + b1.z, a1.y + b1.w);
 }
 
-// The A operand of the three-term split product: node row r (cells complex
-// values) becomes A row r = [hi(Re) | hi(Im) | hi(Re) | hi(Im) | lo(Re) |
-// lo(Im)], each block `cells` wide, lo = bf16(x - hi). One thread per pair of
-// grid bearings of a pair of node rows: their entries are read once (six
-// 16-byte loads), twelve 4-byte stores.
-__device__ __forceinline__ void split_store(uint16_t* row, uint32_t cells, float2 n0, float2 n1)
+// The A operand of the split product: node row r (cells complex values)
+// becomes A row r = [hi(Re) | hi(Im) | .. | lo(Re) | lo(Im) | ..], the halves
+// Kp wide, lo = bf16(x - hi). One thread per pair of grid bearings of a pair
+// of node rows: their entries are read once (six 16-byte loads), eight 4-byte
+// stores.
+__device__ __forceinline__ void split_store(uint16_t* row, uint32_t cells, uint32_t Kp, float2 n0, float2 n1)
 {
     const float x[4] = {n0.x, n0.y, n1.x, n1.y};     // re0, im0, re1, im1
     uint16_t h[4], l[4];
@@ -542,10 +542,8 @@ __device__ __forceinline__ void split_store(uint16_t* row, uint32_t cells, float
     const uint32_t lr = (uint32_t)l[0] | ((uint32_t)l[2] << 16), li = (uint32_t)l[1] | ((uint32_t)l[3] << 16);
     *reinterpret_cast<uint32_t*>(row) = hr;
     *reinterpret_cast<uint32_t*>(row + cells) = hi;
-    *reinterpret_cast<uint32_t*>(row + 2 * cells) = hr;
-    *reinterpret_cast<uint32_t*>(row + 3 * cells) = hi;
-    *reinterpret_cast<uint32_t*>(row + 4 * cells) = lr;
-    *reinterpret_cast<uint32_t*>(row + 5 * cells) = li;
+    *reinterpret_cast<uint32_t*>(row + Kp) = lr;
+    *reinterpret_cast<uint32_t*>(row + Kp + cells) = li;
 }
 
 __global__ void k_prec_split(const float4* __restrict__ G, uint32_t rows, uint32_t cells, uint32_t pitch, uint32_t Kp,
@@ -560,13 +558,13 @@ __global__ void k_prec_split(const float4* __restrict__ G, uint32_t rows, uint32
     float2 a0, a1, b0, b1;                           // rows 2m, 2m + 1 at grid bearings 2 k2, 2 k2 + 1
     pair_values(G, m, 2 * k2, pitch, a0, b0);
     pair_values(G, m, 2 * k2 + 1, pitch, a1, b1);
-    split_store(A + (size_t)(2 * m) * Kp + 2 * k2, cells, a0, a1);
-    if(2 * m + 1 < rows) split_store(A + (size_t)(2 * m + 1) * Kp + 2 * k2, cells, b0, b1);
+    split_store(A + (size_t)(2 * m) * 2 * Kp + 2 * k2, cells, Kp, a0, a1);
+    if(2 * m + 1 < rows) split_store(A + (size_t)(2 * m + 1) * 2 * Kp + 2 * k2, cells, Kp, b0, b1);
 }
 
 // FP16 per-row-scaled split: grid row r is scaled by 2^(14 - e), e =
 // floor(log2(max |component|)), so that its largest component lies in
-// [2^14, 2^15), then split into fp16 [hi | hi | lo] (lo = x - hi, so hi + lo
+// [2^14, 2^15), then split into fp16 [hi | lo] (lo = x - hi, so hi + lo
 // carries 22 significant bits); row_scale[r] = 2^(e - 14) undoes the scaling
 // exactly in the GEMM epilogue. One CTA per pair of node rows: both rows'
 // maxima, then the split.
@@ -615,12 +613,11 @@ k_prec_split_f16(const float4* __restrict__ G, uint32_t rows, uint32_t cells, ui
         const float xr = v.x * sc, xi = v.y * sc;
         const __half hr = __float2half_rn(xr), hi = __float2half_rn(xi);
         const __half lr = __float2half_rn(xr - __half2float(hr)), li = __float2half_rn(xi - __half2float(hi));
-        row[k] = __half_as_ushort(hr);             row[cells + k] = __half_as_ushort(hi);
-        row[2 * cells + k] = __half_as_ushort(hr); row[3 * cells + k] = __half_as_ushort(hi);
-        row[4 * cells + k] = __half_as_ushort(lr); row[5 * cells + k] = __half_as_ushort(li);
+        row[k] = __half_as_ushort(hr);      row[cells + k] = __half_as_ushort(hi);
+        row[Kp + k] = __half_as_ushort(lr); row[Kp + cells + k] = __half_as_ushort(li);
     };
-    uint16_t* row0 = A + (size_t)(2 * m) * Kp;
-    uint16_t* row1 = row0 + Kp;
+    uint16_t* row0 = A + (size_t)(2 * m) * 2 * Kp;
+    uint16_t* row1 = row0 + 2 * Kp;
     for(uint32_t k = threadIdx.x; k < cells; k += blockDim.x) {
         float2 v0, v1;
         pair_values(G, m, k, pitch, v0, v1);
@@ -764,6 +761,12 @@ k_prec_filter(const float2* __restrict__ C, uint32_t ldc2, uint32_t c_rows, size
             if(k < (int)nB) out[(size_t)r * nB + k] = on ? acc[q][h] : make_float2(0.f, 0.f);
         }
     }
+}
+
+using FilterFn = decltype(&k_prec_filter<1>);
+FilterFn filter_kernel(int parts)
+{
+    return parts == 8 ? k_prec_filter<8> : parts == 4 ? k_prec_filter<4> : parts == 2 ? k_prec_filter<2> : k_prec_filter<1>;
 }
 
 // Round-to-nearest-even float -> IEEE-754 binary16 bit pattern (from the
@@ -990,7 +993,7 @@ void free_dev(T*& p)
 void free_precision(Context& c)
 {
     free_dev(c.d_G); free_dev(c.d_flags); free_dev(c.d_A); free_dev(c.d_B);
-    free_dev(c.d_C); free_dev(c.d_taps);
+    free_dev(c.d_C); free_dev(c.d_taps); free_dev(c.d_blocks);
     free_dev(c.d_row_scale); free_dev(c.d_col_scale);
     free_dev(c.d_hot); free_dev(c.d_hotcnt); free_dev(c.d_rep);
     c.prec_f16 = false;
@@ -1102,30 +1105,25 @@ rtacx_status configure_precision(Context& ctx, const rtacx_precision_desc* d)
         cudaGetLastError();
         ctx.acc_staged_blocks[m] = (uint32_t)std::max(bs, 0);
     }
-    if(raise_smem_limit((const void*)k_prec_filter<1>, filter_smem_bytes(kFiltTapsMax)) != cudaSuccess ||
-       raise_smem_limit((const void*)k_prec_filter<2>, filter_smem_bytes(kFiltTapsMax)) != cudaSuccess) {
-        ctx.error = "cannot reserve shared memory for the range filter";
-        return RTACX_ERR_CUDA;
-    }
+    for(int parts = 1; parts <= 8; parts *= 2)
+        if(raise_smem_limit((const void*)filter_kernel(parts), filter_smem_bytes(kFiltTapsMax)) != cudaSuccess) {
+            ctx.error = "cannot reserve shared memory for the range filter";
+            return RTACX_ERR_CUDA;
+        }
 
     // GEMM operand shapes: M = grid rows, N = 2 nB (re / im of each bearing),
-    // K = 6 cells (the three split products of [Re | Im] grid values).
+    // K = 2 cells ([Re | Im] grid values) for each of the three split products.
     ctx.Mpad = (ctx.grid_rows + 127) / 128 * 128;
     ctx.Npad = (2 * nB + 255) / 256 * 256;
-    ctx.Kp = (6 * cells + 63) / 64 * 64;
-    // Split K in two when the 128 x 256 output tiles cover at most half of
-    // the SMs (the node grid of a 4096-range ping: 68 tiles on 152 SMs): twice
-    // the CTAs, each over half of K; the range filter adds the two partials.
-    ctx.ksplit = ((uint64_t)(ctx.Npad / 256) * (ctx.Mpad / 128) * 2 <= (uint64_t)ctx.sm_count &&
-                  (ctx.Kp / 64) % 2 == 0) ? 2u : 1u;
+    ctx.Kp = (2 * cells + 63) / 64 * 64;
 
-    // B operand: row n = 2b (real) / 2b + 1 (imag); K blocks [hi | lo | hi]
-    // of [real part of G | imaginary part of G]. FP16 form: each row n is
+    // B operand: row n = 2b (real) / 2b + 1 (imag); halves [hi | lo] of [real
+    // part of G | imaginary part of G]. FP16 form: each row n is
     // first scaled by 2^(14 - e_n) (largest |value| in [2^14, 2^15)) and
     // col_scale[n] = 2^(e_n - 14) undoes it in the GEMM epilogue.
     const bool f16 = (d->flags & RTACX_PRECISION_FP16_ROWSCALE) != 0;
     const bool hot = (d->flags & RTACX_PRECISION_HOT_RANGE) != 0;
-    std::vector<uint16_t> B((size_t)ctx.Npad * ctx.Kp, 0);
+    std::vector<uint16_t> B((size_t)ctx.Npad * 2 * ctx.Kp, 0);
     std::vector<float> col_scale(ctx.Npad, 1.0f);
     for(uint32_t b = 0; b < nB; b++)
         for(int o = 0; o < 2; o++) {
@@ -1144,7 +1142,7 @@ rtacx_status configure_precision(Context& ctx, const rtacx_precision_desc* d)
                     col_scale[2 * b + o] = std::ldexp(1.0f, -se);
                 }
             }
-            uint16_t* row = B.data() + (size_t)(2 * b + o) * ctx.Kp;
+            uint16_t* row = B.data() + (size_t)(2 * b + o) * 2 * ctx.Kp;
             for(uint32_t k = 0; k < cells; k++)
                 for(int h = 0; h < 2; h++) {
                     const float v = value(k, h) * scale;
@@ -1152,8 +1150,7 @@ rtacx_status configure_precision(Context& ctx, const rtacx_precision_desc* d)
                     if(f16) { bh = host_f16_bits(v); bl = host_f16_bits(v - host_f16_value(bh)); }
                     else { bh = host_bf16_bits(v); bl = host_bf16_bits(v - host_bf16_value(bh)); }
                     row[h * cells + k] = bh;
-                    row[2 * cells + h * cells + k] = bl;
-                    row[4 * cells + h * cells + k] = bh;
+                    row[ctx.Kp + h * cells + k] = bl;
                 }
         }
 
@@ -1163,8 +1160,8 @@ rtacx_status configure_precision(Context& ctx, const rtacx_precision_desc* d)
     };
     const size_t grid_bytes = grid_quads(ctx.grid_rows, g.pitch) * sizeof(float4);
     if(!alloc(ctx.d_G, grid_bytes) || !alloc(ctx.d_flags, (size_t)(nR + 31) / 32 * 4) ||
-       !alloc(ctx.d_A, (size_t)ctx.Mpad * ctx.Kp * 2) || !alloc(ctx.d_B, B.size() * 2) ||
-       !alloc(ctx.d_taps, taps.size() * sizeof(float)) || !alloc(ctx.d_C, (size_t)ctx.ksplit * ctx.Mpad * ctx.Npad * sizeof(float)) ||
+       !alloc(ctx.d_A, (size_t)ctx.Mpad * ctx.Kp * 4) || !alloc(ctx.d_B, B.size() * 2) ||
+       !alloc(ctx.d_taps, taps.size() * sizeof(float)) ||
        (f16 && (!alloc(ctx.d_row_scale, (size_t)ctx.Mpad * sizeof(float)) ||
                 !alloc(ctx.d_col_scale, (size_t)ctx.Npad * sizeof(float)))) ||
        (hot && (!alloc(ctx.d_hot, sizeof(int2)) || !alloc(ctx.d_hotcnt, (size_t)ctx.grid_rows * 4) ||
@@ -1173,7 +1170,17 @@ rtacx_status configure_precision(Context& ctx, const rtacx_precision_desc* d)
         ctx.error = "out of device memory for the precision form";
         return RTACX_ERR_OUT_OF_MEMORY;
     }
-    if(cudaMemset(ctx.d_A, 0, (size_t)ctx.Mpad * ctx.Kp * 2) != cudaSuccess ||
+    const rtacx_status planned = plan_gemm_split(ctx.error, ctx.gemm, ctx.d_A, ctx.d_B, B.data(), (int)ctx.Mpad, (int)ctx.Npad,
+                                                 (int)ctx.Kp, f16, ctx.sm_count);
+    if(planned != RTACX_OK) { free_precision(ctx); return planned; }
+    if(!alloc(ctx.d_C, (size_t)ctx.gemm.ksplit * ctx.Mpad * ctx.Npad * sizeof(float)) ||
+       !alloc(ctx.d_blocks, ctx.gemm.lists.size() * sizeof(uint16_t))) {
+        free_precision(ctx);
+        ctx.error = "out of device memory for the precision form";
+        return RTACX_ERR_OUT_OF_MEMORY;
+    }
+    if(cudaMemset(ctx.d_A, 0, (size_t)ctx.Mpad * ctx.Kp * 4) != cudaSuccess ||
+       cudaMemcpy(ctx.d_blocks, ctx.gemm.lists.data(), ctx.gemm.lists.size() * sizeof(uint16_t), cudaMemcpyHostToDevice) != cudaSuccess ||
        cudaMemcpy(ctx.d_B, B.data(), B.size() * 2, cudaMemcpyHostToDevice) != cudaSuccess ||
        cudaMemcpy(ctx.d_taps, taps.data(), taps.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
        (f16 && (cudaMemcpy(ctx.d_col_scale, col_scale.data(), col_scale.size() * sizeof(float),
@@ -1186,7 +1193,6 @@ rtacx_status configure_precision(Context& ctx, const rtacx_precision_desc* d)
         ctx.error = "uploading the precision tables failed";
         return RTACX_ERR_CUDA;
     }
-    if(gemm_smem_bytes() > 227 * 1024) { ctx.error = "GEMM tile exceeds shared memory"; return RTACX_ERR_UNSUPPORTED; }
     if(hot && raise_smem_limit((const void*)k_hot_pick, (ctx.grid_rows + 1) * sizeof(uint32_t)) != cudaSuccess) {
         free_precision(ctx);
         ctx.error = "cannot reserve shared memory for the hot-range scan";
@@ -1286,14 +1292,14 @@ rtacx_status precision_finish(Context& ctx, float* out, cudaStream_t stream)
     }
     ctx.mark(1, true, stream);
     ctx.mark(3, false, stream);
-    rtacx_status st = gemm_tn(ctx.error, ctx.d_A, ctx.d_B, ctx.d_C, (int)ctx.Mpad, (int)ctx.Npad, (int)ctx.Kp,
-                              (int)ctx.Npad, stream, ctx.d_err, ctx.prec_f16, ctx.prec_f16 ? ctx.d_row_scale : nullptr,
-                              ctx.prec_f16 ? ctx.d_col_scale : nullptr, (int)ctx.ksplit);
+    rtacx_status st = gemm_split(ctx.error, ctx.gemm, ctx.d_blocks, ctx.d_C, (int)ctx.Mpad, (int)ctx.Npad, (int)ctx.Kp, stream,
+                                 ctx.d_err, ctx.prec_f16, ctx.prec_f16 ? ctx.d_row_scale : nullptr,
+                                 ctx.prec_f16 ? ctx.d_col_scale : nullptr);
     if(st != RTACX_OK) return st;
     ctx.mark(3, true, stream);
     ctx.mark(2, false, stream);
     const dim3 fgrid((nB + kFiltCols - 1) / kFiltCols, (range_nodes(nR) + kFiltRows - 1) / kFiltRows);
-    auto filter = ctx.ksplit == 2 ? k_prec_filter<2> : k_prec_filter<1>;
+    auto filter = filter_kernel(ctx.gemm.ksplit);
     RTACX_CUDA(launch_chained(filter, fgrid, kFiltThreads, filter_smem_bytes(ctx.taps), stream,
                               reinterpret_cast<const float2*>(ctx.d_C), ctx.Npad / 2, ctx.grid_rows,
                               (size_t)ctx.Mpad * ctx.Npad / 2, ctx.d_flags, ctx.overlap, ctx.d_taps, ctx.taps, nR, nB,
