@@ -20,8 +20,8 @@
 //                      [hi | lo] of the three-term split product
 //                      (k_prec_split_f16: fp16 with a power-of-two scale per
 //                      row).
-//   gemm_tn            C = A x B^T on tcgen05 (rtacx_umma.cu), B the
-//                      [hi | lo | hi] split of the complex directivity laid
+//   gemm_split         C = A x B^T on tcgen05 (rtacx_umma.cu), B the
+//                      [hi | lo] split of the complex directivity laid
 //                      out so that column 2b of C is the real and 2b + 1 the
 //                      imaginary part of the grid contracted onto bearing b.
 //   k_prec_filter      the range taps of each output-row parity over C's
@@ -529,37 +529,49 @@ __device__ __forceinline__ void pair_values(const float4* __restrict__ G, uint32
 
 // The A operand of the split product: node row r (cells complex values)
 // becomes A row r = [hi(Re) | hi(Im) | .. | lo(Re) | lo(Im) | ..], the halves
-// Kp wide, lo = bf16(x - hi). One thread per pair of grid bearings of a pair
-// of node rows: their entries are read once (six 16-byte loads), eight 4-byte
-// stores.
-__device__ __forceinline__ void split_store(uint16_t* row, uint32_t cells, uint32_t Kp, float2 n0, float2 n1)
-{
-    const float x[4] = {n0.x, n0.y, n1.x, n1.y};     // re0, im0, re1, im1
-    uint16_t h[4], l[4];
-#pragma unroll
-    for(int i = 0; i < 4; i++) { h[i] = bf16_bits(x[i]); l[i] = bf16_bits(x[i] - bf16_value(h[i])); }
-    const uint32_t hr = (uint32_t)h[0] | ((uint32_t)h[2] << 16), hi = (uint32_t)h[1] | ((uint32_t)h[3] << 16);
-    const uint32_t lr = (uint32_t)l[0] | ((uint32_t)l[2] << 16), li = (uint32_t)l[1] | ((uint32_t)l[3] << 16);
-    *reinterpret_cast<uint32_t*>(row) = hr;
-    *reinterpret_cast<uint32_t*>(row + cells) = hi;
-    *reinterpret_cast<uint32_t*>(row + Kp) = lr;
-    *reinterpret_cast<uint32_t*>(row + Kp + cells) = li;
-}
-
-__global__ void k_prec_split(const float4* __restrict__ G, uint32_t rows, uint32_t cells, uint32_t pitch, uint32_t Kp,
-                             uint16_t* __restrict__ A)
+// Kp wide, lo = bf16(x - hi). A warp reads 64 bearing intervals of a pair of
+// node rows as four coalesced rows of 32 entries (lane: row lane & 1, interval
+// lane / 2); an interval's value adds the right share of the interval two
+// lanes down, and lanes of neighbouring bearings trade halves so that each
+// stores 4-byte pairs, the even one hi, the odd one lo.
+constexpr int kSplitThreads = 256;
+__global__ void __launch_bounds__(kSplitThreads)
+k_prec_split(const float4* __restrict__ G, uint32_t rows, uint32_t cells, uint32_t pitch, uint32_t Kp,
+             uint16_t* __restrict__ A)
 {
     const uint32_t m = blockIdx.y;                   // node rows 2m, 2m + 1
-    const uint32_t k2 = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31, q0 = (blockIdx.x * (kSplitThreads / 32) + (threadIdx.x >> 5)) * 64;
     chain_next();
     chain_wait();
     G = after_chain(G);
-    if(2 * m >= rows || 2 * k2 >= cells) return;
-    float2 a0, a1, b0, b1;                           // rows 2m, 2m + 1 at grid bearings 2 k2, 2 k2 + 1
-    pair_values(G, m, 2 * k2, pitch, a0, b0);
-    pair_values(G, m, 2 * k2 + 1, pitch, a1, b1);
-    split_store(A + (size_t)(2 * m) * 2 * Kp + 2 * k2, cells, Kp, a0, a1);
-    if(2 * m + 1 < rows) split_store(A + (size_t)(2 * m + 1) * 2 * Kp + 2 * k2, cells, Kp, b0, b1);
+    if(2 * m >= rows || q0 >= cells) return;
+    const float4* e = G + grid_at((int)(2 * m), 0, pitch);
+    float4 a[5];                                     // a[0]: lanes 30, 31 hold interval q0 - 1
+    a[0] = lane >= 30 && q0 > 0 ? e[2 * (size_t)q0 + lane - 32] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for(int j = 0; j < 4; j++) {
+        const uint32_t q = q0 + 16 * j + (lane >> 1);
+        a[j + 1] = q < cells ? e[2 * (size_t)q0 + 32 * j + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const uint32_t row = 2 * m + (lane & 1);
+    const bool odd = (lane & 2) != 0;                // odd bearing of its pair
+    uint16_t* out = A + (size_t)row * 2 * Kp + (odd ? Kp : 0);
+#pragma unroll
+    for(int j = 0; j < 4; j++) {
+        const float rz = __shfl_sync(0xffffffffu, lane >= 30 ? a[j].z : a[j + 1].z, (lane - 2) & 31);
+        const float rw = __shfl_sync(0xffffffffu, lane >= 30 ? a[j].w : a[j + 1].w, (lane - 2) & 31);
+        const float re = a[j + 1].x + rz, im = a[j + 1].y + rw;
+        const uint16_t hr = bf16_bits(re), hi = bf16_bits(im);
+        const uint16_t lr = bf16_bits(re - bf16_value(hr)), li = bf16_bits(im - bf16_value(hi));
+        const uint32_t own_h = (uint32_t)hr | ((uint32_t)hi << 16), own_l = (uint32_t)lr | ((uint32_t)li << 16);
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? own_h : own_l, 2);
+        const uint32_t x0 = odd ? got : own_h, x1 = odd ? own_l : got;   // the pair's even and odd bearing
+        const uint32_t q = q0 + 16 * j + ((lane >> 1) & ~1u);
+        if(row < rows && q < cells) {
+            *reinterpret_cast<uint32_t*>(out + q) = __byte_perm(x0, x1, 0x5410);
+            *reinterpret_cast<uint32_t*>(out + cells + q) = __byte_perm(x0, x1, 0x7632);
+        }
+    }
 }
 
 // FP16 per-row-scaled split: grid row r is scaled by 2^(14 - e), e =
@@ -626,50 +638,48 @@ k_prec_split_f16(const float4* __restrict__ G, uint32_t rows, uint32_t cells, ui
     }
 }
 
-constexpr int kFiltRows = 64, kFiltCols = 64, kFiltTapsMax = 64, kFiltThreads = 512;
+constexpr int kFiltCols = 64, kFiltTapsMax = 64;
 
-size_t filter_smem_bytes(uint32_t ntaps)
+size_t filter_smem_bytes(uint32_t ntaps, int rows)
 {
     const size_t nt = std::min<uint32_t>(std::max<uint32_t>(ntaps, 1u), (uint32_t)kFiltTapsMax);
-    return (kFiltRows + nt - 1) * kFiltCols * sizeof(float2) + 2 * kFiltTapsMax * sizeof(float2) +
-           2 * kFiltRows * sizeof(int);
+    return (rows + nt - 1) * kFiltCols * sizeof(float2) + 2 * kFiltTapsMax * sizeof(float2) + 2 * rows * sizeof(int);
 }
 
 // Range filter on the contracted grid: out(r, b) = sum_t taps[r % 2][t]
 // C[r / 2 + t + 1][b] (C row j holds range node j - tap_center - 1), or 0
-// when row r's reference window is empty. One CTA per 64 node rows x 64
-// bearings, both output-row parities (warps 0-7 the even rows 2 m, warps
-// 8-15 the odd rows 2 m + 1, from the same staged node rows). Per chunk of
+// when row r's reference window is empty. One CTA per kRows (64, or 16 where
+// 64 would leave most SMs without a CTA) node rows x 64 bearings, both
+// output-row parities (the first half of the warps the even rows 2 m, the
+// second the odd rows 2 m + 1, from the same staged node rows). Per chunk of
 // up to 64 taps the C rows it needs are staged in shared memory once,
-// row-major: every warp first loads all of its rows (up to 8, two 256-byte
+// row-major: every warp first loads up to 8 of its rows (two 256-byte
 // row segments each, the GEMM's K partials added) and only then stores
 // them, so the loads are in flight together. Lane l owns columns l and
 // l + 32; each warp filters 8 node rows of its parity with a sliding window
 // of eight staged rows per column in registers (one shared load per tap and
 // column).
-constexpr int kFiltWarps = kFiltThreads / 32;
-constexpr int kFiltRowsPerWarp = (kFiltRows + kFiltTapsMax - 1 + kFiltWarps - 1) / kFiltWarps;
-
-template <int kParts>
-__global__ void __launch_bounds__(kFiltThreads, 1)
+template <int kParts, int kRows>
+__global__ void __launch_bounds__(8 * kRows, 1)
 k_prec_filter(const float2* __restrict__ C, uint32_t ldc2, uint32_t c_rows, size_t part2,
               const uint32_t* __restrict__ nonempty, int ov, const float2* __restrict__ taps, uint32_t ntaps,
               uint32_t nR, uint32_t nB, float2* __restrict__ out)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     const int ntc = min((int)max(ntaps, 1u), kFiltTapsMax);
-    float2* sG = reinterpret_cast<float2*>(s_raw);                    // [kFiltRows + ntc - 1][kFiltCols]
-    float2* sT = sG + (size_t)(kFiltRows + ntc - 1) * kFiltCols;       // [2][kFiltTapsMax]
-    int* sW = reinterpret_cast<int*>(sT + 2 * kFiltTapsMax);            // [2][kFiltRows]
+    float2* sG = reinterpret_cast<float2*>(s_raw);                    // [kRows + ntc - 1][kFiltCols]
+    float2* sT = sG + (size_t)(kRows + ntc - 1) * kFiltCols;       // [2][kFiltTapsMax]
+    int* sW = reinterpret_cast<int*>(sT + 2 * kFiltTapsMax);            // [2][kRows]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int par = warp >> 3, wl = warp & 7;                           // parity, warp within it
-    const int r0 = blockIdx.y * kFiltRows, k0 = blockIdx.x * kFiltCols;
+    constexpr int kWarps = kRows / 4;                                   // half of them per parity, eight rows each
+    const int par = warp / (kWarps / 2), wl = warp % (kWarps / 2);      // parity, warp within it
+    const int r0 = blockIdx.y * kRows, k0 = blockIdx.x * kFiltCols;
     chain_next();
     chain_wait();
     C = after_chain(C);
     nonempty = after_chain(nonempty);
-    if(tid < 2 * kFiltRows) {
-        const int p = tid / kFiltRows, m = tid % kFiltRows;
+    if(tid < 2 * kRows) {
+        const int p = tid / kRows, m = tid % kRows;
         const int r = 2 * (r0 + m) + p;
         sW[tid] = r < (int)nR ? (row_has_window(nonempty, nR, ov, r) ? 1 : 0) : 0;
     }
@@ -679,13 +689,15 @@ k_prec_filter(const float2* __restrict__ C, uint32_t ldc2, uint32_t c_rows, size
 
     for(int tc = 0; tc < (int)ntaps; tc += ntc) {
         const int nt = min(ntc, (int)ntaps - tc);
-        const int rows_s = kFiltRows + nt - 1;
+        const int rows_s = kRows + nt - 1;
         __syncthreads();
-        if(tid < 2 * nt) sT[(tid / nt) * kFiltTapsMax + tid % nt] = taps[(size_t)(tid / nt) * ntaps + tc + tid % nt];
-        float2 v[kFiltRowsPerWarp][2];
+        for(int i = tid; i < 2 * nt; i += 8 * kRows) sT[(i / nt) * kFiltTapsMax + i % nt] = taps[(size_t)(i / nt) * ntaps + tc + i % nt];
+        constexpr int kRowsPerWarp = 8;                                 // staged rows whose loads are in flight together
+        for(int s0 = 0; s0 < rows_s; s0 += kWarps * kRowsPerWarp) {
+        float2 v[kRowsPerWarp][2];
 #pragma unroll
-        for(int i = 0; i < kFiltRowsPerWarp; i++) {
-            const int rr = warp + kFiltWarps * i;
+        for(int i = 0; i < kRowsPerWarp; i++) {
+            const int rr = s0 + warp + kWarps * i;
             const uint32_t j = (uint32_t)(r0 + tc + rr + 1);        // C row of staged row rr
             const bool live = rr < rows_s && j < c_rows;
             const float2* row = C + (size_t)(live ? j : 0) * ldc2;
@@ -704,12 +716,13 @@ k_prec_filter(const float2* __restrict__ C, uint32_t ldc2, uint32_t c_rows, size
             }
         }
 #pragma unroll
-        for(int i = 0; i < kFiltRowsPerWarp; i++) {
-            const int rr = warp + kFiltWarps * i;
+        for(int i = 0; i < kRowsPerWarp; i++) {
+            const int rr = s0 + warp + kWarps * i;
             if(rr < rows_s) {
                 sG[rr * kFiltCols + lane] = v[i][0];
                 sG[rr * kFiltCols + 32 + lane] = v[i][1];
             }
+        }
         }
         __syncthreads();
         const float2* tp = sT + par * kFiltTapsMax;
@@ -754,7 +767,7 @@ k_prec_filter(const float2* __restrict__ C, uint32_t ldc2, uint32_t c_rows, size
     for(int q = 0; q < 8; q++) {
         const int r = 2 * (r0 + wl * 8 + q) + par;
         if(r >= (int)nR) continue;
-        const bool on = sW[par * kFiltRows + wl * 8 + q] != 0;
+        const bool on = sW[par * kRows + wl * 8 + q] != 0;
 #pragma unroll
         for(int h = 0; h < 2; h++) {
             const int k = k0 + 32 * h + lane;
@@ -763,10 +776,12 @@ k_prec_filter(const float2* __restrict__ C, uint32_t ldc2, uint32_t c_rows, size
     }
 }
 
-using FilterFn = decltype(&k_prec_filter<1>);
-FilterFn filter_kernel(int parts)
+using FilterFn = decltype(&k_prec_filter<1, 64>);
+FilterFn filter_kernel(int parts, int rows)
 {
-    return parts == 8 ? k_prec_filter<8> : parts == 4 ? k_prec_filter<4> : parts == 2 ? k_prec_filter<2> : k_prec_filter<1>;
+    if(rows == 16)
+        return parts == 8 ? k_prec_filter<8, 16> : parts == 4 ? k_prec_filter<4, 16> : parts == 2 ? k_prec_filter<2, 16> : k_prec_filter<1, 16>;
+    return parts == 8 ? k_prec_filter<8, 64> : parts == 4 ? k_prec_filter<4, 64> : parts == 2 ? k_prec_filter<2, 64> : k_prec_filter<1, 64>;
 }
 
 // Round-to-nearest-even float -> IEEE-754 binary16 bit pattern (from the
@@ -1106,10 +1121,11 @@ rtacx_status configure_precision(Context& ctx, const rtacx_precision_desc* d)
         ctx.acc_staged_blocks[m] = (uint32_t)std::max(bs, 0);
     }
     for(int parts = 1; parts <= 8; parts *= 2)
-        if(raise_smem_limit((const void*)filter_kernel(parts), filter_smem_bytes(kFiltTapsMax)) != cudaSuccess) {
-            ctx.error = "cannot reserve shared memory for the range filter";
-            return RTACX_ERR_CUDA;
-        }
+        for(int rows : {16, 64})
+            if(raise_smem_limit((const void*)filter_kernel(parts, rows), filter_smem_bytes(kFiltTapsMax, rows)) != cudaSuccess) {
+                ctx.error = "cannot reserve shared memory for the range filter";
+                return RTACX_ERR_CUDA;
+            }
 
     // GEMM operand shapes: M = grid rows, N = 2 nB (re / im of each bearing),
     // K = 2 cells ([Re | Im] grid values) for each of the three split products.
@@ -1282,8 +1298,8 @@ rtacx_status precision_finish(Context& ctx, float* out, cudaStream_t stream)
     }
     ctx.mark(1, false, stream);
     if(!ctx.prec_f16) {
-        const dim3 sgrid((cells / 2 + 255) / 256, (ctx.grid_rows + 1) / 2);
-        RTACX_CUDA(launch_chained(k_prec_split, sgrid, 256, 0, stream, ctx.d_G, ctx.grid_rows, cells, ctx.grid.pitch,
+        const dim3 sgrid((cells + kSplitThreads * 2 - 1) / (kSplitThreads * 2), (ctx.grid_rows + 1) / 2);
+        RTACX_CUDA(launch_chained(k_prec_split, sgrid, kSplitThreads, 0, stream, ctx.d_G, ctx.grid_rows, cells, ctx.grid.pitch,
                                   ctx.Kp, ctx.d_A));
     }
     else {
@@ -1298,9 +1314,10 @@ rtacx_status precision_finish(Context& ctx, float* out, cudaStream_t stream)
     if(st != RTACX_OK) return st;
     ctx.mark(3, true, stream);
     ctx.mark(2, false, stream);
-    const dim3 fgrid((nB + kFiltCols - 1) / kFiltCols, (range_nodes(nR) + kFiltRows - 1) / kFiltRows);
-    auto filter = filter_kernel(ctx.gemm.ksplit);
-    RTACX_CUDA(launch_chained(filter, fgrid, kFiltThreads, filter_smem_bytes(ctx.taps), stream,
+    const uint32_t col_tiles = (nB + kFiltCols - 1) / kFiltCols;
+    const uint32_t frows = 2 * col_tiles * ((range_nodes(nR) + 63) / 64) < (uint32_t)ctx.sm_count ? 16 : 64;
+    const dim3 fgrid(col_tiles, (range_nodes(nR) + frows - 1) / frows);
+    RTACX_CUDA(launch_chained(filter_kernel(ctx.gemm.ksplit, (int)frows), fgrid, 8 * frows, filter_smem_bytes(ctx.taps, (int)frows), stream,
                               reinterpret_cast<const float2*>(ctx.d_C), ctx.Npad / 2, ctx.grid_rows,
                               (size_t)ctx.Mpad * ctx.Npad / 2, ctx.d_flags, ctx.overlap, ctx.d_taps, ctx.taps, nR, nB,
                               reinterpret_cast<float2*>(out)));
