@@ -509,7 +509,9 @@ struct FusedBatch {
 // Plan of the precision form's contraction (plan_gemm_split).
 struct GemmPlan {
     CUtensorMap ma, mb;
-    int bn = 0, ksplit = 1;             // tile width; K parts (partial products summed by the filter)
+    int bn = 0, ksplit = 1;             // tile width; K parts
+    bool adds() const { return ksplit > 2; }               // many parts: added into one (zeroed) result
+    int parts() const { return adds() ? 1 : ksplit; }      // partial products left for the filter to sum
     std::vector<uint16_t> lists;        // [column tiles][1 + blocks of K]: count, then the blocks where B is not zero
 };
 
@@ -618,7 +620,7 @@ struct Context {
     uint32_t diag_drop_stage = 0xFFFFFFFFu; // failure-path test: stage whose copy the staged accumulation skips
     uint16_t* d_A = nullptr;            // [Mpad][2 Kp] bf16 [hi | lo] split of the binned grid
     uint16_t* d_B = nullptr;            // [Npad][2 Kp] bf16 [hi | lo] split of the directivity
-    float* d_C = nullptr;               // [gemm.ksplit][Mpad][Npad] GEMM partial outputs: the grid contracted over bearings
+    float* d_C = nullptr;               // [gemm.parts()][Mpad][Npad] GEMM partial outputs: the grid contracted over bearings
     float2* d_taps = nullptr;           // [2][taps] range taps per output-row parity at node offsets t - tap_center
     // FP16 per-row-scaled contraction (RTACX_PRECISION_FP16_ROWSCALE): A and B
     // hold fp16 splits instead of bf16 ones.

@@ -30,6 +30,7 @@
 //                      complex64 ping.
 // The range filter runs after the contraction (the two commute): it then
 // works on bearing_count columns instead of the grid's.
+#include "rtacx_bin_device.cuh"
 #include "rtacx_internal.cuh"
 
 #include <cuda_fp16.h>
@@ -353,8 +354,10 @@ int accumulate_echo_model(uint32_t flags)
 }
 
 // Zeroes the grid (16-byte stores, grid-stride) and the non-empty bitmap of
-// a new ping in one launch.
-__global__ void k_prec_clear(float4* __restrict__ G, uint64_t quads, uint32_t* __restrict__ bits, uint32_t words)
+// a new ping (and the contraction's result where K parts add into it) in one
+// launch.
+__global__ void k_prec_clear(float4* __restrict__ G, uint64_t quads, uint32_t* __restrict__ bits, uint32_t words,
+                             float4* __restrict__ C, uint64_t c_quads)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -362,6 +365,7 @@ __global__ void k_prec_clear(float4* __restrict__ G, uint64_t quads, uint32_t* _
     chain_wait();
     for(uint64_t i = i0; i < quads; i += stride) G[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     for(uint64_t i = i0; i < words; i += stride) bits[i] = 0u;
+    for(uint64_t i = i0; i < c_quads; i += stride) C[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // Hot-range detection (RTACX_PRECISION_HOT_RANGE): grid-row counts of a
@@ -482,25 +486,6 @@ __global__ void k_hot_zero(const int2* __restrict__ hot, uint32_t pitch, float4*
     const uint64_t total = (uint64_t)after_chain(hot)->y * kHotReplicas * pitch;
     for(uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x)
         rep[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-}
-
-__device__ __forceinline__ bool bit_set(const uint32_t* bits, long long j)
-{
-    return (bits[j >> 5] >> (j & 31)) & 1u;
-}
-
-// Does row r's reference window hold at least two non-empty range bins?
-// The window of src/Binner.cu:90-102 covers [max(0, r - ov), min(nR - 1,
-// r + ov)] shrunk to its first and last non-empty bins, and it is an empty
-// view when fewer than two bins are non-empty.
-__device__ __noinline__ bool row_has_window(const uint32_t* __restrict__ nonempty, uint32_t nR, int ov, int r)
-{
-    if(ov < 0) return false;
-    const int lo = max(0, r - ov);
-    const int hi = (int)min((long long)nR - 1, (long long)r + ov);
-    int seen = 0;
-    for(int j = lo; j <= hi && seen < 2; j++) seen += bit_set(nonempty, j) ? 1 : 0;
-    return seen >= 2;
 }
 
 // Round-to-nearest-even fp32 -> bf16 (bit pattern).
@@ -638,9 +623,9 @@ k_prec_split_f16(const float4* __restrict__ G, uint32_t rows, uint32_t cells, ui
     }
 }
 
-constexpr int kFiltCols = 64, kFiltTapsMax = 64;
+constexpr int kFiltTapsMax = 64;
 
-size_t filter_smem_bytes(uint32_t ntaps, int rows)
+size_t filter_smem_bytes(uint32_t ntaps, int rows, int kFiltCols)
 {
     const size_t nt = std::min<uint32_t>(std::max<uint32_t>(ntaps, 1u), (uint32_t)kFiltTapsMax);
     return (rows + nt - 1) * kFiltCols * sizeof(float2) + 2 * kFiltTapsMax * sizeof(float2) + 2 * rows * sizeof(int);
@@ -648,8 +633,9 @@ size_t filter_smem_bytes(uint32_t ntaps, int rows)
 
 // Range filter on the contracted grid: out(r, b) = sum_t taps[r % 2][t]
 // C[r / 2 + t + 1][b] (C row j holds range node j - tap_center - 1), or 0
-// when row r's reference window is empty. One CTA per kRows (64, or 16 where
-// 64 would leave most SMs without a CTA) node rows x 64 bearings, both
+// when row r's reference window is empty. One CTA per kRows node rows x
+// kFiltCols bearings (64 x 64, or 16 x 32 where that would leave most SMs
+// without a CTA: 512 ranges x 128 bearings 16 -> 8 us), both
 // output-row parities (the first half of the warps the even rows 2 m, the
 // second the odd rows 2 m + 1, from the same staged node rows). Per chunk of
 // up to 64 taps the C rows it needs are staged in shared memory once,
@@ -659,12 +645,13 @@ size_t filter_smem_bytes(uint32_t ntaps, int rows)
 // l + 32; each warp filters 8 node rows of its parity with a sliding window
 // of eight staged rows per column in registers (one shared load per tap and
 // column).
-template <int kParts, int kRows>
+template <int kParts, int kRows, int kFiltCols>
 __global__ void __launch_bounds__(8 * kRows, 1)
 k_prec_filter(const float2* __restrict__ C, uint32_t ldc2, uint32_t c_rows, size_t part2,
               const uint32_t* __restrict__ nonempty, int ov, const float2* __restrict__ taps, uint32_t ntaps,
               uint32_t nR, uint32_t nB, float2* __restrict__ out)
 {
+    constexpr int kHalves = kFiltCols / 32;                             // columns per lane
     extern __shared__ __align__(16) unsigned char s_raw[];
     const int ntc = min((int)max(ntaps, 1u), kFiltTapsMax);
     float2* sG = reinterpret_cast<float2*>(s_raw);                    // [kRows + ntc - 1][kFiltCols]
@@ -681,11 +668,13 @@ k_prec_filter(const float2* __restrict__ C, uint32_t ldc2, uint32_t c_rows, size
     if(tid < 2 * kRows) {
         const int p = tid / kRows, m = tid % kRows;
         const int r = 2 * (r0 + m) + p;
-        sW[tid] = r < (int)nR ? (row_has_window(nonempty, nR, ov, r) ? 1 : 0) : 0;
+        sW[tid] = r < (int)nR ? (row_on(nonempty, (int)nR, ov, r) ? 1 : 0) : 0;
     }
-    float2 acc[8][2];
+    float2 acc[8][kHalves];
 #pragma unroll
-    for(int q = 0; q < 8; q++) { acc[q][0] = make_float2(0.f, 0.f); acc[q][1] = make_float2(0.f, 0.f); }
+    for(int q = 0; q < 8; q++)
+#pragma unroll
+        for(int h = 0; h < kHalves; h++) acc[q][h] = make_float2(0.f, 0.f);
 
     for(int tc = 0; tc < (int)ntaps; tc += ntc) {
         const int nt = min(ntc, (int)ntaps - tc);
@@ -694,7 +683,7 @@ k_prec_filter(const float2* __restrict__ C, uint32_t ldc2, uint32_t c_rows, size
         for(int i = tid; i < 2 * nt; i += 8 * kRows) sT[(i / nt) * kFiltTapsMax + i % nt] = taps[(size_t)(i / nt) * ntaps + tc + i % nt];
         constexpr int kRowsPerWarp = 8;                                 // staged rows whose loads are in flight together
         for(int s0 = 0; s0 < rows_s; s0 += kWarps * kRowsPerWarp) {
-        float2 v[kRowsPerWarp][2];
+        float2 v[kRowsPerWarp][kHalves];
 #pragma unroll
         for(int i = 0; i < kRowsPerWarp; i++) {
             const int rr = s0 + warp + kWarps * i;
@@ -702,7 +691,7 @@ k_prec_filter(const float2* __restrict__ C, uint32_t ldc2, uint32_t c_rows, size
             const bool live = rr < rows_s && j < c_rows;
             const float2* row = C + (size_t)(live ? j : 0) * ldc2;
 #pragma unroll
-            for(int h = 0; h < 2; h++) {
+            for(int h = 0; h < kHalves; h++) {
                 const int k = k0 + 32 * h + lane;
                 float2 x = make_float2(0.f, 0.f);
                 if(live && k < (int)nB) {
@@ -719,15 +708,15 @@ k_prec_filter(const float2* __restrict__ C, uint32_t ldc2, uint32_t c_rows, size
         for(int i = 0; i < kRowsPerWarp; i++) {
             const int rr = s0 + warp + kWarps * i;
             if(rr < rows_s) {
-                sG[rr * kFiltCols + lane] = v[i][0];
-                sG[rr * kFiltCols + 32 + lane] = v[i][1];
+#pragma unroll
+                for(int h = 0; h < kHalves; h++) sG[rr * kFiltCols + 32 * h + lane] = v[i][h];
             }
         }
         }
         __syncthreads();
         const float2* tp = sT + par * kFiltTapsMax;
 #pragma unroll
-        for(int h = 0; h < 2; h++) {
+        for(int h = 0; h < kHalves; h++) {
             const float2* col = sG + h * 32 + lane + wl * 8 * kFiltCols;
             float2 g[8];
 #pragma unroll
@@ -769,19 +758,18 @@ k_prec_filter(const float2* __restrict__ C, uint32_t ldc2, uint32_t c_rows, size
         if(r >= (int)nR) continue;
         const bool on = sW[par * kRows + wl * 8 + q] != 0;
 #pragma unroll
-        for(int h = 0; h < 2; h++) {
+        for(int h = 0; h < kHalves; h++) {
             const int k = k0 + 32 * h + lane;
             if(k < (int)nB) out[(size_t)r * nB + k] = on ? acc[q][h] : make_float2(0.f, 0.f);
         }
     }
 }
 
-using FilterFn = decltype(&k_prec_filter<1, 64>);
-FilterFn filter_kernel(int parts, int rows)
+using FilterFn = decltype(&k_prec_filter<1, 64, 64>);
+FilterFn filter_kernel(int parts, bool small)
 {
-    if(rows == 16)
-        return parts == 8 ? k_prec_filter<8, 16> : parts == 4 ? k_prec_filter<4, 16> : parts == 2 ? k_prec_filter<2, 16> : k_prec_filter<1, 16>;
-    return parts == 8 ? k_prec_filter<8, 64> : parts == 4 ? k_prec_filter<4, 64> : parts == 2 ? k_prec_filter<2, 64> : k_prec_filter<1, 64>;
+    if(small) return parts == 2 ? k_prec_filter<2, 16, 32> : k_prec_filter<1, 16, 32>;
+    return parts == 2 ? k_prec_filter<2, 64, 64> : k_prec_filter<1, 64, 64>;
 }
 
 // Round-to-nearest-even float -> IEEE-754 binary16 bit pattern (from the
@@ -1120,9 +1108,10 @@ rtacx_status configure_precision(Context& ctx, const rtacx_precision_desc* d)
         cudaGetLastError();
         ctx.acc_staged_blocks[m] = (uint32_t)std::max(bs, 0);
     }
-    for(int parts = 1; parts <= 8; parts *= 2)
-        for(int rows : {16, 64})
-            if(raise_smem_limit((const void*)filter_kernel(parts, rows), filter_smem_bytes(kFiltTapsMax, rows)) != cudaSuccess) {
+    for(int parts = 1; parts <= 2; parts++)
+        for(bool small : {false, true})
+            if(raise_smem_limit((const void*)filter_kernel(parts, small),
+                                filter_smem_bytes(kFiltTapsMax, small ? 16 : 64, small ? 32 : 64)) != cudaSuccess) {
                 ctx.error = "cannot reserve shared memory for the range filter";
                 return RTACX_ERR_CUDA;
             }
@@ -1189,7 +1178,7 @@ rtacx_status configure_precision(Context& ctx, const rtacx_precision_desc* d)
     const rtacx_status planned = plan_gemm_split(ctx.error, ctx.gemm, ctx.d_A, ctx.d_B, B.data(), (int)ctx.Mpad, (int)ctx.Npad,
                                                  (int)ctx.Kp, f16, ctx.sm_count);
     if(planned != RTACX_OK) { free_precision(ctx); return planned; }
-    if(!alloc(ctx.d_C, (size_t)ctx.gemm.ksplit * ctx.Mpad * ctx.Npad * sizeof(float)) ||
+    if(!alloc(ctx.d_C, (size_t)ctx.gemm.parts() * ctx.Mpad * ctx.Npad * sizeof(float)) ||
        !alloc(ctx.d_blocks, ctx.gemm.lists.size() * sizeof(uint16_t))) {
         free_precision(ctx);
         ctx.error = "out of device memory for the precision form";
@@ -1225,7 +1214,8 @@ rtacx_status precision_begin(Context& ctx, cudaStream_t stream)
 {
     const uint64_t quads = grid_quads(ctx.grid_rows, ctx.grid.pitch);
     const uint32_t blocks = (uint32_t)std::min<uint64_t>((quads + 255) / 256, (uint64_t)ctx.sm_count * 32);
-    RTACX_CUDA(launch_chained(k_prec_clear, blocks, 256, 0, stream, ctx.d_G, quads, ctx.d_flags, (ctx.nR + 31) / 32));
+    RTACX_CUDA(launch_chained(k_prec_clear, blocks, 256, 0, stream, ctx.d_G, quads, ctx.d_flags, (ctx.nR + 31) / 32,
+                              reinterpret_cast<float4*>(ctx.d_C), ctx.gemm.adds() ? (uint64_t)ctx.Mpad * ctx.Npad / 4 : 0));
     return RTACX_OK;
 }
 
@@ -1314,10 +1304,12 @@ rtacx_status precision_finish(Context& ctx, float* out, cudaStream_t stream)
     if(st != RTACX_OK) return st;
     ctx.mark(3, true, stream);
     ctx.mark(2, false, stream);
-    const uint32_t col_tiles = (nB + kFiltCols - 1) / kFiltCols;
-    const uint32_t frows = 2 * col_tiles * ((range_nodes(nR) + 63) / 64) < (uint32_t)ctx.sm_count ? 16 : 64;
-    const dim3 fgrid(col_tiles, (range_nodes(nR) + frows - 1) / frows);
-    RTACX_CUDA(launch_chained(filter_kernel(ctx.gemm.ksplit, (int)frows), fgrid, 8 * frows, filter_smem_bytes(ctx.taps, (int)frows), stream,
+    const uint32_t nodes = range_nodes(nR);
+    const bool small = 2u * ((nB + 63) / 64) * ((nodes + 63) / 64) < (uint32_t)ctx.sm_count;
+    const uint32_t frows = small ? 16 : 64, fcols = small ? 32 : 64;
+    const dim3 fgrid((nB + fcols - 1) / fcols, (nodes + frows - 1) / frows);
+    RTACX_CUDA(launch_chained(filter_kernel(ctx.gemm.parts(), small), fgrid, 8 * frows,
+                              filter_smem_bytes(ctx.taps, (int)frows, (int)fcols), stream,
                               reinterpret_cast<const float2*>(ctx.d_C), ctx.Npad / 2, ctx.grid_rows,
                               (size_t)ctx.Mpad * ctx.Npad / 2, ctx.d_flags, ctx.overlap, ctx.d_taps, ctx.taps, nR, nB,
                               reinterpret_cast<float2*>(out)));

@@ -91,7 +91,7 @@ __device__ __forceinline__ void umma_16bit(uint32_t tmem_d, uint64_t adesc, uint
 template <int BN>
 __device__ __forceinline__ void store_tile(uint32_t tmem, float* __restrict__ C, int m0, int n0, int ldc, int warp, int lane,
                                            const float* __restrict__ row_scale, const float* __restrict__ col_scale,
-                                           bool any)
+                                           bool any, bool add)
 {
     const int row = m0 + warp * 32 + lane;
     float* crow = C + (size_t)row * ldc + n0;
@@ -116,6 +116,13 @@ __device__ __forceinline__ void store_tile(uint32_t tmem, float* __restrict__ C,
             }
         }
         float4* dst = reinterpret_cast<float4*>(crow + c * 32);
+        if(add) {
+#pragma unroll
+            for(int q = 0; q < 8; q++)
+                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
+                             ::"l"(dst + q), "f"(v[4 * q]), "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3]) : "memory");
+            continue;
+        }
 #pragma unroll
         for(int q = 0; q < 8; q++) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
     }
@@ -188,7 +195,7 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
     const bool ok = mbar_wait(accum_bar, 0, abort_flag);
     __syncwarp();
     tc_fence_after();
-    if(__all_sync(0xffffffffu, ok ? 1 : 0)) store_tile<BN>(tmem, C, m0, n0, ldc, warp, lane, nullptr, nullptr, true);
+    if(__all_sync(0xffffffffu, ok ? 1 : 0)) store_tile<BN>(tmem, C, m0, n0, ldc, warp, lane, nullptr, nullptr, true, false);
     else if(lane == 0 && err) atomicOr(err, kErrGemmTimeout);
     tc_fence_before();
     __syncthreads();
@@ -202,7 +209,7 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
 // along K; the hi and the lo tiles have a barrier each, so that hi hi starts
 // before the lo tiles are in. blockIdx.z: its share of the column tile's list
 // of blocks (blocks: [column tiles][1 + all blocks], the count first), into its
-// own partial product C + z rows ldc.
+// own partial product C + z rows ldc, or (add) added into C.
 template <int BN_, int STAGES_>
 struct SplitTile {
     static constexpr int BN = BN_, STAGES = STAGES_;
@@ -217,7 +224,7 @@ template <bool kF16, typename T>
 __global__ void __launch_bounds__(kThreads, 1)
 k_gemm_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, float* __restrict__ C,
              int rows, int K, int ldc, const uint16_t* __restrict__ blocks, const float* __restrict__ row_scale,
-             const float* __restrict__ col_scale, uint32_t* __restrict__ err)
+             const float* __restrict__ col_scale, int add, uint32_t* __restrict__ err)
 {
     constexpr int BN = T::BN, STAGES = T::STAGES;
     constexpr uint32_t TMEM_COLS = BN;
@@ -234,7 +241,7 @@ k_gemm_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     const int total = list[0];
     const int begin = total * (int)blockIdx.z / (int)gridDim.z, count = total * ((int)blockIdx.z + 1) / (int)gridDim.z - begin;
     list += 1 + begin;
-    C += (size_t)blockIdx.z * (size_t)rows * ldc;
+    if(!add) C += (size_t)blockIdx.z * (size_t)rows * ldc;
     auto hi_bar = [&](int s) { return smem_u32(bars + s); };
     auto lo_bar = [&](int s) { return smem_u32(bars + STAGES + s); };
     auto empty_bar = [&](int s) { return smem_u32(bars + 2 * STAGES + s); };
@@ -303,7 +310,7 @@ k_gemm_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     __syncwarp();
     tc_fence_after();
     if(__all_sync(0xffffffffu, ok ? 1 : 0))
-        store_tile<BN>(tmem, C, m0, n0, ldc, warp, lane, row_scale, col_scale, count > 0);
+        store_tile<BN>(tmem, C, m0, n0, ldc, warp, lane, row_scale, col_scale, count > 0, add != 0);
     else if(lane == 0 && err) atomicOr(err, kErrGemmTimeout);
     tc_fence_before();
     __syncthreads();
@@ -449,13 +456,15 @@ rtacx_status plan_gemm_split(std::string& error, GemmPlan& g, const void* A, con
     return RTACX_OK;
 }
 
-// C + z M N (z < g.ksplit) = partial products of the planned contraction, in
+// C + z M N (z < g.parts()) = partial products of the planned contraction (added
+// into a zeroed C where g.adds()), in
 // A's and B's current values (16-byte aligned scales optional).
 rtacx_status gemm_split(std::string& error, const GemmPlan& g, const uint16_t* d_blocks, float* C, int M, int N, int K,
                         cudaStream_t stream, uint32_t* err, bool f16, const float* row_scale, const float* col_scale)
 {
     const cudaError_t e = launch_chained(split_kernel(g.bn, f16), dim3(N / g.bn, M / BM, g.ksplit), kThreads,
-                                         split_smem(g.bn), stream, g.ma, g.mb, C, M, K, N, d_blocks, row_scale, col_scale, err);
+                                         split_smem(g.bn), stream, g.ma, g.mb, C, M, K, N, d_blocks, row_scale, col_scale,
+                                         g.adds() ? 1 : 0, err);
     if(e != cudaSuccess) { cudaGetLastError(); error = std::string("k_gemm_split: ") + cudaGetErrorString(e); return RTACX_ERR_CUDA; }
     return RTACX_OK;
 }
