@@ -308,21 +308,6 @@ __device__ __forceinline__ uint32_t range_key(const KeyParams& k, float travel, 
     return (uint32_t)res;
 }
 
-// range_key without the side, for kernels that hold several samples per
-// thread: the common case (between -1 and nR, at most 2^20) by floor_small,
-// the rest (NaN among it) by the conversion.
-__device__ __forceinline__ uint32_t range_key_fast(const KeyParams& k, float travel)
-{
-    const float x = fmaf(k.a, travel, k.b);
-    if(x > -1.0f && x < (float)k.nR) {
-        int whole;
-        floor_small(fmaxf(x, 0.0f), whole);
-        return (uint32_t)whole;
-    }
-    int side;
-    return range_key(k, travel, side);
-}
-
 // Bearing sub-bin (extension of the reference key, see the oracle for the
 // same formula): 0 if !(q >= 1), n - 1 if q >= n, else (int)q.
 __device__ __forceinline__ uint32_t bearing_bin(float scale, float offset, uint32_t n, float bearing)

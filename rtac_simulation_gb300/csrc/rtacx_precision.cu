@@ -54,7 +54,6 @@ constexpr int kAccThreads = 256;
 // of their CTA and warp, and k_hot_fold adds the replicas back into the grid
 // before the contraction.
 constexpr int kHotRows = 128, kHotReplicas = 8;
-constexpr int kAccLoads = 4;                     // independent record loads per thread in flight
 constexpr int kAccEchoModels = 6;                // echo models of the staged accumulation
 // Grid rows are stored cells + kRowPad entries apart (128 bytes of padding,
 // so that the row pitch is not a power of two): 4 % faster accumulation on
@@ -115,62 +114,95 @@ size_t accumulate_smem_bytes(uint32_t nR)
     return (size_t)((nR + 31) / 32) * sizeof(uint32_t);
 }
 
-// General accumulation: any record alignment, echo model read at run time,
-// the hot-range replicas. Grid-stride over the samples, kAccLoads records per
-// thread in flight; non-empty range bins (reference keys) in a shared bitmap
-// OR-ed into the global one once per CTA.
+constexpr uint32_t kNoEntry = 0xFFFFFFFFu;
+constexpr uint32_t kReplicaEntry = 0x80000000u;  // an entry of the hot rows' replicas instead of the grid
+
+// Adds one record per lane (live: the lane has one) to the grid; whole warps.
+// Lanes 2k and 2k + 1 deposit together: first the even lane's sample (row jg
+// from the even lane, jg + 1 from the odd one), then the odd lane's, so each
+// reduction instruction sends a sample's two rows of an interval as one
+// sector when jg is even. Each lane keeps one node's share of its own sample
+// and trades the other's. `replica` maps a row to an entry of the hot rows'
+// replicas (kNoEntry: the row is not hot).
+template <typename Replica>
+__device__ __forceinline__ void deposit_warp(const GridParams& g, const BinParams& p, uint32_t echo, const float4& rec,
+                                             bool live, float4* G, float4* rep, uint64_t keep_pol, Replica&& replica)
+{
+    int jg, q;
+    float alpha, w;
+    const bool ok = grid_coords(g, rec.z, rec.w, jg, alpha, q, w) && live;
+    const float2 v = apply_echo(p, make_float2(rec.x, rec.y), rec.z, echo);
+    const uint32_t e = ((uint32_t)(jg >> 1) * g.pitch + (uint32_t)q) * 2u;
+    uint32_t at0 = e + (uint32_t)(jg & 1), at1 = e + ((jg & 1) ? 2u * g.pitch : 1u);
+    const uint32_t r0 = replica(jg, q), r1 = replica(jg + 1, q);
+    at0 = !ok ? kNoEntry : r0 != kNoEntry ? r0 : at0;
+    at1 = !ok ? kNoEntry : r1 != kNoEntry ? r1 : at1;
+    const float a0 = 1.0f - alpha;
+    const float4 add = make_float4(a0 * v.x, a0 * v.y, alpha * v.x, alpha * v.y);
+    const bool odd = (threadIdx.x & 1u) != 0u;
+    const uint32_t keep = odd ? at1 : at0;
+    const float2 keep_v = odd ? make_float2(add.z, add.w) : make_float2(add.x, add.y);
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? at0 : at1, 1);
+    float2 got_v;
+    got_v.x = __shfl_xor_sync(0xffffffffu, odd ? add.x : add.z, 1);
+    got_v.y = __shfl_xor_sync(0xffffffffu, odd ? add.y : add.w, 1);
+    const float got_w = __shfl_xor_sync(0xffffffffu, w, 1);
+    const uint32_t first = odd ? got : keep, second = odd ? keep : got;
+    auto entry = [&](uint32_t at) { return at & kReplicaEntry ? rep + (at & ~kReplicaEntry) : G + at; };
+    if(first != kNoEntry) deposit(entry(first), odd ? got_w : w, odd ? got_v : keep_v, keep_pol);
+    if(second != kNoEntry) deposit(entry(second), odd ? w : got_w, odd ? keep_v : got_v, keep_pol);
+}
+
+// General accumulation: any record alignment, the echo model read at run
+// time, the hot-range replicas. Warps take 32 records at a time, two loads
+// ahead in registers; non-empty range bins (reference keys) in a shared bitmap
+// OR-ed into the global one once per CTA. Clustered 2^26 samples on a 271 MB
+// grid (8192 ranges x 1024 bearings), with replicas: 1336 us with two
+// reductions per sample from its own lane, 1176 us deposited by lane pairs.
+// Bound there by the reductions that miss the L2; 2, 16 or 32 replicas instead
+// of 8 take 1238, 1227 and 1332 us, and passes over halves or thirds of the
+// grid that would fit the L2 take 1220 and 1359 us (the samples are read again).
 __global__ void __launch_bounds__(kAccThreads)
 k_prec_accumulate(const float* __restrict__ samples, uint64_t n, BinParams p, GridParams g,
                   float4* __restrict__ G, uint32_t* __restrict__ nonempty, const int2* __restrict__ hot,
                   float4* __restrict__ rep)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t* s_bits = reinterpret_cast<uint32_t*>(s_raw);
+    const uint32_t words = (p.key.nR + 31) / 32;
+    const uint64_t keep = policy_evict_last();
+    for(uint32_t i = threadIdx.x; i < words; i += blockDim.x) s_bits[i] = 0u;
     int hot_lo = 0, hot_len = 0;
     chain_next();
     chain_wait();
     samples = after_chain(samples);
     hot = after_chain(hot);
     if(hot) { const int2 h = *hot; hot_lo = h.x; hot_len = h.y; }
-    const uint32_t rsel = (blockIdx.x + (threadIdx.x >> 5)) & (kHotReplicas - 1);   // by CTA and warp
-    const uint32_t pitch = g.pitch;
-    // Entry (jg, q): the grid's, or in this warp's replica of a hot row
-    // (replica rows are plain rows of `pitch` entries).
-    auto entry = [&](int jg, int q) -> float4* {
-        const uint32_t hj = (uint32_t)(jg - hot_lo);
-        return hj < (uint32_t)hot_len ? rep + ((size_t)hj * kHotReplicas + rsel) * pitch + q : G + grid_at(jg, q, pitch);
-    };
-    const uint32_t words = (p.key.nR + 31) / 32;
-    const uint64_t keep = policy_evict_last();
-    for(uint32_t i = threadIdx.x; i < words; i += blockDim.x) s_bits[i] = 0u;
     __syncthreads();
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for(uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i0 < n; i0 += stride * kAccLoads) {
-        float4 rec[kAccLoads];
-#pragma unroll
-        for(int u = 0; u < kAccLoads; u++) {
-            const uint64_t i = i0 + (uint64_t)u * stride;
-            rec[u] = i < n ? load_record(samples, i, p) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for(int u = 0; u < kAccLoads; u++) {
-            if(i0 + (uint64_t)u * stride >= n) continue;
-            int side;
-            const uint32_t j = range_key(p.key, rec[u].z, side);
-            if(j == kOutOfRange) continue;
-            atomicOr(&s_bits[j >> 5], 1u << (j & 31));
-            int jg, q;
-            float alpha, w;
-            if(!grid_coords(g, rec[u].z, rec[u].w, jg, alpha, q, w)) continue;
-            const float2 v = apply_echo(p, make_float2(rec[u].x, rec[u].y), rec[u].z);
-            const float a0 = 1.0f - alpha;
-            deposit(entry(jg, q), w, make_float2(a0 * v.x, a0 * v.y), keep);
-            deposit(entry(jg + 1, q), w, make_float2(alpha * v.x, alpha * v.y), keep);
-        }
+    const uint32_t rsel = (blockIdx.x + warp) & (kHotReplicas - 1);   // by CTA and warp
+    // Replica rows are stored in pairs like the grid's (hot_lo is even).
+    auto replica = [&](int row, int q) -> uint32_t {
+        const uint32_t hj = (uint32_t)(row - hot_lo);
+        return hj < (uint32_t)hot_len ? ((((hj >> 1) * kHotReplicas + rsel) * g.pitch + (uint32_t)q) * 2u + (hj & 1u)) | kReplicaEntry
+                                      : kNoEntry;
+    };
+    const uint64_t stride = (uint64_t)gridDim.x * kAccThreads;
+    auto load = [&](uint64_t i) { return i < n ? load_record(samples, i, p) : make_float4(0.f, 0.f, 0.f, 0.f); };
+    uint64_t i = (uint64_t)blockIdx.x * kAccThreads + threadIdx.x;
+    float4 next0 = load(i), next1 = load(i + stride);
+    for(; i - lane < n; i += stride) {
+        const float4 rec = next0;
+        next0 = next1;
+        next1 = load(i + 2 * stride);
+        int side;
+        const uint32_t key = i < n ? range_key(p.key, rec.z, side) : kOutOfRange;
+        if(key != kOutOfRange && !(s_bits[key >> 5] >> (key & 31) & 1u)) atomicOr(&s_bits[key >> 5], 1u << (key & 31));
+        deposit_warp(g, p, p.echo_flags, rec, key != kOutOfRange, G, rep, keep, replica);
     }
     __syncthreads();
-    for(uint32_t i = threadIdx.x; i < words; i += blockDim.x)
-        if(s_bits[i]) atomicOr(&nonempty[i], s_bits[i]);
+    for(uint32_t w = threadIdx.x; w < words; w += blockDim.x)
+        if(s_bits[w]) atomicOr(&nonempty[w], s_bits[w]);
 }
 
 // The accumulation for the common case: 16-byte aligned records, no hot
@@ -178,10 +210,8 @@ k_prec_accumulate(const float* __restrict__ samples, uint64_t n, BinParams p, Gr
 // shared memory by bulk copies (cp.async.bulk, the TMA engine): every warp has
 // its own ring of kStages stages of kStageRecs records, so that no barrier
 // of the CTA is in the loop and the bytes in flight per SM depend neither on
-// registers nor on how long the threads compute. Each thread computes the
-// key, grid coordinates and weighted values of its records of a stage without
-// branches (invalid and tail records only clear a predicate), then issues the
-// bitmap bits and the reductions; the results are those of k_prec_accumulate.
+// registers nor on how long the threads compute; the results are those of
+// k_prec_accumulate.
 // Warp w of the grid takes stages w, w + warps, ...; its lane 0 issues the
 // copy of the stage kStages ahead as soon as every lane has read the stage it
 // refills. Each wait is bounded (kAccWaitCycles); a timeout sets
@@ -190,10 +220,9 @@ k_prec_accumulate(const float* __restrict__ samples, uint64_t n, BinParams p, Gr
 constexpr int kStageRecs = 32;                   // 512 B of records per stage: one per lane
 constexpr int kStages = 4;
 constexpr int kStagedThreads = 512, kStagedWarps = kStagedThreads / 32;
-constexpr int kStagedPerThread = kStageRecs / 32;
+static_assert(kStageRecs == 32, "one record per lane");
 constexpr int kDiagStageRecs = 1024;             // records of a stage of rtacx_diag_drop_accumulation_stage
 constexpr long long kAccWaitCycles = 2000000000ll;   // about one second
-constexpr uint32_t kNoEntry = 0xFFFFFFFFu;
 
 size_t staged_smem_bytes(uint32_t nR)
 {
@@ -215,7 +244,6 @@ k_prec_accumulate_staged(const float4* __restrict__ samples, uint64_t n, BinPara
     const uint32_t words = (p.key.nR + 31) / 32;
     const uint64_t stages = (n + kStageRecs - 1) / kStageRecs;
     const uint64_t stride = (uint64_t)gridDim.x * kStagedWarps, c0 = (uint64_t)blockIdx.x * kStagedWarps + warp;
-    const uint32_t pitch = g.pitch;
     const uint64_t stream_pol = policy_evict_first(), keep_pol = policy_evict_last();
     auto issue = [&](uint64_t c, int slot) {
         if(c / (kDiagStageRecs / kStageRecs) == drop_stage) return;   // failure-path test: this copy never comes
@@ -252,29 +280,9 @@ k_prec_accumulate_staged(const float4* __restrict__ samples, uint64_t n, BinPara
         if(__any_sync(0xffffffffu, aborted)) { aborted = true; break; }
         const uint64_t left = n - c * kStageRecs;
         const uint32_t count = left < (uint64_t)kStageRecs ? (uint32_t)left : (uint32_t)kStageRecs;
-        uint32_t key[kStagedPerThread];
-        uint32_t at0[kStagedPerThread], at1[kStagedPerThread];   // grid entries of the sample's two nodes (kNoEntry: none)
-        float wgt[kStagedPerThread];
-        float4 add[kStagedPerThread];
-#pragma unroll
-        for(int u = 0; u < kStagedPerThread; u++) {
-            const uint32_t idx = (uint32_t)lane + (uint32_t)u * 32u;
-            const float4 rec = s_ring[slot * kStageRecs + idx];
-            int side;
-            const uint32_t k = range_key(p.key, rec.z, side);
-            const bool live = idx < count && k != kOutOfRange;
-            key[u] = live ? k : kOutOfRange;
-            int jg, q;
-            float alpha, w;
-            const bool ok = grid_coords(g, rec.z, rec.w, jg, alpha, q, w) && live;
-            const float2 v = apply_echo(p, make_float2(rec.x, rec.y), rec.z, kEcho);
-            const uint32_t e = ((uint32_t)(jg >> 1) * pitch + (uint32_t)q) * 2u;
-            at0[u] = ok ? e + (uint32_t)(jg & 1) : kNoEntry;
-            at1[u] = ok ? e + ((jg & 1) ? 2u * pitch : 1u) : kNoEntry;
-            wgt[u] = w;
-            const float a0 = 1.0f - alpha;
-            add[u] = make_float4(a0 * v.x, a0 * v.y, alpha * v.x, alpha * v.y);
-        }
+        const float4 rec = s_ring[slot * kStageRecs + lane];
+        int side;
+        const uint32_t key = (uint32_t)lane < count ? range_key(p.key, rec.z, side) : kOutOfRange;
         // Every lane has read the slot: refill it kStages stages ahead.
         __syncwarp();
         if(lane == 0) {
@@ -282,28 +290,9 @@ k_prec_accumulate_staged(const float4* __restrict__ samples, uint64_t n, BinPara
             const uint64_t next = c + (uint64_t)kStages * stride;
             if(next < stages) issue(next, slot);
         }
-        // Lanes 2k and 2k + 1 deposit together: first the even lane's
-        // sample (row jg from the even lane, jg + 1 from the odd one), then
-        // the odd lane's, so each reduction instruction sends a sample's two
-        // rows of an interval as one sector when jg is even. Each lane keeps
-        // one node's share of its own sample and trades the other's.
-        const bool odd = (lane & 1) != 0;
-#pragma unroll
-        for(int u = 0; u < kStagedPerThread; u++) {
-            // (Set once the first samples are in: a read instead of an atomic.)
-            if(key[u] != kOutOfRange && !(s_bits[key[u] >> 5] >> (key[u] & 31) & 1u))
-                atomicOr(&s_bits[key[u] >> 5], 1u << (key[u] & 31));
-            const uint32_t keep = odd ? at1[u] : at0[u];
-            const float2 keep_v = odd ? make_float2(add[u].z, add[u].w) : make_float2(add[u].x, add[u].y);
-            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? at0[u] : at1[u], 1);
-            float2 got_v;
-            got_v.x = __shfl_xor_sync(0xffffffffu, odd ? add[u].x : add[u].z, 1);
-            got_v.y = __shfl_xor_sync(0xffffffffu, odd ? add[u].y : add[u].w, 1);
-            const float got_w = __shfl_xor_sync(0xffffffffu, wgt[u], 1);
-            const uint32_t first = odd ? got : keep, second = odd ? keep : got;
-            if(first != kNoEntry) deposit(G + first, odd ? got_w : wgt[u], odd ? got_v : keep_v, keep_pol);
-            if(second != kNoEntry) deposit(G + second, odd ? wgt[u] : got_w, odd ? keep_v : got_v, keep_pol);
-        }
+        // (Set once the first samples are in: a read instead of an atomic.)
+        if(key != kOutOfRange && !(s_bits[key >> 5] >> (key & 31) & 1u)) atomicOr(&s_bits[key >> 5], 1u << (key & 31));
+        deposit_warp(g, p, kEcho, rec, key != kOutOfRange, G, G, keep_pol, [](int, int) { return kNoEntry; });
     }
     if(aborted && lane == 0) {
         atomicOr(err, kErrAccumulateTimeout);
@@ -440,7 +429,7 @@ __global__ void __launch_bounds__(kHotPickThreads) k_hot_pick(uint32_t* __restri
     __syncthreads();
     const uint32_t H = min((uint32_t)kHotRows, nR);
     unsigned long long best = 0ull;   // (window count << 32) | (0xFFFFFFFF - start): ties go to the lowest start
-    for(uint32_t s = threadIdx.x; s + H <= nR; s += blockDim.x) {
+    for(uint32_t s = 2 * threadIdx.x; s + H <= nR; s += 2 * blockDim.x) {   // whole row pairs
         const uint32_t w = s_pre[s + H] - s_pre[s];
         const unsigned long long key = ((unsigned long long)w << 32) | (0xFFFFFFFFu - s);
         best = key > best ? key : best;
@@ -455,7 +444,8 @@ __global__ void __launch_bounds__(kHotPickThreads) k_hot_pick(uint32_t* __restri
 }
 
 // Adds the replicas of the hot rows into the grid once every sample is in
-// (nothing when the interval is empty). Replica rows of `pitch` entries.
+// (nothing when the interval is empty). Replica rows are stored in pairs like
+// the grid's: [row pair][replica][pitch][2].
 __global__ void k_hot_fold(const int2* __restrict__ hot, uint32_t pitch, const float4* __restrict__ rep,
                            float4* __restrict__ G)
 {
@@ -465,16 +455,16 @@ __global__ void k_hot_fold(const int2* __restrict__ hot, uint32_t pitch, const f
     G = after_chain(G);
     const int2 h = *after_chain(hot);
     const uint64_t total = (uint64_t)h.y * pitch;
+    const uint64_t row2 = 2 * (uint64_t)pitch;       // entries of a row pair
+    float4* first = G + grid_at(h.x, 0, pitch);
     for(uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t row = i / pitch, k = i % pitch;
-        const float4* rb = rep + row * kHotReplicas * pitch + k;
-        float4* g = G + grid_at(h.x + (int)row, (int)k, pitch);
-        float4 acc = *g;
+        const float4* rb = rep + i / row2 * kHotReplicas * row2 + i % row2;
+        float4 acc = first[i];
         for(int r = 0; r < kHotReplicas; r++) {
-            const float4 e = rb[(uint64_t)r * pitch];
+            const float4 e = rb[(uint64_t)r * row2];
             acc.x += e.x; acc.y += e.y; acc.z += e.z; acc.w += e.w;
         }
-        *g = acc;
+        first[i] = acc;
     }
 }
 
@@ -1224,7 +1214,6 @@ rtacx_status precision_begin(Context& ctx, cudaStream_t stream)
 rtacx_status precision_accumulate(Context& ctx, const void* samples, uint64_t n, cudaStream_t stream)
 {
     if(!n) return RTACX_OK;
-    const uint64_t want = (n + kAccThreads * kAccLoads - 1) / (kAccThreads * kAccLoads);
     if(!ctx.prec_hot && ctx.bin.vec4 && (reinterpret_cast<uintptr_t>(samples) & 15u) == 0) {
         const int m = accumulate_echo_model(ctx.bin.echo_flags);
         if(ctx.acc_staged_blocks[m] > 0) {
@@ -1239,7 +1228,8 @@ rtacx_status precision_accumulate(Context& ctx, const void* samples, uint64_t n,
             return RTACX_OK;
         }
     }
-    const uint32_t blocks = (uint32_t)std::min<uint64_t>(want, (uint64_t)ctx.sm_count * ctx.acc_blocks_per_sm);
+    const uint32_t blocks = (uint32_t)std::min<uint64_t>((n + kAccThreads - 1) / kAccThreads,
+                                                         (uint64_t)ctx.sm_count * ctx.acc_blocks_per_sm);
     RTACX_CUDA(launch_chained(k_prec_accumulate, blocks, kAccThreads, ctx.acc_smem, stream,
                               static_cast<const float*>(samples), n, ctx.bin, ctx.grid, ctx.d_G, ctx.d_flags,
                               ctx.prec_hot ? ctx.d_hot : nullptr, ctx.d_rep));
