@@ -30,27 +30,47 @@ namespace {
 
 constexpr double kPi = 3.14159265358979323846;
 
-__device__ __forceinline__ float mirror_coord(float u)
+// atan2f. The smaller of |x| and |y| over the larger, q in [0, 1], with one
+// Newton correction of the quotient; atan(q) = q + q^3 P(q^2), P the degree-8
+// least-squares polynomial weighted towards equal relative error (2.6e-9 in
+// exact arithmetic, 0.94 ulp in float with q exact); then the octant.
+// Magnitudes whose reciprocal or product could leave the normal range, zeros,
+// infinities and NaN take the library function.
+__device__ __forceinline__ float atan2_fast(float y, float x)
 {
-    const float t = u - 2.0f * floorf(0.5f * u);   // [0, 2)
-    return t <= 1.0f ? t : 2.0f - t;
+    const float ax = fabsf(x), ay = fabsf(y), mx = fmaxf(ax, ay), mn = fminf(ax, ay);
+    if(!(mx > 1e-30f && mx < 1e30f)) return atan2f(y, x);
+    const float r = __fdividef(1.0f, mx);
+    float q = mn * r;
+    q = fmaf(fmaf(-q, mx, mn), r, q);
+    const float s = q * q;
+    float p = -0.0017935627838596702f;
+    p = fmaf(p, s, 0.010914341546595097f);
+    p = fmaf(p, s, -0.031177351251244545f);
+    p = fmaf(p, s, 0.05795709788799286f);
+    p = fmaf(p, s, -0.08403421193361282f);
+    p = fmaf(p, s, 0.1095217615365982f);
+    p = fmaf(p, s, -0.14264239370822906f);
+    p = fmaf(p, s, 0.19998547434806824f);
+    p = fmaf(p, s, -0.33333298563957214f);
+    float a = fmaf(q * s, p, q);
+    // pi / 2 and pi as float plus the rest.
+    if(ay > ax) a = (1.57079637f - a) - 4.37113883e-8f;
+    if(__float_as_int(x) < 0) a = (3.14159274f - a) - 8.74227766e-8f;
+    return copysignf(a, y);
 }
 
-__device__ __forceinline__ int mirror_index(int i, int n)
-{
-    if(i < 0) return min(-i - 1, n - 1);
-    if(i >= n) return max(2 * n - i - 1, 0);
-    return i;
-}
-
-// Bilinear lookup of a [h][w] table at normalized (u, v), mirror addressing.
+// Bilinear lookup of a [h][w] table at normalized (u, v) in [-1, 1] (an angle
+// over pi), mirror addressing: the mirrored coordinate is |u|, and only the
+// texels one step beyond either edge fold back, onto the edge.
 __device__ __forceinline__ float directivity_lookup(const float* __restrict__ tab, int w, int h, float u, float v)
 {
-    const float x = mirror_coord(u) * (float)w - 0.5f, y = mirror_coord(v) * (float)h - 0.5f;
-    const float fx = floorf(x), fy = floorf(y);
-    const float ax = x - fx, ay = y - fy;
-    const int x0 = mirror_index((int)fx, w), x1 = mirror_index((int)fx + 1, w);
-    const int y0 = mirror_index((int)fy, h), y1 = mirror_index((int)fy + 1, h);
+    int x0, y0;
+    const float x = fabsf(u) * (float)w - 0.5f, y = fabsf(v) * (float)h - 0.5f;
+    const float ax = x - floor_small(x, x0), ay = y - floor_small(y, y0);
+    const int x1 = min(x0 + 1, w - 1), y1 = min(y0 + 1, h - 1);
+    x0 = min(max(x0, 0), w - 1);
+    y0 = min(max(y0, 0), h - 1);
     const float t00 = __ldg(tab + (size_t)y0 * w + x0), t01 = __ldg(tab + (size_t)y0 * w + x1);
     const float t10 = __ldg(tab + (size_t)y1 * w + x0), t11 = __ldg(tab + (size_t)y1 * w + x1);
     const float top = fmaf(ax, t01 - t00, t00), bot = fmaf(ax, t11 - t10, t10);
@@ -66,52 +86,76 @@ struct ReceiverParams {
     int dims;
 };
 
+// One hit to its record (a null record without a hit).
+__device__ __forceinline__ float4 make_sample(const rtacx_echo& e, const ReceiverParams& rp, const float* __restrict__ dir_tab)
+{
+    const float d = e.distance;
+    if(!(d >= 1.0e-4f)) return make_float4(0.0f, 0.0f, -1.0f, 0.0f);
+    float2 v = make_float2(e.re, e.im);
+    if(rp.flags & RTACX_ECHO_PHASE) {
+        // Below 2^22 cycles the float-rounded cycle count is within
+        // one of the nearest integer and the one-FMA reduction lands in
+        // [-0.5, 0.5]; longer (or infinite) travels take the full FP64
+        // reduction. |phase| <= pi: the hardware sine / cosine are
+        // accurate to ~4e-7 there.
+        float frac;
+        if(d * rp.cycles_hi < 4194304.0f) frac = carrier_fraction_f64(d, rp.cycles, rp.cycles_hi);
+        else {
+            const double cyc = (double)d * rp.cycles;
+            frac = (float)(cyc - rint(cyc));
+        }
+        float sn, cs;
+        __sincosf(frac * 6.28318530717958647692f, &sn, &cs);
+        v = make_float2(v.x * cs - v.y * sn, v.x * sn + v.y * cs);
+    }
+    if(rp.flags & RTACX_ECHO_SPREADING) {
+        const float inv = __fdividef(1.0f, d * d);
+        v = make_float2(v.x * inv, v.y * inv);
+    }
+    // receiver frame: R^T * dir (column k of R dotted with dir)
+    const float lx = fmaf(rp.R[0], e.dir_x, fmaf(rp.R[3], e.dir_y, rp.R[6] * e.dir_z));
+    const float ly = fmaf(rp.R[1], e.dir_x, fmaf(rp.R[4], e.dir_y, rp.R[7] * e.dir_z));
+    const float lz = fmaf(rp.R[2], e.dir_x, fmaf(rp.R[5], e.dir_y, rp.R[8] * e.dir_z));
+    // atan2 is odd in its first argument: atan2(-ly, lx) = -atan2(ly, lx).
+    const float az = atan2_fast(ly, lx);
+    if(rp.dir_w > 0) {
+        const float g = directivity_lookup(dir_tab, rp.dir_w, rp.dir_h, az * 0.318309886183790671538f,
+                                           atan2_fast(lz, lx) * 0.318309886183790671538f);
+        v = make_float2(v.x * g, v.y * g);
+    }
+    return make_float4(v.x, v.y, d, -az);
+}
+
+// Two hits per thread in flight; PAIRS: the 24-byte hits as three 8-byte
+// loads (8-byte aligned hits). Bound by issue (224 instructions per hit next
+// to its 40 bytes): 2^22 hits with phase, spreading and directivity 41.0 us
+// with 4-byte loads, one hit at a time and the library's atan2f, 37.6 without
+// the latter's replacement, 36.7 as it is; with the directivity table in
+// shared memory 41.6.
+template <bool PAIRS>
 __global__ void k_make_samples(const rtacx_echo* __restrict__ hits, uint64_t n, ReceiverParams rp,
                                const float* __restrict__ dir_tab, float* __restrict__ out)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for(uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-        const rtacx_echo e = hits[i];
-        float re = 0.0f, im = 0.0f, travel = -1.0f, bearing = 0.0f;
-        const float d = e.distance;
-        if(d >= 1.0e-4f) {
-            float2 v = make_float2(e.re, e.im);
-            if(rp.flags & RTACX_ECHO_PHASE) {
-                // Below 2^22 cycles the float-rounded cycle count is within
-                // one of the nearest integer and the one-FMA reduction lands in
-                // [-0.5, 0.5]; longer (or infinite) travels take the full FP64
-                // reduction. |phase| <= pi: the hardware sine / cosine are
-                // accurate to ~4e-7 there.
-                float frac;
-                if(d * rp.cycles_hi < 4194304.0f) frac = carrier_fraction_f64(d, rp.cycles, rp.cycles_hi);
-                else {
-                    const double cyc = (double)d * rp.cycles;
-                    frac = (float)(cyc - rint(cyc));
-                }
-                float sn, cs;
-                __sincosf(frac * 6.28318530717958647692f, &sn, &cs);
-                v = make_float2(v.x * cs - v.y * sn, v.x * sn + v.y * cs);
-            }
-            if(rp.flags & RTACX_ECHO_SPREADING) {
-                const float inv = __fdividef(1.0f, d * d);
-                v = make_float2(v.x * inv, v.y * inv);
-            }
-            // receiver frame: R^T * dir (column k of R dotted with dir)
-            const float lx = fmaf(rp.R[0], e.dir_x, fmaf(rp.R[3], e.dir_y, rp.R[6] * e.dir_z));
-            const float ly = fmaf(rp.R[1], e.dir_x, fmaf(rp.R[4], e.dir_y, rp.R[7] * e.dir_z));
-            const float lz = fmaf(rp.R[2], e.dir_x, fmaf(rp.R[5], e.dir_y, rp.R[8] * e.dir_z));
-            // atan2 is odd in its first argument: atan2(-ly, lx) = -atan2(ly, lx).
-            const float az = atan2f(ly, lx);
-            if(rp.dir_w > 0) {
-                const float g = directivity_lookup(dir_tab, rp.dir_w, rp.dir_h, az * 0.318309886183790671538f,
-                                                   atan2f(lz, lx) * 0.318309886183790671538f);
-                v = make_float2(v.x * g, v.y * g);
-            }
-            re = v.x; im = v.y; travel = d;
-            bearing = -az;
+    auto load = [&](uint64_t i) {
+        rtacx_echo e;
+        if(PAIRS) {
+            const float2* q = reinterpret_cast<const float2*>(hits + i);
+            const float2 a = __ldcs(q), b = __ldcs(q + 1), c = __ldcs(q + 2);
+            e = rtacx_echo{a.x, a.y, b.x, b.y, c.x, c.y};
         }
-        if(rp.dims == 2) reinterpret_cast<float4*>(out)[i] = make_float4(re, im, travel, bearing);
-        else { out[3 * i] = re; out[3 * i + 1] = im; out[3 * i + 2] = travel; }
+        else e = hits[i];
+        return e;
+    };
+    auto store = [&](uint64_t i, const float4& r) {
+        if(rp.dims == 2) __stcs(reinterpret_cast<float4*>(out) + i, r);
+        else { out[3 * i] = r.x; out[3 * i + 1] = r.y; out[3 * i + 2] = r.z; }
+    };
+    for(uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += 2 * stride) {
+        const bool two = i + stride < n;
+        const rtacx_echo e0 = load(i), e1 = two ? load(i + stride) : rtacx_echo{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        store(i, make_sample(e0, rp, dir_tab));
+        if(two) store(i + stride, make_sample(e1, rp, dir_tab));
     }
 }
 
@@ -212,7 +256,8 @@ rtacx_status make_samples(Context& c, const rtacx_echo* hits, uint64_t n, void* 
     rp.cycles_hi = (float)rp.cycles;
     rp.dims = c.dims;
     const uint32_t blocks = (uint32_t)std::min<uint64_t>((n + 255) / 256, (uint64_t)c.sm_count * 16);
-    k_make_samples<<<blocks, 256, 0, stream>>>(hits, n, rp, c.d_dir, static_cast<float*>(samples));
+    auto fn = reinterpret_cast<uintptr_t>(hits) % 8 == 0 ? k_make_samples<true> : k_make_samples<false>;
+    fn<<<blocks, 256, 0, stream>>>(hits, n, rp, c.d_dir, static_cast<float*>(samples));
     const cudaError_t e = cudaGetLastError();
     if(e != cudaSuccess) { c.error = std::string("k_make_samples: ") + cudaGetErrorString(e); return RTACX_ERR_CUDA; }
     return RTACX_OK;
