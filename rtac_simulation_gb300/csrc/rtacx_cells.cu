@@ -27,6 +27,7 @@ constexpr int kCellThreads = 256, kCellWarps = kCellThreads / 32;
 constexpr size_t kMaxCellBytes = (size_t)1 << 30;      // cell rows of one context
 constexpr double kMaxKnot = 0.01;
 constexpr uint32_t kCellBins = 12288;
+constexpr uint32_t kMinUnit = 8;
 
 size_t cells_smem(int W, bool pairs)
 {
@@ -35,7 +36,7 @@ size_t cells_smem(int W, bool pairs)
 
 template <int BPL, bool SHARED, bool PAIR>
 __global__ void __launch_bounds__(kCellThreads, BPL == 2 ? 3 : 2)
-k_cells(const CellPing ping, const uint32_t* __restrict__ total, uint32_t unit)
+k_cells(const CellPing ping, const uint32_t* __restrict__ total)
 {
     CellPing P = ping;
     extern __shared__ __align__(16) unsigned char s_raw[];
@@ -49,12 +50,14 @@ k_cells(const CellPing ping, const uint32_t* __restrict__ total, uint32_t unit)
     BeamLookup beam;
     beam.init(P.beam_axis);
     const uint32_t m = *after_chain(total);
-    for(uint64_t u = (uint64_t)(blockIdx.x * kCellWarps + (threadIdx.x >> 5)) * unit; u < m;
-        u += (uint64_t)gridDim.x * kCellWarps * unit)
+    // Equal units, so that the resident warps all end in the same round.
+    const uint32_t warps = gridDim.x * kCellWarps, rounds = (uint32_t)(((uint64_t)m + (uint64_t)warps * kUnit - 1) / ((uint64_t)warps * kUnit));
+    const uint32_t unit = max(kMinUnit, (uint32_t)(((uint64_t)m + (uint64_t)warps * rounds - 1) / max((uint64_t)warps * rounds, (uint64_t)1)));
+    for(uint64_t u = (uint64_t)(blockIdx.x * kCellWarps + (threadIdx.x >> 5)) * unit; u < m; u += (uint64_t)warps * unit)
         accumulate_unit<BPL, SHARED, PAIR>(P, (uint32_t)u, min(unit, m - (uint32_t)u), blockIdx.y, gridDim.y, S, tab, beam);
 }
 
-using CellsFn = void (*)(const CellPing, const uint32_t*, uint32_t);
+using CellsFn = void (*)(const CellPing, const uint32_t*);
 template <bool PAIR>
 CellsFn cells_fn_of(int bpl, bool shared_out)
 {
@@ -441,7 +444,9 @@ bool configure_cells(Context& c, double beam_support)
     if(ok) ok = raise_smem_limit((const void*)cells_fn(bpl, shared_out, c.cell_pairs), cells_smem(W, c.cell_pairs)) == cudaSuccess &&
                 (c.cell_pairs ||
                  raise_smem_limit((const void*)k_cells_filter, filter_smem(H)) == cudaSuccess);
-    if(!ok) { free_cells(c); return false; }
+    if(ok) ok = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.cell_ctas, cells_fn(bpl, shared_out, c.cell_pairs), kCellThreads,
+                                                              cells_smem(W, c.cell_pairs)) == cudaSuccess && c.cell_ctas > 0;
+    if(!ok) { cudaGetLastError(); free_cells(c); return false; }
     set_ping_params(c);
     c.cells_on = true;
     return true;
@@ -500,17 +505,16 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
         c.sorted_cells_n = n;
         c.sorted_input_order = false;
         c.mark(5, false, stream);
-        // Units of fewer samples while that leaves the SMs' warps without one;
-        // wide beams' windows are then also shared out over blockIdx.y.
-        const uint32_t warps = (uint32_t)c.sm_count * 3u * kCellWarps;
-        uint32_t unit = kUnit;
-        while(unit > 32 && n < (uint64_t)warps * unit * 2) unit /= 2;
-        const uint64_t ctas = (n + (uint64_t)unit * kCellWarps - 1) / ((uint64_t)unit * kCellWarps);
-        const uint32_t gx = (uint32_t)std::min<uint64_t>(ctas, (uint64_t)c.sm_count * 12u);
-        const uint32_t gy = c.cell_shared ? (uint32_t)std::min<uint64_t>((uint64_t)P.windows,
-                                                std::max<uint64_t>(1, (uint64_t)c.sm_count * 3u / gx)) : 1u;
+        // As many CTAs as are resident (twice that for wide beams, whose units
+        // are long: the SMs' shares even out, 2^22 samples 1240 -> 1222 us);
+        // wide beams' windows are also shared out over blockIdx.y where the
+        // samples alone leave SMs idle.
+        const uint32_t resident = (uint32_t)(c.sm_count * c.cell_ctas);
+        const uint32_t gx = (uint32_t)std::min<uint64_t>((n + kMinUnit * kCellWarps - 1) / (kMinUnit * kCellWarps),
+                                                             c.cell_shared ? 2 * resident : resident);
+        const uint32_t gy = c.cell_shared ? std::min((uint32_t)P.windows, std::max(1u, resident / gx)) : 1u;
         e = launch_chained(cells_fn(c.cell_bpl, c.cell_shared, c.cell_pairs), dim3(gx, gy), kCellThreads,
-                           cells_smem(P.beam_axis.n, c.cell_pairs), stream, P, c.d_offsets + bin.nBins, unit);
+                           cells_smem(P.beam_axis.n, c.cell_pairs), stream, P, c.d_offsets + bin.nBins);
         const dim3 fgrid(P.pitch / 32, (c.nR + kFilterWarps * kFilterRows - 1) / (kFilterWarps * kFilterRows));
         if(e == cudaSuccess)
             e = c.cell_pairs ? launch_chained(k_pairs_join, c.nR, std::min(256u, P.pitch), 0, stream, P, c.d_nonempty)

@@ -551,6 +551,7 @@ struct Context {
     // Cell form of a 2D ping (rtacx_cells.cu).
     bool cells_on = false;
     int cell_bpl = 2;                   // bearings per lane
+    int cell_ctas = 1;                  // resident CTAs of the accumulation per SM
     bool cell_shared = false;           // windows shared out: every sample reaches every window
     bool cell_pairs = false;            // row pairs instead of knot cells
     bool cell_rows = false;             // 1D without knot cells: row by row
