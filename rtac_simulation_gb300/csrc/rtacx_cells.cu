@@ -10,7 +10,8 @@
 // rtacx_reduce, us): 2^20 samples, 512 x 1024, 33 taps, narrow beams: 1384 ->
 // 135; 2^22 samples, 512 x 4096, wide beams: 14433 -> 1247; 150003 samples,
 // 387 x 777, 24 taps: 246 -> 62; 20000 samples, 256 x 500, row pairs: 91 -> 38. k_cells is bound by the beam lookups' shared
-// memory and issue slots, at one lookup per (sample, bearing). 1D, us: 20000
+// memory (single tables) and by the FMA pipe (16 copies), at one lookup per
+// (sample, bearing). 1D, us: 20000
 // samples 1049 ranges (row by row) 32.1 -> 13.5; 3e6 samples 4096 ranges, 65
 // taps 380 -> 43.
 #include "rtacx_cells.cuh"
@@ -23,8 +24,16 @@ namespace rtacx {
 
 namespace {
 
-constexpr int kCellThreads = 256, kCellWarps = kCellThreads / 32;
+// Warps per CTA: 8, two or three CTAs per SM; with a replicated table one CTA
+// of as many warps. Narrow beams' tables (up to 606 taps for 64-bearing
+// windows, 1006 for 128) fit 16 times: a copy for each pair of banks, so that
+// a lookup takes two wavefronts instead of three and more, and four samples'
+// lookups in flight pay off. 2^20 samples, 512 x 1024: 111 -> 101 us; 150003
+// samples, 387 x 777: 49 -> 46.6. Fewer warps (20): 109.
+__host__ __device__ constexpr int cell_warps(int bpl, int copies) { return copies == 1 ? 8 : bpl == 2 ? 24 : 16; }
+constexpr int kTableCopies = 16;
 constexpr size_t kMaxCellBytes = (size_t)1 << 30;      // cell rows of one context
+constexpr size_t kMaxCellSmem = 226 * 1024;
 constexpr double kMaxKnot = 0.01;
 constexpr uint32_t kCellBins = 12288;
 // Fewest samples of a warp's unit (20000 samples, 256 x 500, us per ping: 8
@@ -33,45 +42,49 @@ constexpr uint32_t kCellBins = 12288;
 // samples, 512 x 1024, 135 -> 124 us.
 constexpr uint32_t kMinUnit = 32;
 
-size_t cells_smem(int W, bool pairs)
+size_t cells_smem(int W, bool pairs, int bpl, int copies)
 {
-    return kCellWarps * (pairs ? sizeof(CellWarpSmem<true>) : sizeof(CellWarpSmem<false>)) + (size_t)(W + 2) * sizeof(float2);
+    return cell_warps(bpl, copies) * (pairs ? sizeof(CellWarpSmem<true>) : sizeof(CellWarpSmem<false>)) +
+           (size_t)(W + 2) * copies * sizeof(float2);
 }
 
-template <int BPL, bool SHARED, bool PAIR>
-__global__ void __launch_bounds__(kCellThreads, BPL == 2 ? 3 : 2)
+template <int BPL, bool SHARED, bool PAIR, int COPIES>
+__global__ void __launch_bounds__(32 * cell_warps(BPL, COPIES), COPIES > 1 ? 1 : BPL == 2 ? 3 : 2)
 k_cells(const CellPing ping, const uint32_t* __restrict__ total)
 {
+    constexpr int kWarps = cell_warps(BPL, COPIES);
     CellPing P = ping;
     extern __shared__ __align__(16) unsigned char s_raw[];
     CellWarpSmem<PAIR>& S = reinterpret_cast<CellWarpSmem<PAIR>*>(s_raw)[threadIdx.x >> 5];
-    float2* tab = reinterpret_cast<float2*>(s_raw + kCellWarps * sizeof(CellWarpSmem<PAIR>));
+    float2* tab = reinterpret_cast<float2*>(s_raw + kWarps * sizeof(CellWarpSmem<PAIR>));
     chain_next();
-    load_beam_table(tab, P.beam, P.beam_axis.n, threadIdx.x, kCellThreads);
+    load_beam_table<COPIES>(tab, P.beam, P.beam_axis.n, threadIdx.x, 32 * kWarps);
     __syncthreads();
     chain_wait();
     P.sorted = after_chain(P.sorted);
-    BeamLookup beam;
+    BeamLookup<COPIES> beam;
     beam.init(P.beam_axis);
+    tab += threadIdx.x & (COPIES - 1);
     const uint32_t m = *after_chain(total);
     // Equal units, so that the resident warps all end in the same round.
-    const uint32_t warps = gridDim.x * kCellWarps, rounds = (uint32_t)(((uint64_t)m + (uint64_t)warps * kUnit - 1) / ((uint64_t)warps * kUnit));
-    const uint32_t unit = max(kMinUnit, (uint32_t)(((uint64_t)m + (uint64_t)warps * rounds - 1) / max((uint64_t)warps * rounds, (uint64_t)1)));
-    for(uint64_t u = (uint64_t)(blockIdx.x * kCellWarps + (threadIdx.x >> 5)) * unit; u < m; u += (uint64_t)warps * unit)
+    const uint64_t warps = (uint64_t)gridDim.x * kWarps, rounds = (m + warps * kUnit - 1) / (warps * kUnit);
+    const uint32_t unit = max((uint32_t)kMinUnit, (uint32_t)((m + warps * rounds - 1) / max(warps * rounds, (uint64_t)1)));
+    for(uint64_t u = (uint64_t)(blockIdx.x * kWarps + (threadIdx.x >> 5)) * unit; u < m; u += warps * unit)
         accumulate_unit<BPL, SHARED, PAIR>(P, (uint32_t)u, min(unit, m - (uint32_t)u), blockIdx.y, gridDim.y, S, tab, beam);
 }
 
 using CellsFn = void (*)(const CellPing, const uint32_t*);
-template <bool PAIR>
-CellsFn cells_fn_of(int bpl, bool shared_out)
+CellsFn cells_fn(int bpl, bool shared_out, bool pairs, int copies)
 {
-    if(shared_out) return bpl == 4 ? k_cells<4, true, PAIR> : k_cells<2, true, PAIR>;
-    return bpl == 4 ? k_cells<4, false, PAIR> : k_cells<2, false, PAIR>;
+    if(copies > 1) return bpl == 4 ? k_cells<4, false, false, kTableCopies> : k_cells<2, false, false, kTableCopies>;
+    if(pairs)
+        return shared_out ? (bpl == 4 ? k_cells<4, true, true, 1> : k_cells<2, true, true, 1>)
+                          : (bpl == 4 ? k_cells<4, false, true, 1> : k_cells<2, false, true, 1>);
+    return shared_out ? (bpl == 4 ? k_cells<4, true, false, 1> : k_cells<2, true, false, 1>)
+                      : (bpl == 4 ? k_cells<4, false, false, 1> : k_cells<2, false, false, 1>);
 }
-CellsFn cells_fn(int bpl, bool shared_out, bool pairs)
-{
-    return pairs ? cells_fn_of<true>(bpl, shared_out) : cells_fn_of<false>(bpl, shared_out);
-}
+CellsFn cells_fn(const Context& c) { return cells_fn(c.cell_bpl, c.cell_shared, c.cell_pairs, c.cell_copies); }
+size_t cells_smem(const Context& c) { return cells_smem((int)c.W, c.cell_pairs, c.cell_bpl, c.cell_copies); }
 
 // Zeroes what a ping's passes add into: the bin totals, the range-bin bitmap,
 // the cell rows and the ping (8-byte stores: the ping's alignment).
@@ -384,6 +397,7 @@ bool configure_cells(Context& c, double beam_support)
     const bool shared_out = bpl == 0;
     if(shared_out) bpl = nB > 64 ? 4 : 2;
     const int len = 32 * bpl;
+    const int copies = !shared_out && !c.cell_pairs && cells_smem(W, false, bpl, kTableCopies) <= kMaxCellSmem ? kTableCopies : 1;
     // Order of the bearings in a window. For one sample the table entries of
     // two bearings differ by their distance in taps, whatever the sample;
     // lanes whose distances differ modulo the 16 eight-byte banks of shared
@@ -393,6 +407,7 @@ bool configure_cells(Context& c, double beam_support)
     // (counted for the tables of the imaging sensors).
     const double kb = (double)c.red.beam_axis.k_hi;
     auto deal = [&](std::vector<int> order, std::vector<int>& pos, size_t at) {
+        if(copies > 1) { std::copy(order.begin(), order.end(), pos.begin() + at); return; }
         auto bank = [&](int i) { const double x = (double)c.bearings[i] * kb; return x - 16.0 * std::floor(x / 16.0); };
         std::stable_sort(order.begin(), order.end(), [&](int a, int d) { return bank(a) < bank(d); });
         const size_t groups = std::max<size_t>(1, (order.size() + 15) / 16);
@@ -411,6 +426,7 @@ bool configure_cells(Context& c, double beam_support)
     }
     c.cell_bpl = bpl;
     c.cell_shared = shared_out;
+    c.cell_copies = copies;
     c.cell.windows = (int)(pos.size() / len);
     // Sort order: window x cell block, with as many bins as the pipelined
     // scatter takes at one reservation batch per thread.
@@ -440,16 +456,16 @@ bool configure_cells(Context& c, double beam_support)
         col_bearing[col[p]] = pos[p];
     }
     const size_t cell_bytes = (size_t)cp.cells * pitch * sizeof(float4);
-    if(cell_bytes > kMaxCellBytes || cells_smem(W, c.cell_pairs) > 200 * 1024 ||
+    if(cell_bytes > kMaxCellBytes || cells_smem(c) > kMaxCellSmem ||
        (!c.cell_pairs && filter_smem(H) > 200 * 1024)) return false;
     bool ok = put(c.d_cell_taps, cell_taps(c, f)) && put(c.d_row_dev, f.dev) && put(c.d_nonempty, std::vector<uint32_t>((nR + 127) / 128 * 4, 0u)) &&
               put(c.d_pos_theta, theta) && put(c.d_pos_col, col) && put(c.d_col_bearing, col_bearing);
     if(ok && cudaMalloc(&c.d_cells, cell_bytes) != cudaSuccess) { cudaGetLastError(); ok = false; }
-    if(ok) ok = raise_smem_limit((const void*)cells_fn(bpl, shared_out, c.cell_pairs), cells_smem(W, c.cell_pairs)) == cudaSuccess &&
+    if(ok) ok = raise_smem_limit((const void*)cells_fn(c), cells_smem(c)) == cudaSuccess &&
                 (c.cell_pairs ||
                  raise_smem_limit((const void*)k_cells_filter, filter_smem(H)) == cudaSuccess);
-    if(ok) ok = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.cell_ctas, cells_fn(bpl, shared_out, c.cell_pairs), kCellThreads,
-                                                              cells_smem(W, c.cell_pairs)) == cudaSuccess && c.cell_ctas > 0;
+    if(ok) ok = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.cell_ctas, cells_fn(c), 32 * cell_warps(bpl, copies),
+                                                              cells_smem(c)) == cudaSuccess && c.cell_ctas > 0;
     if(!ok) { cudaGetLastError(); free_cells(c); return false; }
     set_ping_params(c);
     c.cells_on = true;
@@ -513,12 +529,12 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
         // are long: the SMs' shares even out, 2^22 samples 1240 -> 1222 us);
         // wide beams' windows are also shared out over blockIdx.y where the
         // samples alone leave SMs idle.
+        const uint32_t warps = (uint32_t)cell_warps(c.cell_bpl, c.cell_copies);
         const uint32_t resident = (uint32_t)(c.sm_count * c.cell_ctas);
-        const uint32_t gx = (uint32_t)std::min<uint64_t>((n + kMinUnit * kCellWarps - 1) / (kMinUnit * kCellWarps),
+        const uint32_t gx = (uint32_t)std::min<uint64_t>((n + kMinUnit * warps - 1) / (kMinUnit * warps),
                                                              c.cell_shared ? 2 * resident : resident);
         const uint32_t gy = c.cell_shared ? std::min((uint32_t)P.windows, std::max(1u, resident / gx)) : 1u;
-        e = launch_chained(cells_fn(c.cell_bpl, c.cell_shared, c.cell_pairs), dim3(gx, gy), kCellThreads,
-                           cells_smem(P.beam_axis.n, c.cell_pairs), stream, P, c.d_offsets + bin.nBins);
+        e = launch_chained(cells_fn(c), dim3(gx, gy), 32 * warps, cells_smem(c), stream, P, c.d_offsets + bin.nBins);
         const dim3 fgrid(P.pitch / 32, (c.nR + kFilterWarps * kFilterRows - 1) / (kFilterWarps * kFilterRows));
         if(e == cudaSuccess)
             e = c.cell_pairs ? launch_chained(k_pairs_join, c.nR, std::min(256u, P.pitch), 0, stream, P, c.d_nonempty)

@@ -101,17 +101,21 @@ __device__ __forceinline__ float2 pulse_at(const float2* __restrict__ pad, const
 // An even table's texel coordinates are half-integers: its entries are stored
 // from the middle of the piece, so that the constant of the fraction is a
 // whole number either way (see BeamLookup).
+// COPIES 16: entry i of copy k at 16 i + k, so that lanes that read the copy of
+// their own pair of banks never conflict (see k_cells).
+template <int COPIES = 1>
 __device__ __forceinline__ void load_beam_table(float2* tab, const float* __restrict__ beam_pad, int W, int tid,
                                                 int threads)
 {
-    for(int i = tid; i <= W + 1; i += threads) {
+    for(int k = tid; k < (W + 2) * COPIES; k += threads) {
+        const int i = k / COPIES;
         float2 e = make_float2(0.f, 0.f);
         if(i <= W) {
             const float lo = beam_pad[i], hi = beam_pad[i + 1];
             e.y = hi - lo;
             e.x = (W & 1) ? lo : fmaf(0.5f, e.y, lo);
         }
-        tab[i] = e;
+        tab[k] = e;
     }
 }
 
@@ -123,6 +127,8 @@ __device__ __forceinline__ void load_beam_table(float2* tab, const float* __rest
 constexpr float kRoundMagic = 12582912.0f;          // 1.5 * 2^23
 constexpr uint32_t kRoundMagicBits = 0x4B400000u;
 
+// tab: the table, at the lane's copy.
+template <int COPIES = 1>
 struct BeamLookup {
     f32x2 k2, k_lo2, c2, magic2, frac2, minus2;
     uint32_t last;                                   // W + 1
@@ -147,8 +153,8 @@ struct BeamLookup {
         const f32x2 y = add2(fma2(d, k2, c2), magic2);
         const f32x2 a = fma2(d, k2, fma2(d, k_lo2, fma2(y, minus2, frac2)));
         const float2 yu = unpack2(y), au = unpack2(a);
-        const float2 e0 = tab[min(__float_as_uint(yu.x) - kRoundMagicBits, last)];
-        const float2 e1 = tab[min(__float_as_uint(yu.y) - kRoundMagicBits, last)];
+        const float2 e0 = tab[min(__float_as_uint(yu.x) - kRoundMagicBits, last) * COPIES];
+        const float2 e1 = tab[min(__float_as_uint(yu.y) - kRoundMagicBits, last) * COPIES];
         return pack2(fmaf(au.x, e0.y, e0.x), fmaf(au.y, e1.y, e1.x));
     }
 };
@@ -179,9 +185,9 @@ struct CellWarpSmem {
 
 // One sample next to a knot, row by row: the lanes take 32 rows at a time,
 // then every row's weight is broadcast and reduced into the (zeroed) ping.
-template <int BPL>
+template <int BPL, int COPIES>
 __device__ __forceinline__ void reduce_row_by_row(const CellPing& P, float4 w, float theta, int C, const float2* tab,
-                                                  const BeamLookup& beam, const f32x2 (&minus_tb)[BPL / 2],
+                                                  const BeamLookup<COPIES>& beam, const f32x2 (&minus_tb)[BPL / 2],
                                                   const int* bearing)
 {
     const int lane = threadIdx.x & 31;
@@ -217,10 +223,10 @@ __device__ __forceinline__ void reduce_row_by_row(const CellPing& P, float4 w, f
 // Accumulates samples [first, first + count) (count <= kUnit) of the sorted
 // order into the cell rows. SHARED: for the windows win0, win0 + win_step, ...;
 // otherwise for each sample's own window.
-template <int BPL, bool SHARED, bool PAIR>
+template <int BPL, bool SHARED, bool PAIR, int COPIES>
 __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t first, uint32_t count, int win0,
                                                 int win_step, CellWarpSmem<PAIR>& S, const float2* tab,
-                                                const BeamLookup& beam)
+                                                const BeamLookup<COPIES>& beam)
 {
     constexpr int NP = BPL / 2;
     const int lane = threadIdx.x & 31;
@@ -311,9 +317,12 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
             for(int w = w_begin; w < w_end; w += win_step) {
                 const int pos0 = w * 32 * BPL + lane;
                 f32x2 minus_tb[NP];
+                int2 col[NP];
 #pragma unroll
-                for(int p = 0; p < NP; p++)
+                for(int p = 0; p < NP; p++) {
                     minus_tb[p] = pack2(-P.pos_theta[pos0 + 64 * p], -P.pos_theta[pos0 + 64 * p + 32]);
+                    if(!SHARED) col[p] = make_int2(P.pos_col[pos0 + 64 * p], P.pos_col[pos0 + 64 * p + 32]);
+                }
                 int s = 0;
                 for(uint32_t left = filled; left; left &= left - 1u) {
                     const int k = __ffs(left) - 1;
@@ -323,7 +332,7 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
                     for(int p = 0; p < NP; p++)
 #pragma unroll
                         for(int e = 0; e < 4; e++) acc[p][e] = 0ull;
-#pragma unroll BPL
+#pragma unroll COPIES > 1 ? 4 : BPL
                     for(; s < end; s++) {
                         const ulonglong2 e0 = S.list[s].v[0], e1 = S.list[s].v[1];
                         f32x2 e2 = 0ull;
@@ -349,9 +358,10 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
                     for(int p = 0; p < NP; p++) {
                         const float2 a = unpack2(acc[p][0]), b = unpack2(acc[p][1]);
                         const float2 c = unpack2(acc[p][2]), d = unpack2(acc[p][3]);
-                        const int x = P.pos_col[pos0 + 64 * p], y = P.pos_col[pos0 + 64 * p + 32];
-                        if(x >= 0) red_add_f4(row + x, a.x, b.x, c.x, d.x);
-                        if(y >= 0) red_add_f4(row + y, a.y, b.y, c.y, d.y);
+                        // (shared-out windows reload the columns: registers)
+                        if(SHARED) col[p] = make_int2(P.pos_col[pos0 + 64 * p], P.pos_col[pos0 + 64 * p + 32]);
+                        if(col[p].x >= 0) red_add_f4(row + col[p].x, a.x, b.x, c.x, d.x);
+                        if(col[p].y >= 0) red_add_f4(row + col[p].y, a.y, b.y, c.y, d.y);
                     }
                 }
             }

@@ -551,6 +551,7 @@ struct Context {
     // Cell form of a 2D ping (rtacx_cells.cu).
     bool cells_on = false;
     int cell_bpl = 2;                   // bearings per lane
+    int cell_copies = 1;                // copies of the beam table in the accumulation's shared memory
     int cell_ctas = 1;                  // resident CTAs of the accumulation per SM
     bool cell_shared = false;           // windows shared out: every sample reaches every window
     bool cell_pairs = false;            // row pairs instead of knot cells

@@ -981,7 +981,7 @@ __device__ __noinline__ void batch_cells_item(const CellPing& P, int form, int b
     float2* tab = reinterpret_cast<float2*>(smem_raw + kWarps * per_warp);
     load_beam_table(tab, P.beam, P.beam_axis.n, threadIdx.x, kThreads);
     __syncthreads();
-    BeamLookup beam;
+    BeamLookup<> beam;
     beam.init(P.beam_axis);
     unsigned char* own = smem_raw + warp * per_warp;
     auto& S = *reinterpret_cast<CellWarpSmem<false>*>(own);

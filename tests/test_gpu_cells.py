@@ -57,6 +57,15 @@ def test_cells_match_fp64_oracle(oracle, n, nR, nB, taps, beam_taps, wide):
     assert rel_l2(got, want) <= TOL, rel_l2(got, want)
 
 
+@pytest.mark.parametrize("nB,beam_taps", [(65, 605), (65, 606), (65, 607), (3, 1), (3, 2), (640, 1006), (640, 1007)])
+def test_tables_around_the_replicated_limit(oracle, nB, beam_taps):
+    """Beam tables on both sides of the largest that is kept in 16 copies (for
+    64- and 128-bearing windows), and the smallest, samples of all warps."""
+    wk = ping(70001, 90, nB, 9, False, beam_taps)
+    got = gpu_reduce(make_context(wk), wk.samples, wk.out_shape)
+    assert rel_l2(got, oracle.reduce(wk.samples, wk.sensor)) <= TOL
+
+
 @pytest.mark.parametrize("change", ["half_margin", "half_tap", "long_pulse"])
 def test_sensors_off_the_cell_rule_match_fp64_oracle(oracle, change):
     """A margin that cuts the pulse's window, taps that are not one range
