@@ -202,10 +202,10 @@ bool configure_common(Context& c, const Common& s, float pulse_scale)
 
 bool allocate_bins(Context& c)
 {
-    c.sort = sort_shape(c, c.bin.nBins);
+    c.sort = sort_shape(c, c.bin.nBins, false);
     uint32_t bins = c.bin.nBins;
     if(c.cells_on) {
-        c.cell_sort = sort_shape(c, c.cell_bin.nBins);
+        c.cell_sort = sort_shape(c, c.cell_bin.nBins, c.dims == 2);
         bins = std::max(bins, c.cell_bin.nBins);
     }
     const size_t cols = (size_t)bins * kCursorStride;
@@ -268,6 +268,7 @@ void rtacx_destroy(rtacx_ctx* ctx)
     cudaSetDevice(c.device);
     free_config(c);
     free_dev(c.d_sorted);
+    free_dev(c.d_ranks);
     free_dev(c.d_dir);
     free_dev(c.d_rast_v); free_dev(c.d_rast_vis); free_dev(c.d_rast_large);
     free_streaming(c);

@@ -44,6 +44,7 @@ namespace rtacx {
 namespace {
 
 constexpr int kScanThreads = 1024;
+constexpr uint64_t kMaxRanked = 1ull << 21;          // samples of a ranked sort, at most
 
 __global__ void k_count(const float* __restrict__ samples, uint64_t n, BinParams p,
                         uint32_t* __restrict__ totals, unsigned long long* __restrict__ oor,
@@ -54,6 +55,144 @@ __global__ void k_count(const float* __restrict__ samples, uint64_t n, BinParams
     chain_next();
     chain_wait();
     count_chunk(after_chain(samples), n, p, blockIdx.x, gridDim.x, totals, oor, sh, s_oor, nonempty);
+}
+
+// Ranked sort of the cell form: the count pass also finds every sample's rank
+// in its bin, so that the scatter writes each record straight to
+// offsets[bin] + rank, without a second histogram, a tile sort and cursors.
+//   k_count_ranked    ranks among the CTA's (at most kRankTile) samples of the
+//                     bin (shared histogram, key and rank kept in one
+//                     register), the CTA's count of each pair of bins added to
+//                     the totals by one 64-bit atomic, whose old value is what
+//                     its ranks start at; the ranks are stored in input order.
+//   k_scatter_ranked  records to offsets[bin] + rank (echo model applied). The
+//                     16-byte stores fill their sectors in the L2.
+// The histogram in shared memory keeps samples of few bins (a wall, a wreck)
+// from queueing at one L2 address. Bound by latency (the samples' loads, the
+// atomics' return, the ranks' loads) and the launches. Whole pings against the
+// tile sort, us: 20000 samples, 256 x 500 26.0 -> 22.1; 150003, 387 x 777 46.7
+// -> 41.3; 2^20, 512 x 1024 100.7 -> 95.5; 2^22, 512 x 4096 1180 -> 1191 (the
+// single 16-byte stores cost more than coalesced runs), hence kMaxRanked.
+constexpr int kRankThreads = 1024, kRankLoads = 16, kRankTile = kRankThreads * kRankLoads;
+constexpr int kRankKeyBits = 14;                     // nBins <= 2^14, a CTA's ranks < 2^18
+static_assert(kRankTile <= 1 << (32 - kRankKeyBits), "key and rank share a word");
+
+__global__ void __launch_bounds__(kRankThreads, 1)
+k_count_ranked(const float* __restrict__ samples, uint64_t n, BinParams p, uint32_t* __restrict__ totals,
+               uint32_t* __restrict__ nonempty, uint32_t* __restrict__ ranks)
+{
+    extern __shared__ __align__(8) uint32_t sh[];
+    const uint32_t tid = threadIdx.x, pairs = (p.nBins + 1) / 2, words = (p.key.nR + 31) / 32;
+    const uint32_t blocks = (p.nBins + kScanBlock - 1) / kScanBlock;
+    uint32_t *s_bits = sh + 2 * pairs, *s_blk = s_bits + words;
+    uint2* s_pair = reinterpret_cast<uint2*>(sh);
+    chain_next();
+    for(uint32_t b = tid; b < 2 * pairs + words + blocks; b += kRankThreads) sh[b] = 0u;
+    __syncthreads();
+    chain_wait();
+    samples = after_chain(samples);
+    const uint64_t chunk = (n + gridDim.x - 1) / gridDim.x, begin = blockIdx.x * chunk, end = min(begin + chunk, n);
+    uint32_t kr[kRankLoads];                     // key | rank in the CTA << kRankKeyBits
+#pragma unroll
+    for(int g = 0; g < kRankLoads; g += 4) {
+        float4 rec[4];
+        if(begin + (uint64_t)g * kRankThreads >= end) {
+#pragma unroll
+            for(int u = 0; u < 4; u++) kr[g + u] = kOutOfRange;
+            continue;
+        }
+#pragma unroll
+        for(int u = 0; u < 4; u++) {
+            const uint64_t i = begin + (uint64_t)(g + u) * kRankThreads + tid;
+            rec[u] = i < end ? load_record(samples, i, p) : make_float4(0.f, 0.f, INFINITY, 0.f);
+        }
+#pragma unroll
+        for(int u = 0; u < 4; u++) {
+            int side;
+            const uint32_t r = range_key(p.key, rec[u].z, side);
+            const uint32_t k = begin + (uint64_t)(g + u) * kRankThreads + tid < end ? sample_key(p, rec[u].z, rec[u].w, side)
+                                                                                : kOutOfRange;
+            kr[g + u] = kOutOfRange;
+            if(k == kOutOfRange) continue;
+            kr[g + u] = k | atomicAdd(&sh[k], 1u) << kRankKeyBits;
+            const uint32_t bit = 1u << (r & 31u);
+            if(!(s_bits[r >> 5] & bit)) atomicOr(&s_bits[r >> 5], bit);
+        }
+    }
+    __syncthreads();
+    // The CTA's counts into the totals; the bins' entries become the first ranks.
+    constexpr int kBatch = 4;
+    for(uint32_t w0 = tid & ~31u; w0 < pairs; w0 += kBatch * kRankThreads) {
+        const uint32_t b0 = w0 + (tid & 31u);
+        uint2 c[kBatch];
+        unsigned long long old[kBatch];
+#pragma unroll
+        for(int q = 0; q < kBatch; q++) {
+            const uint32_t b = b0 + q * kRankThreads;
+            c[q] = b < pairs ? s_pair[b] : make_uint2(0u, 0u);
+            // (an odd last bin's neighbour is the first block sum)
+            if(!(c[q].x | c[q].y)) old[q] = 0ull;
+            else if(2 * b + 1 < p.nBins) old[q] = atomicAdd(reinterpret_cast<unsigned long long*>(totals) + b,
+                                                            (unsigned long long)c[q].y << 32 | c[q].x);
+            else old[q] = atomicAdd(&totals[2 * b], c[q].x);
+        }
+#pragma unroll
+        for(int q = 0; q < kBatch; q++) {
+            const uint32_t b = b0 + q * kRankThreads;
+            if(b < pairs) s_pair[b] = make_uint2((uint32_t)old[q], (uint32_t)(old[q] >> 32));
+            // (a warp's pairs lie in one block of kScanBlock bins)
+            const uint32_t sum = __reduce_add_sync(0xffffffffu, c[q].x + c[q].y);
+            if((tid & 31) == 0 && sum) atomicAdd(&s_blk[2 * b / kScanBlock], sum);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for(int u = 0; u < kRankLoads; u++) {
+        const uint64_t i = begin + (uint64_t)u * kRankThreads + tid;
+        if(kr[u] != kOutOfRange) ranks[i] = sh[kr[u] & ((1u << kRankKeyBits) - 1u)] + (kr[u] >> kRankKeyBits);
+    }
+    for(uint32_t b = tid; b < words; b += kRankThreads)
+        if(s_bits[b]) atomicOr(&nonempty[b], s_bits[b]);
+    for(uint32_t b = tid; b < blocks; b += kRankThreads)
+        if(s_blk[b]) atomicAdd(&totals[p.nBins + b], s_blk[b]);
+}
+
+template <bool ECHO>
+__global__ void __launch_bounds__(256)
+k_scatter_ranked(const float* __restrict__ samples, uint64_t n, BinParams p, const uint32_t* __restrict__ ranks,
+                 const uint32_t* __restrict__ offsets, float4* __restrict__ sorted, uint32_t* __restrict__ err)
+{
+    constexpr int U = 4;
+    chain_next();
+    chain_wait();
+    samples = after_chain(samples);
+    ranks = after_chain(ranks);
+    offsets = after_chain(offsets);
+    const uint32_t total = offsets[p.nBins];
+    const uint64_t stride = (uint64_t)gridDim.x * 256;
+    for(uint64_t i0 = blockIdx.x * (uint64_t)256 + threadIdx.x; i0 < n; i0 += U * stride) {
+        float4 rec[U];
+        uint32_t rank[U];
+#pragma unroll
+        for(int u = 0; u < U; u++) {
+            const uint64_t i = i0 + u * stride;
+            if(i < n) { rec[u] = load_record(samples, i, p); rank[u] = ranks[i]; }
+        }
+#pragma unroll
+        for(int u = 0; u < U; u++) {
+            if(i0 + u * stride >= n) break;
+            int side;
+            const uint32_t k = sample_key(p, rec[u].z, rec[u].w, side);
+            if(k == kOutOfRange) continue;
+            const uint32_t pos = offsets[k] + rank[u];
+            if(ECHO) {
+                const float2 v = apply_echo(p, make_float2(rec[u].x, rec[u].y), rec[u].z);
+                rec[u].x = v.x; rec[u].y = v.y;
+            }
+            if(pos < total) sorted[pos] = rec[u];
+            else atomicOr(err, kErrScatterOverflow);
+        }
+    }
 }
 
 // Exclusive scan of totals[0, nBins) into offsets[0, nBins] by one CTA of
@@ -310,6 +449,11 @@ __global__ void k_reset_batch(const PingDev* __restrict__ pings, uint32_t n_ping
     if(i < n_pings) { pings[i].oor[0] = 0ull; pings[i].oor[1] = 0ull; }
 }
 
+size_t ranked_smem(const BinParams& p)
+{
+    return ((p.nBins + 1) / 2 * 2 + (p.key.nR + 31) / 32 + (p.nBins + kScanBlock - 1) / kScanBlock) * sizeof(uint32_t);
+}
+
 uint32_t hist_grid(uint32_t ctas, uint64_t n)
 {
     // At least ~1024 samples per CTA so that the per-CTA histogram set-up
@@ -341,6 +485,18 @@ bool ensure_capacity(Context& ctx, uint64_t n)
     if(ctx.d_sorted) cudaFree(ctx.d_sorted);
     ctx.d_sorted = p;
     ctx.capacity = cap;
+    // Ranks for the cell form's sort, up to what it takes; without them the
+    // samples go through the tile sort.
+    if(ctx.n_ranks < std::min<uint64_t>(cap, kMaxRanked)) {
+        if(ctx.d_ranks) cudaFree(ctx.d_ranks);
+        ctx.d_ranks = nullptr;
+        ctx.n_ranks = std::min<uint64_t>(cap, kMaxRanked);
+        if(cudaMalloc(&ctx.d_ranks, ctx.n_ranks * sizeof(uint32_t)) != cudaSuccess) {
+            cudaGetLastError();
+            ctx.d_ranks = nullptr;
+            ctx.n_ranks = 0;
+        }
+    }
     ctx.sorted_cells_n = 0;
     return true;
 }
@@ -547,8 +703,14 @@ rtacx_status run_sort(Context& ctx, const BinParams& p, const SortShape& shape, 
     const size_t smem = (size_t)p.nBins * sizeof(uint32_t);
     const float* s = static_cast<const float*>(samples);
     const uint32_t scan_blocks = (p.nBins + kScanBlock - 1) / kScanBlock;
+    const bool ranked = nonempty && shape.ranked && n <= ctx.n_ranks;
     ctx.mark(0, false, stream);
-    RTACX_CUDA(launch_chained(k_count, grid, shape.hist_threads,
+    if(ranked)
+        RTACX_CUDA(launch_chained(k_count_ranked, (uint32_t)std::max(std::min<uint64_t>((uint64_t)ctx.sm_count, (n + kRankThreads - 1) / kRankThreads),
+                                                                        (n + kRankTile - 1) / kRankTile),
+                                  kRankThreads, ranked_smem(p), stream, s, n, p, ctx.d_totals, nonempty, ctx.d_ranks));
+    else
+        RTACX_CUDA(launch_chained(k_count, grid, shape.hist_threads,
                               smem + (nonempty ? (p.key.nR + 31) / 32 * sizeof(uint32_t) : 0), stream, s, n, p,
                               ctx.d_totals, ctx.d_oor, nonempty));
     ctx.mark(0, true, stream);
@@ -558,7 +720,12 @@ rtacx_status run_sort(Context& ctx, const BinParams& p, const SortShape& shape, 
                               ctx.d_offsets, ctx.d_hist));
     ctx.mark(2, true, stream);
     ctx.mark(3, false, stream);
-    if(shape.scatter_shape) {
+    if(ranked) {
+        const uint32_t g = (uint32_t)std::min<uint64_t>((n + 255) / 256, (uint64_t)ctx.sm_count * 16);
+        RTACX_CUDA(launch_chained(p.echo_flags ? k_scatter_ranked<true> : k_scatter_ranked<false>, g, 256, 0, stream, s, n, p,
+                                  ctx.d_ranks, ctx.d_offsets, ctx.d_sorted, ctx.d_err));
+    }
+    else if(shape.scatter_shape) {
         const ScatterShape& sh = kScatterShapes[shape.scatter_shape - 1];
         const uint32_t g = hist_grid((uint32_t)ctx.sm_count, n);
         const bool one_batch = pipe_bins_per_thread(p.nBins, sh.nt) <= (uint32_t)kReserveBatch;
@@ -669,7 +836,7 @@ rtacx_status launch_bin_batch(std::string& error, const PingDev* pings, uint32_t
 }
 
 // Launch shape of the count / scatter passes for a bin count.
-SortShape sort_shape(const Context& ctx, uint32_t nBins)
+SortShape sort_shape(const Context& ctx, uint32_t nBins, bool ranked)
 {
     SortShape shape;
     const size_t smem = (size_t)nBins * sizeof(uint32_t);
@@ -691,6 +858,9 @@ SortShape sort_shape(const Context& ctx, uint32_t nBins)
     };
     shape.hist_ctas = resident((const void*)k_count);
     shape.scatter_ctas = resident((const void*)k_scatter);
+    const size_t ranked_bytes = (nBins + 2 + (ctx.nR + 31) / 32 + nBins / kScanBlock + 1) * sizeof(uint32_t);
+    shape.ranked = ranked && ranked_bytes <= 100 * 1024 && nBins <= 1u << kRankKeyBits &&
+                   raise_smem_limit((const void*)k_count_ranked, ranked_bytes) == cudaSuccess;
     // Staged scatter: the first shape of kScatterShapes whose shared memory
     // fits.
     int optin = 0, smem_sm = 0;

@@ -419,6 +419,7 @@ struct SortShape {
     uint32_t hist_ctas = 0;             // CTAs of the count pass (and of the batched passes)
     uint32_t scatter_ctas = 0;          // CTAs of the per-tile scatter
     uint32_t hist_threads = 0;
+    bool ranked = false;                // ranks found by the count pass, records scattered straight to their place
     int scatter_shape = 0;              // 1 + index of the staged scatter's shape (0: per-tile scatter)
 };
 
@@ -542,6 +543,8 @@ struct Context {
     // Sample-sized scratch.
     uint64_t capacity = 0;              // samples the sorted scratch holds
     float4* d_sorted = nullptr;
+    uint64_t n_ranks = 0;               // samples d_ranks holds
+    uint32_t* d_ranks = nullptr;        // each sample's rank in its bin (ranked sort)
     SortShape sort;
     size_t acc_smem = 0;                // dynamic shared memory of the precision accumulation
     uint32_t acc_blocks_per_sm = 1;
@@ -650,7 +653,7 @@ rtacx_status run_binning(Context& ctx, const void* samples, uint64_t n, cudaStre
 // also the bitmap of range bins), scan, scatter.
 rtacx_status run_sort(Context& ctx, const BinParams& p, const SortShape& shape, const void* samples, uint64_t n,
                       uint32_t* nonempty, cudaStream_t stream);
-SortShape sort_shape(const Context& ctx, uint32_t nBins);
+SortShape sort_shape(const Context& ctx, uint32_t nBins, bool ranked);
 rtacx_status restore_sorted(Context& ctx, cudaStream_t stream);
 rtacx_status run_bin_outputs(Context& ctx, const void* samples, uint64_t n,
                              uint32_t* keys, uint32_t* segments, uint32_t* windows,

@@ -247,7 +247,7 @@ extern "C" rtacx_status rtacx_reduce_noalloc(int sample_kind, const void* sensor
     ctx.d_ranges = reinterpret_cast<float*>(base + kOffRanges);
     ctx.d_support = reinterpret_cast<int2*>(base + kOffSupport);
     ctx.d_bb_tiles = reinterpret_cast<int2*>(base + kOffTiles);
-    ctx.sort = sort_shape(ctx, ctx.bin.nBins);
+    ctx.sort = sort_shape(ctx, ctx.bin.nBins, false);
     ctx.sort.hist_ctas = std::min(ctx.sort.hist_ctas, kMaxHistCtas);
     ctx.hist_cols = (size_t)ctx.bin.nBins * kCursorStride;
     if(ctx.hist_cols * sizeof(uint32_t) > kHistBytes) return RTACX_ERR_UNSUPPORTED;

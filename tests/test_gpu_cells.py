@@ -57,6 +57,19 @@ def test_cells_match_fp64_oracle(oracle, n, nR, nB, taps, beam_taps, wide):
     assert rel_l2(got, want) <= TOL, rel_l2(got, want)
 
 
+@pytest.mark.parametrize("n", [1023, 1025, 1 << 21, (1 << 21) + 1])
+def test_pings_around_the_ranked_sort_limits(oracle, n):
+    """One count CTA and two, the most samples that are ranked and one more;
+    all samples of a wall in few bins."""
+    for wall in (False, True):
+        wk = ping(n, 41, 33, 3, False)
+        if wall:
+            wk.samples[n // 4:, 2] = 7.03
+            wk.samples[n // 4:, 3] = 0.11
+        got = gpu_reduce(make_context(wk), wk.samples, wk.out_shape)
+        assert rel_l2(got, oracle.reduce(wk.samples, wk.sensor)) <= TOL
+
+
 @pytest.mark.parametrize("nB,beam_taps", [(65, 605), (65, 606), (65, 607), (3, 1), (3, 2), (640, 1006), (640, 1007)])
 def test_tables_around_the_replicated_limit(oracle, nB, beam_taps):
     """Beam tables on both sides of the largest that is kept in 16 copies (for
