@@ -101,13 +101,17 @@ struct Batch {
         return true;
     }
 
-    // Samples of a ping's cell form that one work item takes: about 2048
-    // samples of a 64-bearing window's work, in whole rounds of the CTA's warps.
+    // Samples of a ping's cell form that one work item takes: about kItemSamples
+    // of a 64-bearing window's work, in whole rounds of the CTA's warps (16
+    // pings, 2.5e6 2D samples, us for the phase: 2048 243, its last items
+    // leaving SMs idle; 1024 226; 512 247, units of 64 samples).
+    static constexpr uint64_t kItemSamples = 1024;
     static uint32_t cells_per_item(const Context& c)
     {
         const uint64_t pairs = c.cell_shared ? c.cell.pitch : 32u * (uint32_t)c.cell_bpl;
-        const uint64_t want = 2048u * 64u / std::max<uint64_t>(pairs, 64u);
-        return want >= 2048 ? 2048u : want >= 1024 ? 1024u : want >= 512 ? 512u : 256u;
+        uint64_t want = kItemSamples;
+        while(want > 256 && want * pairs > kItemSamples * 64) want /= 2;
+        return (uint32_t)want;
     }
 
     // Whether the batch runs on the fused kernel with the cell form: when the
@@ -177,6 +181,11 @@ struct Batch {
                 for(uint32_t y = 0; y < rows; y++)
                     for(uint32_t x = 0; x < columns; x++) filters.push_back(make_uint4(i, x, y, 0));
                 gather_smem = std::max(gather_smem, batch_cells_smem(c));
+                if(c.dims == 2 && c.cell_sort.ranked && n <= c.n_ranks) {
+                    d.ranks = c.d_ranks;
+                    d.chunks = (uint32_t)std::max<uint64_t>(1, ceil_div(n, kRankedChunk));
+                    gather_smem = std::max(gather_smem, ranked_smem(d.bin.nBins, c.nR));
+                }
             }
             if(cell_form && c.dims == 1) {
                 d.chunks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sm_count * 8, ceil_div(n, cand.per_cta)));

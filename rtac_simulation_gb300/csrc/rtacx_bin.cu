@@ -74,87 +74,15 @@ __global__ void k_count(const float* __restrict__ samples, uint64_t n, BinParams
 // -> 41.3; 2^20, 512 x 1024 100.7 -> 95.5; 2^22, 512 x 4096 1180 -> 1191 (the
 // single 16-byte stores cost more than coalesced runs), hence kMaxRanked.
 constexpr int kRankThreads = 1024, kRankLoads = 16, kRankTile = kRankThreads * kRankLoads;
-constexpr int kRankKeyBits = 14;                     // nBins <= 2^14, a CTA's ranks < 2^18
-static_assert(kRankTile <= 1 << (32 - kRankKeyBits), "key and rank share a word");
 
 __global__ void __launch_bounds__(kRankThreads, 1)
 k_count_ranked(const float* __restrict__ samples, uint64_t n, BinParams p, uint32_t* __restrict__ totals,
                uint32_t* __restrict__ nonempty, uint32_t* __restrict__ ranks)
 {
     extern __shared__ __align__(8) uint32_t sh[];
-    const uint32_t tid = threadIdx.x, pairs = (p.nBins + 1) / 2, words = (p.key.nR + 31) / 32;
-    const uint32_t blocks = (p.nBins + kScanBlock - 1) / kScanBlock;
-    uint32_t *s_bits = sh + 2 * pairs, *s_blk = s_bits + words;
-    uint2* s_pair = reinterpret_cast<uint2*>(sh);
     chain_next();
-    for(uint32_t b = tid; b < 2 * pairs + words + blocks; b += kRankThreads) sh[b] = 0u;
-    __syncthreads();
     chain_wait();
-    samples = after_chain(samples);
-    const uint64_t chunk = (n + gridDim.x - 1) / gridDim.x, begin = blockIdx.x * chunk, end = min(begin + chunk, n);
-    uint32_t kr[kRankLoads];                     // key | rank in the CTA << kRankKeyBits
-#pragma unroll
-    for(int g = 0; g < kRankLoads; g += 4) {
-        float4 rec[4];
-        if(begin + (uint64_t)g * kRankThreads >= end) {
-#pragma unroll
-            for(int u = 0; u < 4; u++) kr[g + u] = kOutOfRange;
-            continue;
-        }
-#pragma unroll
-        for(int u = 0; u < 4; u++) {
-            const uint64_t i = begin + (uint64_t)(g + u) * kRankThreads + tid;
-            rec[u] = i < end ? load_record(samples, i, p) : make_float4(0.f, 0.f, INFINITY, 0.f);
-        }
-#pragma unroll
-        for(int u = 0; u < 4; u++) {
-            int side;
-            const uint32_t r = range_key(p.key, rec[u].z, side);
-            const uint32_t k = begin + (uint64_t)(g + u) * kRankThreads + tid < end ? sample_key(p, rec[u].z, rec[u].w, side)
-                                                                                : kOutOfRange;
-            kr[g + u] = kOutOfRange;
-            if(k == kOutOfRange) continue;
-            kr[g + u] = k | atomicAdd(&sh[k], 1u) << kRankKeyBits;
-            const uint32_t bit = 1u << (r & 31u);
-            if(!(s_bits[r >> 5] & bit)) atomicOr(&s_bits[r >> 5], bit);
-        }
-    }
-    __syncthreads();
-    // The CTA's counts into the totals; the bins' entries become the first ranks.
-    constexpr int kBatch = 4;
-    for(uint32_t w0 = tid & ~31u; w0 < pairs; w0 += kBatch * kRankThreads) {
-        const uint32_t b0 = w0 + (tid & 31u);
-        uint2 c[kBatch];
-        unsigned long long old[kBatch];
-#pragma unroll
-        for(int q = 0; q < kBatch; q++) {
-            const uint32_t b = b0 + q * kRankThreads;
-            c[q] = b < pairs ? s_pair[b] : make_uint2(0u, 0u);
-            // (an odd last bin's neighbour is the first block sum)
-            if(!(c[q].x | c[q].y)) old[q] = 0ull;
-            else if(2 * b + 1 < p.nBins) old[q] = atomicAdd(reinterpret_cast<unsigned long long*>(totals) + b,
-                                                            (unsigned long long)c[q].y << 32 | c[q].x);
-            else old[q] = atomicAdd(&totals[2 * b], c[q].x);
-        }
-#pragma unroll
-        for(int q = 0; q < kBatch; q++) {
-            const uint32_t b = b0 + q * kRankThreads;
-            if(b < pairs) s_pair[b] = make_uint2((uint32_t)old[q], (uint32_t)(old[q] >> 32));
-            // (a warp's pairs lie in one block of kScanBlock bins)
-            const uint32_t sum = __reduce_add_sync(0xffffffffu, c[q].x + c[q].y);
-            if((tid & 31) == 0 && sum) atomicAdd(&s_blk[2 * b / kScanBlock], sum);
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for(int u = 0; u < kRankLoads; u++) {
-        const uint64_t i = begin + (uint64_t)u * kRankThreads + tid;
-        if(kr[u] != kOutOfRange) ranks[i] = sh[kr[u] & ((1u << kRankKeyBits) - 1u)] + (kr[u] >> kRankKeyBits);
-    }
-    for(uint32_t b = tid; b < words; b += kRankThreads)
-        if(s_bits[b]) atomicOr(&nonempty[b], s_bits[b]);
-    for(uint32_t b = tid; b < blocks; b += kRankThreads)
-        if(s_blk[b]) atomicAdd(&totals[p.nBins + b], s_blk[b]);
+    count_ranked<kRankThreads, kRankLoads>(after_chain(samples), n, p, blockIdx.x, gridDim.x, totals, nonempty, ranks, sh, true);
 }
 
 template <bool ECHO>
@@ -449,11 +377,6 @@ __global__ void k_reset_batch(const PingDev* __restrict__ pings, uint32_t n_ping
     if(i < n_pings) { pings[i].oor[0] = 0ull; pings[i].oor[1] = 0ull; }
 }
 
-size_t ranked_smem(const BinParams& p)
-{
-    return ((p.nBins + 1) / 2 * 2 + (p.key.nR + 31) / 32 + (p.nBins + kScanBlock - 1) / kScanBlock) * sizeof(uint32_t);
-}
-
 uint32_t hist_grid(uint32_t ctas, uint64_t n)
 {
     // At least ~1024 samples per CTA so that the per-CTA histogram set-up
@@ -708,7 +631,7 @@ rtacx_status run_sort(Context& ctx, const BinParams& p, const SortShape& shape, 
     if(ranked)
         RTACX_CUDA(launch_chained(k_count_ranked, (uint32_t)std::max(std::min<uint64_t>((uint64_t)ctx.sm_count, (n + kRankThreads - 1) / kRankThreads),
                                                                         (n + kRankTile - 1) / kRankTile),
-                                  kRankThreads, ranked_smem(p), stream, s, n, p, ctx.d_totals, nonempty, ctx.d_ranks));
+                                  kRankThreads, ranked_smem(p.nBins, p.key.nR), stream, s, n, p, ctx.d_totals, nonempty, ctx.d_ranks));
     else
         RTACX_CUDA(launch_chained(k_count, grid, shape.hist_threads,
                               smem + (nonempty ? (p.key.nR + 31) / 32 * sizeof(uint32_t) : 0), stream, s, n, p,
@@ -858,7 +781,7 @@ SortShape sort_shape(const Context& ctx, uint32_t nBins, bool ranked)
     };
     shape.hist_ctas = resident((const void*)k_count);
     shape.scatter_ctas = resident((const void*)k_scatter);
-    const size_t ranked_bytes = (nBins + 2 + (ctx.nR + 31) / 32 + nBins / kScanBlock + 1) * sizeof(uint32_t);
+    const size_t ranked_bytes = ranked_smem(nBins, ctx.nR);
     shape.ranked = ranked && ranked_bytes <= 100 * 1024 && nBins <= 1u << kRankKeyBits &&
                    raise_smem_limit((const void*)k_count_ranked, ranked_bytes) == cudaSuccess;
     // Staged scatter: the first shape of kScatterShapes whose shared memory

@@ -266,6 +266,7 @@ __device__ __forceinline__ void scan_bin_block(const uint32_t* __restrict__ tota
         if(threadIdx.x == 0) *s_prefix = 0u;
         __syncthreads();
         uint32_t s = 0;
+#pragma unroll 16
         for(uint32_t i = threadIdx.x; i < blk * kScanBlock; i += blockDim.x) s += totals[i];
         for(int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
         if(lane_id() == 0 && s) atomicAdd(s_prefix, s);
@@ -354,6 +355,132 @@ __device__ __forceinline__ void scatter_chunk_global(const float* __restrict__ s
             else atomicOr(err, kErrScatterOverflow);
         }
     });
+}
+
+// Ranks of chunk c of nc (at most THREADS x LOADS samples) among the samples of
+// their bins: a shared histogram gives each sample's rank in the chunk (kept
+// with its key in one register), one 64-bit atomic per pair of bins adds the
+// chunk's counts to the totals and returns what its ranks start at; the ranks
+// are stored in input order. Also the bitmap of range bins and, with
+// block_sums, the sums of kScanBlock bins (totals[nBins + block]).
+constexpr int kRankKeyBits = 14;                     // nBins <= 2^14, a chunk's ranks < 2^18
+template <int THREADS, int LOADS>
+__device__ __forceinline__ void count_ranked(const float* __restrict__ samples, uint64_t n, const BinParams& p, uint32_t c,
+                                             uint32_t nc, uint32_t* __restrict__ totals, uint32_t* __restrict__ nonempty,
+                                             uint32_t* __restrict__ ranks, uint32_t* sh, bool block_sums)
+{
+    static_assert(THREADS * LOADS <= 1 << (32 - kRankKeyBits), "key and rank share a word");
+    const uint32_t tid = threadIdx.x, pairs = (p.nBins + 1) / 2, words = (p.key.nR + 31) / 32;
+    const uint32_t blocks = (p.nBins + kScanBlock - 1) / kScanBlock;
+    uint32_t *s_bits = sh + 2 * pairs, *s_blk = s_bits + words;
+    uint2* s_pair = reinterpret_cast<uint2*>(sh);
+    for(uint32_t b = tid; b < 2 * pairs + words + blocks; b += THREADS) sh[b] = 0u;
+    __syncthreads();
+    const uint64_t chunk = (n + nc - 1) / nc, begin = c * chunk, end = min(begin + chunk, n);
+    uint32_t kr[LOADS];                     // key | rank in the CTA << kRankKeyBits
+#pragma unroll
+    for(int g = 0; g < LOADS; g += 4) {
+        float4 rec[4];
+        if(begin + (uint64_t)g * THREADS >= end) {
+#pragma unroll
+            for(int u = 0; u < 4; u++) kr[g + u] = kOutOfRange;
+            continue;
+        }
+#pragma unroll
+        for(int u = 0; u < 4; u++) {
+            const uint64_t i = begin + (uint64_t)(g + u) * THREADS + tid;
+            rec[u] = i < end ? load_record(samples, i, p) : make_float4(0.f, 0.f, INFINITY, 0.f);
+        }
+#pragma unroll
+        for(int u = 0; u < 4; u++) {
+            int side;
+            const uint32_t r = range_key(p.key, rec[u].z, side);
+            const uint32_t k = begin + (uint64_t)(g + u) * THREADS + tid < end ? sample_key(p, rec[u].z, rec[u].w, side)
+                                                                                : kOutOfRange;
+            kr[g + u] = kOutOfRange;
+            if(k == kOutOfRange) continue;
+            kr[g + u] = k | atomicAdd(&sh[k], 1u) << kRankKeyBits;
+            const uint32_t bit = 1u << (r & 31u);
+            if(!(s_bits[r >> 5] & bit)) atomicOr(&s_bits[r >> 5], bit);
+        }
+    }
+    __syncthreads();
+    // The CTA's counts into the totals; the bins' entries become the first ranks.
+    constexpr int kBatch = 4;
+    for(uint32_t w0 = tid & ~31u; w0 < pairs; w0 += kBatch * THREADS) {
+        const uint32_t b0 = w0 + (tid & 31u);
+        uint2 v[kBatch];
+        unsigned long long old[kBatch];
+#pragma unroll
+        for(int q = 0; q < kBatch; q++) {
+            const uint32_t b = b0 + q * THREADS;
+            v[q] = b < pairs ? s_pair[b] : make_uint2(0u, 0u);
+            // (an odd last bin's neighbour is the first block sum)
+            if(!(v[q].x | v[q].y)) old[q] = 0ull;
+            else if(2 * b + 1 < p.nBins) old[q] = atomicAdd(reinterpret_cast<unsigned long long*>(totals) + b,
+                                                            (unsigned long long)v[q].y << 32 | v[q].x);
+            else old[q] = atomicAdd(&totals[2 * b], v[q].x);
+        }
+#pragma unroll
+        for(int q = 0; q < kBatch; q++) {
+            const uint32_t b = b0 + q * THREADS;
+            if(b < pairs) s_pair[b] = make_uint2((uint32_t)old[q], (uint32_t)(old[q] >> 32));
+            // (a warp's pairs lie in one block of kScanBlock bins)
+            const uint32_t sum = __reduce_add_sync(0xffffffffu, v[q].x + v[q].y);
+            if((tid & 31) == 0 && sum) atomicAdd(&s_blk[2 * b / kScanBlock], sum);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for(int u = 0; u < LOADS; u++) {
+        const uint64_t i = begin + (uint64_t)u * THREADS + tid;
+        if(kr[u] != kOutOfRange) ranks[i] = sh[kr[u] & ((1u << kRankKeyBits) - 1u)] + (kr[u] >> kRankKeyBits);
+    }
+    for(uint32_t b = tid; b < words; b += THREADS)
+        if(s_bits[b]) atomicOr(&nonempty[b], s_bits[b]);
+    for(uint32_t b = tid; b < blocks; b += THREADS)
+        if(block_sums && s_blk[b]) atomicAdd(&totals[p.nBins + b], s_blk[b]);
+}
+
+// Scatter of chunk c of nc straight to offsets[bin] + rank, kRankedLoads records
+// per thread in flight (bound by the latency of the loads). Batch of 16 pings,
+// 2.5e6 2D samples, us: count 75 with one global atomic per sample, 45 with
+// count_ranked; scatter 55 with a cursor atomic per sample, 43.
+constexpr int kRankedLoads = 8;
+
+__device__ __forceinline__ void scatter_chunk_ranked(const float* __restrict__ samples, uint64_t n, const BinParams& p,
+                                                     uint32_t c, uint32_t nc, const uint32_t* ranks,
+                                                     const uint32_t* offsets, float4* __restrict__ sorted,
+                                                     uint32_t* __restrict__ err)
+{
+    const uint32_t total = offsets[p.nBins];
+    const uint64_t chunk = (n + nc - 1) / nc, begin = c * chunk, end = min(begin + chunk, n);
+    for(uint64_t t0 = begin + threadIdx.x; t0 < end; t0 += (uint64_t)kRankedLoads * blockDim.x) {
+        float4 rec[kRankedLoads];
+        uint32_t pos[kRankedLoads];
+#pragma unroll
+        for(int u = 0; u < kRankedLoads; u++) {
+            const uint64_t i = t0 + (uint64_t)u * blockDim.x;
+            rec[u] = i < end ? load_record(samples, i, p) : make_float4(0.f, 0.f, INFINITY, 0.f);
+            pos[u] = i < end ? ranks[i] : 0u;
+        }
+#pragma unroll
+        for(int u = 0; u < kRankedLoads; u++) {
+            int side;
+            const uint32_t k = t0 + (uint64_t)u * blockDim.x < end ? sample_key(p, rec[u].z, rec[u].w, side) : kOutOfRange;
+            pos[u] = k != kOutOfRange ? offsets[k] + pos[u] : kOutOfRange;
+        }
+#pragma unroll
+        for(int u = 0; u < kRankedLoads; u++) {
+            if(pos[u] == kOutOfRange) continue;
+            if(p.echo_flags) {
+                const float2 v = apply_echo(p, make_float2(rec[u].x, rec[u].y), rec[u].z);
+                rec[u].x = v.x; rec[u].y = v.y;
+            }
+            if(pos[u] < total) sorted[pos[u]] = rec[u];
+            else atomicOr(err, kErrScatterOverflow);
+        }
+    }
 }
 
 } // namespace

@@ -427,6 +427,9 @@ struct SortShape {
 // (kPerRow), or in the cell form (rtacx_cells.cuh).
 enum PingForm : int { kPerRow = 0, kCells2D, kPairs2D, kCells1D, kRows1D };
 
+// Samples of a count or scatter item of a batched ping with ranks.
+constexpr uint64_t kRankedChunk = 4096;
+
 // Everything one ping of a batch needs on the device (rtacx_batch_*).
 struct PingDev {
     int form;
@@ -444,6 +447,7 @@ struct PingDev {
     unsigned long long* oor;
     uint32_t* err;
     float4* sorted;
+    uint32_t* ranks;                 // cell form, 2D: each sample's rank in its bin (null: cursors)
     uint32_t nR;
     int overlap;
     const int2* support;
@@ -653,6 +657,11 @@ rtacx_status run_binning(Context& ctx, const void* samples, uint64_t n, cudaStre
 // also the bitmap of range bins), scan, scatter.
 rtacx_status run_sort(Context& ctx, const BinParams& p, const SortShape& shape, const void* samples, uint64_t n,
                       uint32_t* nonempty, cudaStream_t stream);
+// Shared memory of a ranked count: the bins' counts, the bitmap, the block sums.
+inline size_t ranked_smem(uint32_t nBins, uint32_t nR)
+{
+    return ((nBins + 1) / 2 * 2 + (nR + 31) / 32 + (nBins + kScanBlock - 1) / kScanBlock) * sizeof(uint32_t);
+}
 SortShape sort_shape(const Context& ctx, uint32_t nBins, bool ranked);
 rtacx_status restore_sorted(Context& ctx, cudaStream_t stream);
 rtacx_status run_bin_outputs(Context& ctx, const void* samples, uint64_t n,

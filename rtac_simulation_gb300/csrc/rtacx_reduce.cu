@@ -974,12 +974,12 @@ __device__ __forceinline__ uint32_t claim(uint32_t* counter, uint32_t* s_item)
 // ---- the cell form's items in the fused kernel ------------------------------
 // Noinline: one copy for every tile shape of the per-row gather.
 __device__ __noinline__ void batch_cells_item(const CellPing& P, int form, int bpl, int shared, uint32_t first,
-                                              uint32_t end, uint32_t unit, unsigned char* smem_raw)
+                                              uint32_t end, uint32_t unit, bool load, unsigned char* smem_raw)
 {
     const int warp = threadIdx.x >> 5;
     const size_t per_warp = form == kPairs2D ? sizeof(CellWarpSmem<true>) : sizeof(CellWarpSmem<false>);
     float2* tab = reinterpret_cast<float2*>(smem_raw + kWarps * per_warp);
-    load_beam_table(tab, P.beam, P.beam_axis.n, threadIdx.x, kThreads);
+    if(load) load_beam_table(tab, P.beam, P.beam_axis.n, threadIdx.x, kThreads);
     __syncthreads();
     BeamLookup<> beam;
     beam.init(P.beam_axis);
@@ -1047,17 +1047,20 @@ __device__ __noinline__ void batch_filter_item(const PingDev& D, const CellPing&
 //   phase 0  zero every ping's bin totals and out-of-range counts (cell
 //            form: its cell rows and bitmaps)
 //   phase 1  count chunks (a global atomic per sample)       dynamic queue
-//            (cell form: zero its pings first)
+//            (cell form: zero its pings first; ranks in the bins
+//            through a histogram in the gather's shared memory)
 //   phase 2  bin-scan blocks of kScanBlock bins              dynamic queue
 //   phase 3  reference windows (static), scatter chunks      dynamic queue
-//            (a global cursor atomic per sample; 1D cell-form pings: the
-//            samples into their cells or rows)
+//            (a global cursor atomic per sample; cell form: straight to
+//            the sample's rank; 1D: the samples into their cells or rows)
 //   phase 4  gather items, heaviest first (cell form: units  dynamic queue
 //            of sorted samples into the cell rows)
 //   phase 5  cell form: range filters                        dynamic queue
 // separated by bounded grid barriers. The binning phases use no shared
 // histogram, so the dynamic shared memory is the gather's and as many CTAs
 // per SM stay resident as for a gather alone.
+constexpr int kBatchRankLoads = 16;
+static_assert(kThreads * kBatchRankLoads == kRankedChunk, "the plan's chunks");
 template <int TR, int TB, bool CELLS>
 __device__ __forceinline__ void batch_fused(const FusedBatch& fb, unsigned char* smem_raw)
 {
@@ -1100,6 +1103,12 @@ __device__ __forceinline__ void batch_fused(const FusedBatch& fb, unsigned char*
         if(k >= fb.n_chunks) break;
         const uint2 m = fb.chunk_map[k];
         const PingDev& P = fb.pings[m.x];
+        if(CELLS && P.ranks) {
+            const BinParams bin = P.bin;         // in registers: read for every sample
+            count_ranked<kThreads, kBatchRankLoads>(P.samples, P.n, bin, m.y, P.chunks, P.totals, P.nonempty, P.ranks,
+                                                    reinterpret_cast<uint32_t*>(smem_raw), false);
+            continue;
+        }
         count_chunk_global(P.samples, P.n, P.bin, m.y, P.chunks, P.totals, P.oor, s_oor,
                            CELLS && P.form != kPerRow ? P.nonempty : nullptr);
     }
@@ -1125,15 +1134,21 @@ __device__ __forceinline__ void batch_fused(const FusedBatch& fb, unsigned char*
         const uint2 m = fb.chunk_map[k];
         const PingDev& P = fb.pings[m.x];
         if(CELLS && k >= fb.n_chunks) batch_chunk_1d(P, cell_of(P), m.y, smem_raw);
+        else if(CELLS && P.ranks) {
+            const BinParams bin = P.bin;
+            scatter_chunk_ranked(P.samples, P.n, bin, m.y, P.chunks, P.ranks, P.offsets, P.sorted, P.err);
+        }
         else scatter_chunk_global(P.samples, P.n, P.bin, m.y, P.chunks, P.hist, P.offsets, P.sorted, P.err);
     }
     if(!grid_barrier(fb, &s_ok)) return;
 
+    uint32_t loaded = 0xFFFFFFFFu;           // ping whose parameters and beam table the CTA holds
     for(;;) {
         const uint32_t it = claim(&fb.sync->next[3], &s_item);
         if(it >= fb.n_items) break;
         const uint4 item = fb.items[it];
         const PingDev& P = fb.pings[item.x];
+        loaded = item.w == 2 ? loaded : 0xFFFFFFFFu;
         if(item.w == 0) {
             gather_tile_2d<TR, TB>(P.sorted, P.offsets, P.win, P.bb_tiles, P.ranges, P.bearings, P.pulse, P.beam,
                                    P.red, P.bin.nBB, P.out, (int)item.y, (int)item.z, smem_raw);
@@ -1142,8 +1157,11 @@ __device__ __forceinline__ void batch_fused(const FusedBatch& fb, unsigned char*
             const uint32_t total = P.offsets[P.bin.nBins];
             const uint64_t first = (uint64_t)item.y * P.per_item;
             if(first >= total) continue;
-            batch_cells_item(cell_of(P), P.form, P.bpl, P.shared, (uint32_t)first,
-                             (uint32_t)min(first + P.per_item, (uint64_t)total), P.unit, smem_raw);
+            const bool load = loaded != item.x;
+            if(load) cell_of(P);
+            loaded = item.x;
+            batch_cells_item(s_cell, P.form, P.bpl, P.shared, (uint32_t)first,
+                             (uint32_t)min(first + P.per_item, (uint64_t)total), P.unit, load, smem_raw);
         }
         else {
             float2* s_pulse = reinterpret_cast<float2*>(smem_raw);

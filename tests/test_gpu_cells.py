@@ -258,3 +258,22 @@ def test_chained_pings_read_what_the_kernel_ahead_wrote(maker):
     torch.cuda.synchronize()
     for i, g in enumerate(got):
         assert float((g - want[i % 2]).norm() / want[i % 2].norm()) <= 2e-6, i
+
+
+@pytest.mark.parametrize("n", [1, 4095, 4097, 12289, (1 << 21) + 1])
+def test_batches_around_the_ranked_chunks(oracle, n):
+    """A ping of n samples next to a small one: one chunk of the batch's ranked
+    count and more, and more samples than are ranked."""
+    from rtac_simulation_gb300 import _lib
+    pings = [ping(n, 41, 33, 3, False), ping(500, 64, 130, 40, False, seed=4)]
+    ctxs = [make_context(wk) for wk in pings]
+    devs = [torch.from_numpy(wk.samples.reshape(-1)).cuda() for wk in pings]
+    outs = [torch.full(wk.out_shape + (2,), float("nan"), device="cuda") for wk in pings]
+    batch = _lib.Batch(0)
+    batch.plan([(c, d, wk.n, o) for wk, c, d, o in zip(pings, ctxs, devs, outs)], autotune=False)
+    for _ in range(2):
+        batch.run(stream=torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    for wk, o in zip(pings, outs):
+        got = o.cpu().numpy()[..., 0] + 1j * o.cpu().numpy()[..., 1]
+        assert rel_l2(got, oracle.reduce(wk.samples, wk.sensor)) <= TOL
