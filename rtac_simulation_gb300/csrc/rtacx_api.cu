@@ -208,6 +208,10 @@ bool allocate_bins(Context& c)
         c.cell_sort = sort_shape(c, c.cell_bin.nBins, c.dims == 2);
         bins = std::max(bins, c.cell_bin.nBins);
     }
+    if(c.lobe_on) {
+        c.lobe_sort = sort_shape(c, c.lobe_bin.nBins, true);
+        bins = std::max(bins, c.lobe_bin.nBins);
+    }
     const size_t cols = (size_t)bins * kCursorStride;
     return upload<uint32_t>(c, c.d_offsets, nullptr, bins + 1) &&
            upload<uint32_t>(c, c.d_totals, nullptr, bins + bins / 1024 + 1) &&   // + block sums

@@ -676,7 +676,7 @@ rtacx_status restore_sorted(Context& ctx, cudaStream_t stream)
     float4* sorted = ctx.d_sorted;
     if(!ctx.sorted_input_order) {
         k_mark_tail<<<(uint32_t)std::min<uint64_t>((n + 255) / 256, (uint64_t)ctx.sm_count * 16), 256, 0, stream>>>(
-            sorted, ctx.d_offsets + ctx.cell_bin.nBins, n);
+            sorted, ctx.d_offsets + ctx.sorted_bins, n);
         RTACX_CUDA(cudaGetLastError());
     }
     void* tmp = nullptr;

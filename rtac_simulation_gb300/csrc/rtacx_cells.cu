@@ -48,9 +48,10 @@ size_t cells_smem(int W, bool pairs, int bpl, int copies)
            (size_t)(W + 2) * copies * sizeof(float2);
 }
 
-template <int BPL, bool SHARED, bool PAIR, int COPIES>
+// begin (null: 0), end: where the sorted samples that it takes start and end.
+template <int BPL, bool SHARED, bool PAIR, int COPIES, bool FLOOR = false>
 __global__ void __launch_bounds__(32 * cell_warps(BPL, COPIES), COPIES > 1 ? 1 : BPL == 2 ? 3 : 2)
-k_cells(const CellPing ping, const uint32_t* __restrict__ total)
+k_cells(const CellPing ping, const uint32_t* begin, const uint32_t* end, uint32_t min_unit)
 {
     constexpr int kWarps = cell_warps(BPL, COPIES);
     CellPing P = ping;
@@ -58,22 +59,24 @@ k_cells(const CellPing ping, const uint32_t* __restrict__ total)
     CellWarpSmem<PAIR>& S = reinterpret_cast<CellWarpSmem<PAIR>*>(s_raw)[threadIdx.x >> 5];
     float2* tab = reinterpret_cast<float2*>(s_raw + kWarps * sizeof(CellWarpSmem<PAIR>));
     chain_next();
-    load_beam_table<COPIES>(tab, P.beam, P.beam_axis.n, threadIdx.x, 32 * kWarps);
+    load_beam_table<COPIES>(tab, P.beam, P.beam_axis, threadIdx.x, 32 * kWarps);
     __syncthreads();
     chain_wait();
     P.sorted = after_chain(P.sorted);
     BeamLookup<COPIES> beam;
     beam.init(P.beam_axis);
     tab += threadIdx.x & (COPIES - 1);
-    const uint32_t m = *after_chain(total);
+    const uint32_t first = begin ? *after_chain(begin) : 0u, m = *after_chain(end) - first;
     // Equal units, so that the resident warps all end in the same round.
     const uint64_t warps = (uint64_t)gridDim.x * kWarps, rounds = (m + warps * kUnit - 1) / (warps * kUnit);
-    const uint32_t unit = max((uint32_t)kMinUnit, (uint32_t)((m + warps * rounds - 1) / max(warps * rounds, (uint64_t)1)));
+    const uint32_t unit = max(min_unit, (uint32_t)((m + warps * rounds - 1) / max(warps * rounds, (uint64_t)1)));
     for(uint64_t u = (uint64_t)(blockIdx.x * kWarps + (threadIdx.x >> 5)) * unit; u < m; u += warps * unit)
-        accumulate_unit<BPL, SHARED, PAIR>(P, (uint32_t)u, min(unit, m - (uint32_t)u), blockIdx.y, gridDim.y, S, tab, beam);
+        accumulate_unit<BPL, SHARED, PAIR, FLOOR>(P, first + (uint32_t)u, min(unit, m - (uint32_t)u), blockIdx.y, gridDim.y, S,
+                                                  tab, beam);
 }
 
-using CellsFn = void (*)(const CellPing, const uint32_t*);
+using CellsFn = void (*)(const CellPing, const uint32_t*, const uint32_t*, uint32_t);
+CellsFn lobe_fn(int bpl) { return bpl == 4 ? k_cells<4, false, false, kTableCopies, true> : k_cells<2, false, false, kTableCopies, true>; }
 CellsFn cells_fn(int bpl, bool shared_out, bool pairs, int copies)
 {
     if(copies > 1) return bpl == 4 ? k_cells<4, false, false, kTableCopies> : k_cells<2, false, false, kTableCopies>;
@@ -101,6 +104,7 @@ __global__ void k_cells_clear(uint32_t* __restrict__ totals, uint32_t n_totals, 
     for(uint64_t i = i0; i < n_out; i += stride) out[i] = make_float2(0.f, 0.f);
 }
 
+template <bool FLOOR>
 __global__ void __launch_bounds__(32 * kFilterWarps)
 k_cells_filter(const CellPing ping, const uint32_t* nonempty)
 {
@@ -110,7 +114,7 @@ k_cells_filter(const CellPing ping, const uint32_t* nonempty)
     chain_wait();
     P.cells = after_chain(P.cells);
     P.out = after_chain(P.out);
-    filter_tile<kFilterWarps>(P, blockIdx.x, blockIdx.y, reinterpret_cast<float4*>(s_raw), after_chain(nonempty));
+    filter_tile<kFilterWarps, FLOOR>(P, blockIdx.x, blockIdx.y, reinterpret_cast<float4*>(s_raw), after_chain(nonempty));
 }
 
 // One CTA per output row.
@@ -190,6 +194,8 @@ void free_cells(Context& c)
 {
     drop(c.d_cells); drop(c.d_cell_taps); drop(c.d_row_dev); drop(c.d_nonempty);
     drop(c.d_pos_theta); drop(c.d_pos_col); drop(c.d_col_bearing);
+    drop(c.d_lobe); drop(c.d_lobe_theta); drop(c.d_lobe_col);
+    c.lobe_on = false;
     c.cells_on = false;
     c.sorted_cells_n = 0;
 }
@@ -271,6 +277,16 @@ bool knot_cells(Context& c, const RowFit& f)
     return set_cell_axis(c.cell.cp, f, 0.5 * H - 0.5 - f.R0 / f.spacing, 1, nR + H, knot, H);
 }
 
+// Window x cell block bins, the blocks as small as kCellBins allows.
+void set_cell_blocks(BinParams& bin, int cells)
+{
+    for(bin.cell_shift = 0;; bin.cell_shift++) {
+        bin.cell_blocks = (uint32_t)((cells - 1) >> bin.cell_shift) + 1u;
+        if(bin.nBB * bin.cell_blocks <= kCellBins || bin.cell_blocks == 1u) break;
+    }
+    bin.nBins = bin.nBB * bin.cell_blocks;
+}
+
 // Taps of the knot cells' filter.
 std::vector<float4> cell_taps(const Context& c, const RowFit& f)
 {
@@ -298,7 +314,47 @@ void set_ping_params(Context& c)
     P.range_axis = c.red.range_axis; P.beam_axis = c.red.beam_axis;
     P.key = c.key; P.overlap = c.overlap;
     P.nR = c.nR; P.nB = c.nB;
+    P.floor = 0.0f; P.floor_col = -1;
 }
+
+// A beam table that is one level, not zero, at both ends: the texels between
+// its flat tails (the lobe), how far the lobe reaches, and the sample bearings
+// from which every output bearing lies within the table.
+struct Lobe { int first = 0, last = 0; float level = 0.0f, in_lo = 0.0f, in_hi = 0.0f; double support = 0.0; };
+
+bool find_lobe(const Context& c, Lobe& l)
+{
+    const int W = (int)c.W;
+    l.level = c.beam[0];
+    if(W < 8 || l.level == 0.0f || !std::isfinite(l.level) || c.beam[W - 1] != l.level) return false;
+    l.first = 0;
+    l.last = W - 1;
+    while(l.first < W && c.beam[l.first] == l.level) l.first++;
+    while(l.last >= 0 && c.beam[l.last] == l.level) l.last--;
+    if(l.first > l.last) return false;
+    const AxisLerp& ax = c.red.beam_axis;
+    const double k = (double)ax.k_hi + (double)ax.k_lo;
+    auto at = [&](double x) { return (x - (double)ax.c) / k; };
+    l.support = std::max(std::fabs(at(l.first - 1)), std::fabs(at(l.last + 1)));
+    const auto mm = std::minmax_element(c.bearings.begin(), c.bearings.end());
+    l.in_lo = (float)(*mm.second + at(2.0));             // two texels from the ends
+    l.in_hi = (float)(*mm.first + at(W - 3.0));
+    return k > 0.0 && l.support > 0.0 && l.in_lo < l.in_hi;
+}
+
+// Lobe form of a sensor whose wide beam is a lobe on a flat floor: beam =
+// floor + lobe, so a sample inside [in_lo, in_hi] adds floor v to the cell
+// sums of all bearings (one column more, which the filter adds to the others)
+// and the lobe's part to the few bearings that the lobe reaches, in windows
+// like a narrow beam's. The other samples and those next to a knot take the
+// whole table, in the last window of the sort; their bearings lie side by side
+// on the lanes, since row by row the reductions bound it (161 -> 61 us against
+// the order that spares the table's banks). Whole pings without / with, us:
+// 2^22 samples, 512 x 4096 1178 -> 439; 2^20, 600 x 2048 429 -> 138; 2^16, 512 x
+// 128 60 -> 40; 2^16, 300 x 1024 58 -> 47; 2^14, 600 x 300 43 -> 50; 2^14, 300 x
+// 1024 38 -> 52: one more launch and short lists, hence kLobeFrom (samples x
+// bearings).
+constexpr uint64_t kLobeFrom = 1ull << 24;
 
 } // namespace
 
@@ -375,27 +431,34 @@ bool configure_cells(Context& c, double beam_support)
     std::vector<int> sorted_b(nB);
     std::iota(sorted_b.begin(), sorted_b.end(), 0);
     std::stable_sort(sorted_b.begin(), sorted_b.end(), [&](int x, int y) { return c.bearings[x] < c.bearings[y]; });
-    const double lo = (double)*mm.first - beam_support, hi = (double)*mm.second + beam_support;
     std::vector<double> theta_sorted(nB);
     for(int i = 0; i < nB; i++) theta_sorted[i] = c.bearings[sorted_b[i]];
-    const int max_windows = std::max(1, (int)std::min(4096.0, (hi - lo) / (0.5 * beam_support)));
+    double lo = 0.0, hi = 0.0;
     std::vector<int2> span_of;              // [first, end) sorted bearings of each window
-    int bpl = 0;
-    for(int cand = 2; cand <= 4 && !bpl; cand += 2)
-        for(int w = std::max(1, nB / (32 * cand)); w <= max_windows && !bpl; w++) {
-            const double step = (hi - lo) / w, slack = 1e-5 * (hi - lo) + beam_support;   // 1e-5: the float window index
-            bool fits = true;
-            span_of.clear();
-            for(int q = 0; q < w && fits; q++) {
-                const auto f = std::lower_bound(theta_sorted.begin(), theta_sorted.end(), lo + q * step - slack);
-                const auto e = std::upper_bound(f, theta_sorted.end(), lo + (q + 1) * step + slack);
-                span_of.push_back(make_int2((int)(f - theta_sorted.begin()), (int)(e - theta_sorted.begin())));
-                fits = e - f <= 32 * cand;
+    auto find_windows = [&](double support) {
+        lo = (double)*mm.first - support;
+        hi = (double)*mm.second + support;
+        const int max_windows = std::max(1, (int)std::min(4096.0, (hi - lo) / (0.5 * support)));
+        for(int cand = 2; cand <= 4; cand += 2)
+            for(int w = std::max(1, nB / (32 * cand)); w <= max_windows; w++) {
+                const double step = (hi - lo) / w, slack = 1e-5 * (hi - lo) + support;   // 1e-5: the float window index
+                bool fits = true;
+                span_of.clear();
+                for(int q = 0; q < w && fits; q++) {
+                    const auto f = std::lower_bound(theta_sorted.begin(), theta_sorted.end(), lo + q * step - slack);
+                    const auto e = std::upper_bound(f, theta_sorted.end(), lo + (q + 1) * step + slack);
+                    span_of.push_back(make_int2((int)(f - theta_sorted.begin()), (int)(e - theta_sorted.begin())));
+                    fits = e - f <= 32 * cand;
+                }
+                if(fits) return cand;
             }
-            if(fits) bpl = cand;
-        }
+        return 0;
+    };
+    int bpl = find_windows(beam_support);
     const bool shared_out = bpl == 0;
     if(shared_out) bpl = nB > 64 ? 4 : 2;
+    Lobe lobe;
+    const bool with_lobe = shared_out && !c.cell_pairs && nB > 128 && find_lobe(c, lobe);
     const int len = 32 * bpl;
     const int copies = !shared_out && !c.cell_pairs && cells_smem(W, false, bpl, kTableCopies) <= kMaxCellSmem ? kTableCopies : 1;
     // Order of the bearings in a window. For one sample the table entries of
@@ -436,21 +499,19 @@ bool configure_cells(Context& c, double beam_support)
     bin.nBB = shared_out ? 1u : (uint32_t)span_of.size();
     bin.bb_scale = (float)(bin.nBB / (hi - lo));
     bin.bb_offset = (float)(-lo * (bin.nBB / (hi - lo)));
-    for(bin.cell_shift = 0;; bin.cell_shift++) {
-        bin.cell_blocks = (uint32_t)((cp.cells - 1) >> bin.cell_shift) + 1u;
-        if(bin.nBB * bin.cell_blocks <= kCellBins || bin.cell_blocks == 1u) break;
-    }
-    bin.nBins = bin.nBB * bin.cell_blocks;
+    set_cell_blocks(bin, cp.cells);
     c.cell.win_scale = bin.bb_scale;
     c.cell.win_offset = bin.bb_offset;
     // Columns: the lanes' order for shared-out windows (whole rows of 512
     // bytes per reduction), the bearings' own order for overlapping ones.
-    const uint32_t pitch = shared_out ? (uint32_t)pos.size() : (uint32_t)((nB + 31) / 32 * 32);
+    // (and, with one more for the floor, where the lobe form has such).
+    const bool lane_order = shared_out && !with_lobe;
+    const uint32_t pitch = lane_order ? (uint32_t)pos.size() : (uint32_t)((nB + (with_lobe ? 1 : 0) + 31) / 32 * 32);
     c.cell.pitch = pitch;
     std::vector<int> col(pos.size()), col_bearing(pitch, -1);
     std::vector<float> theta(pos.size(), c.bearings[sorted_b[nB - 1]]);
     for(size_t p = 0; p < pos.size(); p++) {
-        col[p] = pos[p] < 0 ? -1 : shared_out ? (int)p : pos[p];
+        col[p] = pos[p] < 0 ? -1 : lane_order ? (int)p : pos[p];
         if(pos[p] < 0) continue;
         theta[p] = c.bearings[pos[p]];
         col_bearing[col[p]] = pos[p];
@@ -463,12 +524,52 @@ bool configure_cells(Context& c, double beam_support)
     if(ok && cudaMalloc(&c.d_cells, cell_bytes) != cudaSuccess) { cudaGetLastError(); ok = false; }
     if(ok) ok = raise_smem_limit((const void*)cells_fn(c), cells_smem(c)) == cudaSuccess &&
                 (c.cell_pairs ||
-                 raise_smem_limit((const void*)k_cells_filter, filter_smem(H)) == cudaSuccess);
+                 raise_smem_limit((const void*)k_cells_filter<false>, filter_smem(H)) == cudaSuccess);
     if(ok) ok = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.cell_ctas, cells_fn(c), 32 * cell_warps(bpl, copies),
                                                               cells_smem(c)) == cudaSuccess && c.cell_ctas > 0;
     if(!ok) { cudaGetLastError(); free_cells(c); return false; }
     set_ping_params(c);
     c.cells_on = true;
+    if(!with_lobe || !(c.lobe_bpl = find_windows(lobe.support))) return true;
+
+    // The lobe form's tables; without them the sensor keeps the whole beam.
+    CellPing& L = c.lobe;
+    L = c.cell;
+    const int n_lobe = lobe.last - lobe.first + 1, l_len = 32 * c.lobe_bpl;
+    L.beam_axis.c = (float)(c.red.beam_axis.c - lobe.first);
+    L.beam_axis.n = n_lobe;
+    const size_t smem = cells_smem(n_lobe, false, c.lobe_bpl, kTableCopies);
+    std::vector<float> table(n_lobe + 2, 0.0f);
+    for(int i = 0; i < n_lobe; i++) table[i + 1] = c.beam[lobe.first + i] - lobe.level;
+    L.windows = (int)span_of.size();
+    // (behind the lobe's windows: the whole beam's, in the bearings' order)
+    const size_t whole = (size_t)L.windows * l_len;
+    std::vector<int> l_col(whole + pos.size(), -1);
+    std::vector<float> l_theta(whole + pos.size(), c.bearings[sorted_b[nB - 1]]);
+    for(int q = 0; q < nB; q++) {
+        l_col[whole + q] = sorted_b[q];
+        l_theta[whole + q] = c.bearings[sorted_b[q]];
+    }
+    for(size_t w = 0; w < span_of.size(); w++)
+        for(int q = span_of[w].x; q < span_of[w].y; q++) {
+            l_col[w * l_len + (q - span_of[w].x)] = sorted_b[q];
+            l_theta[w * l_len + (q - span_of[w].x)] = c.bearings[sorted_b[q]];
+        }
+    BinParams& lb = c.lobe_bin;
+    lb = c.cell_bin;
+    lb.split = 1;
+    lb.in_lo = lobe.in_lo;
+    lb.in_hi = lobe.in_hi;
+    lb.nBB = (uint32_t)L.windows + 1u;
+    lb.bb_scale = L.win_scale = (float)(L.windows / (hi - lo));
+    lb.bb_offset = L.win_offset = (float)(-lo * (L.windows / (hi - lo)));
+    set_cell_blocks(lb, cp.cells);
+    L.floor = lobe.level;
+    L.floor_col = nB;
+    c.lobe_on = smem <= kMaxCellSmem && put(c.d_lobe, table) && put(c.d_lobe_theta, l_theta) && put(c.d_lobe_col, l_col) &&
+                raise_smem_limit((const void*)lobe_fn(c.lobe_bpl), smem) == cudaSuccess &&
+                raise_smem_limit((const void*)k_cells_filter<true>, filter_smem(H)) == cudaSuccess;
+    L.beam = c.d_lobe; L.pos_theta = c.d_lobe_theta; L.pos_col = c.d_lobe_col;
     return true;
 }
 
@@ -509,8 +610,11 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
     CellPing P = c.cell;
     P.sorted = c.d_sorted;
     P.out = out;
-    BinParams bin = c.cell_bin;
+    const bool lobe = c.lobe_on && n * (uint64_t)c.nB >= kLobeFrom;
+    BinParams bin = lobe ? c.lobe_bin : c.cell_bin;
     bin.vec4 = c.bin.vec4;
+    bin.echo_flags = c.cell_bin.echo_flags; bin.echo_cycles = c.cell_bin.echo_cycles;
+    bin.echo_k_hi = c.cell_bin.echo_k_hi; bin.echo_k_lo = c.cell_bin.echo_k_lo;
     const uint32_t totals = bin.nBins + (bin.nBins + kScanBlock - 1) / kScanBlock;
     const uint64_t cells = (uint64_t)P.cp.cells * P.pitch, cells_out = c.cell_pairs && n ? 0 : (uint64_t)c.nR * c.nB;   // (the pairs' join writes every cell)
     c.mark(1, false, stream);
@@ -520,9 +624,10 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
     c.mark(1, true, stream);
     c.sorted_cells_n = 0;
     if(e == cudaSuccess && n) {
-        const rtacx_status st = run_sort(c, bin, c.cell_sort, samples, n, c.d_nonempty, stream);
+        const rtacx_status st = run_sort(c, bin, lobe ? c.lobe_sort : c.cell_sort, samples, n, c.d_nonempty, stream);
         if(st != RTACX_OK) return st;
         c.sorted_cells_n = n;
+        c.sorted_bins = bin.nBins;
         c.sorted_input_order = false;
         c.mark(5, false, stream);
         // As many CTAs as are resident (twice that for wide beams, whose units
@@ -531,14 +636,34 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
         // samples alone leave SMs idle.
         const uint32_t warps = (uint32_t)cell_warps(c.cell_bpl, c.cell_copies);
         const uint32_t resident = (uint32_t)(c.sm_count * c.cell_ctas);
-        const uint32_t gx = (uint32_t)std::min<uint64_t>((n + kMinUnit * warps - 1) / (kMinUnit * warps),
-                                                             c.cell_shared ? 2 * resident : resident);
-        const uint32_t gy = c.cell_shared ? std::min((uint32_t)P.windows, std::max(1u, resident / gx)) : 1u;
-        e = launch_chained(cells_fn(c), dim3(gx, gy), 32 * warps, cells_smem(c), stream, P, c.d_offsets + bin.nBins);
+        uint32_t gx = (uint32_t)std::min<uint64_t>((n + kMinUnit * warps - 1) / (kMinUnit * warps),
+                                                   c.cell_shared ? 2 * resident : resident);
+        uint32_t gy = c.cell_shared ? std::min((uint32_t)P.windows, std::max(1u, resident / gx)) : 1u;
+        const uint32_t* split_at = nullptr;
+        CellPing whole = P;
+        if(lobe) {
+            CellPing L = c.lobe;
+            L.sorted = P.sorted; L.out = out; L.pulse = P.pulse; L.ranges = P.ranges;
+            // The samples left are few and mostly next to knots (row by row):
+            // one per warp, all windows side by side.
+            gy = (uint32_t)P.windows;
+            gx = std::max(1u, 2 * resident / gy);
+            whole.pos_theta = L.pos_theta + (size_t)L.windows * 32 * c.lobe_bpl;
+            whole.pos_col = L.pos_col + (size_t)L.windows * 32 * c.lobe_bpl;
+            split_at = c.d_offsets + (bin.nBB - 1u) * bin.cell_blocks;
+            const uint32_t lw = (uint32_t)cell_warps(c.lobe_bpl, kTableCopies);
+            e = launch_chained(lobe_fn(c.lobe_bpl), (uint32_t)std::min<uint64_t>((n + kMinUnit * lw - 1) / (kMinUnit * lw), (uint64_t)c.sm_count),
+                               32 * lw, cells_smem(L.beam_axis.n, false, c.lobe_bpl, kTableCopies), stream, L,
+                               static_cast<const uint32_t*>(nullptr), split_at, kMinUnit);
+        }
+        if(e == cudaSuccess)
+            e = launch_chained(cells_fn(c), dim3(gx, gy), 32 * warps, cells_smem(c), stream, whole, split_at, c.d_offsets + bin.nBins,
+                               lobe ? 1u : kMinUnit);
+        P.floor_col = lobe ? c.lobe.floor_col : -1;
         const dim3 fgrid(P.pitch / 32, (c.nR + kFilterWarps * kFilterRows - 1) / (kFilterWarps * kFilterRows));
         if(e == cudaSuccess)
             e = c.cell_pairs ? launch_chained(k_pairs_join, c.nR, std::min(256u, P.pitch), 0, stream, P, c.d_nonempty)
-                             : launch_chained(k_cells_filter, fgrid, 32 * kFilterWarps, filter_smem(P.cp.taps), stream, P,
+                             : launch_chained(lobe ? k_cells_filter<true> : k_cells_filter<false>, fgrid, 32 * kFilterWarps, filter_smem(P.cp.taps), stream, P,
                                               c.d_nonempty);
         c.mark(5, true, stream);
     }

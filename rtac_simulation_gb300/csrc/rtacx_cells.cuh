@@ -104,16 +104,18 @@ __device__ __forceinline__ float2 pulse_at(const float2* __restrict__ pad, const
 // COPIES 16: entry i of copy k at 16 i + k, so that lanes that read the copy of
 // their own pair of banks never conflict (see k_cells).
 template <int COPIES = 1>
-__device__ __forceinline__ void load_beam_table(float2* tab, const float* __restrict__ beam_pad, int W, int tid,
+__device__ __forceinline__ void load_beam_table(float2* tab, const float* __restrict__ beam_pad, const AxisLerp& ax, int tid,
                                                 int threads)
 {
+    const int W = ax.n;
+    const bool whole = ax.c == floorf(ax.c);         // texel coordinates are whole numbers (an odd table)
     for(int k = tid; k < (W + 2) * COPIES; k += threads) {
         const int i = k / COPIES;
         float2 e = make_float2(0.f, 0.f);
         if(i <= W) {
             const float lo = beam_pad[i], hi = beam_pad[i + 1];
             e.y = hi - lo;
-            e.x = (W & 1) ? lo : fmaf(0.5f, e.y, lo);
+            e.x = whole ? lo : fmaf(0.5f, e.y, lo);
         }
         tab[k] = e;
     }
@@ -141,7 +143,7 @@ struct BeamLookup {
         magic2 = pack2(kRoundMagic, kRoundMagic);
         // fraction = d k + (ax.c + 1 - index); the half of an even table's
         // coordinate is in its entries instead.
-        const float f = kRoundMagic + ((ax.n & 1) ? ax.c + 1.0f : ax.c + 0.5f);
+        const float f = kRoundMagic + (ax.c == floorf(ax.c) ? ax.c + 1.0f : ax.c + 0.5f);
         frac2 = pack2(f, f);
         minus2 = pack2(-1.0f, -1.0f);
         last = (uint32_t)ax.n + 1u;
@@ -223,7 +225,10 @@ __device__ __forceinline__ void reduce_row_by_row(const CellPing& P, float4 w, f
 // Accumulates samples [first, first + count) (count <= kUnit) of the sorted
 // order into the cell rows. SHARED: for the windows win0, win0 + win_step, ...;
 // otherwise for each sample's own window.
-template <int BPL, bool SHARED, bool PAIR, int COPIES>
+// FLOOR (lobe form): the beam table holds what the lobe stands out of the
+// floor; the floor times the cells' sums of v and alpha v goes into one more
+// column (no sample is next to a knot).
+template <int BPL, bool SHARED, bool PAIR, bool FLOOR = false, int COPIES>
 __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t first, uint32_t count, int win0,
                                                 int win_step, CellWarpSmem<PAIR>& S, const float2* tab,
                                                 const BeamLookup<COPIES>& beam)
@@ -246,7 +251,7 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
             const float4 rec = __ldcs(P.sorted + first + i);
             float alpha;
             const int c = range_cell(P.cp, rec.z, alpha);
-            const bool near = !PAIR && !(alpha >= P.cp.knot && alpha <= 1.0f - P.cp.knot);
+            const bool near = !PAIR && !FLOOR && !(alpha >= P.cp.knot && alpha <= 1.0f - P.cp.knot);
             // Bearings far outside (and NaN) move to a bearing that no beam reaches.
             theta[q] = fminf(fmaxf(rec.w, P.theta_lo), P.theta_hi);
             if(PAIR) {
@@ -327,6 +332,22 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
                 for(uint32_t left = filled; left; left &= left - 1u) {
                     const int k = __ffs(left) - 1;
                     const int end = (int)__shfl_sync(0xffffffffu, upto, k);
+                    if(FLOOR) {
+                        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+                        for(int i = s + lane; i < end; i += 32) {
+                            const float* e = reinterpret_cast<const float*>(&S.list[i]);
+                            const float vx = e[2], vy = e[4], alpha = e[6];
+                            sum.x += vx; sum.y += vy;
+                            sum.z = fmaf(alpha, vx, sum.z); sum.w = fmaf(alpha, vy, sum.w);
+                        }
+                        for(int o = 16; o > 0; o >>= 1) {
+                            sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o); sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
+                            sum.z += __shfl_xor_sync(0xffffffffu, sum.z, o); sum.w += __shfl_xor_sync(0xffffffffu, sum.w, o);
+                        }
+                        if(lane == 0)
+                            red_add_f4(P.cells + (size_t)(base + k) * P.pitch + P.floor_col, P.floor * sum.x, P.floor * sum.y,
+                                       P.floor * sum.z, P.floor * sum.w);
+                    }
                     f32x2 acc[NP][4];
 #pragma unroll
                     for(int p = 0; p < NP; p++)
@@ -368,7 +389,7 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
             base = __reduce_min_sync(0xffffffffu, next);
             __syncwarp();
         }
-        if(!PAIR && near_knot) {
+        if(!PAIR && !FLOOR && near_knot) {
             for(int w = w_begin; w < w_end; w += win_step) {
                 const int pos0 = w * 32 * BPL + lane;
                 f32x2 minus_tb[NP];
@@ -547,7 +568,7 @@ __host__ __device__ __forceinline__ size_t filter_smem(int H)
 
 // Columns [32 tile_c, +32) and rows [8 WARPS tile_r, +8 WARPS) of a ping. Called
 // by 32 WARPS threads; synchronises.
-template <int WARPS>
+template <int WARPS, bool FLOOR = false>
 __device__ __forceinline__ void filter_tile(const CellPing& P, int tile_c, int tile_r, float4* s_raw,
                                             const uint32_t* nonempty)
 {
@@ -586,6 +607,16 @@ __device__ __forceinline__ void filter_tile(const CellPing& P, int tile_c, int t
             else *dst = make_float4(0.f, 0.f, 0.f, 0.f);
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
+        if(FLOOR) {
+            // Lobe form: the floor's column joins every column's sums (each thread's own copies).
+#pragma unroll
+            for(int i = warp; i < kFilterChunk; i += WARPS)
+                if(i < rows) {
+                    const float4 f = __ldcg(P.cells + (size_t)(rows0 + k0 + i) * P.pitch + P.floor_col);
+                    float4& a = s_cells[i * 32 + lane];
+                    a = make_float4(a.x + f.x, a.y + f.y, a.z + f.z, a.w + f.w);
+                }
+        }
         __syncthreads();
         // The thread's cell j (from its first row) is the tile's cell
         // j + warp * kFilterRows; output row r0 + q takes tap j - q there.

@@ -185,6 +185,10 @@ struct BinParams {
     uint32_t cell_blocks;
     int cell_shift;
     CellParams cell;
+    // Split (the lobe form): the last window takes the samples next to a knot
+    // and those whose bearing is outside [in_lo, in_hi].
+    int split;
+    float in_lo, in_hi;
 };
 
 // floorf(x) and it as an integer for |x| < 2^22: rounded to a whole number by
@@ -328,6 +332,10 @@ __device__ __forceinline__ uint32_t sample_key(const BinParams& p, float travel,
     if(p.cell_blocks) {
         float alpha;
         const uint32_t block = (uint32_t)max(range_cell(p.cell, travel, alpha), 0) >> p.cell_shift;
+        if(p.split) {
+            const bool in = bearing >= p.in_lo && bearing <= p.in_hi && alpha >= p.cell.knot && alpha <= 1.0f - p.cell.knot;
+            return (in ? bearing_bin(p.bb_scale, p.bb_offset, p.nBB - 1u, bearing) : p.nBB - 1u) * p.cell_blocks + block;
+        }
         return (p.nBB > 1u ? bearing_bin(p.bb_scale, p.bb_offset, p.nBB, bearing) * p.cell_blocks : 0u) + block;
     }
     if(p.nBB == 1u) return rk;
@@ -412,6 +420,8 @@ struct CellPing {
     int replicas;                    // 1D: copies of the cell rows, taken in turn by the CTAs
     uint32_t nR, nB, pitch;
     int windows;
+    float floor;                     // lobe form: the beam's level outside the lobe; its column of the cell rows
+    int floor_col;                   // (-1: none)
 };
 
 // Launch shape of the count / scatter passes for one number of bins.
@@ -573,6 +583,15 @@ struct Context {
     uint32_t* d_nonempty = nullptr;     // [(nR + 31) / 32] bitmap of non-empty range bins
     BinParams cell_bin{};               // the cell form's order
     SortShape cell_sort;
+    bool lobe_on = false;               // the sensor also has the lobe form
+    int lobe_bpl = 2, lobe_ctas = 1;
+    CellPing lobe{};
+    BinParams lobe_bin{};
+    SortShape lobe_sort;
+    float* d_lobe = nullptr;            // padded table of the lobe
+    float* d_lobe_theta = nullptr;      // positions of its windows
+    int* d_lobe_col = nullptr;
+    uint32_t sorted_bins = 0;           // bins of the order that the last ping left in d_sorted
     uint64_t sorted_cells_n = 0;        // samples of the last ping that left another order in d_sorted (0: none)
     bool sorted_input_order = false;    // ... all of them in input order (1D) instead of the in-range ones in cell order
 

@@ -979,7 +979,7 @@ __device__ __noinline__ void batch_cells_item(const CellPing& P, int form, int b
     const int warp = threadIdx.x >> 5;
     const size_t per_warp = form == kPairs2D ? sizeof(CellWarpSmem<true>) : sizeof(CellWarpSmem<false>);
     float2* tab = reinterpret_cast<float2*>(smem_raw + kWarps * per_warp);
-    if(load) load_beam_table(tab, P.beam, P.beam_axis.n, threadIdx.x, kThreads);
+    if(load) load_beam_table(tab, P.beam, P.beam_axis, threadIdx.x, kThreads);
     __syncthreads();
     BeamLookup<> beam;
     beam.init(P.beam_axis);

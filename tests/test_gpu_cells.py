@@ -57,6 +57,26 @@ def test_cells_match_fp64_oracle(oracle, n, nR, nB, taps, beam_taps, wide):
     assert rel_l2(got, want) <= TOL, rel_l2(got, want)
 
 
+@pytest.mark.parametrize("nB,beam_taps,roll,level", [
+    (129, 701, 0, 0.01), (129, 700, 0, 0.01), (200, 701, 90, 0.01), (200, 700, -141, -0.02), (600, 1501, 0, 0.3),
+])
+def test_lobes_on_a_flat_floor(oracle, nB, beam_taps, roll, level):
+    """Wide beams that are one level outside a lobe, in the middle of the table
+    or not, on both sides of the sample count from which the lobe is taken
+    apart; samples whose bearings leave the table, or are not numbers."""
+    for n in ((1 << 24) // nB, (1 << 24) // nB + 1):
+        wk = ping(n, 90, nB, 9, True, beam_taps)
+        beam = np.roll(wk.sensor["beam"], roll)
+        wk.sensor["beam"] = np.where(beam == np.float32(0.01), np.float32(level), beam).astype(np.float32)
+        wk.samples[100:200, 3] *= 3.0
+        wk.samples[200:210, 3] = np.nan
+        good = wk.samples.copy()
+        good[200:210, :2] = 0.0
+        good[200:210, 3] = 0.0
+        got = gpu_reduce(make_context(wk), wk.samples, wk.out_shape)
+        assert rel_l2(got, oracle.reduce(good, wk.sensor)) <= TOL
+
+
 @pytest.mark.parametrize("n", [1023, 1025, 1 << 21, (1 << 21) + 1])
 def test_pings_around_the_ranked_sort_limits(oracle, n):
     """One count CTA and two, the most samples that are ranked and one more;
