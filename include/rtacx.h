@@ -269,8 +269,8 @@ rtacx_status rtacx_reduce_precision(rtacx_ctx* ctx, const void* samples, uint64_
  * caller (the reference fills `samples()` from host vectors before
  * SensorInstance::compute_output(), include/rtac_simulation/SensorInstance.h:67,
  * and reads `output()` back). `samples` holds n host records (pinned memory
- * lets the copies overlap); they are copied to the device in chunks of
- * RTACX_STREAM_CHUNK records through two staging buffers on an internal copy
+ * lets the copies overlap); they are copied to the device in chunks of at
+ * most RTACX_STREAM_CHUNK records through two staging buffers on an internal copy
  * stream, each copy overlapping the accumulation of the previous chunk, and
  * the ping is copied to `out` (host, range_count x bearing_count complex64).
  * Stream-ordered on `stream`: `out` is valid once the stream completes. */

@@ -20,6 +20,12 @@ namespace {
         }                                                                        \
     } while(0)
 
+// The last copy's accumulation runs alone, so what is left of a ping for one
+// chunk is halved down to this many samples: 2^22 samples 388 us in whole
+// chunks, 380 down to 2^18 or 2^17, 382 down to 2^16 (393 with the first copy
+// behind the grid's clearing). Bound by the link: 67 MB in 345 us.
+constexpr uint64_t kLastChunk = 1ull << 18;
+
 rtacx_status ensure_streaming(Context& c, size_t record_bytes)
 {
     if(!c.copy_stream) RTACX_CUDA(cudaStreamCreateWithFlags(&c.copy_stream, cudaStreamNonBlocking));
@@ -67,17 +73,19 @@ rtacx_status reduce_precision_host(Context& c, const void* samples, uint64_t n, 
     cudaEvent_t fork = c.stream_ev[0], copied[2] = {c.stream_ev[1], c.stream_ev[2]},
                 used[2] = {c.stream_ev[3], c.stream_ev[4]};
 
+    // The first copy does not wait for the grid's clearing.
+    RTACX_CUDA(cudaEventRecord(fork, s));
+    RTACX_CUDA(cudaStreamWaitEvent(c.copy_stream, fork, 0));
     c.mark(5, false, s);
     if((st = precision_begin(c, s)) != RTACX_OK) return st;
     c.mark(5, true, s);
     c.mark(0, false, s);
-    RTACX_CUDA(cudaEventRecord(fork, s));
-    RTACX_CUDA(cudaStreamWaitEvent(c.copy_stream, fork, 0));
-    const uint64_t chunks = (n + RTACX_STREAM_CHUNK - 1) / RTACX_STREAM_CHUNK;
-    for(uint64_t i = 0; i < chunks; i++) {
+    uint64_t cnt;
+    for(uint64_t i = 0, first = 0; first < n; i++, first += cnt) {
         const int b = (int)(i & 1);
-        const uint64_t first = i * (uint64_t)RTACX_STREAM_CHUNK;
-        const uint64_t cnt = std::min<uint64_t>(RTACX_STREAM_CHUNK, n - first);
+        const uint64_t left = n - first;
+        cnt = std::min<uint64_t>(RTACX_STREAM_CHUNK, left);
+        if(left <= RTACX_STREAM_CHUNK && left > 2 * kLastChunk) cnt = left / 2;
         if(i >= 2) RTACX_CUDA(cudaStreamWaitEvent(c.copy_stream, used[b], 0));
         RTACX_CUDA(cudaMemcpyAsync(c.d_stage[b], host + first * rec, cnt * rec, cudaMemcpyHostToDevice, c.copy_stream));
         RTACX_CUDA(cudaEventRecord(copied[b], c.copy_stream));
@@ -86,8 +94,8 @@ rtacx_status reduce_precision_host(Context& c, const void* samples, uint64_t n, 
         if((st = precision_accumulate(c, c.d_stage[b], cnt, s)) != RTACX_OK) return st;
         RTACX_CUDA(cudaEventRecord(used[b], s));
     }
-    if(chunks == 0 && (st = precision_hot_scan(c, nullptr, 0, s)) != RTACX_OK) return st;
-    if(chunks == 0) {   // join the forked copy stream
+    if(n == 0 && (st = precision_hot_scan(c, nullptr, 0, s)) != RTACX_OK) return st;
+    if(n == 0) {   // join the forked copy stream
         RTACX_CUDA(cudaEventRecord(copied[0], c.copy_stream));
         RTACX_CUDA(cudaStreamWaitEvent(s, copied[0], 0));
     }

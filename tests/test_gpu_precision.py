@@ -471,3 +471,14 @@ def test_precision_model_close_to_per_sample_psf(n_ranges):
     diff = rel_l2(prec, plain)
     print(f"binned vs per-sample model ({n_ranges} ranges): rel-L2 {diff:.3e}")
     assert diff <= 1e-2, diff
+
+
+@pytest.mark.parametrize("hot", [False, True])
+@pytest.mark.parametrize("n", [1 << 19, (1 << 19) + 1, (1 << 20) + 3, (1 << 21) + (1 << 19) + 1])
+def test_precision_host_entry_chunk_sizes(n, hot):
+    """Pings around the sizes at which the last chunk is halved."""
+    from rtac_simulation_gb300 import _lib
+    wk = wl.precision_2d(n_samples=n, n_bearings=64, n_ranges=256)
+    ctx = precision_context(wk, flags=_lib.RTACX_PRECISION_HOT_RANGE if hot else 0)
+    dev = gpu_precision(ctx, wk.samples, wk.out_shape)
+    assert rel_l2(gpu_precision_host(ctx, wk.samples, wk.out_shape), dev) <= 1e-5
