@@ -440,6 +440,12 @@ rtacx_status plan_gemm_split(std::string& error, GemmPlan& g, const void* A, con
         }
         for(int ks = 1; ks <= 8; ks *= 2) {
             if(ks > 1 && longest < (size_t)2 * ks) continue;
+            // The tensor cores truncate as they accumulate: a sum of K terms in
+            // one accumulator comes out about 1.65e-9 K too small (2e-5 at K =
+            // 12000), a split one its parts' share. Long sums take two parts:
+            // one is that far off, and with more the ping moves further from
+            // the two-part one than its own error.
+            if(3 * longest * BK > 8000 && ks != 2) continue;
             const double ctas = (double)(N / bn) * (M / BM) * ks, waves = std::ceil(ctas / sm_count);
             const double t = waves * ((double)longest / ks * (bn == 256 ? 1.0 : 0.6) + 4.0) + (double)ks * M * N * 4.0 / 4e6;
             if(t < best) { best = t; g.bn = bn; g.ksplit = ks; g.lists = lists; }
