@@ -52,8 +52,7 @@ DEFAULT_CONFIG = "precision_2d"
 # on a GB300. Reported as `traffic` beside the live `achieved` numbers.
 NCU_TRAFFIC_BYTES = {
     "k_prec_accumulate_staged": 336.287e6 + 5.313e6,
-    "k_gemm_tn": 78.715e6 + 4.004e6,
-    "sort_bin": (268.531e6 + 3.186e6) + (273.130e6 + 220.672e6),   # k_count + k_scatter_pipe
+    "k_gemm_split": None,
 }
 # The accumulation's bound is the L2's reduction throughput, not HBM: ncu on
 # the default workload (profiles/k_prec_accumulate_staged_precision_2d.md)
@@ -62,9 +61,10 @@ NCU_TRAFFIC_BYTES = {
 NCU_ACCUMULATE_L2 = {"l2_throughput_pct": 64.7, "l2_red_sectors_pct": 40.6, "red_sectors_per_sample": 1.57,
                      "red_requests_per_sample": 1.50}
 
-# Plain form: count, bin scan, scatter, windows, then (2D) the tile plan and
-# the split gather or (1D) the row gather.
-KERNELS_PER_PING = {1: 5, 2: 6}
+# Plain form over range cells: clear, count, bin scan, scatter, accumulation
+# (one more for a lobe on a floor, not counted), range filter; 1D: clear,
+# accumulation, range filter.
+KERNELS_PER_PING = {1: 3, 2: 6}
 PRECISION_KERNELS_PER_PING = 5   # clear, staged accumulate, operand split, tensor-core GEMM, range filter
 
 
@@ -178,9 +178,36 @@ def measured_peaks() -> dict:
     return {"hbm_gbs": 6800.0, "bf16_tflops": 1900.0, "source": "fallback", "sm_max_mhz": 2070.0}
 
 
+def plain_flop(wk) -> float:
+    """Algorithmic work of the plain form over range cells: 10 flop (one beam
+    lerp, T and M of a complex value) per (sample, bearing inside the beam
+    support) and 16 (two complex multiply-adds) per (output cell, tap); 1D: 4
+    per sample and 16 per (row, tap)."""
+    s = wk.sensor
+    n, nR, taps = wk.samples.shape[0], s["range_count"], len(s["pulse"])
+    if wk.dims == 1:
+        return 4.0 * n + 16.0 * nR * taps
+    return 10.0 * beam_pairs(wk) + 16.0 * nR * len(s["bearings"]) * taps
+
+
+def beam_pairs(wk) -> float:
+    """Sum over samples of the bearings inside the beam support, of a table that
+    is one level at both ends the bearings where it stands out of that level."""
+    s = wk.sensor
+    th = np.sort(np.asarray(s["bearings"], np.float64))
+    W = len(s["beam"])
+    lobe = np.flatnonzero(np.asarray(s["beam"]) != s["beam"][0])
+    reach = 0.5 * (W + 1)                                  # texels from the middle to the end of the fall to zero
+    if s["beam"][0] != 0 and s["beam"][0] == s["beam"][-1] and lobe.size:
+        reach = max(0.5 * (W - 1) - lobe[0], lobe[-1] - 0.5 * (W - 1)) + 1.0
+    half_b = reach * s["beam_span"] / W
+    b = wk.samples[:, 3].astype(np.float64)
+    return float((np.searchsorted(th, b + half_b, "left") - np.searchsorted(th, b - half_b, "right")).sum())
+
+
 def useful_pairs(wk) -> float:
-    """Algorithmic work of the gather: sum over samples of (output rows inside
-    the pulse support) x (bearings inside the beam support)."""
+    """Output cells that the samples reach: sum over samples of (output rows
+    inside the pulse support) x (bearings inside the beam support)."""
     s = wk.sensor
     R = workloads.linspace(s["range_min"], s["range_max"], s["range_count"]).astype(np.float64)
     scale = float(np.float32(1.0) / np.float32(np.float32(s["pulse_duration"]) * np.float32(s["sound_celerity"])))
@@ -711,19 +738,20 @@ def run_ours(args, world, rank, local):
         line["precision_speedup_vs_plain"] = ((res["plain"]["t_dev"] / res["plain"]["steps"]) /
                                               (res["precision"]["t_dev"] / res["precision"]["steps"]))
 
-    # Rooflines. Plain gather: 8 flop per useful (sample, cell) pair.
+    # Rooflines.
     st = res["plain"]["stage"]
-    pairs = useful_pairs(wk)
+    flop = plain_flop(wk)
     gather_s = st["reduce"] / 1e3
     fp32_peak = 152 * 128 * 2 * peaks["sm_max_mhz"] * 1e6 / 1e12
-    gather_tf = 8.0 * pairs / gather_s / 1e12 if gather_s > 0 else 0.0
-    roof_plain = {"bound": "fp32" if wk.dims == 1 else "issue (operand construction of the tensor-core gather)",
+    gather_tf = flop / gather_s / 1e12 if gather_s > 0 else 0.0
+    roof_plain = {"bound": "latency and L2 reductions" if wk.dims == 1 else "FP32 pipe and shared memory (beam lookups)",
                   "achieved": gather_tf, "peak": fp32_peak, "unit": "TFLOP/s",
                   "frac": gather_tf / fp32_peak, "traffic": None,
-                  "kernel": "k_gather_tc (TF32 x3 tcgen05)" if wk.dims == 2 else "k_gather_1d",
+                  "kernel": "k_cells + k_cells_filter" if wk.dims == 2 else "k_cells_1d + k_cells_filter_1d",
                   "peak_source": "nominal FP32 SIMT (152 SMs x 128 FMA x max clock), the FP32-equivalent "
                                  "denominator of the useful work; no measured FP32 peak",
-                  "algorithmic": "8 flop per useful (sample, output cell) pair, %.3e pairs" % pairs}
+                  "algorithmic": "%.3e flop over range cells (plain_flop); %.3e (sample, output cell) pairs reached"
+                                 % (flop, useful_pairs(wk))}
     bin_bytes = n * (rec_in + 16)
     bin_s = (st["count"] + st["reset"] + st["binscan"] + st["scatter"] + st["windows"]) / 1e3
     bin_gbs = bin_bytes / bin_s / 1e9 if bin_s > 0 else 0.0
@@ -755,7 +783,7 @@ def run_ours(args, world, rank, local):
                                           "two node rows as one sector when they share it: 1.5 requests per "
                                           "sample); HBM carries the samples once")}
         roof_gemm = {"bound": "tensor", "achieved": gemm_tf, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
-                     "frac": gemm_tf / peaks["bf16_tflops"], "traffic": ncu.get("k_gemm_tn"), "kernel": "k_gemm_tn",
+                     "frac": gemm_tf / peaks["bf16_tflops"], "traffic": ncu.get("k_gemm_split"), "kernel": "k_gemm_split",
                      "peak_source": peaks["source"],
                      "algorithmic": f"2*M*N*K with M={Mp} N={Np} K={Kp} (three BF16 split products as one K)"}
         dominant = max(("accumulate", "gemm", "filter", "split"), key=lambda k: ps[k])

@@ -88,7 +88,9 @@ typedef int rtacx_status;
 /* A 2D sensor whose pulse taps lie one output range apart and whose windows
  * hold the pulse takes the range-cell form (one beam lookup per sample and
  * bearing, the pulse as a filter over the cells; float arithmetic), whatever
- * the next flag says. */
+ * the next flag says. A beam table that is one level at both ends is then
+ * taken apart into that level and a lobe on large pings (exactly, up to float
+ * round-off). */
 /* rtacx_sensor_2d.flags: gather with the FP32 CUDA-core kernel instead of the
  * tensor-core one. Otherwise a 2D ping's gather (output tiles of 64 ranges x
  * 128 bearings) forms its sample-by-PSF outer products on the tcgen05 tensor
@@ -349,7 +351,7 @@ rtacx_status rtacx_rasterize(rtacx_ctx* ctx, const rtacx_mesh* mesh, const rtacx
 /* Batched plain form: many pings from heterogeneous sensors (each bound to
  * its own configured 1D or 2D context, whose scratch it uses) in one CUDA
  * graph holding ONE kernel: a cooperative persistent launch (every CTA
- * resident) that zeroes, counts, scans, windows, scatters and gathers every
+ * resident) that zeroes, counts, scans, windows, scatters and reduces every
  * ping, taking work from atomic queues (gather tiles heaviest first) and
  * separating the phases with grid barriers whose waits are bounded (about
  * 1 s): a CTA that gives up sets the batch status word and stops, and so
@@ -362,9 +364,9 @@ rtacx_status rtacx_rasterize(rtacx_ctx* ctx, const rtacx_mesh* mesh, const rtacx
  * into the graph: re-plan when any of them changes) and, with
  * RTACX_BATCH_AUTOTUNE, times every candidate gather tile shape x samples
  * per binning chunk on this batch and keeps the fastest. rtacx_batch_run
- * replays the graph on `stream`. Results equal rtacx_reduce's per ping with
- * RTACX_FLAG_SIMT_GATHER (the batch gathers on the CUDA cores), and the
- * default tensor-core gather's to float round-off. */
+ * replays the graph on `stream`. Pings with a range-cell form take it where
+ * that is most of the batch's work, the others gather on the CUDA cores;
+ * results equal rtacx_reduce's per ping to float round-off. */
 typedef struct rtacx_batch rtacx_batch;
 typedef struct {
     rtacx_ctx* ctx;          /* configured context, one per ping          */

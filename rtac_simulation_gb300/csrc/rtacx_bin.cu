@@ -26,6 +26,8 @@
 //                     without the pipelining, for more bins; k_scatter: the
 //                     reservation without staging, when the per-bin tables do
 //                     not fit next to a tile, and in the batched form).
+//   k_count_ranked, k_scatter_ranked
+//                     the cell form's sort of up to 2^21 samples (see there).
 //   k_windows         reference windows (do_make_bins, src/Binner.cu:82-106)
 //                     as range-bin intervals, intersected with each row's PSF
 //                     support.

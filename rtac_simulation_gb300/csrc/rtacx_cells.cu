@@ -6,14 +6,14 @@
 //                   reference window zeroed (k_pairs_join: row pairs);
 //   k_cells_1d, k_cells_filter_1d, k_rows_off_1d  the same for 1D sensors,
 //                   from the input order.
-// Measured against the tensor-core gather on the same pings (whole
-// rtacx_reduce, us): 2^20 samples, 512 x 1024, 33 taps, narrow beams: 1384 ->
-// 135; 2^22 samples, 512 x 4096, wide beams: 14433 -> 1247; 150003 samples,
-// 387 x 777, 24 taps: 246 -> 62; 20000 samples, 256 x 500, row pairs: 91 -> 38. k_cells is bound by the beam lookups' shared
-// memory (single tables) and by the FMA pipe (16 copies), at one lookup per
-// (sample, bearing). 1D, us: 20000
-// samples 1049 ranges (row by row) 32.1 -> 13.5; 3e6 samples 4096 ranges, 65
-// taps 380 -> 43.
+// Measured against the per-row gathers on the same pings (whole rtacx_reduce,
+// us): 2^20 samples, 512 x 1024, 33 taps, narrow beams: 1380 -> 96; 2^22 samples,
+// 512 x 4096, wide beams on a floor: 14430 -> 443 (1180 with the whole beam);
+// 150003 samples, 387 x 777, 24 taps: 246 -> 42; 20000 samples, 256 x 500, row
+// pairs: 94 -> 22. k_cells is bound by the beam lookups' shared memory (single
+// tables) and by the FMA pipe (16 copies), at one lookup per (sample, bearing).
+// 1D: 20000 samples, 1049 ranges (row by row) 33 -> 11; 3e6 samples, 4096
+// ranges, 65 taps 381 -> 38.
 #include "rtacx_cells.cuh"
 
 #include <algorithm>

@@ -1,4 +1,5 @@
-// Plain sparse PSF reduction (FP32 SIMT).
+// Plain sparse PSF reduction: the per-row gathers, for sensors off the cell
+// form's rule (rtacx_cells.cuh), and the fused batched kernel.
 //
 // Replaces do_sparse_convolve_2d_f (src/SensorInstance2D.cu:44-119) and
 // do_sparse_convolve_1d_f (src/SensorInstance1D.cu:35-89):
