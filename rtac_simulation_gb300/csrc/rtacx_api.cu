@@ -204,8 +204,8 @@ bool allocate_bins(Context& c)
 {
     c.sort = sort_shape(c, c.bin.nBins, false);
     uint32_t bins = c.bin.nBins;
-    if(c.cells_on) {
-        c.cell_sort = sort_shape(c, c.cell_bin.nBins, c.dims == 2);
+    if(c.cells_on && c.dims == 2) {
+        c.cell_sort = sort_shape(c, c.cell_bin.nBins, true);
         bins = std::max(bins, c.cell_bin.nBins);
     }
     if(c.lobe_on) {
@@ -272,7 +272,6 @@ void rtacx_destroy(rtacx_ctx* ctx)
     cudaSetDevice(c.device);
     free_config(c);
     free_dev(c.d_sorted);
-    free_dev(c.d_ranks);
     free_dev(c.d_dir);
     free_dev(c.d_rast_v); free_dev(c.d_rast_vis); free_dev(c.d_rast_large);
     free_streaming(c);

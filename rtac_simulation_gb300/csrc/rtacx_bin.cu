@@ -401,27 +401,20 @@ uint32_t hist_grid(uint32_t ctas, uint64_t n)
 bool ensure_capacity(Context& ctx, uint64_t n)
 {
     if(n <= ctx.capacity) return true;
-    uint64_t cap = std::max<uint64_t>(n, 1024);
+    const uint64_t cap = std::max<uint64_t>(n, 1024), ranks = std::min<uint64_t>(cap, kMaxRanked);
+    // The ranks of the cell form's sort lie behind the records; without them
+    // the samples go through the tile sort.
     float4* p = nullptr;
-    if(cudaMalloc(&p, cap * sizeof(float4)) != cudaSuccess) {
+    const bool ranked = cudaMalloc(&p, cap * sizeof(float4) + ranks * sizeof(uint32_t)) == cudaSuccess;
+    if(!ranked && (cudaGetLastError(), cudaMalloc(&p, cap * sizeof(float4)) != cudaSuccess)) {
         cudaGetLastError();
         return ctx.fail("out of device memory for " + std::to_string(cap) + " sorted samples");
     }
     if(ctx.d_sorted) cudaFree(ctx.d_sorted);
     ctx.d_sorted = p;
     ctx.capacity = cap;
-    // Ranks for the cell form's sort, up to what it takes; without them the
-    // samples go through the tile sort.
-    if(ctx.n_ranks < std::min<uint64_t>(cap, kMaxRanked)) {
-        if(ctx.d_ranks) cudaFree(ctx.d_ranks);
-        ctx.d_ranks = nullptr;
-        ctx.n_ranks = std::min<uint64_t>(cap, kMaxRanked);
-        if(cudaMalloc(&ctx.d_ranks, ctx.n_ranks * sizeof(uint32_t)) != cudaSuccess) {
-            cudaGetLastError();
-            ctx.d_ranks = nullptr;
-            ctx.n_ranks = 0;
-        }
-    }
+    ctx.d_ranks = ranked ? reinterpret_cast<uint32_t*>(p + cap) : nullptr;
+    ctx.n_ranks = ranked ? ranks : 0;
     ctx.sorted_cells_n = 0;
     return true;
 }

@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <numeric>
 
 namespace rtacx {
@@ -170,31 +171,43 @@ __global__ void k_rows_off_1d(const CellPing P, const uint32_t* nonempty)
     if(r < (int)P.nR && !row_on(after_chain(nonempty), (int)P.nR, P.overlap, r)) P.out[r] = make_float2(0.f, 0.f);
 }
 
-template <typename T>
-void drop(T*& p)
-{
-    if(p) cudaFree(p);
-    p = nullptr;
-}
-
-template <typename T>
-bool put(T*& dst, const std::vector<T>& src)
-{
-    if(cudaMalloc(&dst, src.size() * sizeof(T)) != cudaSuccess ||
-       cudaMemcpy(dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
+// The tables and the cell rows of a context in one allocation, filled by one
+// copy (each cudaMalloc and cudaMemcpy of its own costs a configuration 10 to
+// 20 us).
+struct Arena {
+    std::vector<unsigned char> host;
+    template <typename T>
+    size_t add(const std::vector<T>& v)
+    {
+        const size_t at = (host.size() + 255) / 256 * 256;
+        host.resize(at + v.size() * sizeof(T));
+        std::memcpy(host.data() + at, v.data(), v.size() * sizeof(T));
+        return at;
     }
-    return true;
-}
+    // The tables with `cells` more bytes (not initialised) behind them.
+    bool upload(Context& c, size_t cells)
+    {
+        host.resize((host.size() + 255) / 256 * 256);
+        if(cudaMalloc(&c.d_cell_arena, host.size() + cells) != cudaSuccess ||
+           cudaMemcpy(c.d_cell_arena, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        c.d_cells = at<float4>(c, host.size());
+        return true;
+    }
+    template <typename T>
+    static T* at(const Context& c, size_t offset) { return reinterpret_cast<T*>(c.d_cell_arena + offset); }
+};
 
 } // namespace
 
 void free_cells(Context& c)
 {
-    drop(c.d_cells); drop(c.d_cell_taps); drop(c.d_row_dev); drop(c.d_nonempty);
-    drop(c.d_pos_theta); drop(c.d_pos_col); drop(c.d_col_bearing);
-    drop(c.d_lobe); drop(c.d_lobe_theta); drop(c.d_lobe_col);
+    if(c.d_cell_arena) cudaFree(c.d_cell_arena);
+    c.d_cell_arena = nullptr;
+    c.d_cells = nullptr;
+    c.d_nonempty = nullptr;
     c.lobe_on = false;
     c.cells_on = false;
     c.sorted_cells_n = 0;
@@ -309,8 +322,6 @@ void set_ping_params(Context& c)
 {
     CellPing& P = c.cell;
     P.cells = c.d_cells;
-    P.row_dev = c.d_row_dev; P.taps = c.d_cell_taps;
-    P.pos_theta = c.d_pos_theta; P.pos_col = c.d_pos_col; P.col_bearing = c.d_col_bearing;
     P.range_axis = c.red.range_axis; P.beam_axis = c.red.beam_axis;
     P.key = c.key; P.overlap = c.overlap;
     P.nR = c.nR; P.nB = c.nB;
@@ -375,11 +386,14 @@ bool configure_cells_1d(Context& c)
         // First row reached: floor(y) + 1 with y = (travel - reach - R0) / spacing.
         ok = set_cell_axis(c.cell.cp, f, -(reach + f.R0) / f.spacing, c.cell.rows, nR + c.cell.rows - 1, 0.0, (int)c.H);
     }
-    ok = ok && put(c.d_row_dev, f.dev) && put(c.d_cell_taps, cell_taps(c, f)) &&
-         put(c.d_nonempty, std::vector<uint32_t>((nR + 127) / 128 * 4, 0u)) &&
-         put(c.d_cells, std::vector<float4>(c.cell_rows ? 1 : (size_t)kReplicas1D * c.cell.cp.cells)) &&
+    Arena arena;
+    const size_t dev = arena.add(f.dev), taps = arena.add(cell_taps(c, f)), bits = arena.add(std::vector<uint32_t>((nR + 127) / 128 * 4, 0u));
+    ok = ok && arena.upload(c, (c.cell_rows ? 1 : (size_t)kReplicas1D * c.cell.cp.cells) * sizeof(float4)) &&
          raise_smem_limit((const void*)k_cells_filter_1d, filter_smem_1d(c.cell_rows ? 1 : (int)c.H, kFilterRows1D)) == cudaSuccess;
     if(!ok) { free_cells(c); return false; }
+    c.cell.row_dev = Arena::at<float>(c, dev);
+    c.cell.taps = Arena::at<float4>(c, taps);
+    c.d_nonempty = Arena::at<uint32_t>(c, bits);
     set_ping_params(c);
     c.cell.pitch = 1;
     c.cells_on = true;
@@ -519,57 +533,72 @@ bool configure_cells(Context& c, double beam_support)
     const size_t cell_bytes = (size_t)cp.cells * pitch * sizeof(float4);
     if(cell_bytes > kMaxCellBytes || cells_smem(c) > kMaxCellSmem ||
        (!c.cell_pairs && filter_smem(H) > 200 * 1024)) return false;
-    bool ok = put(c.d_cell_taps, cell_taps(c, f)) && put(c.d_row_dev, f.dev) && put(c.d_nonempty, std::vector<uint32_t>((nR + 127) / 128 * 4, 0u)) &&
-              put(c.d_pos_theta, theta) && put(c.d_pos_col, col) && put(c.d_col_bearing, col_bearing);
-    if(ok && cudaMalloc(&c.d_cells, cell_bytes) != cudaSuccess) { cudaGetLastError(); ok = false; }
-    if(ok) ok = raise_smem_limit((const void*)cells_fn(c), cells_smem(c)) == cudaSuccess &&
-                (c.cell_pairs ||
-                 raise_smem_limit((const void*)k_cells_filter<false>, filter_smem(H)) == cudaSuccess);
-    if(ok) ok = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.cell_ctas, cells_fn(c), 32 * cell_warps(bpl, copies),
-                                                              cells_smem(c)) == cudaSuccess && c.cell_ctas > 0;
+    Arena arena;
+    const size_t taps = arena.add(cell_taps(c, f)), dev = arena.add(f.dev), bits = arena.add(std::vector<uint32_t>((nR + 127) / 128 * 4, 0u)),
+                 at_theta = arena.add(theta), at_col = arena.add(col), at_bearing = arena.add(col_bearing);
+
+    // The lobe form's tables.
+    CellPing& L = c.lobe;
+    size_t l_table = 0, at_l_theta = 0, at_l_col = 0, l_smem = 0;
+    if(with_lobe && (c.lobe_bpl = find_windows(lobe.support)) != 0) {
+        const int n_lobe = lobe.last - lobe.first + 1, l_len = 32 * c.lobe_bpl;
+        l_smem = cells_smem(n_lobe, false, c.lobe_bpl, kTableCopies);
+        c.lobe_on = l_smem <= kMaxCellSmem;
+        L.windows = (int)span_of.size();
+        std::vector<float> table(n_lobe + 2, 0.0f);
+        for(int i = 0; i < n_lobe; i++) table[i + 1] = c.beam[lobe.first + i] - lobe.level;
+        // (behind the lobe's windows: the whole beam's, in the bearings' order)
+        const size_t whole = (size_t)L.windows * l_len;
+        std::vector<int> l_col(whole + pos.size(), -1);
+        std::vector<float> l_theta(whole + pos.size(), c.bearings[sorted_b[nB - 1]]);
+        for(int q = 0; q < nB; q++) {
+            l_col[whole + q] = sorted_b[q];
+            l_theta[whole + q] = c.bearings[sorted_b[q]];
+        }
+        for(size_t w = 0; w < span_of.size(); w++)
+            for(int q = span_of[w].x; q < span_of[w].y; q++) {
+                l_col[w * l_len + (q - span_of[w].x)] = sorted_b[q];
+                l_theta[w * l_len + (q - span_of[w].x)] = c.bearings[sorted_b[q]];
+            }
+        l_table = arena.add(table); at_l_theta = arena.add(l_theta); at_l_col = arena.add(l_col);
+    }
+
+    bool ok = arena.upload(c, cell_bytes) &&
+              raise_smem_limit((const void*)cells_fn(c), cells_smem(c)) == cudaSuccess &&
+              (c.cell_pairs || raise_smem_limit((const void*)k_cells_filter<false>, filter_smem(H)) == cudaSuccess) &&
+              cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.cell_ctas, cells_fn(c), 32 * cell_warps(bpl, copies),
+                                                            cells_smem(c)) == cudaSuccess && c.cell_ctas > 0;
     if(!ok) { cudaGetLastError(); free_cells(c); return false; }
+    c.cell.taps = Arena::at<float4>(c, taps);
+    c.cell.row_dev = Arena::at<float>(c, dev);
+    c.d_nonempty = Arena::at<uint32_t>(c, bits);
+    c.cell.pos_theta = Arena::at<float>(c, at_theta);
+    c.cell.pos_col = Arena::at<int>(c, at_col);
+    c.cell.col_bearing = Arena::at<int>(c, at_bearing);
     set_ping_params(c);
     c.cells_on = true;
-    if(!with_lobe || !(c.lobe_bpl = find_windows(lobe.support))) return true;
-
-    // The lobe form's tables; without them the sensor keeps the whole beam.
-    CellPing& L = c.lobe;
+    if(!c.lobe_on) return true;
+    c.lobe_on = raise_smem_limit((const void*)lobe_fn(c.lobe_bpl), l_smem) == cudaSuccess &&
+                raise_smem_limit((const void*)k_cells_filter<true>, filter_smem(H)) == cudaSuccess;
+    const int windows = L.windows;
     L = c.cell;
-    const int n_lobe = lobe.last - lobe.first + 1, l_len = 32 * c.lobe_bpl;
+    L.windows = windows;
+    L.beam = Arena::at<float>(c, l_table);
+    L.pos_theta = Arena::at<float>(c, at_l_theta);
+    L.pos_col = Arena::at<int>(c, at_l_col);
     L.beam_axis.c = (float)(c.red.beam_axis.c - lobe.first);
-    L.beam_axis.n = n_lobe;
-    const size_t smem = cells_smem(n_lobe, false, c.lobe_bpl, kTableCopies);
-    std::vector<float> table(n_lobe + 2, 0.0f);
-    for(int i = 0; i < n_lobe; i++) table[i + 1] = c.beam[lobe.first + i] - lobe.level;
-    L.windows = (int)span_of.size();
-    // (behind the lobe's windows: the whole beam's, in the bearings' order)
-    const size_t whole = (size_t)L.windows * l_len;
-    std::vector<int> l_col(whole + pos.size(), -1);
-    std::vector<float> l_theta(whole + pos.size(), c.bearings[sorted_b[nB - 1]]);
-    for(int q = 0; q < nB; q++) {
-        l_col[whole + q] = sorted_b[q];
-        l_theta[whole + q] = c.bearings[sorted_b[q]];
-    }
-    for(size_t w = 0; w < span_of.size(); w++)
-        for(int q = span_of[w].x; q < span_of[w].y; q++) {
-            l_col[w * l_len + (q - span_of[w].x)] = sorted_b[q];
-            l_theta[w * l_len + (q - span_of[w].x)] = c.bearings[sorted_b[q]];
-        }
+    L.beam_axis.n = lobe.last - lobe.first + 1;
+    L.floor = lobe.level;
+    L.floor_col = nB;
     BinParams& lb = c.lobe_bin;
     lb = c.cell_bin;
     lb.split = 1;
     lb.in_lo = lobe.in_lo;
     lb.in_hi = lobe.in_hi;
-    lb.nBB = (uint32_t)L.windows + 1u;
-    lb.bb_scale = L.win_scale = (float)(L.windows / (hi - lo));
-    lb.bb_offset = L.win_offset = (float)(-lo * (L.windows / (hi - lo)));
+    lb.nBB = (uint32_t)windows + 1u;
+    lb.bb_scale = L.win_scale = (float)(windows / (hi - lo));
+    lb.bb_offset = L.win_offset = (float)(-lo * (windows / (hi - lo)));
     set_cell_blocks(lb, cp.cells);
-    L.floor = lobe.level;
-    L.floor_col = nB;
-    c.lobe_on = smem <= kMaxCellSmem && put(c.d_lobe, table) && put(c.d_lobe_theta, l_theta) && put(c.d_lobe_col, l_col) &&
-                raise_smem_limit((const void*)lobe_fn(c.lobe_bpl), smem) == cudaSuccess &&
-                raise_smem_limit((const void*)k_cells_filter<true>, filter_smem(H)) == cudaSuccess;
-    L.beam = c.d_lobe; L.pos_theta = c.d_lobe_theta; L.pos_col = c.d_lobe_col;
     return true;
 }
 

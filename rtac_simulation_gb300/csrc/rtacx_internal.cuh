@@ -558,7 +558,7 @@ struct Context {
     uint64_t capacity = 0;              // samples the sorted scratch holds
     float4* d_sorted = nullptr;
     uint64_t n_ranks = 0;               // samples d_ranks holds
-    uint32_t* d_ranks = nullptr;        // each sample's rank in its bin (ranked sort)
+    uint32_t* d_ranks = nullptr;        // each sample's rank in its bin (ranked sort), behind d_sorted
     SortShape sort;
     size_t acc_smem = 0;                // dynamic shared memory of the precision accumulation
     uint32_t acc_blocks_per_sm = 1;
@@ -574,12 +574,8 @@ struct Context {
     bool cell_pairs = false;            // row pairs instead of knot cells
     bool cell_rows = false;             // 1D without knot cells: row by row
     CellPing cell{};                    // sorted and out are set per call
+    unsigned char* d_cell_arena = nullptr;   // the cell form's tables and cell rows, one allocation
     float4* d_cells = nullptr;
-    float4* d_cell_taps = nullptr;
-    float* d_row_dev = nullptr;
-    float* d_pos_theta = nullptr;
-    int* d_pos_col = nullptr;
-    int* d_col_bearing = nullptr;
     uint32_t* d_nonempty = nullptr;     // [(nR + 31) / 32] bitmap of non-empty range bins
     BinParams cell_bin{};               // the cell form's order
     SortShape cell_sort;
@@ -588,9 +584,6 @@ struct Context {
     CellPing lobe{};
     BinParams lobe_bin{};
     SortShape lobe_sort;
-    float* d_lobe = nullptr;            // padded table of the lobe
-    float* d_lobe_theta = nullptr;      // positions of its windows
-    int* d_lobe_col = nullptr;
     uint32_t sorted_bins = 0;           // bins of the order that the last ping left in d_sorted
     uint64_t sorted_cells_n = 0;        // samples of the last ping that left another order in d_sorted (0: none)
     bool sorted_input_order = false;    // ... all of them in input order (1D) instead of the in-range ones in cell order
