@@ -460,6 +460,7 @@ rtacx_status rtacx_batch_run(rtacx_batch* b, void* stream)
         Context& c = p.ctx->impl;
         c.sorted_cells_n = B.cells && takes_cells(c, p.n) ? p.n : 0;
         c.sorted_input_order = c.dims == 1;
+        c.sorted_bins = c.cell_bin.nBins;
     }
     return RTACX_OK;
 }

@@ -297,3 +297,26 @@ def test_batches_around_the_ranked_chunks(oracle, n):
     for wk, o in zip(pings, outs):
         got = o.cpu().numpy()[..., 0] + 1j * o.cpu().numpy()[..., 1]
         assert rel_l2(got, oracle.reduce(wk.samples, wk.sensor)) <= TOL
+
+
+def test_sorted_scratch_after_a_batch(oracle):
+    """The documented order from the scratch that a batch left, of sensors whose
+    single pings sort into other bins (a lobe on a floor) or into the same."""
+    from rtac_simulation_gb300 import _lib
+    from test_gpu_sorted import KEY_OOR, composite_keys, record_hash
+    pings = [ping(20000, 257, 129, 9, False), ping(90000, 100, 200, 9, True)]
+    ctxs = [make_context(wk) for wk in pings]
+    gpu_reduce(ctxs[1], pings[1].samples, pings[1].out_shape)
+    devs = [torch.from_numpy(wk.samples.reshape(-1)).cuda() for wk in pings]
+    outs = [torch.empty(wk.out_shape + (2,), device="cuda") for wk in pings]
+    batch = _lib.Batch(0)
+    batch.plan([(c, d, wk.n, o) for wk, c, d, o in zip(pings, ctxs, devs, outs)], autotune=False)
+    batch.run(torch.cuda.current_stream())
+    for wk, ctx in zip(pings, ctxs):
+        buf = torch.zeros((wk.n, 4), device="cuda")
+        ctx.diag_sorted(buf, wk.n, stream=torch.cuda.current_stream())
+        inside = wk.samples[composite_keys(oracle, wk, wk.samples) != KEY_OOR]
+        got = buf.cpu().numpy()[:len(inside)]
+        assert np.all(np.diff(composite_keys(oracle, wk, got).astype(np.int64)) >= 0)
+        assert np.array_equal(np.sort(record_hash(got)), np.sort(record_hash(inside)))
+    batch.close()
