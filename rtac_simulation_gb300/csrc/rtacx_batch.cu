@@ -181,7 +181,7 @@ struct Batch {
                 for(uint32_t y = 0; y < rows; y++)
                     for(uint32_t x = 0; x < columns; x++) filters.push_back(make_uint4(i, x, y, 0));
                 gather_smem = std::max(gather_smem, batch_cells_smem(c));
-                if(c.dims == 2 && c.cell_sort.ranked && n <= c.n_ranks) {
+                if(c.dims == 2 && c.cell_sort.ranked && n <= std::min(c.n_ranks, kMaxRanked)) {
                     d.ranks = c.d_ranks;
                     d.chunks = (uint32_t)std::max<uint64_t>(1, ceil_div(n, kRankedChunk));
                     gather_smem = std::max(gather_smem, ranked_smem(d.bin.nBins, c.nR));

@@ -27,7 +27,7 @@
 //                     reservation without staging, when the per-bin tables do
 //                     not fit next to a tile, and in the batched form).
 //   k_count_ranked, k_scatter_ranked
-//                     the cell form's sort of up to 2^21 samples (see there).
+//                     the cell form's sort of up to 2^21 or 2^22 samples (see there).
 //   k_windows         reference windows (do_make_bins, src/Binner.cu:82-106)
 //                     as range-bin intervals, intersected with each row's PSF
 //                     support.
@@ -46,7 +46,6 @@ namespace rtacx {
 namespace {
 
 constexpr int kScanThreads = 1024;
-constexpr uint64_t kMaxRanked = 1ull << 21;          // samples of a ranked sort, at most
 
 __global__ void k_count(const float* __restrict__ samples, uint64_t n, BinParams p,
                         uint32_t* __restrict__ totals, unsigned long long* __restrict__ oor,
@@ -74,7 +73,7 @@ __global__ void k_count(const float* __restrict__ samples, uint64_t n, BinParams
 // atomics' return, the ranks' loads) and the launches. Whole pings against the
 // tile sort, us: 20000 samples, 256 x 500 26.0 -> 22.1; 150003, 387 x 777 46.7
 // -> 41.3; 2^20, 512 x 1024 100.7 -> 95.5; 2^22, 512 x 4096 1180 -> 1191 (the
-// single 16-byte stores cost more than coalesced runs), hence kMaxRanked.
+// single 16-byte stores cost more than coalesced runs): see kMaxRanked.
 constexpr int kRankThreads = 1024, kRankLoads = 16, kRankTile = kRankThreads * kRankLoads;
 
 __global__ void __launch_bounds__(kRankThreads, 1)
@@ -401,7 +400,7 @@ uint32_t hist_grid(uint32_t ctas, uint64_t n)
 bool ensure_capacity(Context& ctx, uint64_t n)
 {
     if(n <= ctx.capacity) return true;
-    const uint64_t cap = std::max<uint64_t>(n, 1024), ranks = std::min<uint64_t>(cap, kMaxRanked);
+    const uint64_t cap = std::max<uint64_t>(n, 1024), ranks = std::min<uint64_t>(cap, kMaxRankedMany);
     // The ranks of the cell form's sort lie behind the records; without them
     // the samples go through the tile sort.
     float4* p = nullptr;
@@ -621,7 +620,7 @@ rtacx_status run_sort(Context& ctx, const BinParams& p, const SortShape& shape, 
     const size_t smem = (size_t)p.nBins * sizeof(uint32_t);
     const float* s = static_cast<const float*>(samples);
     const uint32_t scan_blocks = (p.nBins + kScanBlock - 1) / kScanBlock;
-    const bool ranked = nonempty && shape.ranked && n <= ctx.n_ranks;
+    const bool ranked = nonempty && shape.ranked && n <= ctx.n_ranks && (n <= kMaxRanked || p.nBins > kManyBins);
     ctx.mark(0, false, stream);
     if(ranked)
         RTACX_CUDA(launch_chained(k_count_ranked, (uint32_t)std::max(std::min<uint64_t>((uint64_t)ctx.sm_count, (n + kRankThreads - 1) / kRankThreads),
@@ -639,7 +638,7 @@ rtacx_status run_sort(Context& ctx, const BinParams& p, const SortShape& shape, 
     ctx.mark(2, true, stream);
     ctx.mark(3, false, stream);
     if(ranked) {
-        const uint32_t g = (uint32_t)std::min<uint64_t>((n + 255) / 256, (uint64_t)ctx.sm_count * 16);
+        const uint32_t g = (uint32_t)std::min<uint64_t>((n + 255) / 256, (uint64_t)ctx.sm_count * 64);
         RTACX_CUDA(launch_chained(p.echo_flags ? k_scatter_ranked<true> : k_scatter_ranked<false>, g, 256, 0, stream, s, n, p,
                                   ctx.d_ranks, ctx.d_offsets, ctx.d_sorted, ctx.d_err));
     }

@@ -8,7 +8,7 @@
 //                   from the input order.
 // Measured against the per-row gathers on the same pings (whole rtacx_reduce,
 // us): 2^20 samples, 512 x 1024, 33 taps, narrow beams: 1380 -> 96; 2^22 samples,
-// 512 x 4096, wide beams on a floor: 14430 -> 443 (1180 with the whole beam);
+// 512 x 4096, wide beams on a floor: 14430 -> 418 (1180 with the whole beam);
 // 150003 samples, 387 x 777, 24 taps: 246 -> 42; 20000 samples, 256 x 500, row
 // pairs: 94 -> 22. k_cells is bound by the beam lookups' shared memory (single
 // tables) and by the FMA pipe (16 copies), at one lookup per (sample, bearing).
@@ -361,7 +361,7 @@ bool find_lobe(const Context& c, Lobe& l)
 // whole table, in the last window of the sort; their bearings lie side by side
 // on the lanes, since row by row the reductions bound it (161 -> 61 us against
 // the order that spares the table's banks). Whole pings without / with, us:
-// 2^22 samples, 512 x 4096 1178 -> 439; 2^20, 600 x 2048 429 -> 138; 2^16, 512 x
+// 2^22 samples, 512 x 4096 1178 -> 418; 2^20, 600 x 2048 429 -> 138; 2^16, 512 x
 // 128 60 -> 40; 2^16, 300 x 1024 58 -> 47; 2^14, 600 x 300 43 -> 50; 2^14, 300 x
 // 1024 38 -> 52: one more launch and short lists, hence kLobeFrom (samples x
 // bearings).
@@ -676,7 +676,7 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
             // The samples left are few and mostly next to knots (row by row):
             // one per warp, all windows side by side.
             gy = (uint32_t)P.windows;
-            gx = std::max(1u, 2 * resident / gy);
+            gx = std::max(1u, 4 * resident / gy);
             whole.pos_theta = L.pos_theta + (size_t)L.windows * 32 * c.lobe_bpl;
             whole.pos_col = L.pos_col + (size_t)L.windows * 32 * c.lobe_bpl;
             split_at = c.d_offsets + (bin.nBB - 1u) * bin.cell_blocks;

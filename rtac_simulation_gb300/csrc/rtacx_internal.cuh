@@ -669,6 +669,13 @@ rtacx_status run_binning(Context& ctx, const void* samples, uint64_t n, cudaStre
 // also the bitmap of range bins), scan, scatter.
 rtacx_status run_sort(Context& ctx, const BinParams& p, const SortShape& shape, const void* samples, uint64_t n,
                       uint32_t* nonempty, cudaStream_t stream);
+// Samples of a ranked sort, at most, and where the tile sort takes more than one
+// batch of reservations per thread (8 bins for each of its 768). Whole pings,
+// us, tile sort / ranked: 2^22 samples on 4129 bins 1180 / 1191; on 10000 to
+// 12000 bins 2^22 330 / 320 and 455 / 444 (441 / 418 with the phase), 2^23 788 /
+// 797 and 590 / 612: the records no longer fit the L2.
+constexpr uint64_t kMaxRanked = 1ull << 21, kMaxRankedMany = 1ull << 22;
+constexpr uint32_t kManyBins = 8 * 768;
 // Shared memory of a ranked count: the bins' counts, the bitmap, the block sums.
 inline size_t ranked_smem(uint32_t nBins, uint32_t nR)
 {

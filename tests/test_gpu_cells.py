@@ -90,6 +90,14 @@ def test_pings_around_the_ranked_sort_limits(oracle, n):
         assert rel_l2(got, oracle.reduce(wk.samples, wk.sensor)) <= TOL
 
 
+@pytest.mark.parametrize("n", [(1 << 21) + 1, (1 << 22) + 1])
+def test_many_bins_around_their_ranked_limit(oracle, n):
+    """More bins than the tile sort reserves in one batch: ranked up to 2^22."""
+    wk = ping(n, 2600, 129, 2, False)
+    got = gpu_reduce(make_context(wk), wk.samples, wk.out_shape)
+    assert rel_l2(got, oracle.reduce(wk.samples, wk.sensor)) <= TOL
+
+
 @pytest.mark.parametrize("nB,beam_taps", [(65, 605), (65, 606), (65, 607), (3, 1), (3, 2), (640, 1006), (640, 1007)])
 def test_tables_around_the_replicated_limit(oracle, nB, beam_taps):
     """Beam tables on both sides of the largest that is kept in 16 copies (for
