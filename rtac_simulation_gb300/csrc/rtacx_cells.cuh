@@ -277,6 +277,9 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
             }
         }
     }
+    // Every lane reads S.w below, also where no sample is listed (all of them
+    // next to knots): the votes converge the lanes but order no memory.
+    __syncwarp();
     near_knot = __any_sync(0xffffffffu, near_knot);
     for(cur = __reduce_min_sync(0xffffffffu, cur); cur != INT_MAX;) {
         const int w_begin = SHARED ? win0 : cur, w_end = SHARED ? P.windows : cur + 1;

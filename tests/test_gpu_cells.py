@@ -77,6 +77,18 @@ def test_lobes_on_a_flat_floor(oracle, nB, beam_taps, roll, level):
         assert rel_l2(got, oracle.reduce(good, wk.sensor)) <= TOL
 
 
+@pytest.mark.parametrize("nB,wide", [(65, False), (640, False), (65, True), (200, True)])
+@pytest.mark.parametrize("n", [1, 33, 5000, 90000])
+def test_pings_of_samples_next_to_knots_alone(oracle, n, nB, wide):
+    """Every travel on a knot (an odd pulse's knots lie on the output ranges):
+    units without a sample for the cell rows, in windows of 64 and 128 bearings,
+    shared-out windows and the lobe form."""
+    wk = ping(n, 90, nB, 9, wide)
+    wk.samples[:, 2] = wl.linspace(0.4, 30.0, 90)[np.arange(n) % 90]
+    got = gpu_reduce(make_context(wk), wk.samples, wk.out_shape)
+    assert rel_l2(got, oracle.reduce(wk.samples, wk.sensor)) <= TOL
+
+
 @pytest.mark.parametrize("n", [1023, 1025, 1 << 21, (1 << 21) + 1])
 def test_pings_around_the_ranked_sort_limits(oracle, n):
     """One count CTA and two, the most samples that are ranked and one more;
