@@ -151,15 +151,18 @@ struct CellParams {
 // Range cell of a travel and its fraction of the cell: floor and fraction of
 // travel * k + b, with the product's exact residual (fmaf) and the low part
 // of k added to the fraction (k * travel reaches the row count, a fraction of
-// which a plain float product would round away). Returns the cell's storage
-// row C + 1 (C = -1: the first cell any row's pulse reaches) or -1 for a
-// travel that reaches no row, NaN and infinities included.
+// which a plain float product would round away). The product is rounded on its
+// own: contracted into the subtraction it would carry the residual a second
+// time, and by another choice of the compiler in another kernel the count and
+// the scatter of a sort would disagree on a sample's key. Returns the cell's
+// storage row C + 1 (C = -1: the first cell any row's pulse reaches) or -1 for
+// a travel that reaches no row, NaN and infinities included.
 __device__ __forceinline__ int range_cell(const CellParams& cp, float travel, float& alpha)
 {
-    const float prod = travel * cp.k_hi;
+    const float prod = __fmul_rn(travel, cp.k_hi);
     const float err = fmaf(travel, cp.k_hi, -prod);
     const float whole = rintf(prod);
-    const float f = (prod - whole) + (err + fmaf(travel, cp.k_lo, cp.b_frac));
+    const float f = __fadd_rn(__fsub_rn(prod, whole), __fadd_rn(err, fmaf(travel, cp.k_lo, cp.b_frac)));
     const float fl = floorf(f);
     alpha = f - fl;
     const float row = whole + fl + cp.b_row;      // whole numbers below 2^22: exact

@@ -89,6 +89,17 @@ def test_pings_of_samples_next_to_knots_alone(oracle, n, nB, wide):
     assert rel_l2(got, oracle.reduce(wk.samples, wk.sensor)) <= TOL
 
 
+@pytest.mark.parametrize("n", [20001, (1 << 21) + 1])
+def test_cells_far_from_the_sensor(oracle, n):
+    """Ranges 1e5 of their spacings away, where a cell coordinate's float
+    rounding is 4e-3 of a cell: the cells' fractions keep the coordinate's
+    residual (1e-3 relative without, or with it twice), and the two sorts' count
+    and scatter agree on every sample's cell block."""
+    wk = ping(n, 1024, 33, 8, False, rmin=100.0, rmax=101.023)
+    got = gpu_reduce(make_context(wk), wk.samples, wk.out_shape)
+    assert rel_l2(got, oracle.reduce(wk.samples, wk.sensor)) <= TOL
+
+
 @pytest.mark.parametrize("n", [1023, 1025, 1 << 21, (1 << 21) + 1])
 def test_pings_around_the_ranked_sort_limits(oracle, n):
     """One count CTA and two, the most samples that are ranked and one more;
