@@ -428,7 +428,7 @@ rtacx_status rtacx_configure_2d(rtacx_ctx* ctx, const rtacx_sensor_2d* s)
     if(c.cells_on) {
         c.cell.pulse = c.d_pulse; c.cell.beam = c.d_beam; c.cell.ranges = c.d_ranges;
     }
-    else {
+    if(!c.cells_on || c.cell_from > 1) {
         const uint64_t tiles = (uint64_t)((c.nB + c.bearing_tile - 1) / c.bearing_tile) * ((c.nR + c.range_tile - 1) / c.range_tile);
         if(!upload<uint32_t>(c, c.d_tile_parts, nullptr, tiles) || !upload<uint32_t>(c, c.d_tile_first, nullptr, tiles + 1) ||
            !upload<uint4>(c, c.d_items, nullptr, tiles * 256) || !upload<uint32_t>(c, c.d_item_counter, nullptr, 1))

@@ -405,12 +405,39 @@ bool configure_cells_1d(Context& c)
 // us, row by row / sorted: 1049 ranges, 5 rows, 2^15 samples 19 / 33, 2^17 31 /
 // 35, 2^19 134 / 51; 4096 ranges, 32 rows, 2^15 32 / 33, 2^17 82 / 40; 9 rows
 // 2^17 30 / 35. They meet near 512 reductions per row, or a million in all.
+// 2D: see cell_from_2d.
 bool takes_cells(const Context& c, uint64_t n)
 {
-    return c.cells_on && (!c.cell_rows || n * (uint64_t)c.cell.rows <= std::min<uint64_t>(512ull * c.nR, 1ull << 20));
+    if(!c.cells_on) return false;
+    if(c.dims == 1) return !c.cell_rows || n * (uint64_t)c.cell.rows <= std::min<uint64_t>(512ull * c.nR, 1ull << 20);
+    return n == 0 || n >= c.cell_from;
 }
 
 int cell_replicas(const Context& c, uint64_t n) { return !c.cell_rows && n >= kReplicateFrom1D ? kReplicas1D : 1; }
+
+// Samples from which a 2D ping takes the cell form. It clears and filters all
+// cell rows whatever the sample count; the gathers' work follows the samples,
+// and the tiles that any sample reaches. Whole pings, us, cell form / gather, 33
+// taps, uniform scene (half of the samples in 1 % of the ranges): 512 x 1024
+// 2^9 56 / 62; 512 x 2048 2^9 66 / 66; 512 x 4096 2^7 91 / 89 (76), 2^9 91 / 85
+// (99), 2^12 89 / 83 (115), 2^13 87 / 89 (122); 1024 x 4096 2^10 144 / 93 (103),
+// 2^14 138 / 117 (130), 2^15 138 / 150 (153), with 9 taps 2^10 103 / 96 (87),
+// 2^12 99 / 91 (116); 1024 x 8192 2^10 244 / 126 (132), 2^15 234 / 199 (218),
+// 2^16 236 / 289 (324). Wide beams: 1024 x 8192 2^14 302 / 224 (234), 2^15 298 /
+// 339 (355). Row pairs, which have no filter: 1024 x 4096 2^8 70 / 62 (64), 2^9
+// 68 / 72 (74); 1024 x 8192 2^10 107 / 101 (101), 2^12 113 / 126 (122). So the
+// cell form takes 40 us and, per million entries, 12 and 0.36 per tap (7.5 for
+// pairs); the gather 65 us (52) at 64 samples, up to 10 more with every
+// doubling, in the end 2 us per 1000 samples (wide beams 4 per 1024 bearings).
+uint64_t cell_from_2d(const Context& c)
+{
+    const double entries = 1e-6 * (double)c.cell.cp.cells * c.cell.pitch;
+    const double cells = 40.0 + entries * (c.cell_pairs ? 7.5 : 12.0 + 0.36 * c.H);
+    double from = 64.0 * std::exp2(std::min((cells - (c.cell_pairs ? 52.0 : 65.0)) / 10.0, 40.0));
+    if(!c.cell_pairs)
+        from = std::min(from, 1e3 * (cells - 55.0 - 9.0 * entries) / (c.cell_shared ? std::max(2.0, c.nB / 256.0) : 2.0));
+    return from > 100.0 ? (uint64_t)from : 0;
+}
 
 // Decides whether a configured 2D sensor takes the cell form and builds its
 // tables: row pairs where no travel reaches three rows, else knot cells where
@@ -577,6 +604,7 @@ bool configure_cells(Context& c, double beam_support)
     c.cell.col_bearing = Arena::at<int>(c, at_bearing);
     set_ping_params(c);
     c.cells_on = true;
+    c.cell_from = cell_from_2d(c);
     if(!c.lobe_on) return true;
     c.lobe_on = raise_smem_limit((const void*)lobe_fn(c.lobe_bpl), l_smem) == cudaSuccess &&
                 raise_smem_limit((const void*)k_cells_filter<true>, filter_smem(H)) == cudaSuccess;

@@ -570,6 +570,7 @@ struct Context {
 
     // Cell form of a 2D ping (rtacx_cells.cu).
     bool cells_on = false;
+    uint64_t cell_from = 0;             // 2D: fewest samples of a ping that takes it
     int cell_bpl = 2;                   // bearings per lane
     int cell_copies = 1;                // copies of the beam table in the accumulation's shared memory
     int cell_ctas = 1;                  // resident CTAs of the accumulation per SM

@@ -200,6 +200,39 @@ def test_row_pairs_match_fp64_oracle(oracle, n, nR, nB, H, wide, margin):
     assert rel_l2(got, want) <= TOL, rel_l2(got, want)
 
 
+def by_rows(ctx):
+    """Whether the context's last (traced) ping went through the per-row
+    gathers, which alone have windows."""
+    return ctx.stage_times()["windows"] > 0.0
+
+
+def row_pairs(wk):
+    """The ping's sensor with a pulse one output range long."""
+    s = wk.sensor
+    res = float(wl.linspace_resolution(s["range_min"], s["range_max"], s["range_count"]))
+    s["pulse"] = np.exp(1j * np.linspace(0.0, 9.0, 20)).astype(np.complex64)
+    s["pulse_duration"] = float(np.float32(np.float32(res) / np.float32(1500.0)))
+    s["margin"] = float(np.float32(1500.0) * np.float32(s["pulse_duration"]))
+    return wk
+
+
+@pytest.mark.parametrize("nB,nR,wide,pairs,few,many", [
+    (512, 4096, False, False, 201, 3001), (512, 6000, True, False, 1000, 20000), (600, 8000, False, True, 33, 3000),
+])
+def test_small_pings_of_large_sensors_gather_per_row(oracle, nB, nR, wide, pairs, few, many):
+    """A few samples against cell rows of a size: the gathers; more of them, or
+    none, the cell form, on one context in turn."""
+    wk = ping(many, nR, nB, 33, wide)
+    if pairs:
+        row_pairs(wk)
+    ctx = make_context(wk)
+    ctx.set_tracing(True)
+    for n in (few, many, 0, 1, few):
+        got = gpu_reduce(ctx, wk.samples[:n], wk.out_shape)
+        assert by_rows(ctx) == (0 < n <= few), n
+        assert rel_l2(got, oracle.reduce(wk.samples[:n], wk.sensor)) <= TOL, n
+
+
 def ping_1d(n, nR, taps, H=0, ext_bins=0.0, seed=5):
     rmin, rmax = 0.4, 30.0
     res = float(wl.linspace_resolution(rmin, rmax, nR))
