@@ -114,17 +114,62 @@ struct Batch {
         return (uint32_t)want;
     }
 
-    // Whether the batch runs on the fused kernel with the cell form: when the
-    // per-row gathers' share of the work (samples x bearings) is at most half,
-    // since that kernel keeps fewer of their CTAs resident.
+    // Estimates of a ping in the fused kernel (us): of the per-row gathers,
+    // with the default tiles and `alone` the time of its tiles one behind the
+    // other on one CTA each, and of the cell form.
+    static double rows_us(const Context& c, uint64_t n, double& alone)
+    {
+        const double samples = (double)n, TR = gather_shape_rows(2), TB = gather_shape_bearings(2);
+        if(c.dims == 1) { alone = 0.0; return 0.09e-3 * samples; }
+        const double tr = std::ceil(c.nR / TR), tb = std::ceil(c.nB / TB);
+        const double pulse_rows = (double)c.duration * c.c * (c.nR - 1.0) / std::max(1e-30, (double)c.rmax - c.rmin);
+        double entered = std::min(tr, 1.0 + pulse_rows / TR), across = tb;      // tiles that a sample enters
+        if(c.bin.nBB > 1) {
+            const double fan = c.bin.nBB / (double)c.bin.bb_scale;
+            across = std::min(tb, tb / fan * ((fan - c.span) * TB / c.nB + c.span + fan / c.bin.nBB));
+        }
+        entered *= across;
+        alone = 0.35 * samples * entered / (tr * tb);
+        return 5e-6 * c.nR * c.nB + samples * entered * TR * TB / 4e6;
+    }
+    static double cells_us(const Context& c, uint64_t n)
+    {
+        if(c.dims == 1) return 0.015e-3 * n;
+        const double entries = 1e-6 * (double)c.cell.cp.cells * c.cell.pitch;
+        return entries * (c.cell_pairs ? 13.0 : 18.0 + 0.4 * c.H) +
+               0.8e-6 * n * (c.cell_shared ? c.cell.pitch : 32.0 * c.cell_bpl);
+    }
+
+    // Whether the batch runs on the fused kernel with the cell form: where that
+    // is estimated to be faster (it clears and filters every cell row, whatever
+    // the samples), and when the per-row gathers' share of the work (samples x
+    // bearings) is at most half, since that kernel keeps fewer of their CTAs
+    // resident. us per batch, per-row / cell form, samples spread evenly (a
+    // floor in view): one ping of 512 x 1024, 33 taps, 2^12 samples 57 / 118 (89
+    // / 113), 2^14 78 / 116 (147 / 109), 2^16 159 / 113 (443 / 108); six of them
+    // 2^12 98 / 210 (127 / 201), 2^14 198 / 202 (245 / 202); six of 512 x 4096
+    // 2^14 251 / 500 (278 / 503), 2^16 647 / 558 (683 / 531); six of 1024 x 8192
+    // 2^15 824 / 1632 (851 / 1636), 2^17 2572 / 1778 (2640 / 1731); six wide beams
+    // of 512 x 1024 2^10 90 / 244 (119 / 248), 2^13 336 / 216 (457 / 228); six row
+    // pairs of 1024 x 4096 2^13 346 / 565 (336 / 562), 2^15 726 / 582 (749 / 646);
+    // six 1D pings 2^8 44 / 30, 2^17 113 / 45. The estimates are fitted to both
+    // scenes, towards the cell form where they differ.
     void choose_form()
     {
-        double per_row = 0.0, cell = 0.0;
+        double per_row = 0.0, cell = 0.0, rows = 0.0, longest = 0.0, form = 28.0;
+        bool any_2d = false;
         for(const rtacx_ping_desc& p : pings) {
             const Context& c = p.ctx->impl;
-            (takes_cells(c, p.n) ? cell : per_row) += (double)p.n * c.nB;
+            const bool takes = takes_cells(c, p.n);
+            (takes ? cell : per_row) += (double)p.n * c.nB;
+            double alone;
+            const double r = rows_us(c, p.n, alone);
+            rows += r;
+            longest = std::max(longest, alone);
+            form += takes ? cells_us(c, p.n) : r;
+            any_2d |= takes && c.dims == 2;
         }
-        cells = !staged && cell > 0.0 && per_row <= cell;
+        cells = !staged && cell > 0.0 && per_row <= cell && form + (any_2d ? 70.0 : 0.0) < 35.0 + std::max(rows, longest);
         per_row_2d = false;
         for(const rtacx_ping_desc& p : pings)
             if(p.ctx->impl.dims == 2 && !(cells && takes_cells(p.ctx->impl, p.n))) per_row_2d = true;

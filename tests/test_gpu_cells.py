@@ -233,6 +233,29 @@ def test_small_pings_of_large_sensors_gather_per_row(oracle, nB, nR, wide, pairs
         assert rel_l2(got, oracle.reduce(wk.samples[:n], wk.sensor)) <= TOL, n
 
 
+@pytest.mark.parametrize("large", [0, 150000])
+def test_batches_of_small_pings(oracle, large):
+    """Small pings of every form alone, which the per-row gathers take, and
+    next to a large one, with which the cell form does."""
+    from rtac_simulation_gb300 import _lib
+    pings = [ping(300, 1024, 512, 33, False), ping(900, 512, 130, 17, True), row_pairs(ping(50, 400, 200, 5, True)),
+             ping(100, 4096, 512, 33, False), ping_1d(999, 64, 17), ping_1d(999, 64, 2, 40, 2.0)]
+    if large:
+        pings.append(ping(large, 257, 129, 33, False))
+    ctxs = [make_context(wk) for wk in pings]
+    devs = [torch.from_numpy(wk.samples.reshape(-1)).cuda() for wk in pings]
+    outs = [torch.full(wk.out_shape + (2,), float("nan"), device="cuda") for wk in pings]
+    batch = _lib.Batch(0)
+    batch.plan([(c, d, wk.n, o) for wk, c, d, o in zip(pings, ctxs, devs, outs)], autotune=False)
+    for _ in range(2):
+        batch.run(torch.cuda.current_stream())
+    batch.status(torch.cuda.current_stream())
+    for wk, o in zip(pings, outs):
+        got = o.cpu().numpy()[..., 0] + 1j * o.cpu().numpy()[..., 1]
+        assert rel_l2(got, oracle.reduce(wk.samples, wk.sensor)) <= TOL, (wk.name, wk.n)
+    batch.close()
+
+
 def ping_1d(n, nR, taps, H=0, ext_bins=0.0, seed=5):
     rmin, rmax = 0.4, 30.0
     res = float(wl.linspace_resolution(rmin, rmax, nR))
