@@ -130,6 +130,29 @@ def test_tables_around_the_replicated_limit(oracle, nB, beam_taps):
     assert rel_l2(got, oracle.reduce(wk.samples, wk.sensor)) <= TOL
 
 
+@pytest.mark.parametrize("spread,span", [(0.01, 0.5), (0.0, 0.1), (0.0, 0.02)])
+def test_clustered_bearings(oracle, spread, span):
+    """Bearings that no windows of 128 can hold (most of them in one direction,
+    narrow beams): right, and configured in a fraction of the 0.1 s that a
+    search through all windows took."""
+    import time
+    wk = ping(5000, 100, 512, 9, False)
+    s = wk.sensor
+    s["bearings"] = np.concatenate([[-1.1], np.linspace(0.0, spread * wl.DEG, 510), [1.1]]).astype(np.float32)
+    s["beam_span"] = span * wl.DEG
+    wk.samples[::2, 3] = np.linspace(-span, span, len(wk.samples[::2])) * wl.DEG
+    wk.samples[1::8, 3] = np.float32(1.1)
+    ctx = make_context(wk)
+    took = []
+    for _ in range(3):
+        t0 = time.perf_counter()
+        ctx.configure_2d(**s)
+        took.append(time.perf_counter() - t0)
+    got = gpu_reduce(ctx, wk.samples, wk.out_shape)
+    assert rel_l2(got, oracle.reduce(wk.samples, s)) <= TOL
+    assert min(took) < 0.02, took
+
+
 @pytest.mark.parametrize("change", ["half_margin", "half_tap", "long_pulse"])
 def test_sensors_off_the_cell_rule_match_fp64_oracle(oracle, change):
     """A margin that cuts the pulse's window, taps that are not one range
