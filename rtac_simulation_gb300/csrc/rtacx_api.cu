@@ -122,26 +122,12 @@ void free_config(Context& c)
     c.psf_tex = 0;
     if(c.psf_array) cudaFreeArray(c.psf_array);
     c.psf_array = nullptr;
-    free_dev(c.d_pulse); free_dev(c.d_beam); free_dev(c.d_bearings); free_dev(c.d_ranges);
-    free_dev(c.d_support); free_dev(c.d_bb_tiles64); free_dev(c.d_bb_tiles128); c.d_bb_tiles = nullptr;
-    free_dev(c.d_offsets); free_dev(c.d_totals);
-    free_dev(c.d_win); free_dev(c.d_hist);
-    free_dev(c.d_tile_parts); free_dev(c.d_tile_first); free_dev(c.d_items); free_dev(c.d_item_counter);
-    c.hist_cols = 0;
+    free_dev(c.d_config);
+    c.d_pulse = nullptr; c.d_beam = nullptr; c.d_bearings = nullptr; c.d_ranges = nullptr; c.d_support = nullptr;
+    c.d_bb_tiles64 = nullptr; c.d_bb_tiles128 = nullptr; c.d_bb_tiles = nullptr;
+    c.d_offsets = nullptr; c.d_totals = nullptr; c.d_win = nullptr; c.d_hist = nullptr;
+    c.d_tile_parts = nullptr; c.d_tile_first = nullptr; c.d_items = nullptr; c.d_item_counter = nullptr;
     c.configured = false;
-}
-
-template <typename T>
-bool upload(Context& c, T*& dst, const T* src, size_t count)
-{
-    free_dev(dst);
-    if(count == 0) count = 1;
-    if(cudaMalloc(&dst, count * sizeof(T)) != cudaSuccess) { cudaGetLastError(); return c.fail("cudaMalloc failed"); }
-    if(src && cudaMemcpy(dst, src, count * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess) {
-        cudaGetLastError();
-        return c.fail("cudaMemcpy failed");
-    }
-    return true;
 }
 
 bool all_finite(const float* p, size_t n)
@@ -159,7 +145,7 @@ struct Common {
 // Validation and the parts shared by the 1D and 2D configurations: Binner
 // reconfiguration (src/SensorInstance.cu:32, src/Binner.cu:15-22), Key
 // parameters, overlap, output range table, pulse table and per-row support.
-bool configure_common(Context& c, const Common& s, float pulse_scale)
+bool configure_common(Context& c, const Common& s, float pulse_scale, ConfigArena& arena)
 {
     if(!(std::isfinite(s.rmin) && std::isfinite(s.rmax) && std::isfinite(s.margin)))
         return c.fail("range_min, range_max and margin must be finite");
@@ -177,30 +163,33 @@ bool configure_common(Context& c, const Common& s, float pulse_scale)
     c.key = host_key_params(s.nR, s.rmin, s.rmax, s.margin);
     c.overlap = (s.nR > 1) ? host_bin_overlap(s.rmin, s.rmax, s.nR, s.margin) : 0;
 
-    std::vector<float> ranges(s.nR);
-    for(uint32_t r = 0; r < s.nR; r++) ranges[r] = host_linspace_at(s.rmin, s.rmax, s.nR, r);
+    c.ranges.resize(s.nR);
+    for(uint32_t r = 0; r < s.nR; r++) c.ranges[r] = host_linspace_at(s.rmin, s.rmax, s.nR, r);
 
     // Range bins that can hold a sample with non-zero pulse weight for row r:
     // |travel - R_r| < extent / 2 * (1 + 1 / H), widened by a relative slack.
     const double ext = 1.0 / (double)pulse_scale;
     const double half = 0.5 * ext * (1.0 + 1.0 / s.H) * (1.0 + 1e-4);
-    std::vector<int2> support(s.nR);
+    c.support.resize(s.nR);
     for(uint32_t r = 0; r < s.nR; r++) {
-        const double R = ranges[r];
+        const double R = c.ranges[r];
         const double slack = 1e-6 * (std::fabs(R) + half) + 1e-30;
         const float lo = (float)(R - half - slack), hi = (float)(R + half + slack);
-        support[r] = make_int2((int)host_range_key_clamped(c.key, lo), (int)host_range_key_clamped(c.key, hi));
+        c.support[r] = make_int2((int)host_range_key_clamped(c.key, lo), (int)host_range_key_clamped(c.key, hi));
     }
     std::vector<float2> pad(s.H + 2, make_float2(0.f, 0.f));
     std::memcpy(pad.data() + 1, s.pulse, 2 * sizeof(float) * s.H);
     c.red.nR = s.nR;
     c.red.range_axis = host_axis_lerp(pulse_scale, s.H);
-    return upload(c, c.d_ranges, ranges.data(), ranges.size()) &&
-           upload(c, c.d_support, support.data(), support.size()) &&
-           upload(c, c.d_pulse, pad.data(), pad.size());
+    arena.table(c.d_ranges, c.ranges);
+    arena.table(c.d_support, c.support);
+    arena.table(c.d_pulse, pad);
+    return true;
 }
 
-bool allocate_bins(Context& c)
+// The scratch that goes by the bins of the sensor's orders; then everything in
+// the arena goes to the device.
+rtacx_status commit_config(Context& c, ConfigArena& arena)
 {
     c.sort = sort_shape(c, c.bin.nBins, false);
     uint32_t bins = c.bin.nBins;
@@ -212,12 +201,19 @@ bool allocate_bins(Context& c)
         c.lobe_sort = sort_shape(c, c.lobe_bin.nBins, true);
         bins = std::max(bins, c.lobe_bin.nBins);
     }
-    const size_t cols = (size_t)bins * kCursorStride;
-    return upload<uint32_t>(c, c.d_offsets, nullptr, bins + 1) &&
-           upload<uint32_t>(c, c.d_totals, nullptr, bins + bins / 1024 + 1) &&   // + block sums
-           upload<int2>(c, c.d_win, nullptr, c.nR) &&
-           upload<uint32_t>(c, c.d_hist, nullptr, cols) &&
-           ((c.hist_cols = cols), true);
+    arena.scratch(c.d_offsets, bins + 1);
+    arena.scratch(c.d_totals, bins + bins / 1024 + 1);   // + block sums
+    arena.scratch(c.d_win, c.nR);
+    arena.scratch(c.d_hist, cursor_word(bins + 1));
+    const cudaError_t e = arena.commit(c.d_config);
+    if(e == cudaSuccess) {
+        if(c.cells_on) bind_cells(c);
+        if(c.capacity) ensure_cells(c);       // (otherwise with the first samples' scratch)
+        return RTACX_OK;
+    }
+    c.error = e == cudaErrorMemoryAllocation ? "out of device memory for the sensor's tables" : "uploading the sensor's tables failed";
+    free_config(c);
+    return e == cudaErrorMemoryAllocation ? RTACX_ERR_OUT_OF_MEMORY : RTACX_ERR_CUDA;
 }
 
 rtacx_status set_device(Context& c)
@@ -302,7 +298,8 @@ rtacx_status rtacx_configure_1d(rtacx_ctx* ctx, const rtacx_sensor_1d* s)
     const float scale = host_pulse_scale(s->pulse_duration, s->sound_celerity, literal);
     Common cm{s->range_min, s->range_max, s->sound_celerity, s->pulse_duration, s->margin,
               s->range_count, s->pulse_len, s->pulse};
-    if(!configure_common(c, cm, scale)) return RTACX_ERR_INVALID_ARGUMENT;
+    ConfigArena arena;
+    if(!configure_common(c, cm, scale, arena)) return RTACX_ERR_INVALID_ARGUMENT;
     if((s->pulse_len + 2) * sizeof(float2) > kMaxGatherSmem) {
         c.error = "pulse table too long for shared memory";
         return RTACX_ERR_UNSUPPORTED;
@@ -313,21 +310,19 @@ rtacx_status rtacx_configure_1d(rtacx_ctx* ctx, const rtacx_sensor_1d* s)
     c.bin = BinParams{c.key, 1u, 0.0f, 0.0f, c.nR, 3u, 0};
     sync_echo(c);
     if(c.nR > kMaxSmemBins) { c.error = "range_count above the shared-memory histogram limit"; return RTACX_ERR_UNSUPPORTED; }
-    std::vector<float> one(1, 0.0f);
-    free_cells(c);
-    if(!upload(c, c.d_beam, one.data(), 1) || !upload(c, c.d_bearings, one.data(), 1) || !allocate_bins(c))
-        return RTACX_ERR_OUT_OF_MEMORY;
-    if((s->flags & RTACX_FLAG_TEXTURE_PSF) && make_pulse_texture_1d(c, s, scale) != RTACX_OK) return RTACX_ERR_CUDA;
+    const float none = 0.0f;
+    arena.table(c.d_beam, &none, 1);
+    arena.table(c.d_bearings, &none, 1);
     if(s->flags & RTACX_FLAG_TEXTURE_CLAMP) {
         // Clamp addressing gives every sample of the window the pulse's edge
         // taps, so each row reads its whole reference window, not only the
         // bins that hold the pulse's support.
-        std::vector<int2> whole(c.nR, make_int2(0, (int)c.nR - 1));
-        if(!upload(c, c.d_support, whole.data(), whole.size())) return RTACX_ERR_OUT_OF_MEMORY;
+        arena.table(c.d_support, std::vector<int2>(c.nR, make_int2(0, (int)c.nR - 1)));
     }
-    if(!(s->flags & RTACX_FLAG_TEXTURE_PSF) && configure_cells_1d(c)) {
-        c.cell.pulse = c.d_pulse; c.cell.ranges = c.d_ranges;
-    }
+    if(!(s->flags & RTACX_FLAG_TEXTURE_PSF)) configure_cells_1d(c, arena);
+    const rtacx_status st = commit_config(c, arena);
+    if(st != RTACX_OK) return st;
+    if((s->flags & RTACX_FLAG_TEXTURE_PSF) && make_pulse_texture_1d(c, s, scale) != RTACX_OK) return RTACX_ERR_CUDA;
     c.configured = true;
     return RTACX_OK;
 }
@@ -350,7 +345,8 @@ rtacx_status rtacx_configure_2d(rtacx_ctx* ctx, const rtacx_sensor_2d* s)
     const float scale = host_pulse_scale(s->pulse_duration, s->sound_celerity, false);
     Common cm{s->range_min, s->range_max, s->sound_celerity, s->pulse_duration, s->margin,
               s->range_count, s->pulse_len, s->pulse};
-    if(!configure_common(c, cm, scale)) return RTACX_ERR_INVALID_ARGUMENT;
+    ConfigArena arena;
+    if(!configure_common(c, cm, scale, arena)) return RTACX_ERR_INVALID_ARGUMENT;
 
     c.dims = 2; c.flags = s->flags;
     c.nB = s->bearing_count; c.W = s->beam_len; c.span = s->beam_span;
@@ -413,27 +409,26 @@ rtacx_status rtacx_configure_2d(rtacx_ctx* ctx, const rtacx_sensor_2d* s)
     };
     const std::vector<int2> bbt64 = tile_ranges(64), bbt128 = tile_ranges(128);
     if(!texture_psf) {
-        configure_cells(c, sb);
+        configure_cells(c, sb, arena);
         sync_echo(c);
     }
     std::vector<float> bpad(c.W + 2, 0.0f);
     std::memcpy(bpad.data() + 1, s->beam, sizeof(float) * c.W);
-    if(!upload(c, c.d_beam, bpad.data(), bpad.size()) ||
-       !upload(c, c.d_bearings, c.bearings.data(), c.bearings.size()) ||
-       !upload(c, c.d_bb_tiles64, bbt64.data(), bbt64.size()) ||
-       !upload(c, c.d_bb_tiles128, bbt128.data(), bbt128.size()) || !allocate_bins(c))
-        return RTACX_ERR_OUT_OF_MEMORY;
-    c.d_bb_tiles = (c.bearing_tile == 64) ? c.d_bb_tiles64 : c.d_bb_tiles128;
-    if(texture_psf && make_psf_texture(c, s) != RTACX_OK) return RTACX_ERR_CUDA;
-    if(c.cells_on) {
-        c.cell.pulse = c.d_pulse; c.cell.beam = c.d_beam; c.cell.ranges = c.d_ranges;
-    }
+    arena.table(c.d_beam, bpad);
+    arena.table(c.d_bearings, c.bearings);
+    arena.table(c.d_bb_tiles64, bbt64);
+    arena.table(c.d_bb_tiles128, bbt128);
     if(!c.cells_on || c.cell_from > 1) {
         const uint64_t tiles = (uint64_t)((c.nB + c.bearing_tile - 1) / c.bearing_tile) * ((c.nR + c.range_tile - 1) / c.range_tile);
-        if(!upload<uint32_t>(c, c.d_tile_parts, nullptr, tiles) || !upload<uint32_t>(c, c.d_tile_first, nullptr, tiles + 1) ||
-           !upload<uint4>(c, c.d_items, nullptr, tiles * 256) || !upload<uint32_t>(c, c.d_item_counter, nullptr, 1))
-            return RTACX_ERR_OUT_OF_MEMORY;
+        arena.scratch(c.d_tile_parts, tiles);
+        arena.scratch(c.d_tile_first, tiles + 1);
+        arena.scratch(c.d_items, tiles * 256);
+        arena.scratch(c.d_item_counter, 1);
     }
+    const rtacx_status st = commit_config(c, arena);
+    if(st != RTACX_OK) return st;
+    c.d_bb_tiles = (c.bearing_tile == 64) ? c.d_bb_tiles64 : c.d_bb_tiles128;
+    if(texture_psf && make_psf_texture(c, s) != RTACX_OK) return RTACX_ERR_CUDA;
     c.configured = true;
     return RTACX_OK;
 }

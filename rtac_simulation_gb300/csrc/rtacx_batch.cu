@@ -212,6 +212,7 @@ struct Batch {
             if(c.dims == 2) d.bb_tiles = (TB == 64) ? c.d_bb_tiles64 : c.d_bb_tiles128;   // ranges for width TB
             if(cell_form) {
                 d.cell = c.cell;
+                d.cell.cells = c.d_cells;
                 d.cell.sorted = c.d_sorted;
                 d.cell.out = d.out;
                 d.cell.replicas = c.dims == 1 ? cell_replicas(c, n) : 1;

@@ -399,6 +399,7 @@ uint32_t hist_grid(uint32_t ctas, uint64_t n)
 
 bool ensure_capacity(Context& ctx, uint64_t n)
 {
+    if(n && ctx.cells_on && !ctx.d_cells) ensure_cells(ctx);
     if(n <= ctx.capacity) return true;
     const uint64_t cap = std::max<uint64_t>(n, 1024), ranks = std::min<uint64_t>(cap, kMaxRankedMany);
     // The ranks of the cell form's sort lie behind the records; without them

@@ -18,7 +18,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstring>
 #include <numeric>
 
 namespace rtacx {
@@ -171,46 +170,33 @@ __global__ void k_rows_off_1d(const CellPing P, const uint32_t* nonempty)
     if(r < (int)P.nR && !row_on(after_chain(nonempty), (int)P.nR, P.overlap, r)) P.out[r] = make_float2(0.f, 0.f);
 }
 
-// The tables and the cell rows of a context in one allocation, filled by one
-// copy (each cudaMalloc and cudaMemcpy of its own costs a configuration 10 to
-// 20 us).
-struct Arena {
-    std::vector<unsigned char> host;
-    template <typename T>
-    size_t add(const std::vector<T>& v)
-    {
-        const size_t at = (host.size() + 255) / 256 * 256;
-        host.resize(at + v.size() * sizeof(T));
-        std::memcpy(host.data() + at, v.data(), v.size() * sizeof(T));
-        return at;
-    }
-    // The tables with `cells` more bytes (not initialised) behind them.
-    bool upload(Context& c, size_t cells)
-    {
-        host.resize((host.size() + 255) / 256 * 256);
-        if(cudaMalloc(&c.d_cell_arena, host.size() + cells) != cudaSuccess ||
-           cudaMemcpy(c.d_cell_arena, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        c.d_cells = at<float4>(c, host.size());
-        return true;
-    }
-    template <typename T>
-    static T* at(const Context& c, size_t offset) { return reinterpret_cast<T*>(c.d_cell_arena + offset); }
-};
-
 } // namespace
 
 void free_cells(Context& c)
 {
-    if(c.d_cell_arena) cudaFree(c.d_cell_arena);
-    c.d_cell_arena = nullptr;
+    if(c.d_cells) cudaFree(c.d_cells);
     c.d_cells = nullptr;
     c.d_nonempty = nullptr;
     c.lobe_on = false;
     c.cells_on = false;
     c.sorted_cells_n = 0;
+}
+
+void ensure_cells(Context& c)
+{
+    if(!c.cells_on || c.d_cells || cudaMalloc(&c.d_cells, c.cell_bytes) == cudaSuccess) return;
+    cudaGetLastError();
+    free_cells(c);
+}
+
+void bind_cells(Context& c)
+{
+    c.cell.pulse = c.d_pulse; c.cell.beam = c.d_beam; c.cell.ranges = c.d_ranges;
+    if(c.lobe_on) {
+        CellPing& L = c.lobe;
+        L.pulse = c.cell.pulse; L.ranges = c.cell.ranges; L.taps = c.cell.taps; L.row_dev = c.cell.row_dev;
+        L.col_bearing = c.cell.col_bearing;
+    }
 }
 
 namespace {
@@ -219,7 +205,6 @@ namespace {
 // each row lies from it, in taps.
 struct RowFit {
     double k = 0.0, spacing = 0.0, R0 = 0.0, worst = 0.0, last = 0.0;   // taps per metre; metres; taps; metres
-    std::vector<double> R;
     std::vector<float> dev;
 };
 
@@ -228,22 +213,20 @@ bool fit_rows(const Context& c, RowFit& f)
     const int nR = (int)c.nR;
     if(nR < 2 || c.H < 1) return false;
     f.k = (double)c.red.range_axis.k_hi + (double)c.red.range_axis.k_lo;
-    f.R.resize(nR);
     double sr = 0.0, sx = 0.0;
     for(int r = 0; r < nR; r++) {
-        f.R[r] = host_linspace_at(c.rmin, c.rmax, c.nR, (uint32_t)r);
-        sr += f.R[r];
-        sx += ((double)r - 0.5 * (nR - 1)) * f.R[r];
+        sr += c.ranges[r];
+        sx += ((double)r - 0.5 * (nR - 1)) * c.ranges[r];
     }
     f.spacing = sx / ((double)nR * ((double)nR * nR - 1.0) / 12.0);
     f.R0 = sr / nR - 0.5 * (nR - 1) * f.spacing;
     if(!(f.spacing > 0.0) || !std::isfinite(f.spacing)) return false;
     f.dev.resize(nR);
     for(int r = 0; r < nR; r++) {
-        const double e = f.k * (f.R0 + r * f.spacing - f.R[r]);
+        const double e = f.k * (f.R0 + r * f.spacing - c.ranges[r]);
         f.dev[r] = (float)e;
         f.worst = std::max(f.worst, std::fabs(e));
-        f.last = std::max(f.last, std::fabs(f.R[r]));
+        f.last = std::max(f.last, std::fabs((double)c.ranges[r]));
     }
     return true;
 }
@@ -280,13 +263,9 @@ bool knot_cells(Context& c, const RowFit& f)
     // spacing's over half the pulse, and the rounding of travel - range.
     const double knot = 1.01 * (f.worst + std::fabs(f.k * f.spacing - 1.0) * (0.5 * H + 1.0)) + 2e-6 + 1.5e-7 * H;
     if(!(knot <= kMaxKnot)) return false;
-    for(int r = 0; r < nR; r++) {
-        const double reach = 0.5 * ((double)H / f.k) * (1.0 + 1.0 / H) * (1.0 + 1e-4);
-        const double slack = 1e-6 * (std::fabs(f.R[r]) + reach) + 1e-30;
-        const int lo = (int)host_range_key_clamped(c.key, (float)(f.R[r] - reach - slack));
-        const int hi = (int)host_range_key_clamped(c.key, (float)(f.R[r] + reach + slack));
-        if(lo < std::max(0ll, (long long)r - c.overlap) || hi > std::min((long long)nR - 1, (long long)r + c.overlap)) return false;
-    }
+    for(int r = 0; r < nR; r++)
+        if(c.support[r].x < std::max(0ll, (long long)r - c.overlap) ||
+           c.support[r].y > std::min((long long)nR - 1, (long long)r + c.overlap)) return false;
     return set_cell_axis(c.cell.cp, f, 0.5 * H - 0.5 - f.R0 / f.spacing, 1, nR + H, knot, H);
 }
 
@@ -321,7 +300,6 @@ std::vector<float4> cell_taps(const Context& c, const RowFit& f)
 void set_ping_params(Context& c)
 {
     CellPing& P = c.cell;
-    P.cells = c.d_cells;
     P.range_axis = c.red.range_axis; P.beam_axis = c.red.beam_axis;
     P.key = c.key; P.overlap = c.overlap;
     P.nR = c.nR; P.nB = c.nB;
@@ -370,7 +348,7 @@ constexpr uint64_t kLobeFrom = 1ull << 24;
 } // namespace
 
 // 1D sensors: knot cells where the pulse's taps allow them, else row by row.
-bool configure_cells_1d(Context& c)
+bool configure_cells_1d(Context& c, ConfigArena& arena)
 {
     free_cells(c);
     RowFit f;
@@ -386,14 +364,12 @@ bool configure_cells_1d(Context& c)
         // First row reached: floor(y) + 1 with y = (travel - reach - R0) / spacing.
         ok = set_cell_axis(c.cell.cp, f, -(reach + f.R0) / f.spacing, c.cell.rows, nR + c.cell.rows - 1, 0.0, (int)c.H);
     }
-    Arena arena;
-    const size_t dev = arena.add(f.dev), taps = arena.add(cell_taps(c, f)), bits = arena.add(std::vector<uint32_t>((nR + 127) / 128 * 4, 0u));
-    ok = ok && arena.upload(c, (c.cell_rows ? 1 : (size_t)kReplicas1D * c.cell.cp.cells) * sizeof(float4)) &&
-         raise_smem_limit((const void*)k_cells_filter_1d, filter_smem_1d(c.cell_rows ? 1 : (int)c.H, kFilterRows1D)) == cudaSuccess;
-    if(!ok) { free_cells(c); return false; }
-    c.cell.row_dev = Arena::at<float>(c, dev);
-    c.cell.taps = Arena::at<float4>(c, taps);
-    c.d_nonempty = Arena::at<uint32_t>(c, bits);
+    if(!ok || raise_smem_limit((const void*)k_cells_filter_1d, filter_smem_1d(c.cell_rows ? 1 : (int)c.H, kFilterRows1D)) != cudaSuccess)
+        return false;
+    arena.table(c.cell.row_dev, f.dev);
+    arena.table(c.cell.taps, cell_taps(c, f));
+    arena.table(c.d_nonempty, std::vector<uint32_t>((nR + 127) / 128 * 4, 0u));
+    c.cell_bytes = (c.cell_rows ? 1 : (size_t)kReplicas1D * c.cell.cp.cells) * sizeof(float4);
     set_ping_params(c);
     c.cell.pitch = 1;
     c.cells_on = true;
@@ -408,7 +384,7 @@ bool configure_cells_1d(Context& c)
 // 2D: see cell_from_2d.
 bool takes_cells(const Context& c, uint64_t n)
 {
-    if(!c.cells_on) return false;
+    if(!c.cells_on || !c.d_cells) return false;
     if(c.dims == 1) return !c.cell_rows || n * (uint64_t)c.cell.rows <= std::min<uint64_t>(512ull * c.nR, 1ull << 20);
     return n == 0 || n >= c.cell_from;
 }
@@ -443,8 +419,8 @@ uint64_t cell_from_2d(const Context& c)
 // tables: row pairs where no travel reaches three rows, else knot cells where
 // the pulse's taps allow them, and the cell rows and the beam table have to
 // fit (everything else keeps the per-row gathers). Returns whether the form
-// is on; a failed allocation leaves it off.
-bool configure_cells(Context& c, double beam_support)
+// is on.
+bool configure_cells(Context& c, double beam_support, ConfigArena& arena)
 {
     free_cells(c);
     const int nR = (int)c.nR, nB = (int)c.nB, H = (int)c.H, W = (int)c.W;
@@ -565,65 +541,56 @@ bool configure_cells(Context& c, double beam_support)
         theta[p] = c.bearings[pos[p]];
         col_bearing[col[p]] = pos[p];
     }
-    const size_t cell_bytes = (size_t)cp.cells * pitch * sizeof(float4);
-    if(cell_bytes > kMaxCellBytes || cells_smem(c) > kMaxCellSmem ||
+    c.cell_bytes = (size_t)cp.cells * pitch * sizeof(float4);
+    if(c.cell_bytes > kMaxCellBytes || cells_smem(c) > kMaxCellSmem ||
        (!c.cell_pairs && filter_smem(H) > 200 * 1024)) return false;
-    Arena arena;
-    const size_t taps = arena.add(cell_taps(c, f)), dev = arena.add(f.dev), bits = arena.add(std::vector<uint32_t>((nR + 127) / 128 * 4, 0u)),
-                 at_theta = arena.add(theta), at_col = arena.add(col), at_bearing = arena.add(col_bearing);
-
-    // The lobe form's tables.
-    CellPing& L = c.lobe;
-    size_t l_table = 0, at_l_theta = 0, at_l_col = 0, l_smem = 0;
-    if(with_lobe && (c.lobe_bpl = find_windows(lobe.support)) != 0) {
-        const int n_lobe = lobe.last - lobe.first + 1, l_len = 32 * c.lobe_bpl;
-        l_smem = cells_smem(n_lobe, false, c.lobe_bpl, kTableCopies);
-        c.lobe_on = l_smem <= kMaxCellSmem;
-        L.windows = (int)span_of.size();
-        std::vector<float> table(n_lobe + 2, 0.0f);
-        for(int i = 0; i < n_lobe; i++) table[i + 1] = c.beam[lobe.first + i] - lobe.level;
-        // (behind the lobe's windows: the whole beam's, in the bearings' order)
-        const size_t whole = (size_t)L.windows * l_len;
-        std::vector<int> l_col(whole + pos.size(), -1);
-        std::vector<float> l_theta(whole + pos.size(), c.bearings[sorted_b[nB - 1]]);
-        for(int q = 0; q < nB; q++) {
-            l_col[whole + q] = sorted_b[q];
-            l_theta[whole + q] = c.bearings[sorted_b[q]];
-        }
-        for(size_t w = 0; w < span_of.size(); w++)
-            for(int q = span_of[w].x; q < span_of[w].y; q++) {
-                l_col[w * l_len + (q - span_of[w].x)] = sorted_b[q];
-                l_theta[w * l_len + (q - span_of[w].x)] = c.bearings[sorted_b[q]];
-            }
-        l_table = arena.add(table); at_l_theta = arena.add(l_theta); at_l_col = arena.add(l_col);
+    if(raise_smem_limit((const void*)cells_fn(c), cells_smem(c)) != cudaSuccess ||
+       (!c.cell_pairs && raise_smem_limit((const void*)k_cells_filter<false>, filter_smem(H)) != cudaSuccess) ||
+       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.cell_ctas, cells_fn(c), 32 * cell_warps(bpl, copies),
+                                                     cells_smem(c)) != cudaSuccess || c.cell_ctas < 1) {
+        cudaGetLastError();
+        return false;
     }
-
-    bool ok = arena.upload(c, cell_bytes) &&
-              raise_smem_limit((const void*)cells_fn(c), cells_smem(c)) == cudaSuccess &&
-              (c.cell_pairs || raise_smem_limit((const void*)k_cells_filter<false>, filter_smem(H)) == cudaSuccess) &&
-              cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.cell_ctas, cells_fn(c), 32 * cell_warps(bpl, copies),
-                                                            cells_smem(c)) == cudaSuccess && c.cell_ctas > 0;
-    if(!ok) { cudaGetLastError(); free_cells(c); return false; }
-    c.cell.taps = Arena::at<float4>(c, taps);
-    c.cell.row_dev = Arena::at<float>(c, dev);
-    c.d_nonempty = Arena::at<uint32_t>(c, bits);
-    c.cell.pos_theta = Arena::at<float>(c, at_theta);
-    c.cell.pos_col = Arena::at<int>(c, at_col);
-    c.cell.col_bearing = Arena::at<int>(c, at_bearing);
+    arena.table(c.cell.taps, cell_taps(c, f));
+    arena.table(c.cell.row_dev, f.dev);
+    arena.table(c.d_nonempty, std::vector<uint32_t>((nR + 127) / 128 * 4, 0u));
+    arena.table(c.cell.pos_theta, theta);
+    arena.table(c.cell.pos_col, col);
+    arena.table(c.cell.col_bearing, col_bearing);
     set_ping_params(c);
     c.cells_on = true;
     c.cell_from = cell_from_2d(c);
-    if(!c.lobe_on) return true;
-    c.lobe_on = raise_smem_limit((const void*)lobe_fn(c.lobe_bpl), l_smem) == cudaSuccess &&
-                raise_smem_limit((const void*)k_cells_filter<true>, filter_smem(H)) == cudaSuccess;
-    const int windows = L.windows;
+
+    // The lobe form's tables.
+    if(!with_lobe || (c.lobe_bpl = find_windows(lobe.support)) == 0) return true;
+    const int n_lobe = lobe.last - lobe.first + 1, l_len = 32 * c.lobe_bpl, windows = (int)span_of.size();
+    const size_t l_smem = cells_smem(n_lobe, false, c.lobe_bpl, kTableCopies);
+    if(l_smem > kMaxCellSmem || raise_smem_limit((const void*)lobe_fn(c.lobe_bpl), l_smem) != cudaSuccess ||
+       raise_smem_limit((const void*)k_cells_filter<true>, filter_smem(H)) != cudaSuccess) return true;
+    c.lobe_on = true;
+    std::vector<float> table(n_lobe + 2, 0.0f);
+    for(int i = 0; i < n_lobe; i++) table[i + 1] = c.beam[lobe.first + i] - lobe.level;
+    // (behind the lobe's windows: the whole beam's, in the bearings' order)
+    const size_t whole = (size_t)windows * l_len;
+    std::vector<int> l_col(whole + pos.size(), -1);
+    std::vector<float> l_theta(whole + pos.size(), c.bearings[sorted_b[nB - 1]]);
+    for(int q = 0; q < nB; q++) {
+        l_col[whole + q] = sorted_b[q];
+        l_theta[whole + q] = c.bearings[sorted_b[q]];
+    }
+    for(int w = 0; w < windows; w++)
+        for(int q = span_of[w].x; q < span_of[w].y; q++) {
+            l_col[w * l_len + (q - span_of[w].x)] = sorted_b[q];
+            l_theta[w * l_len + (q - span_of[w].x)] = c.bearings[sorted_b[q]];
+        }
+    CellPing& L = c.lobe;
     L = c.cell;
     L.windows = windows;
-    L.beam = Arena::at<float>(c, l_table);
-    L.pos_theta = Arena::at<float>(c, at_l_theta);
-    L.pos_col = Arena::at<int>(c, at_l_col);
+    arena.table(L.beam, table);
+    arena.table(L.pos_theta, l_theta);
+    arena.table(L.pos_col, l_col);
     L.beam_axis.c = (float)(c.red.beam_axis.c - lobe.first);
-    L.beam_axis.n = lobe.last - lobe.first + 1;
+    L.beam_axis.n = n_lobe;
     L.floor = lobe.level;
     L.floor_col = nB;
     BinParams& lb = c.lobe_bin;
@@ -641,6 +608,7 @@ bool configure_cells(Context& c, double beam_support)
 static rtacx_status run_cells_1d(Context& c, const void* samples, uint64_t n, float2* out, cudaStream_t stream)
 {
     CellPing P = c.cell;
+    P.cells = c.d_cells;
     P.out = out;
     P.replicas = cell_replicas(c, n);
     const uint64_t cells = c.cell_rows ? 0 : (uint64_t)P.cp.cells * P.replicas;
@@ -673,6 +641,7 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
 {
     if(c.dims == 1) return run_cells_1d(c, samples, n, out, stream);
     CellPing P = c.cell;
+    P.cells = c.d_cells;
     P.sorted = c.d_sorted;
     P.out = out;
     const bool lobe = c.lobe_on && n * (uint64_t)c.nB >= kLobeFrom;
@@ -708,7 +677,7 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
         CellPing whole = P;
         if(lobe) {
             CellPing L = c.lobe;
-            L.sorted = P.sorted; L.out = out; L.pulse = P.pulse; L.ranges = P.ranges;
+            L.cells = P.cells; L.sorted = P.sorted; L.out = out;
             // The samples left are few and mostly next to knots (row by row):
             // one per warp, all windows side by side.
             gy = (uint32_t)P.windows;

@@ -2,7 +2,9 @@
 #pragma once
 
 #include <cstdint>
+#include <cstring>
 #include <string>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -518,6 +520,51 @@ struct GemmPlan {
     std::vector<uint16_t> lists;        // [column tiles][1 + blocks of K]: count, then the blocks where B is not zero
 };
 
+// A sensor's device tables and the scratch that goes by its bins: laid out on
+// the host, then one allocation, one copy (each of its own costs a
+// configuration 2 to 6 us). commit sets the pointers.
+class ConfigArena {
+public:
+    template <typename T>
+    void table(T*& dst, const T* src, size_t count)
+    {
+        const size_t at = (host.size() + 255) / 256 * 256;
+        host.resize(at + count * sizeof(T));
+        std::memcpy(host.data() + at, src, count * sizeof(T));
+        slots.push_back({pointer(dst), at, true});
+    }
+    template <typename T>
+    void table(T*& dst, const std::vector<std::remove_const_t<T>>& v) { table<T>(dst, v.data(), v.size()); }
+    // Not initialised.
+    template <typename T>
+    void scratch(T*& dst, size_t count)
+    {
+        slots.push_back({pointer(dst), behind, false});
+        behind += (count * sizeof(T) + 255) / 256 * 256;
+    }
+    // cudaSuccess, or the error of the allocation or copy (consumed). The copy
+    // has arrived when it returns (one from pageable memory alone may not
+    // have, for streams that do not wait for the default stream).
+    cudaError_t commit(unsigned char*& base)
+    {
+        const size_t tables = (host.size() + 255) / 256 * 256;
+        cudaError_t e = cudaMalloc(&base, tables + behind + 256);
+        if(e == cudaSuccess) e = cudaMemcpy(base, host.data(), host.size(), cudaMemcpyHostToDevice);
+        if(e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+        if(e != cudaSuccess) { cudaGetLastError(); return e; }
+        for(const Slot& s : slots) *s.dst = base + (s.table ? 0 : tables) + s.at;
+        return cudaSuccess;
+    }
+
+private:
+    struct Slot { void** dst; size_t at; bool table; };
+    std::vector<unsigned char> host;
+    std::vector<Slot> slots;
+    size_t behind = 0;
+    template <typename T>
+    static void** pointer(T*& dst) { return reinterpret_cast<void**>(const_cast<std::remove_const_t<T>**>(&dst)); }
+};
+
 // Scratch and configuration owned by one context.
 struct Context {
     int device = 0;
@@ -531,7 +578,8 @@ struct Context {
     // Host copies of the configuration.
     float rmin = 0, rmax = 0, margin = 0, c = 0, duration = 0, span = 0;
     uint32_t nR = 0, nB = 0, H = 0, W = 0;
-    std::vector<float> pulse, beam, bearings;
+    std::vector<float> pulse, beam, bearings, ranges;
+    std::vector<int2> support;          // range bins that can hold a row's PSF support
     KeyParams key{};
     int overlap = 0;
     BinParams bin{};
@@ -539,7 +587,8 @@ struct Context {
     uint32_t bearing_tile = 0;          // bearings per gather tile
     uint32_t range_tile = 0;            // rows per gather tile
 
-    // Device tables (configuration-sized).
+    // Device tables and bin scratch (configuration-sized; all in d_config).
+    unsigned char* d_config = nullptr;
     float2* d_pulse = nullptr;          // pulse padded with a zero tap on each side
     float* d_beam = nullptr;            // beam padded with a zero tap on each side
     float* d_bearings = nullptr;        // [nB]
@@ -565,8 +614,7 @@ struct Context {
     SortShape sort;
     size_t acc_smem = 0;                // dynamic shared memory of the precision accumulation
     uint32_t acc_blocks_per_sm = 1;
-    size_t hist_cols = 0;               // allocated words of d_hist (the write cursors)
-    uint32_t* d_hist = nullptr;         // the scatter's per-bin write cursors (cursor_word), nBins x kCursorStride words
+    uint32_t* d_hist = nullptr;         // the scatter's per-bin write cursors (cursor_word)
 
     // Cell form of a 2D ping (rtacx_cells.cu).
     bool cells_on = false;
@@ -578,13 +626,13 @@ struct Context {
     bool cell_pairs = false;            // row pairs instead of knot cells
     bool cell_rows = false;             // 1D without knot cells: row by row
     CellPing cell{};                    // sorted and out are set per call
-    unsigned char* d_cell_arena = nullptr;   // the cell form's tables and cell rows, one allocation
+    size_t cell_bytes = 0;              // ... and the cell rows, allocated with the sample-sized scratch
     float4* d_cells = nullptr;
     uint32_t* d_nonempty = nullptr;     // [(nR + 31) / 32] bitmap of non-empty range bins
     BinParams cell_bin{};               // the cell form's order
     SortShape cell_sort;
     bool lobe_on = false;               // the sensor also has the lobe form
-    int lobe_bpl = 2, lobe_ctas = 1;
+    int lobe_bpl = 2;
     CellPing lobe{};
     BinParams lobe_bin{};
     SortShape lobe_sort;
@@ -697,8 +745,10 @@ rtacx_status run_windows(Context& ctx, cudaStream_t stream);
 rtacx_status run_reduce(Context& ctx, float* out, cudaStream_t stream);
 
 // Cell form of the plain reduction (rtacx_cells.cu).
-bool configure_cells(Context& ctx, double beam_support);
-bool configure_cells_1d(Context& ctx);
+bool configure_cells(Context& ctx, double beam_support, ConfigArena& arena);
+bool configure_cells_1d(Context& ctx, ConfigArena& arena);
+void bind_cells(Context& ctx);                           // once the arena is committed
+void ensure_cells(Context& ctx);                         // the cell rows; without memory for them the gathers
 bool takes_cells(const Context& ctx, uint64_t n);
 int cell_replicas(const Context& ctx, uint64_t n);       // 1D: copies of the cell rows that a ping uses
 void free_cells(Context& ctx);

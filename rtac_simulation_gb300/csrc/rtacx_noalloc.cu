@@ -249,8 +249,7 @@ extern "C" rtacx_status rtacx_reduce_noalloc(int sample_kind, const void* sensor
     ctx.d_bb_tiles = reinterpret_cast<int2*>(base + kOffTiles);
     ctx.sort = sort_shape(ctx, ctx.bin.nBins, false);
     ctx.sort.hist_ctas = std::min(ctx.sort.hist_ctas, kMaxHistCtas);
-    ctx.hist_cols = (size_t)ctx.bin.nBins * kCursorStride;
-    if(ctx.hist_cols * sizeof(uint32_t) > kHistBytes) return RTACX_ERR_UNSUPPORTED;
+    if((size_t)ctx.bin.nBins * kCursorStride * sizeof(uint32_t) > kHistBytes) return RTACX_ERR_UNSUPPORTED;
 
     // Upload this call's tables (pageable copies: the staging above may be
     // reused as soon as these return) and clear the error word.

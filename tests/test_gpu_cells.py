@@ -256,6 +256,30 @@ def test_small_pings_of_large_sensors_gather_per_row(oracle, nB, nR, wide, pairs
         assert rel_l2(got, oracle.reduce(wk.samples[:n], wk.sensor)) <= TOL, n
 
 
+def test_cell_rows_come_with_the_scratch_of_samples(oracle):
+    """A configured sensor holds no cell rows (135 MB here) until a ping or
+    rtacx_reserve sizes the scratch; a sensor configured on a context that has
+    scratch can be captured at once."""
+    wk = ping(60000, 8192, 1024, 9, False)
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    ctx = make_context(wk)
+    assert free0 - torch.cuda.mem_get_info()[0] < 64 << 20
+    ctx.reserve(wk.n)
+    assert free0 - torch.cuda.mem_get_info()[0] > 120 << 20
+    small = ping(60000, 300, 64, 9, False)
+    ctx.configure_2d(**small.sensor)
+    d = torch.from_numpy(small.samples).cuda()
+    out = torch.zeros(small.out_shape + (2,), device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ctx.reduce(d, small.n, out, stream=torch.cuda.current_stream())
+    graph.replay()
+    torch.cuda.synchronize()
+    got = out.cpu().numpy()[..., 0] + 1j * out.cpu().numpy()[..., 1]
+    assert rel_l2(got, oracle.reduce(small.samples, small.sensor)) <= TOL
+
+
 @pytest.mark.parametrize("large", [0, 150000])
 def test_batches_of_small_pings(oracle, large):
     """Small pings of every form alone, which the per-row gathers take, and
