@@ -427,13 +427,16 @@ rtacx_status rtacx_diag_drop_accumulation_stage(rtacx_ctx* ctx, uint32_t stage);
 
 /* Diagnostic (no counterpart in the reference): copies the first
  * min(max_records, capacity) records of the context's sorted scratch, as
- * left by the last rtacx_bin / rtacx_reduce queued on `stream`, into
+ * left by the last rtacx_bin / rtacx_reduce queued on `stream` (a batch's run
+ * or a replayed graph's included), into
  * `records` (device or pinned host memory, 16 bytes per record): float4
  * {re, im, travel, bearing} (bearing 0 for 1D sensors; the value after the
  * echo model when one is set). The first n - (out-of-range count) records
  * are the binned samples, each once, grouped by composite key (range bin x
  * bearing sub-bins + bearing sub-bin) in ascending order, in any order
- * inside a group. */
+ * inside a group. A sensor with the range-cell form sorts in another order:
+ * there the call first sorts the whole scratch again, with a stream-ordered
+ * allocation (cudaMallocAsync) as large as the scratch. */
 rtacx_status rtacx_diag_sorted(rtacx_ctx* ctx, float* records, uint64_t max_records, void* stream);
 int rtacx_stage_times(rtacx_ctx* ctx, float* ms, int max);
 

@@ -205,7 +205,8 @@ rtacx_status commit_config(Context& c, ConfigArena& arena)
     arena.scratch(c.d_totals, bins + bins / 1024 + 1);   // + block sums
     arena.scratch(c.d_win, c.nR);
     arena.scratch(c.d_hist, cursor_word(bins + 1));
-    const cudaError_t e = arena.commit(c.d_config);
+    cudaError_t e = cudaMemset(c.d_oor + 2, 0, sizeof(unsigned long long));      // (kRangeOrder: another sensor's bins)
+    if(e == cudaSuccess) e = arena.commit(c.d_config);
     if(e == cudaSuccess) {
         if(c.cells_on) bind_cells(c);
         if(c.capacity) ensure_cells(c);       // (otherwise with the first samples' scratch)
@@ -251,8 +252,8 @@ rtacx_status rtacx_create(rtacx_ctx** out, int device)
        cudaDeviceGetAttribute(&c.sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
        cudaMalloc(&c.d_err, sizeof(uint32_t)) != cudaSuccess ||
        cudaMemset(c.d_err, 0, sizeof(uint32_t)) != cudaSuccess ||
-       cudaMalloc(&c.d_oor, 2 * sizeof(unsigned long long)) != cudaSuccess ||
-       cudaMemset(c.d_oor, 0, 2 * sizeof(unsigned long long)) != cudaSuccess) {
+       cudaMalloc(&c.d_oor, 3 * sizeof(unsigned long long)) != cudaSuccess ||
+       cudaMemset(c.d_oor, 0, 3 * sizeof(unsigned long long)) != cudaSuccess) {
         cudaGetLastError();
         rtacx_destroy(ctx);
         return RTACX_ERR_CUDA;

@@ -211,6 +211,7 @@ struct Batch {
             d.pulse = c.d_pulse; d.beam = c.d_beam; d.out = reinterpret_cast<float2*>(pings[i].out);
             if(c.dims == 2) d.bb_tiles = (TB == 64) ? c.d_bb_tiles64 : c.d_bb_tiles128;   // ranges for width TB
             if(cell_form) {
+                d.order = c.dims == 1 ? kInputOrder | n : kBinsOrder | d.bin.nBins;
                 d.cell = c.cell;
                 d.cell.cells = c.d_cells;
                 d.cell.sorted = c.d_sorted;
@@ -500,13 +501,6 @@ rtacx_status rtacx_batch_run(rtacx_batch* b, void* stream)
         cudaGetLastError();
         B.error = "cudaGraphLaunch failed";
         return RTACX_ERR_CUDA;
-    }
-    // The order that the batch leaves in the pings' sorted scratch.
-    for(const rtacx_ping_desc& p : B.pings) {
-        Context& c = p.ctx->impl;
-        c.sorted_cells_n = B.cells && takes_cells(c, p.n) ? p.n : 0;
-        c.sorted_input_order = c.dims == 1;
-        c.sorted_bins = c.cell_bin.nBins;
     }
     return RTACX_OK;
 }

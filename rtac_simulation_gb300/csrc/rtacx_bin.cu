@@ -323,10 +323,15 @@ __global__ void k_oor_out(const unsigned long long* __restrict__ src, uint64_t* 
     if(threadIdx.x < 2) dst[threadIdx.x] = src[threadIdx.x];
 }
 
-// Puts records [*count, n) of the sorted scratch out of every sensor's range.
-__global__ void k_mark_tail(float4* __restrict__ sorted, const uint32_t* __restrict__ count, uint64_t n)
+// Puts the records of the sorted scratch [0, n) behind those that the last
+// ping left there out of every sensor's range.
+__global__ void k_mark_tail(float4* __restrict__ sorted, const unsigned long long* __restrict__ order,
+                            const uint32_t* __restrict__ offsets, uint32_t nBins, uint64_t n)
 {
-    for(uint64_t i = *count + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    const uint32_t of = (uint32_t)*order;
+    const unsigned long long kind = *order - of;
+    const uint32_t count = kind == kInputOrder ? of : offsets[kind == kBinsOrder ? of : nBins];
+    for(uint64_t i = count + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
         sorted[i] = make_float4(0.f, 0.f, INFINITY, 0.f);
 }
 
@@ -375,7 +380,7 @@ __global__ void k_windows_batch(const PingDev* __restrict__ pings, const uint2* 
 __global__ void k_reset_batch(const PingDev* __restrict__ pings, uint32_t n_pings)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if(i < n_pings) { pings[i].oor[0] = 0ull; pings[i].oor[1] = 0ull; }
+    if(i < n_pings) { pings[i].oor[0] = 0ull; pings[i].oor[1] = 0ull; pings[i].oor[2] = pings[i].order; }
 }
 
 uint32_t hist_grid(uint32_t ctas, uint64_t n)
@@ -415,7 +420,6 @@ bool ensure_capacity(Context& ctx, uint64_t n)
     ctx.capacity = cap;
     ctx.d_ranks = ranked ? reinterpret_cast<uint32_t*>(p + cap) : nullptr;
     ctx.n_ranks = ranked ? ranks : 0;
-    ctx.sorted_cells_n = 0;
     return true;
 }
 
@@ -601,8 +605,7 @@ constexpr int kNumScatterShapes = sizeof(kScatterShapes) / sizeof(kScatterShapes
 rtacx_status run_binning(Context& ctx, const void* samples, uint64_t n, cudaStream_t stream)
 {
     const BinParams& p = ctx.bin;
-    ctx.sorted_cells_n = 0;
-    RTACX_CUDA(cudaMemsetAsync(ctx.d_oor, 0, 2 * sizeof(unsigned long long), stream));
+    RTACX_CUDA(cudaMemsetAsync(ctx.d_oor, 0, 3 * sizeof(unsigned long long), stream));   // (and kRangeOrder)
     if(n == 0) {
         RTACX_CUDA(cudaMemsetAsync(ctx.d_offsets, 0, (p.nBins + 1) * sizeof(uint32_t), stream));
         return RTACX_OK;
@@ -661,19 +664,18 @@ rtacx_status run_sort(Context& ctx, const BinParams& p, const SortShape& shape, 
 
 // Brings a sorted scratch that the cell form left in its own order (window x
 // cell block of the in-range records, or, 1D, the input order of all) into
-// the order that rtacx_bin documents: the tail beyond the in-range count is
-// marked out of range, then the reference order's passes run from the scratch itself into
-// a stream-ordered buffer that is copied back.
+// the order that rtacx_bin documents: what lies behind the last ping's records
+// is marked out of range, then the reference order's passes run from the whole
+// scratch itself into a stream-ordered buffer that is copied back. Which order
+// it is in only the device knows; one in that order comes out the same.
 rtacx_status restore_sorted(Context& ctx, cudaStream_t stream)
 {
-    const uint64_t n = ctx.sorted_cells_n;
-    if(!n) return RTACX_OK;
+    const uint64_t n = ctx.capacity;
+    if(!n || !ctx.cells_on || !ctx.d_cells) return RTACX_OK;
     float4* sorted = ctx.d_sorted;
-    if(!ctx.sorted_input_order) {
-        k_mark_tail<<<(uint32_t)std::min<uint64_t>((n + 255) / 256, (uint64_t)ctx.sm_count * 16), 256, 0, stream>>>(
-            sorted, ctx.d_offsets + ctx.sorted_bins, n);
-        RTACX_CUDA(cudaGetLastError());
-    }
+    k_mark_tail<<<(uint32_t)std::min<uint64_t>((n + 255) / 256, (uint64_t)ctx.sm_count * 16), 256, 0, stream>>>(
+        sorted, ctx.d_oor + 2, ctx.d_offsets, ctx.bin.nBins, n);
+    RTACX_CUDA(cudaGetLastError());
     void* tmp = nullptr;
     RTACX_CUDA(cudaMallocAsync(&tmp, n * sizeof(float4), stream));
     const BinParams kept = ctx.bin;

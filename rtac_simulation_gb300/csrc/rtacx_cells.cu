@@ -90,14 +90,17 @@ CellsFn cells_fn(const Context& c) { return cells_fn(c.cell_bpl, c.cell_shared, 
 size_t cells_smem(const Context& c) { return cells_smem((int)c.W, c.cell_pairs, c.cell_bpl, c.cell_copies); }
 
 // Zeroes what a ping's passes add into: the bin totals, the range-bin bitmap,
-// the cell rows and the ping (8-byte stores: the ping's alignment).
-__global__ void k_cells_clear(uint32_t* __restrict__ totals, uint32_t n_totals, uint32_t* __restrict__ bits,
+// the cell rows and the ping (8-byte stores: the ping's alignment). Notes the
+// order that the ping leaves in the sorted scratch.
+__global__ void k_cells_clear(unsigned long long* __restrict__ sorted_order, unsigned long long order,
+                              uint32_t* __restrict__ totals, uint32_t n_totals, uint32_t* __restrict__ bits,
                               uint32_t n_bits, float4* __restrict__ cells, uint64_t n_cells, float2* __restrict__ out,
                               uint64_t n_out)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     chain_next();
     chain_wait();
+    if(i0 == 0) *sorted_order = order;
     for(uint64_t i = i0; i < n_totals; i += stride) totals[i] = 0u;
     for(uint64_t i = i0; i < n_bits; i += stride) bits[i] = 0u;
     for(uint64_t i = i0; i < n_cells; i += stride) cells[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -179,7 +182,6 @@ void free_cells(Context& c)
     c.d_nonempty = nullptr;
     c.lobe_on = false;
     c.cells_on = false;
-    c.sorted_cells_n = 0;
 }
 
 void ensure_cells(Context& c)
@@ -614,11 +616,9 @@ static rtacx_status run_cells_1d(Context& c, const void* samples, uint64_t n, fl
     const uint64_t cells = c.cell_rows ? 0 : (uint64_t)P.cp.cells * P.replicas;
     c.mark(1, false, stream);
     cudaError_t e = launch_chained(k_cells_clear, (uint32_t)std::min<uint64_t>((cells + c.nR + 255) / 256, (uint64_t)c.sm_count * 8),
-                                   256, 0, stream, c.d_totals, 0u, c.d_nonempty, (c.nR + 31) / 32, c.d_cells, cells, out,
+                                   256, 0, stream, c.d_oor + 2, kInputOrder | n, c.d_totals, 0u, c.d_nonempty, (c.nR + 31) / 32, c.d_cells, cells, out,
                                    (uint64_t)c.nR);
     c.mark(1, true, stream);
-    c.sorted_cells_n = n;
-    c.sorted_input_order = true;
     if(e == cudaSuccess && n) {
         c.mark(5, false, stream);
         // One record per thread while that fills the SMs, more beyond.
@@ -653,16 +653,13 @@ rtacx_status run_cells(Context& c, const void* samples, uint64_t n, float2* out,
     const uint64_t cells = (uint64_t)P.cp.cells * P.pitch, cells_out = c.cell_pairs && n ? 0 : (uint64_t)c.nR * c.nB;   // (the pairs' join writes every cell)
     c.mark(1, false, stream);
     cudaError_t e = launch_chained(k_cells_clear, (uint32_t)std::min<uint64_t>((cells + 255) / 256, (uint64_t)c.sm_count * 8),
-                                   256, 0, stream, c.d_totals, totals, c.d_nonempty, (c.nR + 31) / 32, c.d_cells, cells,
+                                   256, 0, stream, c.d_oor + 2, n ? kBinsOrder | bin.nBins : +kInputOrder,
+                                   c.d_totals, totals, c.d_nonempty, (c.nR + 31) / 32, c.d_cells, cells,
                                    out, cells_out);
     c.mark(1, true, stream);
-    c.sorted_cells_n = 0;
     if(e == cudaSuccess && n) {
         const rtacx_status st = run_sort(c, bin, lobe ? c.lobe_sort : c.cell_sort, samples, n, c.d_nonempty, stream);
         if(st != RTACX_OK) return st;
-        c.sorted_cells_n = n;
-        c.sorted_bins = bin.nBins;
-        c.sorted_input_order = false;
         c.mark(5, false, stream);
         // As many CTAs as are resident (twice that for wide beams, whose units
         // are long: the SMs' shares even out, 2^22 samples 1240 -> 1222 us);

@@ -438,6 +438,12 @@ struct SortShape {
     int scatter_shape = 0;              // 1 + index of the staged scatter's shape (0: per-tile scatter)
 };
 
+// Order in which a ping leaves the sorted scratch, kept on the device (d_oor[2])
+// by the pings themselves, so that it is right for replayed graphs too: 0 the
+// order of rtacx_bin, the in-range records by the bins of another order
+// (offsets[bins] of them), or n records in input order.
+enum SortedOrder : unsigned long long { kRangeOrder = 0, kBinsOrder = 1ull << 32, kInputOrder = 2ull << 32 };
+
 // How a ping of a batch is reduced: sorted by range and gathered per row
 // (kPerRow), or in the cell form (rtacx_cells.cuh).
 enum PingForm : int { kPerRow = 0, kCells2D, kPairs2D, kCells1D, kRows1D };
@@ -460,6 +466,7 @@ struct PingDev {
     uint32_t* totals;
     uint32_t* offsets;
     unsigned long long* oor;
+    unsigned long long order;        // SortedOrder that it leaves in `sorted`
     uint32_t* err;
     float4* sorted;
     uint32_t* ranks;                 // cell form, 2D: each sample's rank in its bin (null: cursors)
@@ -603,7 +610,7 @@ struct Context {
     uint32_t* d_offsets = nullptr;      // [nBins + 1] exclusive scan of bin counts
     uint32_t* d_totals = nullptr;       // [nBins]
     int2* d_win = nullptr;              // [nR] effective bin range per row (lo > hi: empty)
-    unsigned long long* d_oor = nullptr;// [2] low / high out-of-range counts
+    unsigned long long* d_oor = nullptr;// [3] low / high out-of-range counts, the sorted scratch's order
     uint32_t* d_err = nullptr;          // device error word
 
     // Sample-sized scratch.
@@ -636,9 +643,6 @@ struct Context {
     CellPing lobe{};
     BinParams lobe_bin{};
     SortShape lobe_sort;
-    uint32_t sorted_bins = 0;           // bins of the order that the last ping left in d_sorted
-    uint64_t sorted_cells_n = 0;        // samples of the last ping that left another order in d_sorted (0: none)
-    bool sorted_input_order = false;    // ... all of them in input order (1D) instead of the in-range ones in cell order
 
     // Split persistent gather of 2D pings (see rtacx_reduce.cu).
     uint32_t* d_tile_parts = nullptr;   // [tiles] sample-stream length of each output tile

@@ -1010,6 +1010,7 @@ __device__ __noinline__ void batch_chunk_1d(const PingDev& D, const CellPing& P,
 {
     uint32_t* s_bits = reinterpret_cast<uint32_t*>(smem_raw);
     const uint32_t words = (P.nR + 31) / 32;
+    if(chunk == 0 && threadIdx.x == 0) D.oor[2] = D.order;
     for(uint32_t i = threadIdx.x; i < words; i += kThreads) s_bits[i] = 0u;
     __syncthreads();
     const uint64_t per = (D.n + D.chunks - 1) / D.chunks, begin = chunk * per, end = min(begin + per, D.n);
@@ -1085,7 +1086,7 @@ __device__ __forceinline__ void batch_fused(const FusedBatch& fb, unsigned char*
         const uint32_t b = m.y * kThreads + threadIdx.x;
         if(b < P.bin.nBins) P.totals[b] = 0u;
         if(b < (P.bin.nBins + kScanBlock - 1) / kScanBlock) P.totals[P.bin.nBins + b] = 0u;
-        if(m.y == 0 && threadIdx.x < 2) P.oor[threadIdx.x] = 0ull;
+        if(m.y == 0 && threadIdx.x < 3) P.oor[threadIdx.x] = threadIdx.x < 2 ? 0ull : P.order;
     }
     if(CELLS)
         for(uint32_t k = blockIdx.x; k < fb.n_zero16; k += gridDim.x) {

@@ -205,6 +205,44 @@ def test_sorted_scratch_after_a_ping_keeps_its_order(oracle):
     assert rel_l2(gpu_reduce(ctx, wk.samples, wk.out_shape), first) <= 1e-6
 
 
+@pytest.mark.parametrize("dims", [1, 2])
+def test_sorted_scratch_after_replayed_pings(oracle, dims):
+    """A captured ping replayed between other calls on its context: the
+    diagnostic copy is in its order after each of them, also when the scratch
+    was put in order (or filled by rtacx_bin) since the capture."""
+    from test_gpu_sorted import KEY_OOR, composite_keys, record_hash
+    wk = ping(20001, 257, 200, 17, False) if dims == 2 else ping_1d(20001, 257, 17)
+    n = wk.n
+    ctx = make_context(wk)
+    ctx.reserve(n + 500)
+    dev = torch.from_numpy(wk.samples).cuda()
+    out = torch.zeros(wk.out_shape + (2,), device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ctx.reduce(dev, n, out, stream=torch.cuda.current_stream())
+
+    def check(samples, count):
+        buf = torch.zeros((n, 4), device="cuda")
+        ctx.diag_sorted(buf, n, stream=torch.cuda.current_stream())
+        recs = np.zeros((count, 4), np.float32)
+        recs[:, :samples.shape[1]] = samples[:count]
+        inside = recs[composite_keys(oracle, wk, recs) != KEY_OOR]
+        got = buf.cpu().numpy()[:len(inside)]
+        assert np.all(np.diff(composite_keys(oracle, wk, got).astype(np.int64)) >= 0)
+        assert np.array_equal(np.sort(record_hash(got)), np.sort(record_hash(inside)))
+
+    stream = torch.cuda.current_stream()
+    for scale in (1.0, 0.9, 0.8):
+        samples = wk.samples.copy()
+        samples[:, 2] *= np.float32(scale)
+        dev.copy_(torch.from_numpy(samples))
+        graph.replay()
+        check(samples, n)
+        check(samples, n)
+        ctx.bin(dev, n // 3, dims, stream=stream)
+        check(samples, n // 3)
+
+
 @pytest.mark.parametrize("margin", [1.0, 0.999, 3.0])
 @pytest.mark.parametrize("wide", [False, True])
 @pytest.mark.parametrize("n,nR,nB,H", [(1, 2, 1, 3), (33, 5, 33, 2), (1000, 64, 65, 17), (30000, 300, 129, 164)])
