@@ -35,7 +35,8 @@ constexpr double kPi = 3.14159265358979323846;
 // least-squares polynomial weighted towards equal relative error (2.6e-9 in
 // exact arithmetic, 0.94 ulp in float with q exact); then the octant.
 // Magnitudes whose reciprocal or product could leave the normal range, zeros,
-// infinities and NaN take the library function.
+// infinities and two NaN take the library function (one NaN next to a number
+// does not come from a direction and a finite rotation).
 __device__ __forceinline__ float atan2_fast(float y, float x)
 {
     const float ax = fabsf(x), ay = fabsf(y), mx = fmaxf(ax, ay), mn = fminf(ax, ay);

@@ -87,8 +87,9 @@ __device__ __forceinline__ void umma_16bit(uint32_t tmem_d, uint64_t adesc, uint
                  : "memory");
 }
 
-// Epilogue of one warp: its TMEM lane quadrant -> rows m0 + 32 warp + lane.
-template <int BN>
+// Epilogue of one warp: its TMEM lane quadrant -> rows m0 + 32 warp + lane. LO:
+// the sum of two accumulators, BN columns apart.
+template <int BN, bool LO>
 __device__ __forceinline__ void store_tile(uint32_t tmem, float* __restrict__ C, int m0, int n0, int ldc, int warp, int lane,
                                            const float* __restrict__ row_scale, const float* __restrict__ col_scale,
                                            bool any, bool add)
@@ -98,11 +99,17 @@ __device__ __forceinline__ void store_tile(uint32_t tmem, float* __restrict__ C,
     const float rs = row_scale ? row_scale[row] : 1.0f;
 #pragma unroll 1
     for(int c = 0; c < BN / 32; c++) {
-        uint32_t r[32];
-        tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c * 32), r);
+        uint32_t r[32], lo[32];
+        const uint32_t at = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c * 32);
+        if(LO) tmem_ld32_two(at, r, at + BN, lo);
+        else tmem_ld32(at, r);
         float v[32];
 #pragma unroll
-        for(int q = 0; q < 32; q++) v[q] = any ? __uint_as_float(r[q]) : 0.0f;
+        for(int q = 0; q < 32; q++) {
+            v[q] = __uint_as_float(r[q]);
+            if(LO) v[q] += __uint_as_float(lo[q]);
+            if(!any) v[q] = 0.0f;
+        }
         if(row_scale) {
 #pragma unroll
             for(int q = 0; q < 32; q++) v[q] *= rs;
@@ -195,7 +202,7 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
     const bool ok = mbar_wait(accum_bar, 0, abort_flag);
     __syncwarp();
     tc_fence_after();
-    if(__all_sync(0xffffffffu, ok ? 1 : 0)) store_tile<BN>(tmem, C, m0, n0, ldc, warp, lane, nullptr, nullptr, true, false);
+    if(__all_sync(0xffffffffu, ok ? 1 : 0)) store_tile<BN, false>(tmem, C, m0, n0, ldc, warp, lane, nullptr, nullptr, true, false);
     else if(lane == 0 && err) atomicOr(err, kErrGemmTimeout);
     tc_fence_before();
     __syncthreads();
@@ -207,7 +214,12 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
 
 // The split contraction. Stage: A hi, A lo, B hi, B lo of one block of 64
 // along K; the hi and the lo tiles have a barrier each, so that hi hi starts
-// before the lo tiles are in. blockIdx.z: its share of the column tile's list
+// before the lo tiles are in. The products with a lo half have an accumulator
+// of their own: the tensor cores truncate as they accumulate, so in one
+// accumulator the two products that add next to nothing to the sum cost it
+// digits too (2^24 samples, 512 x 4096: 1.1e-5 from 64 bits, 7.8e-6 with two, in
+// 224.4 and 224.6 us; the second tile of columns costs small contractions up to
+// 0.4 us). blockIdx.z: its share of the column tile's list
 // of blocks (blocks: [column tiles][1 + all blocks], the count first), into its
 // own partial product C + z rows ldc, or (add) added into C.
 template <int BN_, int STAGES_>
@@ -227,7 +239,7 @@ k_gemm_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
              const float* __restrict__ col_scale, int add, uint32_t* __restrict__ err)
 {
     constexpr int BN = T::BN, STAGES = T::STAGES;
-    constexpr uint32_t TMEM_COLS = BN;
+    constexpr uint32_t TMEM_COLS = 2 * BN;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     unsigned char* base = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
@@ -298,9 +310,9 @@ k_gemm_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
             if(!mbar_wait(lo_bar(s), parity, abort_flag)) break;
             tc_fence_after();
 #pragma unroll
-            for(int kk = 0; kk < BK / 16; kk++) umma_16bit<kF16, BN>(tmem, ahi + 2 * kk, blo + 2 * kk, 1u);
+            for(int kk = 0; kk < BK / 16; kk++) umma_16bit<kF16, BN>(tmem + BN, ahi + 2 * kk, blo + 2 * kk, (i > 0 || kk > 0) ? 1u : 0u);
 #pragma unroll
-            for(int kk = 0; kk < BK / 16; kk++) umma_16bit<kF16, BN>(tmem, alo + 2 * kk, bhi + 2 * kk, 1u);
+            for(int kk = 0; kk < BK / 16; kk++) umma_16bit<kF16, BN>(tmem + BN, alo + 2 * kk, bhi + 2 * kk, 1u);
             umma_commit(empty_bar(s));
         }
         umma_commit(accum_bar);   // arrives once every MMA issued above has completed
@@ -310,7 +322,7 @@ k_gemm_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     __syncwarp();
     tc_fence_after();
     if(__all_sync(0xffffffffu, ok ? 1 : 0))
-        store_tile<BN>(tmem, C, m0, n0, ldc, warp, lane, row_scale, col_scale, count > 0, add != 0);
+        store_tile<BN, true>(tmem, C, m0, n0, ldc, warp, lane, row_scale, col_scale, count > 0, add != 0);
     else if(lane == 0 && err) atomicOr(err, kErrGemmTimeout);
     tc_fence_before();
     __syncthreads();
@@ -409,6 +421,10 @@ size_t split_smem(int bn) { return bn == 256 ? SplitWide::SMEM_BYTES : SplitNarr
 
 } // namespace
 
+// Parts of K, at most (16384 grid bearings' real and imaginary parts are 15 of
+// kMaxTerms), and terms of a part's sum.
+constexpr int kMaxParts = 16, kMaxTerms = 2200;
+
 // Tile width, K split and block lists of the contraction of A [M][2 K] with
 // B [N][2 K] (b: its host copy), M % 128 == 0, N % 256 == 0, K % 64 == 0.
 //
@@ -438,14 +454,14 @@ rtacx_status plan_gemm_split(std::string& error, GemmPlan& g, const void* A, con
                 if(used[(size_t)t * (bn / 128) * nkb + kb] || (bn == 256 && used[((size_t)t * 2 + 1) * nkb + kb])) l[++l[0]] = (uint16_t)kb;
             longest = std::max<size_t>(longest, l[0]);
         }
-        for(int ks = 1; ks <= 8; ks *= 2) {
+        for(int ks = 1; ks <= kMaxParts; ks *= 2) {
             if(ks > 1 && longest < (size_t)2 * ks) continue;
-            // The tensor cores truncate as they accumulate: a sum of K terms in
-            // one accumulator comes out about 1.65e-9 K too small (2e-5 at K =
-            // 12000), a split one its parts' share. Long sums take two parts:
-            // one is that far off, and with more the ping moves further from
-            // the two-part one than its own error.
-            if(3 * longest * BK > 8000 && ks != 2) continue;
+            // A sum of K terms of one sign in one accumulator comes out about 6e-9
+            // K too small (measured with fp16 operands, up to 16384 grid bearings
+            // in 8 parts), a split one its parts' share. So no part takes more
+            // than kMaxTerms (1.32e-5), and the time decides among the splits
+            // that keep to that.
+            if(longest * BK > (size_t)kMaxTerms * ks && ks < kMaxParts) continue;
             const double ctas = (double)(N / bn) * (M / BM) * ks, waves = std::ceil(ctas / sm_count);
             const double t = waves * ((double)longest / ks * (bn == 256 ? 1.0 : 0.6) + 4.0) + (double)ks * M * N * 4.0 / 4e6;
             if(t < best) { best = t; g.bn = bn; g.ksplit = ks; g.lists = lists; }
