@@ -221,8 +221,8 @@ struct Batch {
                 d.bpl = c.cell_bpl;
                 d.shared = c.cell_shared ? 1 : 0;
                 zero(zero16, c.d_nonempty, (c.nR + 127) / 128, 16);
-                if(d.form != kRows1D) zero(zero16, c.d_cells, (uint64_t)c.cell.cp.cells * c.cell.pitch * d.cell.replicas, 16);
-                if(d.form != kPairs2D) zero(zero8, d.out, (uint64_t)c.nR * c.nB, 8);
+                zero(zero16, c.d_cells, c.dims == 1 ? cell_words_1d(c, n) : (uint64_t)c.cell.cp.cells * c.cell.pitch, 16);
+                if(d.form != kPairs2D && d.form != kRows1D) zero(zero8, d.out, (uint64_t)c.nR * c.nB, 8);
                 uint32_t columns;
                 const uint32_t rows = batch_filter_tiles(c, columns);
                 for(uint32_t y = 0; y < rows; y++)

@@ -4,7 +4,7 @@
 //   k_cells         the sorted samples of one ping into the cell rows;
 //   k_cells_filter  the pulse's taps over the cell rows, rows without a
 //                   reference window zeroed (k_pairs_join: row pairs);
-//   k_cells_1d, k_cells_filter_1d, k_rows_off_1d  the same for 1D sensors,
+//   k_cells_1d, k_cells_filter_1d, k_rows_join_1d  the same for 1D sensors,
 //                   from the input order.
 // Measured against the per-row gathers on the same pings (whole rtacx_reduce,
 // us): 2^20 samples, 512 x 1024, 33 taps, narrow beams: 1380 -> 96; 2^22 samples,
@@ -145,8 +145,7 @@ k_cells_1d(const CellPing P, const BinParams p, const float* __restrict__ sample
     __syncthreads();
     chain_wait();
     const uint64_t chunk = (n + gridDim.x - 1) / gridDim.x, begin = blockIdx.x * chunk;
-    accumulate_1d<ROWS>(P, p, after_chain(samples), begin, min(begin + chunk, n), P.cells + (size_t)(blockIdx.x % P.replicas) * P.cp.cells,
-                        s_bits, copy);
+    accumulate_1d<ROWS>(P, p, after_chain(samples), begin, min(begin + chunk, n), copy_1d(P, ROWS, blockIdx.x), s_bits, copy);
     __syncthreads();
     for(uint32_t i = threadIdx.x; i < words; i += kThreads1D)
         if(s_bits[i]) atomicOr(&nonempty[i], s_bits[i]);
@@ -164,13 +163,14 @@ k_cells_filter_1d(const CellPing ping, const uint32_t* nonempty)
     filter_rows_1d<kFilterRows1D>(P, blockIdx.x, reinterpret_cast<float4*>(s_raw), after_chain(nonempty));
 }
 
-// Rows of a 1D ping without a reference window.
-__global__ void k_rows_off_1d(const CellPing P, const uint32_t* nonempty)
+__global__ void k_rows_join_1d(const CellPing ping, const uint32_t* nonempty)
 {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    CellPing P = ping;
     chain_next();
     chain_wait();
-    if(r < (int)P.nR && !row_on(after_chain(nonempty), (int)P.nR, P.overlap, r)) P.out[r] = make_float2(0.f, 0.f);
+    P.cells = after_chain(P.cells);
+    if(r < (int)P.nR) join_rows_1d(P, r, after_chain(nonempty));
 }
 
 } // namespace
@@ -371,7 +371,7 @@ bool configure_cells_1d(Context& c, ConfigArena& arena)
     arena.table(c.cell.row_dev, f.dev);
     arena.table(c.cell.taps, cell_taps(c, f));
     arena.table(c.d_nonempty, std::vector<uint32_t>((nR + 127) / 128 * 4, 0u));
-    c.cell_bytes = (c.cell_rows ? 1 : (size_t)kReplicas1D * c.cell.cp.cells) * sizeof(float4);
+    c.cell_bytes = (size_t)kReplicas1D * (c.cell_rows ? nR * sizeof(float2) : c.cell.cp.cells * sizeof(float4));
     set_ping_params(c);
     c.cell.pitch = 1;
     c.cells_on = true;
@@ -391,7 +391,21 @@ bool takes_cells(const Context& c, uint64_t n)
     return n == 0 || n >= c.cell_from;
 }
 
-int cell_replicas(const Context& c, uint64_t n) { return !c.cell_rows && n >= kReplicateFrom1D ? kReplicas1D : 1; }
+// More than one copy where a row takes more than 8 reductions, or a cell 48 (4
+// copies; 8 from 2^18 samples, below which clearing them costs more than they
+// save).
+int cell_replicas(const Context& c, uint64_t n)
+{
+    if(c.cell_rows) return n * (uint64_t)c.cell.rows > 8ull * c.nR ? kReplicas1D : 1;
+    return n >= (1ull << 18) ? kReplicas1D : n >= 48ull * c.cell.cp.cells ? 4 : 1;
+}
+
+// 16-byte words of the cell rows that a 1D ping uses.
+uint64_t cell_words_1d(const Context& c, uint64_t n)
+{
+    const uint64_t copies = (uint64_t)cell_replicas(c, n);
+    return c.cell_rows ? (copies * c.nR + 1) / 2 : copies * c.cell.cp.cells;
+}
 
 // Samples from which a 2D ping takes the cell form. It clears and filters all
 // cell rows whatever the sample count; the gathers' work follows the samples,
@@ -613,11 +627,11 @@ static rtacx_status run_cells_1d(Context& c, const void* samples, uint64_t n, fl
     P.cells = c.d_cells;
     P.out = out;
     P.replicas = cell_replicas(c, n);
-    const uint64_t cells = c.cell_rows ? 0 : (uint64_t)P.cp.cells * P.replicas;
+    const uint64_t cells = cell_words_1d(c, n), cells_out = c.cell_rows && n ? 0 : c.nR;   // (joined rows are all written)
     c.mark(1, false, stream);
     cudaError_t e = launch_chained(k_cells_clear, (uint32_t)std::min<uint64_t>((cells + c.nR + 255) / 256, (uint64_t)c.sm_count * 8),
                                    256, 0, stream, c.d_oor + 2, kInputOrder | n, c.d_totals, 0u, c.d_nonempty, (c.nR + 31) / 32, c.d_cells, cells, out,
-                                   (uint64_t)c.nR);
+                                   cells_out);
     c.mark(1, true, stream);
     if(e == cudaSuccess && n) {
         c.mark(5, false, stream);
@@ -628,7 +642,7 @@ static rtacx_status run_cells_1d(Context& c, const void* samples, uint64_t n, fl
         e = launch_chained(fn, grid, kThreads1D, bits, stream, P, c.bin, static_cast<const float*>(samples), n,
                            c.d_nonempty, c.d_sorted);
         if(e == cudaSuccess)
-            e = c.cell_rows ? launch_chained(k_rows_off_1d, (c.nR + 255) / 256, 256, 0, stream, P, c.d_nonempty)
+            e = c.cell_rows ? launch_chained(k_rows_join_1d, (c.nR + 255) / 256, 256, 0, stream, P, c.d_nonempty)
                             : launch_chained(k_cells_filter_1d, (c.nR + kFilterRows1D - 1) / kFilterRows1D, 4 * kFilterRows1D,
                                              filter_smem_1d(P.cp.taps, kFilterRows1D), stream, P, c.d_nonempty);
         c.mark(5, true, stream);

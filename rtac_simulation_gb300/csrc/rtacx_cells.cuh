@@ -432,18 +432,27 @@ __device__ __forceinline__ void accumulate_unit(const CellPing& P, uint32_t firs
 // ---- 1D sensors --------------------------------------------------------------
 // Without bearings a sample's sums are two complex numbers, so nothing is
 // gained by sorting: each sample is one 16-byte reduction {v, alpha v} into
-// its cell (ROWS: one 8-byte reduction per output row it reaches), straight
-// from the input order. Samples [begin, end) by one CTA, kLoads1D records per
-// thread in flight. cells: the copy of the cell rows that the CTA adds into
-// (see kReplicas1D). s_bits: the CTA's bitmap of range bins. The records (echo
+// its cell (ROWS: one 8-byte reduction per output row it reaches, into float2
+// rows), straight from the input order. Samples [begin, end) by one CTA,
+// kLoads1D records per thread in flight. cells: the copy of the cell rows that
+// the CTA adds into (copy_1d). s_bits: the CTA's bitmap of range bins. The records (echo
 // model applied) are kept in `copy` for the diagnostic copy of the sorted scratch.
 constexpr int kLoads1D = 4;
-// Copies of the cell rows on large pings: with one, 3e6 samples on 4161 cells
-// queue at the same L2 addresses (whole ping 55.5 us; 41.6 with 8 copies, 41.1
-// with 32, 33 without the reductions); below 2^18 samples the copies' clearing
-// costs more than it saves.
+// Copies of the cell rows, taken in turn by the CTAs. On large pings one queues
+// at its L2 addresses: 3e6 samples on 4161 cells, whole ping, 55.5 us; 41.6 with
+// 8 copies, 41.1 with 32, 33 without the reductions. And a word that many
+// samples add into one after the other loses digits: 1.3e5 samples on 2070 to
+// 2113 cells (63 each) 4.1e-7 and 4.4e-7 from 64 bits with one copy, 2.7e-7 and
+// 3.3e-7 with 4, 2.7e-7 and 3.0e-7 with 8; 10.6 and 11.4 us, 10.3 and 11.4, 10.8
+// and 12.2. Row by row, 20000 samples on 1049 rows (95 each): 1.7e-7, 8 copies
+// 9e-8.
 constexpr int kReplicas1D = 8;
-constexpr uint64_t kReplicateFrom1D = 1ull << 18;
+
+__device__ __forceinline__ float4* copy_1d(const CellPing& P, bool rows, uint32_t cta)
+{
+    const size_t k = cta % (uint32_t)P.replicas;
+    return rows ? reinterpret_cast<float4*>(reinterpret_cast<float2*>(P.cells) + k * P.nR) : P.cells + k * P.cp.cells;
+}
 
 template <bool ROWS>
 __device__ __forceinline__ void accumulate_1d(const CellPing& P, const BinParams& p, const float* __restrict__ samples,
@@ -482,7 +491,8 @@ __device__ __forceinline__ void accumulate_1d(const CellPing& P, const BinParams
                 for(int r = max(r0, 0); r < min(r0 + P.rows, (int)P.nR); r++) {
                     if(abs((int)key - r) > P.overlap) continue;
                     const float2 f = pulse_at(P.pulse, P.range_axis, t - P.ranges[r]);
-                    if(f.x != 0.0f || f.y != 0.0f) red_add_f2(P.out + r, v.x * f.x - v.y * f.y, v.x * f.y + v.y * f.x);
+                    if(f.x != 0.0f || f.y != 0.0f)
+                        red_add_f2(reinterpret_cast<float2*>(cells) + r, v.x * f.x - v.y * f.y, v.x * f.y + v.y * f.x);
                 }
                 continue;
             }
@@ -501,6 +511,18 @@ __device__ __forceinline__ void accumulate_1d(const CellPing& P, const BinParams
             }
         }
     }
+}
+
+// Output row r of a ping summed row by row.
+__device__ __forceinline__ void join_rows_1d(const CellPing& P, int r, const uint32_t* nonempty)
+{
+    float2 v = make_float2(0.f, 0.f);
+#pragma unroll 8
+    for(int k = 0; k < P.replicas; k++) {
+        const float2 x = __ldcg(reinterpret_cast<const float2*>(P.cells) + (size_t)k * P.nR + r);
+        v.x += x.x; v.y += x.y;
+    }
+    P.out[r] = row_on(nonempty, (int)P.nR, P.overlap, r) ? v : make_float2(0.f, 0.f);
 }
 
 // Range filter of a 1D ping: four threads per output row, every fourth tap

@@ -406,7 +406,7 @@ struct ReduceParams {
 struct CellPing {
     CellParams cp;
     const float4* sorted;
-    float4* cells;                   // [cp.cells][pitch] {T, M}
+    float4* cells;                   // [cp.cells][pitch] {T, M}; 1D row by row: float2 rows [replicas][nR]
     float2* out;
     const float2* pulse;             // padded pulse table
     const float* beam;               // padded beam table
@@ -755,6 +755,7 @@ void bind_cells(Context& ctx);                           // once the arena is co
 void ensure_cells(Context& ctx);                         // the cell rows; without memory for them the gathers
 bool takes_cells(const Context& ctx, uint64_t n);
 int cell_replicas(const Context& ctx, uint64_t n);       // 1D: copies of the cell rows that a ping uses
+uint64_t cell_words_1d(const Context& ctx, uint64_t n);  // ... their 16-byte words
 void free_cells(Context& ctx);
 rtacx_status run_cells(Context& ctx, const void* samples, uint64_t n, float2* out, cudaStream_t stream);
 

@@ -1014,7 +1014,7 @@ __device__ __noinline__ void batch_chunk_1d(const PingDev& D, const CellPing& P,
     for(uint32_t i = threadIdx.x; i < words; i += kThreads) s_bits[i] = 0u;
     __syncthreads();
     const uint64_t per = (D.n + D.chunks - 1) / D.chunks, begin = chunk * per, end = min(begin + per, D.n);
-    float4* cells = P.cells + (size_t)(chunk % P.replicas) * P.cp.cells;
+    float4* cells = copy_1d(P, D.form == kRows1D, chunk);
     if(D.form == kRows1D) accumulate_1d<true>(P, D.bin, D.samples, begin, end, cells, s_bits, D.sorted);
     else accumulate_1d<false>(P, D.bin, D.samples, begin, end, cells, s_bits, D.sorted);
     __syncthreads();
@@ -1038,7 +1038,7 @@ __device__ __noinline__ void batch_filter_item(const PingDev& D, const CellPing&
     case kCells1D: filter_rows_1d<kBatchRows1D>(P, (int)item.z, s, D.nonempty); break;
     case kRows1D: {
         const int r = r0 + (int)threadIdx.x;
-        if(r < (int)P.nR && !row_on(D.nonempty, (int)P.nR, P.overlap, r)) P.out[r] = make_float2(0.f, 0.f);
+        if(r < (int)P.nR) join_rows_1d(P, r, D.nonempty);
         break;
     }
     default: break;

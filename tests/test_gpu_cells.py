@@ -369,6 +369,16 @@ def test_1d_pings_match_fp64_oracle(oracle, n, nR, taps, H, ext):
         assert rel_l2(got, want) <= TOL, rel_l2(got, want)
 
 
+def test_row_sums_of_1d_pings_keep_their_digits(oracle):
+    """About 95 reductions per output row, in one word one after the other
+    2e-7 off: the rms of a rounded sum of n terms of either sign is 2^-24 /
+    sqrt(3) sqrt(n / 2), 2.4e-7 for 95 and 8e-8 for the 12 of a copy, with three
+    roundings per product and eight copies together under 1.4e-7."""
+    wk = wl.ea400_reference_1d(n_samples=20000)
+    got = gpu_reduce(make_context(wk), wk.samples, wk.out_shape)
+    assert rel_l2(got, oracle.reduce(wk.samples, wk.sensor)) <= 1.4e-7
+
+
 def test_1d_sorted_scratch_after_a_ping(oracle):
     from test_gpu_sorted import KEY_OOR, composite_keys, record_hash
     wk = ping_1d(5000, 257, 17)
