@@ -522,6 +522,7 @@ struct FusedBatch {
 struct GemmPlan {
     CUtensorMap ma, mb;
     int bn = 0, ksplit = 1;             // tile width; K parts
+    bool lo_apart = false;              // the lo products in an accumulator of their own
     bool adds() const { return ksplit > 2; }               // many parts: added into one (zeroed) result
     int parts() const { return adds() ? 1 : ksplit; }      // partial products left for the filter to sum
     std::vector<uint16_t> lists;        // [column tiles][1 + blocks of K]: count, then the blocks where B is not zero

@@ -87,28 +87,35 @@ __device__ __forceinline__ void umma_16bit(uint32_t tmem_d, uint64_t adesc, uint
                  : "memory");
 }
 
-// Epilogue of one warp: its TMEM lane quadrant -> rows m0 + 32 warp + lane. LO:
-// the sum of two accumulators, BN columns apart.
-template <int BN, bool LO>
+// Epilogue of one warp: its TMEM lane quadrant -> rows m0 + 32 warp + lane. lo_at
+// (not 0): the sum of two accumulators, so many columns apart.
+template <int BN>
 __device__ __forceinline__ void store_tile(uint32_t tmem, float* __restrict__ C, int m0, int n0, int ldc, int warp, int lane,
                                            const float* __restrict__ row_scale, const float* __restrict__ col_scale,
-                                           bool any, bool add)
+                                           bool any, bool add, uint32_t lo_at = 0)
 {
     const int row = m0 + warp * 32 + lane;
     float* crow = C + (size_t)row * ldc + n0;
     const float rs = row_scale ? row_scale[row] : 1.0f;
 #pragma unroll 1
     for(int c = 0; c < BN / 32; c++) {
-        uint32_t r[32], lo[32];
+        uint32_t r[32];
         const uint32_t at = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c * 32);
-        if(LO) tmem_ld32_two(at, r, at + BN, lo);
-        else tmem_ld32(at, r);
         float v[32];
+        if(lo_at) {
+            uint32_t lo[32];
+            tmem_ld32_two(at, r, at + lo_at, lo);
 #pragma unroll
-        for(int q = 0; q < 32; q++) {
-            v[q] = __uint_as_float(r[q]);
-            if(LO) v[q] += __uint_as_float(lo[q]);
-            if(!any) v[q] = 0.0f;
+            for(int q = 0; q < 32; q++) v[q] = __uint_as_float(r[q]) + __uint_as_float(lo[q]);
+        }
+        else {
+            tmem_ld32(at, r);
+#pragma unroll
+            for(int q = 0; q < 32; q++) v[q] = __uint_as_float(r[q]);
+        }
+        if(!any) {
+#pragma unroll
+            for(int q = 0; q < 32; q++) v[q] = 0.0f;
         }
         if(row_scale) {
 #pragma unroll
@@ -202,7 +209,7 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
     const bool ok = mbar_wait(accum_bar, 0, abort_flag);
     __syncwarp();
     tc_fence_after();
-    if(__all_sync(0xffffffffu, ok ? 1 : 0)) store_tile<BN, false>(tmem, C, m0, n0, ldc, warp, lane, nullptr, nullptr, true, false);
+    if(__all_sync(0xffffffffu, ok ? 1 : 0)) store_tile<BN>(tmem, C, m0, n0, ldc, warp, lane, nullptr, nullptr, true, false);
     else if(lane == 0 && err) atomicOr(err, kErrGemmTimeout);
     tc_fence_before();
     __syncthreads();
@@ -214,12 +221,12 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
 
 // The split contraction. Stage: A hi, A lo, B hi, B lo of one block of 64
 // along K; the hi and the lo tiles have a barrier each, so that hi hi starts
-// before the lo tiles are in. The products with a lo half have an accumulator
-// of their own: the tensor cores truncate as they accumulate, so in one
-// accumulator the two products that add next to nothing to the sum cost it
-// digits too (2^24 samples, 512 x 4096: 1.1e-5 from 64 bits, 7.8e-6 with two, in
-// 224.4 and 224.6 us; the second tile of columns costs small contractions up to
-// 0.4 us). blockIdx.z: its share of the column tile's list
+// before the lo tiles are in. In long sums (lo_at = BN) the products with a lo
+// half have an accumulator of their own: the tensor cores truncate as they
+// accumulate, so in one accumulator the two products that add next to nothing
+// to the sum cost it digits too (2^24 samples, 512 x 4096: 1.0e-5 from 64 bits,
+// 7.3e-6 with two, the time within 0.2 us; short sums keep one, since reading
+// two would cost them 0.2 of 19.5 us). blockIdx.z: its share of the column tile's list
 // of blocks (blocks: [column tiles][1 + all blocks], the count first), into its
 // own partial product C + z rows ldc, or (add) added into C.
 template <int BN_, int STAGES_>
@@ -236,7 +243,7 @@ template <bool kF16, typename T>
 __global__ void __launch_bounds__(kThreads, 1)
 k_gemm_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, float* __restrict__ C,
              int rows, int K, int ldc, const uint16_t* __restrict__ blocks, const float* __restrict__ row_scale,
-             const float* __restrict__ col_scale, int add, uint32_t* __restrict__ err)
+             const float* __restrict__ col_scale, int add, uint32_t lo_at, uint32_t* __restrict__ err)
 {
     constexpr int BN = T::BN, STAGES = T::STAGES;
     constexpr uint32_t TMEM_COLS = 2 * BN;
@@ -310,9 +317,9 @@ k_gemm_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
             if(!mbar_wait(lo_bar(s), parity, abort_flag)) break;
             tc_fence_after();
 #pragma unroll
-            for(int kk = 0; kk < BK / 16; kk++) umma_16bit<kF16, BN>(tmem + BN, ahi + 2 * kk, blo + 2 * kk, (i > 0 || kk > 0) ? 1u : 0u);
+            for(int kk = 0; kk < BK / 16; kk++) umma_16bit<kF16, BN>(tmem + lo_at, ahi + 2 * kk, blo + 2 * kk, (!lo_at || i > 0 || kk > 0) ? 1u : 0u);
 #pragma unroll
-            for(int kk = 0; kk < BK / 16; kk++) umma_16bit<kF16, BN>(tmem + BN, alo + 2 * kk, bhi + 2 * kk, 1u);
+            for(int kk = 0; kk < BK / 16; kk++) umma_16bit<kF16, BN>(tmem + lo_at, alo + 2 * kk, bhi + 2 * kk, 1u);
             umma_commit(empty_bar(s));
         }
         umma_commit(accum_bar);   // arrives once every MMA issued above has completed
@@ -322,7 +329,7 @@ k_gemm_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     __syncwarp();
     tc_fence_after();
     if(__all_sync(0xffffffffu, ok ? 1 : 0))
-        store_tile<BN, true>(tmem, C, m0, n0, ldc, warp, lane, row_scale, col_scale, count > 0, add != 0);
+        store_tile<BN>(tmem, C, m0, n0, ldc, warp, lane, row_scale, col_scale, count > 0, add != 0, lo_at);
     else if(lane == 0 && err) atomicOr(err, kErrGemmTimeout);
     tc_fence_before();
     __syncthreads();
@@ -424,6 +431,8 @@ size_t split_smem(int bn) { return bn == 256 ? SplitWide::SMEM_BYTES : SplitNarr
 // Parts of K, at most (16384 grid bearings' real and imaginary parts are 15 of
 // kMaxTerms), and terms of a part's sum.
 constexpr int kMaxParts = 16, kMaxTerms = 2200;
+// Terms of a part's sum from which the lo products have their own accumulator.
+constexpr int kLoApart = 512;
 
 // Tile width, K split and block lists of the contraction of A [M][2 K] with
 // B [N][2 K] (b: its host copy), M % 128 == 0, N % 256 == 0, K % 64 == 0.
@@ -464,7 +473,7 @@ rtacx_status plan_gemm_split(std::string& error, GemmPlan& g, const void* A, con
             if(longest * BK > (size_t)kMaxTerms * ks && ks < kMaxParts) continue;
             const double ctas = (double)(N / bn) * (M / BM) * ks, waves = std::ceil(ctas / sm_count);
             const double t = waves * ((double)longest / ks * (bn == 256 ? 1.0 : 0.6) + 4.0) + (double)ks * M * N * 4.0 / 4e6;
-            if(t < best) { best = t; g.bn = bn; g.ksplit = ks; g.lists = lists; }
+            if(t < best) { best = t; g.bn = bn; g.ksplit = ks; g.lists = lists; g.lo_apart = longest * BK > (size_t)kLoApart * ks; }
         }
     }
     if(!make_map(&g.ma, A, (uint64_t)M, 2 * (uint64_t)K, BM, f16) || !make_map(&g.mb, B, (uint64_t)N, 2 * (uint64_t)K, g.bn, f16)) {
@@ -486,7 +495,7 @@ rtacx_status gemm_split(std::string& error, const GemmPlan& g, const uint16_t* d
 {
     const cudaError_t e = launch_chained(split_kernel(g.bn, f16), dim3(N / g.bn, M / BM, g.ksplit), kThreads,
                                          split_smem(g.bn), stream, g.ma, g.mb, C, M, K, N, d_blocks, row_scale, col_scale,
-                                         g.adds() ? 1 : 0, err);
+                                         g.adds() ? 1 : 0, (uint32_t)(g.lo_apart ? g.bn : 0), err);
     if(e != cudaSuccess) { cudaGetLastError(); error = std::string("k_gemm_split: ") + cudaGetErrorString(e); return RTACX_ERR_CUDA; }
     return RTACX_OK;
 }
