@@ -56,10 +56,12 @@ NCU_TRAFFIC_BYTES = {
 }
 # The accumulation's bound is the L2's reduction throughput, not HBM: ncu on
 # the default workload (profiles/k_prec_accumulate_staged_precision_2d.md)
-# shows 1.50 L2 reduction requests (1.57 sectors) per sample and the L2 at
-# 65 % of its peak throughput while DRAM carries the algorithmic bytes once.
-NCU_ACCUMULATE_L2 = {"l2_throughput_pct": 64.7, "l2_red_sectors_pct": 40.6, "red_sectors_per_sample": 1.57,
-                     "red_requests_per_sample": 1.50}
+# shows the L2 at 71 % of its peak throughput (tag requests; its reduction
+# sectors at 66 %, 2.31 per sample over both dies' slices, for 1.50 requests
+# of the SMs), the issue slots 76 % busy, and DRAM carrying the algorithmic
+# bytes once.
+NCU_ACCUMULATE_L2 = {"l2_throughput_pct": 71.1, "l2_red_sectors_pct": 66.0, "red_sectors_per_sample": 2.31,
+                     "red_requests_per_sample": 1.50, "issue_pct": 75.8}
 
 # Plain form over range cells: clear, count, bin scan, scatter, accumulation
 # (one more for a lobe on a floor, not counted), range filter; 1D: clear,
@@ -721,7 +723,7 @@ def run_ours(args, world, rank, local):
         "config": {"workload": wk_desc(wk),
                    "form": ("precision: bin onto range nodes two bins apart x a 4x bearing grid, BF16x3 tcgen05 "
                             "complex contraction (K split in two), FP32 polyphase range filter, FP64 carrier phase"
-                            if head == "precision" else "plain (FP32 SIMT sparse PSF gather)"),
+                            if head == "precision" else "plain (FP32: range cells, or the per-row gathers off their rule)"),
                    "l2": ("inputs larger than L2 (%.0f MB of samples)" if n * rec_in > 129e6 else
                           "inputs smaller than L2 (%.0f MB of samples): timed warm, not flushed") % (n * rec_in / 1e6),
                    "timing": ("one ping at a time on one stream (two pings in flight on two contexts and "
@@ -785,7 +787,7 @@ def run_ours(args, world, rank, local):
         roof_gemm = {"bound": "tensor", "achieved": gemm_tf, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
                      "frac": gemm_tf / peaks["bf16_tflops"], "traffic": ncu.get("k_gemm_split"), "kernel": "k_gemm_split",
                      "peak_source": peaks["source"],
-                     "algorithmic": f"2*M*N*K with M={Mp} N={Np} K={Kp} (three BF16 split products as one K)"}
+                     "algorithmic": f"2*M*N*K with M={Mp} N={Np} K={Kp} (three BF16 split products of hi and lo tiles loaded once)"}
         dominant = max(("accumulate", "gemm", "filter", "split"), key=lambda k: ps[k])
         line["roofline"] = roof_gemm if dominant == "gemm" else roof_acc
         line["roofline"]["dominant_stage"] = dominant

@@ -88,9 +88,12 @@ typedef int rtacx_status;
 /* A 2D sensor whose pulse taps lie one output range apart and whose windows
  * hold the pulse takes the range-cell form (one beam lookup per sample and
  * bearing, the pulse as a filter over the cells; float arithmetic), whatever
- * the next flag says. A beam table that is one level at both ends is then
- * taken apart into that level and a lobe on large pings (exactly, up to float
- * round-off). */
+ * the next flag says, unless a ping has few samples for the size of the sensor
+ * (its cells are all cleared and filtered): that one is gathered. A beam table
+ * that is one level at both ends is taken apart into that level and a lobe on
+ * large pings (exactly, up to float round-off). A sample value that is not
+ * finite makes ranges and bearings that the sample reaches not finite, and
+ * others near them, which ones going by the form. */
 /* rtacx_sensor_2d.flags: gather with the FP32 CUDA-core kernel instead of the
  * tensor-core one. Otherwise a 2D ping's gather (output tiles of 64 ranges x
  * 128 bearings) forms its sample-by-PSF outer products on the tcgen05 tensor
@@ -225,7 +228,9 @@ rtacx_status rtacx_set_echo_model(rtacx_ctx* ctx, const rtacx_echo_model* model)
  * Each sample costs two 16-byte vector reductions: the grid is stored by
  * bearing interval (the shares of its two bearings side by side). The
  * contraction runs in BF16 with three split products (hi*hi + hi*lo +
- * lo*hi) and FP32 accumulation on tcgen05 tensor cores; the rest is FP32.
+ * lo*hi) and FP32 accumulation on tcgen05 tensor cores, over the blocks of D
+ * that are not zero (a grid value that is not finite does not reach bearings
+ * of the others); the rest is FP32.
  * NULL tables are derived from the 2D sensor: taps[p][t] the least-squares
  * (L2) projection of the pulse response pulse(x - p res) (texture-equivalent
  * lerp, seen from a node) onto the hat functions of the nodes (the weight of
@@ -365,8 +370,9 @@ rtacx_status rtacx_rasterize(rtacx_ctx* ctx, const rtacx_mesh* mesh, const rtacx
  * RTACX_BATCH_AUTOTUNE, times every candidate gather tile shape x samples
  * per binning chunk on this batch and keeps the fastest. rtacx_batch_run
  * replays the graph on `stream`. Pings with a range-cell form take it where
- * that is most of the batch's work, the others gather on the CUDA cores;
- * results equal rtacx_reduce's per ping to float round-off. */
+ * that is most of the batch's work and estimated to be faster than gathering
+ * them, the others gather on the CUDA cores; results equal rtacx_reduce's per
+ * ping to float round-off. */
 typedef struct rtacx_batch rtacx_batch;
 typedef struct {
     rtacx_ctx* ctx;          /* configured context, one per ping          */

@@ -570,9 +570,9 @@ __device__ __forceinline__ void filter_rows_1d(const CellPing& P, int tile, floa
 }
 
 // ---- range filter over the cell rows ----------------------------------------
-// A CTA of WARPS warps filters 32 columns x WARPS * kFilterRows output rows. The cell rows it needs are staged in shared memory by 16-byte
-// asynchronous copies, kFilterChunk rows at a time, all of them in flight
-// together. Each thread holds one column and kFilterRows consecutive output
+// A CTA of WARPS warps filters 32 columns x WARPS * kFilterRows output rows. The
+// cell rows it needs are staged in shared memory by 16-byte asynchronous
+// copies, kFilterChunk rows at a time, all of them in flight together. Each thread holds one column and kFilterRows consecutive output
 // rows and walks the staged cells; the taps of its rows slide through
 // registers (the tap of row q at a cell is the tap of row q + 1 at the next).
 // What is in the ping already is loaded before the cells arrive. Bound by
@@ -591,8 +591,8 @@ __host__ __device__ __forceinline__ size_t filter_smem(int H)
     return (size_t)cell_tap_entries(H) * sizeof(float4) + (size_t)kFilterChunk * 32 * sizeof(float4);
 }
 
-// Columns [32 tile_c, +32) and rows [8 WARPS tile_r, +8 WARPS) of a ping. Called
-// by 32 WARPS threads; synchronises.
+// Columns [32 tile_c, +32) and rows [WARPS kFilterRows tile_r, + WARPS
+// kFilterRows) of a ping. Called by 32 WARPS threads; synchronises.
 template <int WARPS, bool FLOOR = false>
 __device__ __forceinline__ void filter_tile(const CellPing& P, int tile_c, int tile_r, float4* s_raw,
                                             const uint32_t* nonempty)
